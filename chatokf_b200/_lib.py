@@ -7,9 +7,12 @@ beside this file only, so a stale copy elsewhere is never picked up.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
+import sysconfig
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libokfcuda.so"
+CALL_PATH = LIB_PATH.with_name("_okfcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 OKF_OK = 0
 STATUS = {
@@ -148,5 +151,29 @@ def load() -> ctypes.CDLL:
             fn = getattr(L, name)  # AttributeError here = header and library out of step
             fn.restype = res
             fn.argtypes = args
+        call._load(L)
         _lib = L
     return _lib
+
+
+class _Call:
+    """The C module behind CudaEnc's and QB's methods (csrc/okf_pycall.c), filled in by load()."""
+
+    def _load(self, L: ctypes.CDLL) -> None:
+        if not CALL_PATH.exists():
+            raise ImportError(f"{CALL_PATH} is missing: build it with `python -m chatokf_b200.build`")
+        import torch
+
+        spec = importlib.util.spec_from_file_location("_okfcall", CALL_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        # a torch without CUDA lacks these two; nothing that needs a stream runs there
+        dev, raw = (getattr(torch._C, n, None) for n in ("_cuda_getDevice", "_cuda_getCurrentRawStream"))
+        mod.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in SIGNATURES},
+                 (torch.float32, torch.float16, torch.bfloat16), dev, raw)
+        for name in ("gemm", "gemv", "parallel_begin", "parallel_end", "dequant", "embed", "argmax", "norm", "silu",
+                     "matmul_at", "matmul_host"):
+            setattr(self, name, getattr(mod, name))
+
+
+call = _Call()

@@ -4,7 +4,9 @@
 
 The library links the CUDA runtime statically and exports only the C ABI of
 include/okf_cuda.h.  Objects go to chatokf_b200/csrc/build/ (git-ignored); the
-shared library sits beside this file so it travels with the package.
+shared library sits beside this file so it travels with the package.  Beside it
+goes _okfcall, the C module through which Python calls the library's hot entry
+points.
 """
 from __future__ import annotations
 
@@ -13,6 +15,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -20,6 +23,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = CSRC / "build"
 LIB = PKG / "libokfcuda.so"
+PYCALL = CSRC / "okf_pycall.c"
+PYMOD = PKG / ("_okfcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = [
@@ -39,14 +44,29 @@ def sources() -> list[Path]:
     return sorted(CSRC.glob("*.cu"))
 
 
-def _deps_mtime() -> float:
-    deps = list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
+def _headers_mtime() -> float:
+    deps = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h"))
     deps.append(PKG.parent / "include" / "okf_cuda.h")
     return max(p.stat().st_mtime for p in deps)
 
 
+def _stale(out: Path, src_mtime: float) -> bool:
+    return not out.exists() or out.stat().st_mtime < max(src_mtime, _headers_mtime())
+
+
 def needs_build() -> bool:
-    return (not LIB.exists()) or LIB.stat().st_mtime < _deps_mtime()
+    return (_stale(LIB, max(p.stat().st_mtime for p in sources()))
+            or _stale(PYMOD, PYCALL.stat().st_mtime))
+
+
+def build_pycall() -> None:
+    cmd = [shutil.which("gcc") or "cc", "-O2", "-Wall", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-I", sysconfig.get_paths()["include"], str(PYCALL), "-o", str(PYMOD) + ".tmp"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError(f"compiling {PYCALL.name} failed")
+    os.replace(str(PYMOD) + ".tmp", PYMOD)
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -58,6 +78,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
     def compile_one(src: Path) -> Path:
         obj = OBJ / (src.stem + ".o")
+        if not force and not _stale(obj, src.stat().st_mtime):
+            return obj
         cmd = [cc, *ARCH, *NVCC_FLAGS, *extra, "-c", str(src), "-o", str(obj)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if verbose or r.returncode:
@@ -77,6 +99,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("link of libokfcuda.so failed")
     os.replace(tmp, LIB)
+    build_pycall()
     return LIB
 
 

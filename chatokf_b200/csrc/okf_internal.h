@@ -58,16 +58,20 @@ struct okf_ctx {
 
 namespace okf {
 
+// Makes `dev` current for the calls in a scope.  The usual case, it is current already, costs one
+// look at the thread's state.
 struct DeviceGuard {
     int prev = -1;
-    bool ok = true;
+    bool ok = true, moved = false;
     explicit DeviceGuard(int dev) {
         if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
-        if (prev != dev) ok = cudaSetDevice(dev) == cudaSuccess;
+        if (prev != dev) {
+            ok = cudaSetDevice(dev) == cudaSuccess;
+            moved = true;
+        }
     }
     ~DeviceGuard() {
-        int cur = -1;
-        if (prev >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != prev) cudaSetDevice(prev);
+        if (moved && prev >= 0) cudaSetDevice(prev);
     }
 };
 

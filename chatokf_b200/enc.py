@@ -9,8 +9,6 @@ libokfcuda.so.
 """
 from __future__ import annotations
 
-import contextlib
-
 import ctypes
 from dataclasses import dataclass
 
@@ -18,7 +16,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import OkfError
+from ._lib import OkfError, call
 from .gguf_types import GGUFType, block_elems, row_byte_count
 
 F32, F16, BF16 = 0, 1, 2
@@ -59,7 +57,7 @@ class Context:
         rc = self.lib.okf_init(int(device), ctypes.byref(h))
         if rc:
             raise OkfError(rc, "okf_init")
-        self.h = h
+        self.h, self._addr = h, h.value
         self.device = int(device)
 
     def _check(self, rc: int, what: str):
@@ -69,7 +67,7 @@ class Context:
     def close(self):
         if getattr(self, "h", None):
             self.lib.okf_destroy(self.h)
-            self.h = None
+            self.h, self._addr = None, 0
 
     def __del__(self):
         try:
@@ -126,11 +124,12 @@ class Weights:
 
     def __init__(self, ctx: Context, h, nbytes: int, keep):
         self.ctx, self.h, self.nbytes, self._keep = ctx, h, nbytes, keep
+        self._addr = h.value
 
     def free(self):
         if self.h and self.ctx.h:
             self.ctx.lib.okf_weights_free(self.ctx.h, self.h)
-        self.h = None
+        self.h, self._addr = None, 0
 
     def __del__(self):
         try:
@@ -144,8 +143,30 @@ def _stream_ptr(stream) -> int:
     return int(s.cuda_stream)
 
 
+class _Region:
+    """What CudaEnc.parallel() hands to `with`: okf_parallel_begin / okf_parallel_end."""
+
+    __slots__ = ("enc",)
+
+    def __init__(self, enc):
+        self.enc = enc
+
+    def __enter__(self):
+        rc = call.parallel_begin(self.enc)
+        if rc:
+            self.enc.ctx._check(rc, "okf_parallel_begin")
+        return self.enc
+
+    def __exit__(self, *exc):
+        rc = call.parallel_end(self.enc)
+        if rc:
+            self.enc.ctx._check(rc, "okf_parallel_end")
+        return False
+
+
 class CudaEnc:
-    """Drop-in for MetalEnc's quantized linear operators on one stream."""
+    """Drop-in for MetalEnc's quantized linear operators on one stream (the current one
+    when none is given)."""
 
     NARROW_MAX = 8  # MetalEnc.narrowMax is 5 (MetalEnc.swift:172); widened to the verify batch of 8
 
@@ -156,30 +177,20 @@ class CudaEnc:
              x_off_bytes: int = 0, out_off_bytes: int = 0):
         """MetalEnc.gemv(w, x:, out:, off:, xOffBytes:, outOffBytes:)."""
         assert out.dtype == torch.float32
-        c = self.ctx
-        c._check(c.lib.okf_gemv(c.h, int(w.type), off.h, w.offset, w.K, w.M,
-                                x.data_ptr() + x_off_bytes, _DT[x.dtype],
-                                out.data_ptr() + out_off_bytes, _stream_ptr(self.stream)), "okf_gemv")
-
-    def _gemm(self, fn, name, w, X, out, off, N):
-        c = self.ctx
-        c._check(fn(c.h, int(w.type), off.h, w.offset, w.K, w.M, X.data_ptr(), _DT[X.dtype], int(N),
-                    out.data_ptr(), _DT[out.dtype], _stream_ptr(self.stream)), name)
+        rc = call.gemv(self, w, x, out, off, x_off_bytes, out_off_bytes)
+        if rc:
+            self.ctx._check(rc, "okf_gemv")
 
     def gemm(self, w: GGUFTensor, X: torch.Tensor, out: torch.Tensor, off: Weights, N: int):
         """MetalEnc.gemm(w, X:, out:, off:, N:): out[n*M + m]."""
-        self._gemm(self.ctx.lib.okf_gemm, "okf_gemm", w, X, out, off, N)
+        rc = call.gemm(self, 0, w, X, out, off, N)
+        if rc:
+            self.ctx._check(rc, "okf_gemm")
 
-    @contextlib.contextmanager
     def parallel(self):
         """MetalEnc.parallel { ... } (LLM/Base/MetalEnc.swift:42-47): the calls inside
         have no order among themselves; narrow matvecs of the same x leave as one launch."""
-        c = self.ctx
-        c._check(c.lib.okf_parallel_begin(c.h), "okf_parallel_begin")
-        try:
-            yield self
-        finally:
-            c._check(c.lib.okf_parallel_end(c.h), "okf_parallel_end")
+        return _Region(self)
 
     def gemm_gather(self, w: GGUFTensor, X: torch.Tensor, gather, off: Weights, N: int = 1):
         """okf_gemm_gather: this rank's rows of a row-sharded matrix, stored straight into
@@ -196,21 +207,24 @@ class CudaEnc:
 
     def gemmTile(self, w: GGUFTensor, X: torch.Tensor, out: torch.Tensor, off: Weights, N: int):
         """MetalEnc.gemmTile: the tensor-core tile at any N (kernel bench)."""
-        self._gemm(self.ctx.lib.okf_gemm_tile, "okf_gemm_tile", w, X, out, off, N)
+        rc = call.gemm(self, 1, w, X, out, off, N)
+        if rc:
+            self.ctx._check(rc, "okf_gemm_tile")
 
     def gemm_noalloc(self, w: GGUFTensor, X: torch.Tensor, out: torch.Tensor, off: Weights, N: int):
         """okf_gemm_noalloc: the matmul with its scratch in a fixed array of the library,
         for callers that may not allocate device memory (N * M <= 2 Mi outputs)."""
-        self._gemm(self.ctx.lib.okf_gemm_noalloc, "okf_gemm_noalloc", w, X, out, off, N)
+        rc = call.gemm(self, 2, w, X, out, off, N)
+        if rc:
+            self.ctx._check(rc, "okf_gemm_noalloc")
 
     def dequantRow(self, off: Weights, out: torch.Tensor, n: int, type: int,
                    weight_off: int = 0, out_off_bytes: int = 0):
         """MetalEnc.dequantRow(weightOff:, out:, n:, type:, outOffBytes:)."""
         assert out.dtype == torch.float32
-        c = self.ctx
-        c._check(c.lib.okf_dequant(c.h, int(type), off.h, int(weight_off), int(n),
-                                   out.data_ptr() + out_off_bytes, _stream_ptr(self.stream)), "okf_dequant")
-
+        rc = call.dequant(self, off, out, n, type, weight_off, out_off_bytes)
+        if rc:
+            self.ctx._check(rc, "okf_dequant")
 
     # ---- the linears' neighbours ----------------------------------------------------
 
@@ -219,29 +233,29 @@ class CudaEnc:
         """MetalEnc.embedBatch(ids:, weightOff:, out:, nEmbd:, N:, type:): out[n] = row ids[n],
         unpacked exactly.  `rows` is the height of the embedding matrix (ids are checked against it)."""
         assert ids.dtype == torch.int32 and out.dtype == torch.float32
-        c = self.ctx
-        c._check(c.lib.okf_embed_batch(c.h, int(type), off.h, int(weight_off), int(nEmbd), int(rows), ids.data_ptr(),
-                                       int(N), out.data_ptr(), _stream_ptr(self.stream)), "okf_embed_batch")
+        rc = call.embed(self, ids, off, out, nEmbd, N, type, rows, weight_off)
+        if rc:
+            self.ctx._check(rc, "okf_embed_batch")
 
     def argmaxRows(self, x: torch.Tensor, out: torch.Tensor, n: int, rows: int):
         """MetalEnc.argmaxRows(x:, out:, n:, rows:): ties to the lower index."""
         assert x.dtype == torch.float32 and out.dtype == torch.int32
-        c = self.ctx
-        c._check(c.lib.okf_argmax_rows(c.h, x.data_ptr(), int(n), int(rows), out.data_ptr(),
-                                       _stream_ptr(self.stream)), "okf_argmax_rows")
+        rc = call.argmax(self, x, out, n, rows)
+        if rc:
+            self.ctx._check(rc, "okf_argmax_rows")
 
     def addRmsnormBatch(self, x: torch.Tensor, r, weight: torch.Tensor, y: torch.Tensor, n: int, rows: int,
                         eps: float, x_stride: int | None = None, y_stride: int | None = None):
         """MetalEnc.addRmsnormBatch / rmsnormBatch (r = None): x += r; y = rmsnorm(x) * weight."""
-        c = self.ctx
-        c._check(c.lib.okf_add_rmsnorm(c.h, x.data_ptr(), r.data_ptr() if r is not None else None, weight.data_ptr(),
-                                       y.data_ptr(), int(n), int(rows), float(eps), int(x_stride or n),
-                                       int(y_stride or n), _stream_ptr(self.stream)), "okf_add_rmsnorm")
+        rc = call.norm(self, x, r, weight, y, n, rows, eps, x_stride or n, y_stride or n)
+        if rc:
+            self.ctx._check(rc, "okf_add_rmsnorm")
 
     def siluMul(self, a: torch.Tensor, b: torch.Tensor, n: int):
         """MetalEnc.siluMul: a = silu(a) * b."""
-        c = self.ctx
-        c._check(c.lib.okf_silu_mul(c.h, a.data_ptr(), b.data_ptr(), int(n), _stream_ptr(self.stream)), "okf_silu_mul")
+        rc = call.silu(self, a, b, n)
+        if rc:
+            self.ctx._check(rc, "okf_silu_mul")
 
     def srq(self, src: torch.Tensor, dst: torch.Tensor, n: int, side):
         """srqTo / srqInPlace: side = (scale, lo, hi) as SRQ.Side."""
@@ -269,34 +283,28 @@ class QB:
         self.ctx = ctx
 
     def matvec(self, w: GGUFTensor, off: Weights, x: np.ndarray, out: np.ndarray | None = None) -> np.ndarray:
-        x = np.ascontiguousarray(x, dtype=np.float32)
-        assert x.size == w.K
         if out is None:
             out = np.empty(w.M, dtype=np.float32)
-        assert out.dtype == np.float32 and out.size == w.M and out.flags.c_contiguous
-        c = self.ctx
-        c._check(c.lib.okf_matvec_host(c.h, int(w.type), off.h, w.offset, w.K, w.M,
-                                       x.ctypes.data, out.ctypes.data), "okf_matvec_host")
-        return out
+        return self.matmul(w, off, x, 1, out)
 
     def matmul(self, w: GGUFTensor, off: Weights, X: np.ndarray, N: int, out: np.ndarray | None = None) -> np.ndarray:
-        X = np.ascontiguousarray(X, dtype=np.float32)
-        assert X.size == N * w.K
         if out is None:
             out = np.empty((N, w.M), dtype=np.float32)
-        assert out.dtype == np.float32 and out.size == N * w.M and out.flags.c_contiguous
-        c = self.ctx
-        c._check(c.lib.okf_matmul_host(c.h, int(w.type), off.h, w.offset, w.K, w.M,
-                                       X.ctypes.data, int(N), out.ctypes.data), "okf_matmul_host")
+        rc = call.matmul_host(self.ctx, w, off, X, N, out)
+        if rc is None:  # not float32 in C order
+            X = np.ascontiguousarray(X, dtype=np.float32)
+            rc = call.matmul_host(self.ctx, w, off, X, N, out)
+            assert rc is not None, "out is a writable float32 array in C order"
+        if rc:
+            self.ctx._check(rc, "okf_matmul_host")
         return out
 
     def matmul_at(self, w: GGUFTensor, off: Weights, x_addr: int, N: int, out_addr: int) -> None:
         """okf_matmul_host on raw host addresses (N x K floats in, N x M floats out), as a host
         that keeps its own buffers calls it: nothing is checked, converted or allocated here."""
-        c = self.ctx
-        rc = c.lib.okf_matmul_host(c.h, int(w.type), off.h, w.offset, w.K, w.M, x_addr, N, out_addr)
+        rc = call.matmul_at(self.ctx, w, off, x_addr, N, out_addr)
         if rc:
-            c._check(rc, "okf_matmul_host")
+            self.ctx._check(rc, "okf_matmul_host")
 
     def dequant(self, w: GGUFTensor, off: Weights, row: int, count: int) -> np.ndarray:
         """QB.dequant(w, row:, count:, into:): `count` weights from the row start."""
