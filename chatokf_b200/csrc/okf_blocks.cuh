@@ -195,6 +195,15 @@ __device__ __forceinline__ void decode32(const uint8_t *row, uint32_t gran, floa
     }
 }
 
+// Programmatic dependent launch: let the next kernel in the stream start its
+// weight prefetch while this one drains, and wait for the previous kernel's
+// results before touching activations or outputs.  Both are no-ops when the
+// launch does not carry the attribute.
+__device__ __forceinline__ void pdl_launch_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }

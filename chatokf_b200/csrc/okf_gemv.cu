@@ -1533,7 +1533,7 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
 // 8 rows always start on a 16-byte boundary -- otherwise rows are cut into
 // segments of at least 1 KB, one copy per row.  `tiles_per_cta` is the most tiles
 // any CTA of the launch gets.
-constexpr uint32_t kSharedBudget = 112 * 1024;
+constexpr uint32_t kSharedBudget = 112 * 1024;  // two of them leave 2 KB of an SM: enough for the small kernels between matvecs
 
 static bool gemv_layout_with(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t tiles_per_cta, uint32_t tab_copies,
                              uint32_t budget, GemvArgs &a, GemvLayout &L) {
@@ -1645,18 +1645,48 @@ static bool gemv_layout_in(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_
     return have;
 }
 
-static bool gemv_layout(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t tiles_per_cta, GemvArgs &a,
-                        GemvLayout &L) {
+static bool gemv_layout_search(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t tiles_per_cta, GemvArgs &a,
+                               GemvLayout &L) {
     // (Tried for several columns of long rows, whose panel of x does not fit beside the ring in
     // half an SM's shared memory: taking the SM alone with the whole panel resident.  Slower:
     // the next kernel can then not prefetch under this one.)
     return gemv_layout_in(ty, nunit, n, sep, tiles_per_cta, kSharedBudget, a, L);
 }
 
-// CTAs of a launch: one per SM, each with its share of the tiles -- except when there are only
-// a few more tiles than SMs (160 on 148): then two tiles in a row on a dozen SMs would set the
-// launch's time, and one CTA per tile is used instead; an SM has room for two of them side by
-// side, and they do not slow each other down much (a CTA alone issues on a third of the cycles).
+// The search costs the host about as much as a launch and an engine asks for the same few
+// shapes on every token, so each thread keeps the plans it found last.
+static bool gemv_layout(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t tiles_per_cta, GemvArgs &a,
+                        GemvLayout &L) {
+    struct Entry {
+        int ty;
+        uint32_t nunit, n, tiles_per_cta, cb, nchunk;
+        bool sep, used, ok;
+        GemvLayout L;
+    };
+    constexpr uint32_t kEntries = 64;
+    static thread_local Entry cache[kEntries];
+    uint32_t h = ((uint32_t)ty * 31 + nunit) * 31 + n;
+    h = (h * 31 + tiles_per_cta) * 2 + (sep ? 1 : 0);
+    Entry &e = cache[(h * 2654435761u) >> 26];
+    static_assert(kEntries == 64, "six bits of the hash");
+    if (!(e.used && e.ty == ty && e.nunit == nunit && e.n == n && e.tiles_per_cta == tiles_per_cta && e.sep == sep)) {
+        GemvArgs t = {};
+        e = {ty, nunit, n, tiles_per_cta, 0, 0, sep, true, false, {}};
+        e.ok = gemv_layout_search(ty, nunit, n, sep, tiles_per_cta, t, e.L);
+        e.cb = t.cb;
+        e.nchunk = t.nchunk;
+    }
+    if (!e.ok) return false;
+    a.cb = e.cb;
+    a.nchunk = e.nchunk;
+    L = e.L;
+    return true;
+}
+
+// CTAs of a launch: one per SM, each with its share of the tiles, with two exceptions.
+// When there are only a few more tiles than SMs (160 on 148) two tiles in a row on a dozen SMs would
+// set the launch's time, and one CTA per tile is used instead; an SM has room for two of them side
+// by side, and they do not slow each other down much (a CTA alone issues on a third of the cycles).
 // (One column only: with several columns two CTAs on an SM, each staging its slices of x at
 // barriers, were 16 % slower than two tiles in a row.)
 static uint32_t gemv_ctas(uint32_t tiles, int sms, bool sep) {
@@ -1677,17 +1707,7 @@ static cudaError_t launch_t(GemvArgs a, const GemvGather &G, cudaStream_t s, int
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(G.nranks ? kGemvThreadsMax : kGemvThreads);
-    cfg.dynamicSmemBytes = L.smem_bytes;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemv_kernel<TY, XDT, SEP>, a, L, G);
+    return launch_pdl(gemv_kernel<TY, XDT, SEP>, ctas, G.nranks ? kGemvThreadsMax : kGemvThreads, L.smem_bytes, s, 1, a, L, G);
 }
 
 template <int TY>

@@ -5,6 +5,30 @@
 
 namespace okf {
 
+// Launch with programmatic dependent launch: the kernel may start while the one before it in the
+// stream is finishing, and has to call pdl_wait() before it touches anything another kernel writes
+// or reads.  A chain stays in order as long as every kernel of it does: one that has passed its
+// wait knows that everything before its predecessor is complete.  `cluster` > 1 adds a cluster of
+// that many CTAs along x.
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, unsigned cluster,
+                              A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Simple kernels: one warp per row (matvec), one fp32 register tile per thread
 // (matmul).  They define the numerics the fast kernels are checked against on
 // the device and serve shapes the fast kernels do not take.

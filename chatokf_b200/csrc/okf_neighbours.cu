@@ -8,6 +8,17 @@
 // silu_mul (Kernels.metal:3280-3285) and srq_to / srq_inplace (Kernels.metal:4743-4767).
 // All of them are bound by memory, not arithmetic: one pass over their operands with
 // 16-byte accesses where the shapes allow it.
+//
+// In decode each of them works on a few kilobytes between two matvecs, and what counts is the
+// gap it leaves: all are launched with programmatic dependent launch and trigger their
+// successor at once, so that the next matvec's weights are on their way while these run.
+// (Four FFN blocks of 2560 / 9728 in Q4_K, one token, on the GPU alone: 123 us when these
+// kernels were launched plainly, 86 us so.)  They also have to fit beside two matvec CTAs, which
+// leave 10240 registers and 2 KB of an SM: where one does not, a CTA of the matvec behind it cannot
+// start on that SM, lands as a third one elsewhere, and the whole launch takes twice as long
+// (logits of 2560 -> 151936 with an arg-max of 512 threads per CTA: 177 us instead of 132).
+#include <cooperative_groups.h>
+
 #include "okf_internal.h"
 #include "okf_kernels.h"
 
@@ -23,10 +34,12 @@ __global__ void __launch_bounds__(256) embed_kernel(const uint8_t *__restrict__ 
                                                     uint32_t k, uint32_t n, uint32_t rows, float *__restrict__ out,
                                                     int *bad) {
     __shared__ uint64_t grid_s[256];
+    pdl_launch_dependents();
     if constexpr (TY == T_IQ2_XXS) {
         grid_s[threadIdx.x] = g_iq2xxs_grid[threadIdx.x];
         __syncthreads();
     }
+    pdl_wait();
     const uint32_t gpr = k / 32;  // granules per row
     const size_t row_bytes = (size_t)(k / Geom<TY>::per) * Geom<TY>::bytes;
     const uint64_t total = (uint64_t)n * gpr, stride = (uint64_t)gridDim.x * blockDim.x;
@@ -54,8 +67,7 @@ static cudaError_t embed_t(const uint8_t *w, const int *ids, uint32_t k, uint32_
     if (total == 0) return cudaSuccess;
     uint64_t blocks = (total + 255) / 256;
     if (blocks > 148ull * 32) blocks = 148ull * 32;
-    embed_kernel<TY><<<(unsigned)blocks, 256, 0, s>>>(w, ids, k, n, rows, out, bad);
-    return cudaGetLastError();
+    return launch_pdl(embed_kernel<TY>, (unsigned)blocks, 256, 0, s, 1, w, ids, k, n, rows, out, bad);
 }
 
 static cudaError_t launch_embed(int ty, const uint8_t *w, const int *ids, uint32_t k, uint32_t n, uint32_t rows, float *out,
@@ -74,24 +86,36 @@ static cudaError_t launch_embed(int ty, const uint8_t *w, const int *ids, uint32
 }
 
 // ---- arg-max over rows --------------------------------------------------------------
-// One CTA per row.  The largest value wins, ties go to the lower index, NaNs never win
-// (an all-NaN row gives 0): what the host arg-max it replaces does.
+// The largest value wins, ties go to the lower index, NaNs never win (an all-NaN row gives 0):
+// what the host arg-max it replaces does.  A row is walked by a cluster of CTAs, each taking
+// every cluster-size-th stretch, whose winners meet in the first CTA's shared memory.
 __device__ __forceinline__ void argmax_take(float &bv, int &bi, float ov, int oi) {
     if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
 }
 
-__global__ void __launch_bounds__(512) argmax_rows_kernel(const float *__restrict__ x, int *__restrict__ out, uint32_t n) {
-    __shared__ float bestv[16];
-    __shared__ int besti[16];
-    const float *row = x + (size_t)blockIdx.x * n;
+// A logits row is 600 KB at a vocabulary of 151936, more than one SM can take from L2 in the time
+// of a launch; rows below kArgmaxSplit stay with one CTA.
+constexpr uint32_t kArgmaxCluster = 8, kArgmaxSplit = 16384;
+__global__ void __launch_bounds__(256, 6) argmax_rows_kernel(const float *__restrict__ x, int *__restrict__ out, uint32_t n,
+                                                          uint32_t parts) {
+    __shared__ float bestv[8 + kArgmaxCluster];  // per warp, then per CTA of the cluster
+    __shared__ int besti[8 + kArgmaxCluster];
+    pdl_launch_dependents();
+    namespace cg = cooperative_groups;
+    if (parts > 1) cg::this_cluster().barrier_arrive();  // "this CTA has started": seen before anyone writes to another's memory
+    const uint32_t rank = blockIdx.x % parts, r = blockIdx.x / parts;
+    const float *row = x + (size_t)r * n;
     float bv = -INFINITY;
-    int bi = 0;
+    int bi = 0x7FFFFFFF;
+    const uint32_t first = rank * blockDim.x + threadIdx.x, step = parts * blockDim.x;
+    pdl_wait();
     // 16-byte loads where the row allows them; each thread walks its indices in rising
     // order, so a strict > keeps the lowest index among its equals
     const bool vec = (n & 3u) == 0 && ((uintptr_t)row & 15u) == 0;
     if (vec) {
         const float4 *r4 = reinterpret_cast<const float4 *>(row);
-        for (uint32_t i = threadIdx.x; i < n / 4; i += blockDim.x) {
+#pragma unroll 4
+        for (uint32_t i = first; i < n / 4; i += step) {
             const float4 v = __ldg(r4 + i);
             if (v.x > bv) { bv = v.x; bi = (int)(4 * i); }
             if (v.y > bv) { bv = v.y; bi = (int)(4 * i + 1); }
@@ -99,8 +123,9 @@ __global__ void __launch_bounds__(512) argmax_rows_kernel(const float *__restric
             if (v.w > bv) { bv = v.w; bi = (int)(4 * i + 3); }
         }
     } else {
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const float v = row[i];
+#pragma unroll 4
+        for (uint32_t i = first; i < n; i += step) {
+            const float v = __ldg(row + i);
             if (v > bv) { bv = v; bi = (int)i; }
         }
     }
@@ -112,24 +137,47 @@ __global__ void __launch_bounds__(512) argmax_rows_kernel(const float *__restric
         besti[threadIdx.x >> 5] = bi;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0)
         for (uint32_t w = 1; w < blockDim.x / 32; w++) argmax_take(bv, bi, bestv[w], besti[w]);
-        out[blockIdx.x] = bi;
+    if (parts > 1) {
+        cg::cluster_group cl = cg::this_cluster();
+        cl.barrier_wait();
+        if (threadIdx.x == 0) {
+            cl.map_shared_rank(bestv, 0)[8 + rank] = bv;
+            cl.map_shared_rank(besti, 0)[8 + rank] = bi;
+        }
+        cl.sync();
+        if (rank != 0) return;
+        if (threadIdx.x == 0)
+            for (uint32_t w = 1; w < parts; w++) argmax_take(bv, bi, bestv[8 + w], besti[8 + w]);
     }
+    if (threadIdx.x == 0) out[r] = bi == 0x7FFFFFFF ? 0 : bi;  // nothing above -inf: index 0
 }
 
 // ---- residual add + RMS norm ----------------------------------------------------------
 // x[row] += r[row] (skipped when r is null); y[row] = x[row] * scale * w with
-// scale = 1 / sqrt(mean(x^2) + eps).  One CTA per row; the row is read from HBM once
-// (the second sweep hits L1 / L2).
+// scale = 1 / sqrt(mean(x^2) + eps).  One CTA per row.
+__device__ __forceinline__ float norm_scale(float ss, uint32_t n, float eps, float *part) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    float tot = (threadIdx.x & 31) < blockDim.x / 32 ? part[threadIdx.x & 31] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    return 1.f / sqrtf(tot / (float)n + eps);
+}
+// any length and alignment: the row is read from HBM once, the second sweep hits L1 / L2
 __global__ void __launch_bounds__(256) add_rmsnorm_kernel(float *x, const float *__restrict__ r,
                                                           const float *__restrict__ w, float *y, uint32_t n,
                                                           float eps, uint32_t x_stride, uint32_t y_stride) {
-    __shared__ float part[8];
+    __shared__ float part[32];
+    pdl_launch_dependents();
     float *xr = x + (size_t)blockIdx.x * x_stride;
     const float *rr = r ? r + (size_t)blockIdx.x * x_stride : nullptr;
     float *yr = y + (size_t)blockIdx.x * y_stride;
     float ss = 0.f;
+    pdl_wait();
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
         float v = xr[i];
         if (rr) {
@@ -138,24 +186,65 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(float *x, const float 
         }
         ss = fmaf(v, v, ss);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    float tot = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; i++) tot += part[i];
-    const float scale = 1.f / sqrtf(tot / (float)n + eps);
+    const float scale = norm_scale(ss, n, eps, part);
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) yr[i] = xr[i] * scale * w[i];
+}
+// Rows of up to 8192 floats, everything 16-byte aligned: a thread keeps its (at most two) groups of
+// four in registers, so there is one round trip to L2, for x, r and w together, and one sum.
+__global__ void __launch_bounds__(1024, 2) add_rmsnorm_vec_kernel(float *x, const float *__restrict__ r,
+                                                               const float *__restrict__ w, float *y, uint32_t n,
+                                                               float eps, uint32_t x_stride, uint32_t y_stride) {
+    __shared__ float part[32];
+    pdl_launch_dependents();
+    float4 *xr = reinterpret_cast<float4 *>(x + (size_t)blockIdx.x * x_stride);
+    const float4 *rr = r ? reinterpret_cast<const float4 *>(r + (size_t)blockIdx.x * x_stride) : nullptr;
+    float4 *yr = reinterpret_cast<float4 *>(y + (size_t)blockIdx.x * y_stride);
+    const float4 *w4 = reinterpret_cast<const float4 *>(w);
+    float4 v[2], g[2];
+    float ss = 0.f;
+    pdl_wait();
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const uint32_t i = threadIdx.x + j * blockDim.x;
+        v[j] = g[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < n / 4) {
+            v[j] = xr[i];
+            g[j] = w4[i];
+            if (rr) {
+                const float4 a = rr[i];
+                v[j].x += a.x; v[j].y += a.y; v[j].z += a.z; v[j].w += a.w;
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        ss = fmaf(v[j].x, v[j].x, fmaf(v[j].y, v[j].y, fmaf(v[j].z, v[j].z, fmaf(v[j].w, v[j].w, ss))));
+        const uint32_t i = threadIdx.x + j * blockDim.x;
+        if (rr && i < n / 4) xr[i] = v[j];
+    }
+    const float s = norm_scale(ss, n, eps, part);
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const uint32_t i = threadIdx.x + j * blockDim.x;
+        if (i < n / 4) yr[i] = make_float4(v[j].x * s * g[j].x, v[j].y * s * g[j].y, v[j].z * s * g[j].z, v[j].w * s * g[j].w);
+    }
 }
 
 // ---- SiLU gating: a = silu(a) * b ------------------------------------------------------
-__global__ void __launch_bounds__(256) silu_mul_kernel(float *a, const float *__restrict__ b, size_t n) {
-    const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float v = a[i];
-        a[i] = v / (1.f + expf(-v)) * b[i];
+__device__ __forceinline__ float silu_times(float v, float b) { return v / (1.f + expf(-v)) * b; }
+// `vec`: both pointers 16-byte aligned; the last n % 4 elements are taken one by one
+__global__ void __launch_bounds__(256) silu_mul_kernel(float *a, const float *__restrict__ b, size_t n, bool vec) {
+    pdl_launch_dependents();
+    const size_t stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t n4 = vec ? n / 4 : 0;
+    pdl_wait();
+    for (size_t i = first; i < n4; i += stride) {
+        float4 v = reinterpret_cast<const float4 *>(a)[i];
+        const float4 g = reinterpret_cast<const float4 *>(b)[i];
+        v.x = silu_times(v.x, g.x); v.y = silu_times(v.y, g.y); v.z = silu_times(v.z, g.z); v.w = silu_times(v.w, g.w);
+        reinterpret_cast<float4 *>(a)[i] = v;
     }
+    for (size_t i = n4 * 4 + first; i < n; i += stride) a[i] = silu_times(a[i], b[i]);
 }
 
 // ---- clamp / fake-quant around a linear -------------------------------------------------
@@ -163,8 +252,10 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(float *a, const float *__
 // [lo, hi] without rounding (SRQ.apply, LLM/Gemma/Gemma4Quant.swift:413-427).  Every step
 // rounds once, as the Swift code does, so the result is bit-exact.
 __global__ void __launch_bounds__(256) srq_kernel(const float *src, float *dst, size_t n, float scale, float lo, float hi) {
+    pdl_launch_dependents();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const float inv = scale != 0.f ? __fdiv_rn(1.f, scale) : 0.f;
+    pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const float v = src[i];
         if (scale != 0.f) {
@@ -212,8 +303,8 @@ int okf_argmax_rows(okf_ctx *ctx, const float *x, uint32_t n, uint32_t rows, int
     if (fault_fires(ctx)) return OKF_E_INJECTED;
     DeviceGuard g(ctx->device);
     if (!g.ok) return cuda_fail(ctx, cudaErrorInvalidDevice);
-    argmax_rows_kernel<<<rows, 512, 0, (cudaStream_t)stream>>>(x, out, n);
-    cudaError_t e = cudaGetLastError();
+    const uint32_t parts = n >= kArgmaxSplit && rows <= 0x7FFFFFFFu / kArgmaxCluster ? kArgmaxCluster : 1;
+    cudaError_t e = launch_pdl(argmax_rows_kernel, rows * parts, 256, 0, (cudaStream_t)stream, parts, x, out, n, parts);
     if (e != cudaSuccess) return cuda_fail(ctx, e);
     ctx->launches++;
     return OKF_OK;
@@ -227,8 +318,11 @@ int okf_add_rmsnorm(okf_ctx *ctx, float *x, const float *r, const float *weight,
     if (fault_fires(ctx)) return OKF_E_INJECTED;
     DeviceGuard g(ctx->device);
     if (!g.ok) return cuda_fail(ctx, cudaErrorInvalidDevice);
-    add_rmsnorm_kernel<<<rows, 256, 0, (cudaStream_t)stream>>>(x, r, weight, y, n, eps, x_stride, y_stride);
-    cudaError_t e = cudaGetLastError();
+    const bool vec = n % 4 == 0 && n <= 8192 && x_stride % 4 == 0 && y_stride % 4 == 0 &&
+                     (((uintptr_t)x | (uintptr_t)r | (uintptr_t)weight | (uintptr_t)y) & 15) == 0;
+    const unsigned threads = vec ? ((n + 7) / 8 + 31) / 32 * 32 : 256;  // two groups of four a thread
+    cudaError_t e = launch_pdl(vec ? add_rmsnorm_vec_kernel : add_rmsnorm_kernel, rows, threads, 0,
+                               (cudaStream_t)stream, 1, x, r, weight, y, n, eps, x_stride, y_stride);
     if (e != cudaSuccess) return cuda_fail(ctx, e);
     ctx->launches++;
     return OKF_OK;
@@ -240,8 +334,8 @@ int okf_silu_mul(okf_ctx *ctx, float *a, const float *b, size_t n, okf_stream st
     if (fault_fires(ctx)) return OKF_E_INJECTED;
     DeviceGuard g(ctx->device);
     if (!g.ok) return cuda_fail(ctx, cudaErrorInvalidDevice);
-    silu_mul_kernel<<<flat_blocks(n), 256, 0, (cudaStream_t)stream>>>(a, b, n);
-    cudaError_t e = cudaGetLastError();
+    const bool vec = (((uintptr_t)a | (uintptr_t)b) & 15) == 0;
+    cudaError_t e = launch_pdl(silu_mul_kernel, flat_blocks(vec ? (n + 3) / 4 : n), 256, 0, (cudaStream_t)stream, 1, a, b, n, vec);
     if (e != cudaSuccess) return cuda_fail(ctx, e);
     ctx->launches++;
     return OKF_OK;
@@ -259,8 +353,7 @@ int okf_srq(okf_ctx *ctx, const float *src, float *dst, size_t n, const okf_srq_
     if (fault_fires(ctx)) return OKF_E_INJECTED;
     DeviceGuard g(ctx->device);
     if (!g.ok) return cuda_fail(ctx, cudaErrorInvalidDevice);
-    srq_kernel<<<flat_blocks(n), 256, 0, (cudaStream_t)stream>>>(src, dst, n, side->scale, side->lo, side->hi);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pdl(srq_kernel, flat_blocks(n), 256, 0, (cudaStream_t)stream, 1, src, dst, n, side->scale, side->lo, side->hi);
     if (e != cudaSuccess) return cuda_fail(ctx, e);
     ctx->launches++;
     return OKF_OK;
