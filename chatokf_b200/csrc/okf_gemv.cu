@@ -1689,9 +1689,16 @@ static bool gemv_layout(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t t
 // by side, and they do not slow each other down much (a CTA alone issues on a third of the cycles).
 // (One column only: with several columns two CTAs on an SM, each staging its slices of x at
 // barriers, were 16 % slower than two tiles in a row.)
+// From eight tiles per SM on, two CTAs share every SM: eight warps wait for one another's
+// instructions on two thirds of the cycles, sixteen fill them (Q4_K 2560 -> 65536 22.3 -> 18.5 us,
+// Q8_0 2048 -> 65536 37.2 -> 25.2, IQ2_XXS 5120 -> 34816 31.1 -> 27.7, four columns 73.7 -> 63.1).
+// Below that the second panel of x and the lost room for the next launch's first copies cost as
+// much as they gain (Q4_K 2560 -> 9728, four tiles per SM: 6.0 us both ways).
+constexpr uint32_t kTwoCtasTiles = 8;
 static uint32_t gemv_ctas(uint32_t tiles, int sms, bool sep) {
     const uint32_t n = (uint32_t)sms;
     if (tiles <= n) return tiles;
+    if (tiles >= kTwoCtasTiles * n) return 2 * n;
     return sep && tiles <= n + n / 4 ? tiles : n;
 }
 
