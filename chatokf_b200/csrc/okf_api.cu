@@ -110,7 +110,12 @@ int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uin
             if (e != cudaSuccess) return cuda_fail(ctx, e);
             return OKF_OK;
         } else {
-            if (!simple) ctx->fallbacks++;  // a shape or alignment the tensor-core matvec does not take
+            if (!simple) ctx->fallbacks++;  // a shape or alignment the kernels above do not take
+            if (!simple && gemv_ragged_supported(ty, k, m, wp, x, xdt, n, ctx->sms)) {
+                e = launch_gemv_fast(ty, wp, k, m, x, xdt, n, (float *)out, ctx->dev_status, s, ctx->sms, ctx->device,
+                                     &ctx->launches);
+                return e == cudaSuccess ? OKF_OK : cuda_fail(ctx, e);
+            }
             e = launch_gemv_simple(ty, wp, k, m, x, xdt, n, (float *)out, s);
         }
     } else if (!(ctx->flags & OKF_FLAG_SIMPLE_KERNELS) && gemm_tc_supported(ty, k, m, wp, x, xdt, n)) {

@@ -28,10 +28,11 @@
 // g % 2 of x).  Thread c of a quad owns the k of quarter c and feeds x only into
 // that quarter's columns, so the accumulator a thread reads back is the sum over
 // exactly the 64 k whose block scales it decoded.
-//   Two to four columns ("WIDE"): MMA column g stands for (activation column g / 2,
-// byte g % 2); one MMA per 32-wide block, fed by all four threads of the quad.
-// More than four columns are run as passes.
+//   Several columns ("WIDE"): x is the A operand, see okf_gemv_wide.cuh.
+#include <cooperative_groups.h>
+
 #include "okf_gemv_mma.cuh"
+#include "okf_gemv_wide.cuh"
 #include "okf_kernels.h"
 
 namespace okf {
@@ -54,11 +55,12 @@ struct GemvLayout {
     uint32_t tps;          // tiles per stage (mode 0 only, else 1)
     uint32_t ragged;       // mode 2: row segments do not start on 16-byte boundaries
     uint32_t group;        // tiles summed per barrier
-    uint32_t nc;           // real activation columns of this pass
-    uint32_t ecols;        // byte columns of the x panel in shared memory: hi and lo of every activation column
+    uint32_t nc;           // activation columns of this pass
+    uint32_t nc_inv;       // i / nc = i * nc_inv >> 16 for the few hundred (tile, column) pairs of a group
     uint32_t es;           // bytes between columns of the x panel
     uint32_t panel;        // k-chunks whose slice of x is staged together
-    uint32_t xs_off, info_off, red_off, tab_off;  // byte offsets in dynamic shared memory
+    uint32_t clog;         // log2 of the CTAs of a cluster, each with its share of K of the cluster's tiles (0: no clusters)
+    uint32_t xs_off, info_off, red_off, tab_off, part_off;  // byte offsets in dynamic shared memory
     uint32_t tab_copies;   // IQ2_XXS: copies of every codebook entry, side by side (a power of two)
     uint32_t smem_bytes;
 };
@@ -73,6 +75,7 @@ constexpr uint32_t kConsumers = kGemvWarps * 32;
 // bank groups.
 constexpr uint32_t kXqUnit = 256;
 constexpr float kXqMax = 32512.f;  // 127 * 256: hi stays a signed byte after rounding
+constexpr float kXq3Max = 8323072.f;  // 127 * 65536, three bytes
 // SEP x panel: per byte column and unit, four quarters of 80 bytes: 64 bytes of x in k
 // order, then (first byte column only) the quarter's record {scale, scale * sum of x over
 // its first 32-wide block, over its second, -}.  One address register reaches a
@@ -91,97 +94,6 @@ __host__ __device__ inline uint32_t sep_col_stride(uint32_t units) {
 }
 __host__ __device__ inline uint32_t xq_piece_offset(uint32_t c, uint32_t piece) {
     return c * 64 + ((piece ^ (c >> 1)) & 3u) * 16;
-}
-
-__device__ __forceinline__ uint4 lds128(const uint8_t *p) { return *reinterpret_cast<const uint4 *>(p); }
-
-// Shared-memory loads by 32-bit shared-window address: the one-column path does
-// all its address arithmetic in 32 bits.
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint2 lds64(uint32_t a) {
-    uint2 v;
-    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ uint32_t lds16(uint32_t a) {
-    uint32_t v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a));
-    return v;
-}
-// 4 * NW bytes from a 2-byte aligned shared address: aligned words and a funnel shift
-template <int NW>
-__device__ __forceinline__ void lds_a2(uint32_t a, uint32_t (&out)[NW]) {
-    const uint32_t base = a & ~3u, sh = (a & 2u) * 8u;
-    uint32_t w[NW + 1];
-#pragma unroll
-    for (int i = 0; i <= NW; i++) w[i] = lds32(base + 4 * i);
-#pragma unroll
-    for (int i = 0; i < NW; i++) out[i] = __funnelshift_r(w[i], w[i + 1], sh);
-}
-__device__ __forceinline__ uint2 lds64(const uint8_t *p) { return *reinterpret_cast<const uint2 *>(p); }
-__device__ __forceinline__ int ubyte(uint32_t v, int i) { return (int)__byte_perm(v, 0, 0x4440 + i); }
-__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
-    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void sts32(uint32_t a, uint32_t x) {
-    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(x) : "memory");
-}
-__device__ __forceinline__ void sts16(uint32_t a, uint32_t x) {
-    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "r"(x) : "memory");
-}
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t v;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(v) : "r"(a), "r"(b), "r"(sel));
-    return v;
-}
-
-// 4 * NW bytes from a 2-byte aligned shared-memory address, as aligned 32-bit
-// loads plus a funnel shift when the address is 2 mod 4.
-template <int NW>
-__device__ __forceinline__ void lds_a2(const uint8_t *p, uint32_t (&out)[NW]) {
-    const uint32_t *base = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3);
-    const uint32_t sh = ((uint32_t)reinterpret_cast<uintptr_t>(p) & 2u) * 8u;
-    uint32_t w[NW + 1];
-#pragma unroll
-    for (int i = 0; i <= NW; i++) w[i] = base[i];
-#pragma unroll
-    for (int i = 0; i < NW; i++) out[i] = __funnelshift_r(w[i], w[i + 1], sh);
-}
-
-// 6-bit (scale, min) of Q4_K sub-blocks 2c and 2c+1 (ggml get_scale_min_k4,
-// LLM/Quantize/KQuants.swift:86-101), as byte pairs in the low 16 bits.
-__device__ __forceinline__ void q4k_scale_min(const uint4 &h, uint32_t c, uint32_t &sc, uint32_t &mn) {
-    const uint32_t sh = (c & 1) * 16;
-    const uint32_t a = h.y >> sh, b = h.z >> sh, e = h.w >> sh;
-    if (c < 2) {
-        sc = a & 0x3F3Fu;
-        mn = b & 0x3F3Fu;
-    } else {
-        sc = (e & 0x0F0Fu) | ((a >> 2) & 0x3030u);
-        mn = ((e >> 4) & 0x0F0Fu) | ((b >> 2) & 0x3030u);
-    }
-}
-// The same for two rows at once: bytes {row a: 2c, 2c+1, row b: 2c, 2c+1}.
-__device__ __forceinline__ void q4k_scale_min2(const uint4 &ha, const uint4 &hb, uint32_t c, uint32_t &sc,
-                                               uint32_t &mn) {
-    const uint32_t sel = (c & 1) ? 0x7632u : 0x5410u;
-    const uint32_t a = __byte_perm(ha.y, hb.y, sel), b = __byte_perm(ha.z, hb.z, sel), e = __byte_perm(ha.w, hb.w, sel);
-    if (c < 2) {
-        sc = a & 0x3F3F3F3Fu;
-        mn = b & 0x3F3F3F3Fu;
-    } else {
-        sc = (e & 0x0F0F0F0Fu) | ((a >> 2) & 0x30303030u);
-        mn = ((e >> 4) & 0x0F0F0F0Fu) | ((b >> 2) & 0x30303030u);
-    }
 }
 
 // ---- integer MMA: D (16 x 8, s32) += A (16 x 32, bytes) * B (32 x 8, signed bytes) ----
@@ -213,20 +125,6 @@ __device__ __forceinline__ void imma0(int (&d)[4], uint32_t a0, uint32_t a1, uin
             : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
             : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
-// IQ2_XXS: byte masks (0xFF = negative) of the eight weights a 7-bit sign index stands
-// for; the eighth sign is the parity of the seven (LLM/Quantize/IQ2Grid.swift:73-85).
-// n * 0x00204081 puts bit j of a nibble on bit 8j (and on bits that the AND drops; no
-// two of its terms meet, so nothing carries); times 0xFF a set bit fills its byte.
-// Computed rather than looked up: look-ups at data-dependent addresses collide on
-// shared-memory banks, and the multiplies run on the otherwise idle FMA pipe.
-__device__ __forceinline__ uint2 iq2_sign_masks(uint32_t idx7) {
-    const uint32_t lo = idx7 & 15u, hi = (idx7 >> 4) | ((__popc(idx7) & 1u) << 3);
-    uint2 m;
-    m.x = ((lo * 0x00204081u) & 0x01010101u) * 0xFFu;
-    m.y = ((hi * 0x00204081u) & 0x01010101u) * 0xFFu;
-    return m;
-}
-
 // sum over the hi and lo bytes of x: columns 2c (hi) and 2c+1 (lo) of one row
 __device__ __forceinline__ float join_hi_lo(int hi, int lo) { return (float)(hi * 256 + lo); }
 
@@ -237,11 +135,9 @@ struct SepConst {
     uint32_t hoff;          // Q2_0: where the block that share lies in starts
     uint32_t sel, m1, m2;   // Q4_K: how to pick this thread's 6-bit scales and mins out of the 12 bytes
     bool low;               // Q4_K: sub-blocks 0..3 (plain 6-bit fields) or 4..7 (split fields)
-    uint32_t tab_lane;      // IQ2_XXS: shared address of this lane's copy of codebook entry 0
-    uint32_t tab_stride;    // IQ2_XXS: bytes between table entries (copies of one entry lie side by side)
 };
 template <int TY>
-__device__ __forceinline__ SepConst sep_const(uint32_t c, uint32_t lane, uint32_t tab, uint32_t tab_copies) {
+__device__ __forceinline__ SepConst sep_const(uint32_t c) {
     SepConst k = {};
     if constexpr (TY == T_Q4_K || TY == T_Q5_K) {
         k.qoff = (TY == T_Q4_K ? 16 : 48) + 32 * c;
@@ -264,21 +160,8 @@ __device__ __forceinline__ SepConst sep_const(uint32_t c, uint32_t lane, uint32_
         k.qoff = k.hoff + 2 + 16 * (c & 1);
     } else {
         k.qoff = 2 + 16 * c;
-        k.tab_lane = tab + (lane & (tab_copies - 1)) * 8;
-        k.tab_stride = tab_copies * 8;
     }
     return k;
-}
-
-// IQ2_XXS: byte masks (0xFF = negative) of the eight weights a 7-bit sign index stands
-// for; the eighth sign is the parity of the seven (LLM/Quantize/IQ2Grid.swift:73-85).
-// One multiply puts sign bit j on the top bit of byte j (the shifted copies of a 7-bit
-// number do not overlap, so nothing carries), and a byte permute in its
-// sign-replicating mode fills each byte with its top bit.
-__device__ __forceinline__ void iq2_sign_bytes(uint32_t idx7, uint32_t &lo, uint32_t &hi) {
-    const uint32_t par = (uint32_t)__popc(idx7) << 31;
-    lo = prmt(idx7 * 0x10204080u, 0u, 0xBA98u);        // signs 0..3: shifts 7, 14, 21, 28
-    hi = prmt(idx7 * 0x00020408u + par, 0u, 0xBA98u);  // signs 4..6: shifts 3, 10, 17; parity on bit 31
 }
 
 // IQ4_NL: the sixteen codebook values (LLM/Gemma/Gemma4Quant.swift:5-9) for four nibbles (one per
@@ -300,7 +183,7 @@ __device__ __forceinline__ uint32_t iq4nl_lookup(uint32_t v) {
 // the first 32-wide block of the quarter, over the second, -} as float bits.
 // acc: rows g and g + 8.
 template <int TY>
-__device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepConst &K, const uint32_t (&xf)[16],
+__device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepConst &K, const Iq2Tab &tab, const uint32_t (&xf)[16],
                                          const uint4 &xi, float (&acc)[2]) {
     const float xs = __uint_as_float(xi.x);
     if constexpr (TY == T_Q4_K) {
@@ -546,32 +429,28 @@ __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepCons
         lds_a2<4>(ua + K.qoff, wa);
         lds_a2<4>(ub + K.qoff, wb);
         const float da = f16bits(lds16(ua + K.hoff)), db = f16bits(lds16(ub + K.hoff));
-        int t[4] = {0, 0, 0, 0};  // both 32-wide halves together, times 64
+        int d[4][4];  // per code position, both 32-wide halves; position s carries a factor 4^s
 #pragma unroll
-        for (int sub = 0; sub < 2; sub++) {
-#pragma unroll
-            for (int s = 0; s < 4; s++) {
-                const uint32_t m = 0x03030303u << (2 * s);
-                int d[4];
-                imma0<false>(d, wa[2 * sub] & m, wb[2 * sub] & m, wa[2 * sub + 1] & m, wb[2 * sub + 1] & m,
-                             xf[8 * sub + s], xf[8 * sub + 4 + s]);
-#pragma unroll
-                for (int e = 0; e < 4; e++) t[e] = t[e] + d[e] * (64 >> (2 * s));
-            }
+        for (int s = 0; s < 4; s++) {
+            const uint32_t m = 0x03030303u << (2 * s);
+            imma0<false>(d[s], wa[0] & m, wb[0] & m, wa[1] & m, wb[1] & m, xf[s], xf[4 + s]);
         }
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+            const uint32_t m = 0x03030303u << (2 * s);
+            imma<false>(d[s], wa[2] & m, wb[2] & m, wa[3] & m, wb[3] & m, xf[8 + s], xf[12 + s]);
+        }
+        int t[4];  // times 64
+#pragma unroll
+        for (int e = 0; e < 4; e++) t[e] = ((d[0][e] * 4 + d[1][e]) * 4 + d[2][e]) * 4 + d[3][e];
         const float xsum = __uint_as_float(xi.y) + __uint_as_float(xi.z);  // scale * sum of x over the quarter
         acc[0] += da * (xs * 0.015625f * join_hi_lo(t[0], t[1]) - xsum);
         acc[1] += db * (xs * 0.015625f * join_hi_lo(t[2], t[3]) - xsum);
     } else {
         // IQ2_XXS {f16 d; 8 x (u32 a0: four codebook indices, u32 a1: four 7-bit sign
         // indices + 4-bit scale)} (LLM/Quantize/IQ2XXS.swift:34-53).  Thread c takes
-        // sub-blocks 2c and 2c+1.  A codebook entry is eight magnitude bytes = the two
-        // A registers of one row; the byte masks of a sign index (0xFF = negative) are
-        // computed (a table of them, tried, gained 2 % at K = 5120 and cost 8 % at K = 17408,
-        // where it crowds the ring out of shared memory).  Signs: XOR with the mask turns a
-        // magnitude m into the signed byte -(m + 1); a second MMA on the masks themselves
-        // (255 per negative weight) gives 255 x the sum of x over the negative weights, which
-        // puts the missing 1 back: sum(sign * m * x) = D1 + D2 / 255.
+        // sub-blocks 2c and 2c+1.  A codebook entry is eight signed bytes = the two A registers
+        // of a row.
         uint32_t wa[4], wb[4];
         lds_a2<4>(ua + K.qoff, wa);
         lds_a2<4>(ub + K.qoff, wb);
@@ -580,25 +459,17 @@ __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepCons
 #pragma unroll
         for (int sb = 0; sb < 2; sb++) {
             const uint32_t a0a = wa[2 * sb], a1a = wa[2 * sb + 1], a0b = wb[2 * sb], a1b = wb[2 * sb + 1];
-            int d1[4], d2[4];
+            int d[4];
 #pragma unroll
             for (int l = 0; l < 4; l++) {
-                const uint2 ea = lds64(K.tab_lane + prmt(a0a, 0u, 0x4440u + l) * K.tab_stride);
-                const uint2 eb = lds64(K.tab_lane + prmt(a0b, 0u, 0x4440u + l) * K.tab_stride);
-                uint2 ma, mb;
-                iq2_sign_bytes((a1a >> (7 * l)) & 127u, ma.x, ma.y);
-                iq2_sign_bytes((a1b >> (7 * l)) & 127u, mb.x, mb.y);
+                const uint2 ea = tab.bytes(prmt(a0a, 0u, 0x4440u + l), a1a >> (7 * l));
+                const uint2 eb = tab.bytes(prmt(a0b, 0u, 0x4440u + l), a1b >> (7 * l));
                 const uint32_t x0 = xf[8 * sb + 2 * l], x1 = xf[8 * sb + 2 * l + 1];
-                if (l == 0) {
-                    imma0<true>(d1, ea.x ^ ma.x, eb.x ^ mb.x, ea.y ^ ma.y, eb.y ^ mb.y, x0, x1);
-                    imma0<false>(d2, ma.x, mb.x, ma.y, mb.y, x0, x1);
-                } else {
-                    imma<true>(d1, ea.x ^ ma.x, eb.x ^ mb.x, ea.y ^ ma.y, eb.y ^ mb.y, x0, x1);
-                    imma<false>(d2, ma.x, mb.x, ma.y, mb.y, x0, x1);
-                }
+                if (l == 0) imma0<true>(d, ea.x, eb.x, ea.y, eb.y, x0, x1);
+                else imma<true>(d, ea.x, eb.x, ea.y, eb.y, x0, x1);
             }
-            sum[sb][0] = fmaf(join_hi_lo(d2[0], d2[1]), 1.f / 255.f, join_hi_lo(d1[0], d1[1]));
-            sum[sb][1] = fmaf(join_hi_lo(d2[2], d2[3]), 1.f / 255.f, join_hi_lo(d1[2], d1[3]));
+            sum[sb][0] = join_hi_lo(d[0], d[1]);
+            sum[sb][1] = join_hi_lo(d[2], d[3]);
         }
         const float sa0 = 0.5f + (float)(wa[1] >> 28), sa1 = 0.5f + (float)(wa[3] >> 28);
         const float sb0 = 0.5f + (float)(wb[1] >> 28), sb1 = 0.5f + (float)(wb[3] >> 28);
@@ -607,304 +478,7 @@ __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepCons
     }
 }
 
-// ---- per-unit arithmetic, up to four columns ("WIDE") ---------------------------
-// MMA column g stands for (activation column g / 2, byte g % 2 of x); all four
-// threads of a quad feed every MMA, thread c with the eight k [8c, 8c + 8) of a
-// 32-wide block (Q2_0: k = 16w + 4b + c for word w, byte b).  One MMA per block:
-// what comes back to thread (g, c) is the block's integer sum for rows g, g + 8
-// and activation column c, hi and lo byte.  Block scales multiply these sums as
-// integers where they are integers (Q4_K), else in fp32.
-// xf: this thread's 64 bytes of x for the unit, block b in xf[2b], xf[2b+1].
-// xw: {xs, -, -, -, X0..X7}: the unit's scale for column c and the integer sums
-// of x over its eight blocks.  acc: rows g, g + 8 of column c.
-
-template <int TY>
-__device__ __forceinline__ void unit_wide(const uint8_t *ua, const uint8_t *ub, uint32_t c, const uint32_t (&xf)[16],
-                                          const float *xw, const uint2 *tab, uint32_t tab_copies, float (&acc)[2]) {
-    const float xs = xw[0];
-    if constexpr (TY == T_Q4_K) {
-        const uint4 ha = lds128(ua), hb = lds128(ub);
-        // 6-bit scales and mins of the eight sub-blocks, four to a word (get_scale_min_k4)
-        const uint32_t sa03 = ha.y & 0x3F3F3F3Fu, ma03 = ha.z & 0x3F3F3F3Fu;
-        const uint32_t sa47 = (ha.w & 0x0F0F0F0Fu) | ((ha.y >> 2) & 0x30303030u);
-        const uint32_t ma47 = ((ha.w >> 4) & 0x0F0F0F0Fu) | ((ha.z >> 2) & 0x30303030u);
-        const uint32_t sb03 = hb.y & 0x3F3F3F3Fu, mb03 = hb.z & 0x3F3F3F3Fu;
-        const uint32_t sb47 = (hb.w & 0x0F0F0F0Fu) | ((hb.y >> 2) & 0x30303030u);
-        const uint32_t mb47 = ((hb.w >> 4) & 0x0F0F0F0Fu) | ((hb.z >> 2) & 0x30303030u);
-        const int4 x03 = *reinterpret_cast<const int4 *>(xw + 4), x47 = *reinterpret_cast<const int4 *>(xw + 8);
-        const int xb[8] = {x03.x, x03.y, x03.z, x03.w, x47.x, x47.y, x47.z, x47.w};
-        const uint32_t ml = 0x0F0F0F0Fu, mh = 0xF0F0F0F0u;
-        int te[4] = {0, 0, 0, 0}, to[4] = {0, 0, 0, 0};  // sum of scale * block sum: low-nibble / high-nibble blocks
-        int mina = 0, minb = 0;
-#pragma unroll
-        for (int p = 0; p < 4; p++) {  // 32 bytes of nibbles: block 2p in the low ones, 2p+1 in the high ones
-            const uint2 wa = lds64(ua + 16 + 32 * p + 8 * c), wb = lds64(ub + 16 + 32 * p + 8 * c);
-            const int sa0 = ubyte(p < 2 ? sa03 : sa47, (2 * p) & 3), sa1 = ubyte(p < 2 ? sa03 : sa47, (2 * p + 1) & 3);
-            const int sb0 = ubyte(p < 2 ? sb03 : sb47, (2 * p) & 3), sb1 = ubyte(p < 2 ? sb03 : sb47, (2 * p + 1) & 3);
-            int d[4];
-            imma0<false>(d, wa.x & ml, wb.x & ml, wa.y & ml, wb.y & ml, xf[4 * p], xf[4 * p + 1]);
-            te[0] += sa0 * d[0]; te[1] += sa0 * d[1]; te[2] += sb0 * d[2]; te[3] += sb0 * d[3];
-            imma0<false>(d, wa.x & mh, wb.x & mh, wa.y & mh, wb.y & mh, xf[4 * p + 2], xf[4 * p + 3]);
-            to[0] += sa1 * d[0]; to[1] += sa1 * d[1]; to[2] += sb1 * d[2]; to[3] += sb1 * d[3];
-            mina += ubyte(p < 2 ? ma03 : ma47, (2 * p) & 3) * xb[2 * p] + ubyte(p < 2 ? ma03 : ma47, (2 * p + 1) & 3) * xb[2 * p + 1];
-            minb += ubyte(p < 2 ? mb03 : mb47, (2 * p) & 3) * xb[2 * p] + ubyte(p < 2 ? mb03 : mb47, (2 * p + 1) & 3) * xb[2 * p + 1];
-        }
-        const float da = f16bits(ha.x & 0xFFFF), dma = f16bits(ha.x >> 16);
-        const float db = f16bits(hb.x & 0xFFFF), dmb = f16bits(hb.x >> 16);
-        // The scaled sums no longer fit 256 * hi + lo in 32 bits: join them in fp32.  The
-        // high-nibble sums are exact multiples of 16, taken out by a shift; everything
-        // converted is below 2^24 in magnitude.
-        auto join = [](int hi, int lo) { return fmaf((float)hi, 256.f, (float)lo); };
-        acc[0] += xs * (da * (join(te[0], te[1]) + join(to[0] >> 4, to[1] >> 4)) - dma * (float)mina);
-        acc[1] += xs * (db * (join(te[2], te[3]) + join(to[2] >> 4, to[3] >> 4)) - dmb * (float)minb);
-    } else if constexpr (TY == T_Q5_K) {
-        // Q4_K's layout with qh[32] after the header and a fifth bit per weight: bit j of qh[l]
-        // for sub-block j (LLM/Quantize/KQuants.swift:127-158); this thread's l are 8c .. 8c + 7
-        const uint2 ga = lds64(ua + 16 + 8 * c), gb = lds64(ub + 16 + 8 * c);
-        const uint4 ha = lds128(ua), hb = lds128(ub);
-        // 6-bit scales and mins of the eight sub-blocks, four to a word (get_scale_min_k4)
-        const uint32_t sa03 = ha.y & 0x3F3F3F3Fu, ma03 = ha.z & 0x3F3F3F3Fu;
-        const uint32_t sa47 = (ha.w & 0x0F0F0F0Fu) | ((ha.y >> 2) & 0x30303030u);
-        const uint32_t ma47 = ((ha.w >> 4) & 0x0F0F0F0Fu) | ((ha.z >> 2) & 0x30303030u);
-        const uint32_t sb03 = hb.y & 0x3F3F3F3Fu, mb03 = hb.z & 0x3F3F3F3Fu;
-        const uint32_t sb47 = (hb.w & 0x0F0F0F0Fu) | ((hb.y >> 2) & 0x30303030u);
-        const uint32_t mb47 = ((hb.w >> 4) & 0x0F0F0F0Fu) | ((hb.z >> 2) & 0x30303030u);
-        const int4 x03 = *reinterpret_cast<const int4 *>(xw + 4), x47 = *reinterpret_cast<const int4 *>(xw + 8);
-        const int xb[8] = {x03.x, x03.y, x03.z, x03.w, x47.x, x47.y, x47.z, x47.w};
-        const uint32_t ml = 0x0F0F0F0Fu;
-        int te[4] = {0, 0, 0, 0}, to[4] = {0, 0, 0, 0};  // sum of scale * block sum: low-nibble / high-nibble blocks
-        int mina = 0, minb = 0;
-#pragma unroll
-        for (int p = 0; p < 4; p++) {  // 32 bytes of nibbles: block 2p in the low ones, 2p+1 in the high ones
-            const uint2 wa = lds64(ua + 48 + 32 * p + 8 * c), wb = lds64(ub + 48 + 32 * p + 8 * c);
-            const uint32_t b1 = 0x01010101u;
-            const uint32_t la0 = (wa.x & ml) | (((ga.x >> (2 * p)) & b1) << 4), la1 = (wa.y & ml) | (((ga.y >> (2 * p)) & b1) << 4);
-            const uint32_t lb0 = (wb.x & ml) | (((gb.x >> (2 * p)) & b1) << 4), lb1 = (wb.y & ml) | (((gb.y >> (2 * p)) & b1) << 4);
-            const uint32_t ha0 = ((wa.x >> 4) & ml) | (((ga.x >> (2 * p + 1)) & b1) << 4), ha1 = ((wa.y >> 4) & ml) | (((ga.y >> (2 * p + 1)) & b1) << 4);
-            const uint32_t hb0 = ((wb.x >> 4) & ml) | (((gb.x >> (2 * p + 1)) & b1) << 4), hb1 = ((wb.y >> 4) & ml) | (((gb.y >> (2 * p + 1)) & b1) << 4);
-            const int sa0 = ubyte(p < 2 ? sa03 : sa47, (2 * p) & 3), sa1 = ubyte(p < 2 ? sa03 : sa47, (2 * p + 1) & 3);
-            const int sb0 = ubyte(p < 2 ? sb03 : sb47, (2 * p) & 3), sb1 = ubyte(p < 2 ? sb03 : sb47, (2 * p + 1) & 3);
-            int d[4];
-            imma0<false>(d, la0, lb0, la1, lb1, xf[4 * p], xf[4 * p + 1]);
-            te[0] += sa0 * d[0]; te[1] += sa0 * d[1]; te[2] += sb0 * d[2]; te[3] += sb0 * d[3];
-            imma0<false>(d, ha0, hb0, ha1, hb1, xf[4 * p + 2], xf[4 * p + 3]);
-            to[0] += sa1 * d[0]; to[1] += sa1 * d[1]; to[2] += sb1 * d[2]; to[3] += sb1 * d[3];
-            mina += ubyte(p < 2 ? ma03 : ma47, (2 * p) & 3) * xb[2 * p] + ubyte(p < 2 ? ma03 : ma47, (2 * p + 1) & 3) * xb[2 * p + 1];
-            minb += ubyte(p < 2 ? mb03 : mb47, (2 * p) & 3) * xb[2 * p] + ubyte(p < 2 ? mb03 : mb47, (2 * p + 1) & 3) * xb[2 * p + 1];
-        }
-        const float da = f16bits(ha.x & 0xFFFF), dma = f16bits(ha.x >> 16);
-        const float db = f16bits(hb.x & 0xFFFF), dmb = f16bits(hb.x >> 16);
-        // The scaled sums no longer fit 256 * hi + lo in 32 bits: join them in fp32.
-        auto join = [](int hi, int lo) { return fmaf((float)hi, 256.f, (float)lo); };
-        acc[0] += xs * (da * (join(te[0], te[1]) + join(to[0], to[1])) - dma * (float)mina);
-        acc[1] += xs * (db * (join(te[2], te[3]) + join(to[2], to[3])) - dmb * (float)minb);
-    } else if constexpr (TY == T_IQ4_NL) {
-        float fa = 0.f, fb = 0.f;
-        const uint32_t sh = 4 * (c >> 1);  // threads 0, 1: low nibbles (k 0..15); 2, 3: high (k 16..31)
-#pragma unroll
-        for (int b = 0; b < 8; b++) {  // block b: {f16 d; u8 qs[16]}, this thread's eight bytes at 2 + 8 (c & 1)
-            uint32_t qa[2], qb[2];
-            lds_a2<2>(ua + 18 * b + 2 + 8 * (c & 1), qa);
-            lds_a2<2>(ub + 18 * b + 2 + 8 * (c & 1), qb);
-            int d[4];
-            imma0<true>(d, iq4nl_lookup((qa[0] >> sh) & 0x0F0F0F0Fu), iq4nl_lookup((qb[0] >> sh) & 0x0F0F0F0Fu),
-                        iq4nl_lookup((qa[1] >> sh) & 0x0F0F0F0Fu), iq4nl_lookup((qb[1] >> sh) & 0x0F0F0F0Fu), xf[2 * b], xf[2 * b + 1]);
-            fa += f16bits(ld_u16(ua + 18 * b)) * join_hi_lo(d[0], d[1]);
-            fb += f16bits(ld_u16(ub + 18 * b)) * join_hi_lo(d[2], d[3]);
-        }
-        acc[0] += xs * fa;
-        acc[1] += xs * fb;
-    } else if constexpr (TY == T_Q6_K) {
-        // Block b = half n = b / 4 of the unit, granule r = b % 4 (see the one-column path).  This
-        // thread's eight weights l = 8c .. 8c + 7 share one of the block's two 16-wide scales,
-        // threads 0, 1 the first and 2, 3 the second: two MMAs per block, each fed by the two
-        // threads of one scale (the others pass zeros), so that each sum meets its own scale.
-        float fa = 0.f, fb = 0.f;
-        const bool first = c < 2;
-#pragma unroll
-        for (int b = 0; b < 8; b++) {
-            const int n = b >> 2, r = b & 3;
-            uint32_t la[2], lb[2], ha[2], hb[2];
-            lds_a2<2>(ua + 64 * n + 32 * (r & 1) + 8 * c, la);
-            lds_a2<2>(ub + 64 * n + 32 * (r & 1) + 8 * c, lb);
-            lds_a2<2>(ua + 128 + 32 * n + 8 * c, ha);
-            lds_a2<2>(ub + 128 + 32 * n + 8 * c, hb);
-            uint32_t qa[2], qb[2];
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const uint32_t va = (((la[i] >> (r >= 2 ? 4 : 0)) & 0x0F0F0F0Fu) | (((ha[i] >> (2 * r)) & 0x03030303u) << 4)) ^ 0x20202020u;
-                const uint32_t vb = (((lb[i] >> (r >= 2 ? 4 : 0)) & 0x0F0F0F0Fu) | (((hb[i] >> (2 * r)) & 0x03030303u) << 4)) ^ 0x20202020u;
-                qa[i] = va | ((va & 0x20202020u) * 6u);  // q - 32 as a signed byte
-                qb[i] = vb | ((vb & 0x20202020u) * 6u);
-            }
-            const uint32_t sca = ld_u16(ua + 192 + 8 * n + 2 * r), scb = ld_u16(ub + 192 + 8 * n + 2 * r);
-            int d0[4], d1[4];
-            imma0<true>(d0, first ? qa[0] : 0u, first ? qb[0] : 0u, first ? qa[1] : 0u, first ? qb[1] : 0u, xf[2 * b], xf[2 * b + 1]);
-            imma0<true>(d1, first ? 0u : qa[0], first ? 0u : qb[0], first ? 0u : qa[1], first ? 0u : qb[1], xf[2 * b], xf[2 * b + 1]);
-            fa += (float)(int)(int8_t)(sca & 0xFF) * join_hi_lo(d0[0], d0[1]) + (float)(int)(int8_t)(sca >> 8) * join_hi_lo(d1[0], d1[1]);
-            fb += (float)(int)(int8_t)(scb & 0xFF) * join_hi_lo(d0[2], d0[3]) + (float)(int)(int8_t)(scb >> 8) * join_hi_lo(d1[2], d1[3]);
-        }
-        acc[0] += xs * f16bits(ld_u16(ua + 208)) * fa;
-        acc[1] += xs * f16bits(ld_u16(ub + 208)) * fb;
-    } else if constexpr (TY == T_Q4_0) {
-        const int4 x03 = *reinterpret_cast<const int4 *>(xw + 4), x47 = *reinterpret_cast<const int4 *>(xw + 8);
-        const int xb[8] = {x03.x, x03.y, x03.z, x03.w, x47.x, x47.y, x47.z, x47.w};
-        float fa = 0.f, fb = 0.f;
-        const uint32_t sh = 4 * (c >> 1);  // threads 0, 1: low nibbles (k 0..15); 2, 3: high (k 16..31)
-#pragma unroll
-        for (int b = 0; b < 8; b++) {  // block b: {f16 d; u8 qs[16]}, this thread's eight bytes at 2 + 8 (c & 1)
-            uint32_t qa[2], qb[2];
-            lds_a2<2>(ua + 18 * b + 2 + 8 * (c & 1), qa);
-            lds_a2<2>(ub + 18 * b + 2 + 8 * (c & 1), qb);
-            int d[4];
-            imma0<false>(d, (qa[0] >> sh) & 0x0F0F0F0Fu, (qb[0] >> sh) & 0x0F0F0F0Fu, (qa[1] >> sh) & 0x0F0F0F0Fu,
-                         (qb[1] >> sh) & 0x0F0F0F0Fu, xf[2 * b], xf[2 * b + 1]);
-            // (q - 8) * d: eight times the block's sum of x leaves again
-            fa += f16bits(ld_u16(ua + 18 * b)) * (float)(d[0] * 256 + d[1] - 8 * xb[b]);
-            fb += f16bits(ld_u16(ub + 18 * b)) * (float)(d[2] * 256 + d[3] - 8 * xb[b]);
-        }
-        acc[0] += xs * fa;
-        acc[1] += xs * fb;
-    } else if constexpr (TY == T_Q8_0) {
-        float fa = 0.f, fb = 0.f;
-#pragma unroll
-        for (int b = 0; b < 8; b++) {  // block b: {f16 d; i8 q[32]}, this thread's quants at 2 + 8c
-            uint32_t qa[2], qb[2];
-            lds_a2<2>(ua + 34 * b + 2 + 8 * c, qa);
-            lds_a2<2>(ub + 34 * b + 2 + 8 * c, qb);
-            int d[4];
-            imma0<true>(d, qa[0], qb[0], qa[1], qb[1], xf[2 * b], xf[2 * b + 1]);
-            fa += f16bits(ld_u16(ua + 34 * b)) * join_hi_lo(d[0], d[1]);
-            fb += f16bits(ld_u16(ub + 34 * b)) * join_hi_lo(d[2], d[3]);
-        }
-        acc[0] += xs * fa;
-        acc[1] += xs * fb;
-    } else if constexpr (TY == T_Q2_0) {
-        const int4 x03 = *reinterpret_cast<const int4 *>(xw + 4), x47 = *reinterpret_cast<const int4 *>(xw + 8);
-        const int xsum[2] = {x03.x + x03.y + x03.z + x03.w, x47.x + x47.y + x47.z + x47.w};
-        float fa = 0.f, fb = 0.f;
-#pragma unroll
-        for (int blk = 0; blk < 2; blk++) {  // block of 128 codes: {f16 d; u8 qs[32]}
-            const uint8_t *pa = ua + 34 * blk, *pb = ub + 34 * blk;
-            int t[4] = {0, 0, 0, 0};
-#pragma unroll
-            for (int sb = 0; sb < 4; sb++) {  // 8 bytes = 32 codes; this thread takes code c of every byte
-                uint32_t wa[2], wb[2];
-                lds_a2<2>(pa + 2 + 8 * sb, wa);
-                lds_a2<2>(pb + 2 + 8 * sb, wb);
-                const uint32_t m = 0x03030303u, sh = 2 * c;
-                int d[4];
-                imma0<false>(d, (wa[0] >> sh) & m, (wb[0] >> sh) & m, (wa[1] >> sh) & m, (wb[1] >> sh) & m,
-                             xf[8 * blk + 2 * sb], xf[8 * blk + 2 * sb + 1]);
-#pragma unroll
-                for (int e = 0; e < 4; e++) t[e] += d[e];
-            }
-            // (code - 1) * d: the sum of x over the block leaves again
-            fa += f16bits(ld_u16(pa)) * (join_hi_lo(t[0], t[1]) - (float)xsum[blk]);
-            fb += f16bits(ld_u16(pb)) * (join_hi_lo(t[2], t[3]) - (float)xsum[blk]);
-        }
-        acc[0] += xs * fa;
-        acc[1] += xs * fb;
-    } else {
-        // IQ2_XXS: codebook entry c of every sub-block is this thread's eight weights
-        float fa = 0.f, fb = 0.f;
-#pragma unroll
-        for (int b = 0; b < 8; b++) {
-            uint32_t wa[2], wb[2];  // a0: four codebook indices, a1: four 7-bit sign indices + 4-bit scale
-            lds_a2<2>(ua + 2 + 8 * b, wa);
-            lds_a2<2>(ub + 2 + 8 * b, wb);
-            const uint2 ea = tab[((wa[0] >> (8 * c)) & 0xFF) * tab_copies], eb = tab[((wb[0] >> (8 * c)) & 0xFF) * tab_copies];
-            const uint2 ma = iq2_sign_masks((wa[1] >> (7 * c)) & 127u), mb = iq2_sign_masks((wb[1] >> (7 * c)) & 127u);
-            int pos[4], neg[4];
-            imma0<false>(pos, ea.x, eb.x, ea.y, eb.y, xf[2 * b], xf[2 * b + 1]);
-            imma0<false>(neg, ea.x & ma.x, eb.x & mb.x, ea.y & ma.y, eb.y & mb.y, xf[2 * b], xf[2 * b + 1]);
-            fa += (0.5f + (float)(wa[1] >> 28)) * join_hi_lo(pos[0] - 2 * neg[0], pos[1] - 2 * neg[1]);
-            fb += (0.5f + (float)(wb[1] >> 28)) * join_hi_lo(pos[2] - 2 * neg[2], pos[3] - 2 * neg[3]);
-        }
-        acc[0] += xs * 0.25f * f16bits(ld_u16(ua)) * fa;
-        acc[1] += xs * 0.25f * f16bits(ld_u16(ub)) * fb;
-    }
-}
-
 // ---- staging x ------------------------------------------------------------------
-// One item is 16 consecutive k of one column; the 16 neighbouring items (lanes) of
-// a 256-wide unit agree on its scale, two neighbours make one 32-wide block.
-template <int XDT> struct XRaw { uint4 v[XDT == DT_F32 ? 4 : 2]; };
-
-template <int XDT>
-__device__ __forceinline__ XRaw<XDT> load16(const void *x, size_t src, bool live) {
-    XRaw<XDT> r;
-    constexpr int NV = XDT == DT_F32 ? 4 : 2;
-    const uint4 *p = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(x) + src * (XDT == DT_F32 ? 4 : 2));
-#pragma unroll
-    for (int j = 0; j < NV; j++) r.v[j] = live ? __ldg(p + j) : make_uint4(0u, 0u, 0u, 0u);
-    return r;
-}
-
-// The 16 integers, the unit's scale (NaN if the unit holds a NaN, so that it
-// spreads to the results as it would in a plain dot product) and the 32-wide
-// block's integer sum.
-template <int XDT>
-__device__ __forceinline__ void quantize16(const XRaw<XDT> &raw, int (&q)[16], float &xs, int &qsum) {
-    float v[16];
-    if constexpr (XDT == DT_F32) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            v[4 * j] = __uint_as_float(raw.v[j].x); v[4 * j + 1] = __uint_as_float(raw.v[j].y);
-            v[4 * j + 2] = __uint_as_float(raw.v[j].z); v[4 * j + 3] = __uint_as_float(raw.v[j].w);
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            const uint32_t w[4] = {raw.v[j].x, raw.v[j].y, raw.v[j].z, raw.v[j].w};
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                if constexpr (XDT == DT_F16) {
-                    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[e]));
-                    v[8 * j + 2 * e] = f.x; v[8 * j + 2 * e + 1] = f.y;
-                } else {
-                    v[8 * j + 2 * e] = __uint_as_float(w[e] << 16);
-                    v[8 * j + 2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u);
-                }
-            }
-        }
-    }
-    // largest magnitude of the 256-wide unit (16 neighbouring items); a NaN anywhere
-    // makes the probe below a NaN
-    float m8[8], bad8[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        m8[j] = fmaxf(fabsf(v[j]), fabsf(v[j + 8]));
-        bad8[j] = v[j] + v[j + 8];  // NaN if either is (inf - inf cannot matter: infs give NaN results anyway)
-    }
-#pragma unroll
-    for (int w = 4; w >= 1; w >>= 1)
-#pragma unroll
-        for (int j = 0; j < w; j++) {
-            m8[j] = fmaxf(m8[j], m8[j + w]);
-            bad8[j] = bad8[j] + bad8[j + w];
-        }
-    float amax = m8[0], nanprobe = bad8[0];
-#pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        nanprobe += __shfl_xor_sync(0xffffffffu, nanprobe, o);
-    }
-    const bool bad = nanprobe != nanprobe && !(amax == __int_as_float(0x7F800000));
-    // an infinite amax gives 0 and xs = inf; a unit whose largest magnitude is below 1e-30
-    // counts as zeros (32512 / amax would overflow, and its products vanish in fp32 anyway)
-    const float inv = amax > 1e-30f ? __fdividef(kXqMax, amax) : 0.f;
-    xs = bad ? __int_as_float(0x7FC00000) : amax * (1.f / kXqMax);
-    int s4[4] = {0, 0, 0, 0};
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-        q[j] = __float2int_rn(v[j] * inv);
-        s4[j & 3] += q[j];
-    }
-    qsum = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-    qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
-}
-
 // SEP: one column as a hi and a lo byte column.  An item is 8 consecutive k; the
 // 32 items of a 256-wide unit are the 32 lanes of one warp, so the unit's largest
 // magnitude is one warp reduction.  Magnitudes are compared as integers (the bit
@@ -917,6 +491,27 @@ __device__ __forceinline__ void quantize16(const XRaw<XDT> &raw, int (&q)[16], f
 // {scale, scale * sum of x over its first 32-wide block, over its second} follows its 64
 // bytes in the first byte column.
 template <int XDT> struct XRaw8 { uint4 v[XDT == DT_F32 ? 2 : 1]; };
+template <int XDT>
+__device__ __forceinline__ void x_floats(const XRaw8<XDT> &raw, float (&v)[8]) {
+    if constexpr (XDT == DT_F32) {
+        v[0] = __uint_as_float(raw.v[0].x); v[1] = __uint_as_float(raw.v[0].y);
+        v[2] = __uint_as_float(raw.v[0].z); v[3] = __uint_as_float(raw.v[0].w);
+        v[4] = __uint_as_float(raw.v[1].x); v[5] = __uint_as_float(raw.v[1].y);
+        v[6] = __uint_as_float(raw.v[1].z); v[7] = __uint_as_float(raw.v[1].w);
+    } else {
+        const uint32_t w[4] = {raw.v[0].x, raw.v[0].y, raw.v[0].z, raw.v[0].w};
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            if constexpr (XDT == DT_F16) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[e]));
+                v[2 * e] = f.x; v[2 * e + 1] = f.y;
+            } else {
+                v[2 * e] = __uint_as_float(w[e] << 16);
+                v[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u);
+            }
+        }
+    }
+}
 
 template <int TY, int XDT>
 __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const void *x, uint32_t u_first, uint32_t nu,
@@ -943,24 +538,7 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
             const uint32_t i = base + r * kConsumers;
             if (i >= items) break;  // the same for the whole warp: a warp holds one unit
             float v[8];
-            if constexpr (XDT == DT_F32) {
-                v[0] = __uint_as_float(raw[r].v[0].x); v[1] = __uint_as_float(raw[r].v[0].y);
-                v[2] = __uint_as_float(raw[r].v[0].z); v[3] = __uint_as_float(raw[r].v[0].w);
-                v[4] = __uint_as_float(raw[r].v[1].x); v[5] = __uint_as_float(raw[r].v[1].y);
-                v[6] = __uint_as_float(raw[r].v[1].z); v[7] = __uint_as_float(raw[r].v[1].w);
-            } else {
-                const uint32_t w[4] = {raw[r].v[0].x, raw[r].v[0].y, raw[r].v[0].z, raw[r].v[0].w};
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    if constexpr (XDT == DT_F16) {
-                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[e]));
-                        v[2 * e] = f.x; v[2 * e + 1] = f.y;
-                    } else {
-                        v[2 * e] = __uint_as_float(w[e] << 16);
-                        v[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u);
-                    }
-                }
-            }
+            x_floats<XDT>(raw[r], v);
             uint32_t mb = 0;
 #pragma unroll
             for (int j = 0; j < 8; j++) mb = max(mb, __float_as_uint(v[j]) & 0x7FFFFFFFu);
@@ -1005,160 +583,137 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
     }
 }
 
-// WIDE: up to four columns, each as a hi and a lo byte column (panel columns 2j and
-// 2j + 1).  Inside a unit of a byte column, thread c's 64 bytes start at 64c: eight
-// bytes per 32-wide block, block after block, the 16-byte pieces of threads 2 and 3
-// swapped in pairs as in the one-column panel.  The eight bytes of a block are its
-// k [8c, 8c + 8) in order (Q2_0: k = 16w + 4b + c for word w, byte b).
-// xw[(unit * 4 + column) * 12]: {xs, -, -, -, X0 .. X7}.
-template <int TY, int XDT>
-__device__ __forceinline__ void stage_x_wide(uint8_t *xs, float *xw, const GemvLayout &L, const void *x, uint32_t kdim,
+// WIDE: every column as two or three byte columns of the panel, `es` bytes from one to the next.  An item is 8 consecutive k; the 32 items of a (column, unit)
+// pair are the lanes of one warp.  Two bytes: the integers of the one-column panel.  Three: q of 24
+// bits, |q| <= 127 * 2^16.  Inside a unit of a byte column thread c's 64 bytes start at 64c: eight bytes per
+// 32-wide block in the type's WideOrder, block after block, the 16-byte pieces of threads 2 and 3
+// swapped in pairs (see kXqUnit).
+template <int TY, int MODE, int XDT>
+__device__ __forceinline__ void stage_x_wide(uint32_t xs32, uint32_t es, uint32_t info32, const void *x, uint32_t kdim, uint32_t ncols,
                                              uint32_t u_first, uint32_t nu, uint32_t tid) {
-    if constexpr (TY != T_Q2_0) {
-        // An item is 8 consecutive k = the eight bytes thread c = item % 4 of a quad feeds into block
-        // item / 4; the 32 items of a (column, unit) pair are the lanes of one warp, so the unit's
-        // largest magnitude is one warp reduction and a block's sum two shuffles, as in the
-        // one-column panel.  The loads of four pairs go out before the first is worked on.
-        const uint32_t warp = tid >> 5, e8 = tid & 31, blk = e8 >> 2, c = e8 & 3;
-        const uint32_t pairs = L.nc * nu;
-        constexpr uint32_t kFlight = 4;
-        constexpr uint32_t kMagicBits = 0x4B400080u;  // 1.5 * 2^23 + 128 as a float
-        const uint32_t piece = xq_piece_offset(c, blk >> 1) + (blk & 1) * 8;
-        for (uint32_t base = warp; base < pairs; base += kFlight * kGemvWarps) {
-            XRaw8<XDT> raw[kFlight];
-            uint32_t col_of[kFlight], u_of[kFlight];
-#pragma unroll
-            for (uint32_t r = 0; r < kFlight; r++) {
-                const uint32_t pr = base + r * kGemvWarps;
-                const bool live = pr < pairs;
-                col_of[r] = live ? pr / nu : 0;
-                u_of[r] = live ? pr - col_of[r] * nu : 0;
-                const uint4 *src = reinterpret_cast<const uint4 *>(
-                    reinterpret_cast<const uint8_t *>(x) +
-                    ((size_t)col_of[r] * kdim + (size_t)(u_first + u_of[r]) * 256 + e8 * 8) * (XDT == DT_F32 ? 4 : 2));
-#pragma unroll
-                for (int j = 0; j < (XDT == DT_F32 ? 2 : 1); j++)
-                    raw[r].v[j] = live ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (uint32_t r = 0; r < kFlight; r++) {
-                if (base + r * kGemvWarps >= pairs) break;  // the same for the whole warp
-                float v[8];
-                if constexpr (XDT == DT_F32) {
-                    v[0] = __uint_as_float(raw[r].v[0].x); v[1] = __uint_as_float(raw[r].v[0].y);
-                    v[2] = __uint_as_float(raw[r].v[0].z); v[3] = __uint_as_float(raw[r].v[0].w);
-                    v[4] = __uint_as_float(raw[r].v[1].x); v[5] = __uint_as_float(raw[r].v[1].y);
-                    v[6] = __uint_as_float(raw[r].v[1].z); v[7] = __uint_as_float(raw[r].v[1].w);
-                } else {
-                    const uint32_t w[4] = {raw[r].v[0].x, raw[r].v[0].y, raw[r].v[0].z, raw[r].v[0].w};
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        if constexpr (XDT == DT_F16) {
-                            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[e]));
-                            v[2 * e] = f.x; v[2 * e + 1] = f.y;
-                        } else {
-                            v[2 * e] = __uint_as_float(w[e] << 16);
-                            v[2 * e + 1] = __uint_as_float(w[e] & 0xFFFF0000u);
-                        }
-                    }
-                }
-                uint32_t mb = 0;
-#pragma unroll
-                for (int j = 0; j < 8; j++) mb = max(mb, __float_as_uint(v[j]) & 0x7FFFFFFFu);
-                mb = __reduce_max_sync(0xffffffffu, mb);
-                const float amax = __uint_as_float(mb);
-                // as in the one-column panel: below 1e-30 the unit counts as zeros, an infinite
-                // amax gives inv = 0 and an infinite scale, a NaN gives inv = 0 and a NaN scale
-                const float inv = amax > 1e-30f ? __fdividef(kXqMax, amax) : 0.f;
-                const float scale = amax * (1.f / kXqMax);
-                uint32_t t[8], tsum = 0;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    t[j] = __float_as_uint(fmaf(v[j], inv, __uint_as_float(kMagicBits)));
-                    tsum += t[j];
-                }
-                int qsum = (int)(tsum - 8u * kMagicBits);
-                qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
-                qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
-                uint8_t *dst = xs + (2 * col_of[r]) * L.es + u_of[r] * kXqUnit + piece;
-                *reinterpret_cast<uint2 *>(dst) =
-                    make_uint2(prmt(prmt(t[0], t[1], 0x0051u), prmt(t[2], t[3], 0x0051u), 0x5410u),
-                               prmt(prmt(t[4], t[5], 0x0051u), prmt(t[6], t[7], 0x0051u), 0x5410u));
-                *reinterpret_cast<uint2 *>(dst + L.es) =
-                    make_uint2(prmt(prmt(t[0], t[1], 0x0040u), prmt(t[2], t[3], 0x0040u), 0x5410u) ^ 0x80808080u,
-                               prmt(prmt(t[4], t[5], 0x0040u), prmt(t[6], t[7], 0x0040u), 0x5410u) ^ 0x80808080u);
-                float *w12 = xw + ((size_t)u_of[r] * 4 + col_of[r]) * 12;
-                if (c == 0) reinterpret_cast<int *>(w12)[4 + blk] = qsum;
-                if (e8 == 0) w12[0] = scale;
-            }
-        }
-        return;
-    }
-    const uint32_t items_per_col = nu * 16;
-    const uint32_t total = (L.nc * items_per_col + 31) & ~31u;
-    constexpr uint32_t kFlight = 3;  // items a thread has in flight: the loads go out first
-    auto where = [&](uint32_t i, bool &live, uint32_t &col, uint32_t &it) {
-        live = i < L.nc * items_per_col;
-        col = live ? i / items_per_col : 0;
-        it = live ? i % items_per_col : 0;
+    using W = WideMode<MODE>;
+    constexpr int NB = W::nb;
+    constexpr uint32_t IW = wide_info_words(TY, NB);
+    const uint32_t warp = tid >> 5, e8 = tid & 31, blk = e8 >> 2, e4 = e8 & 3;
+    const uint32_t pairs = ncols * nu;
+    constexpr uint32_t kFlight = 4;
+    constexpr uint32_t kMagicBits = 0x4B400080u;  // 1.5 * 2^23 + 128 as a float
+    // (column, unit) pairs are walked unit first, kGemvWarps at a time
+    auto step = [&](uint32_t &col, uint32_t &u) {
+        u += kGemvWarps;
+        while (u >= nu) { u -= nu; col++; }
     };
-    for (uint32_t base_i = tid; base_i < total; base_i += kFlight * kConsumers) {
-      XRaw<XDT> raw[kFlight];
+    uint32_t col = 0, u = warp;
+    while (u >= nu) { u -= nu; col++; }
+    for (uint32_t base = warp; base < pairs; base += kFlight * kGemvWarps) {
+        XRaw8<XDT> raw[kFlight];
+        uint32_t lcol = col, lu = u;
 #pragma unroll
-      for (uint32_t r = 0; r < kFlight; r++) {
-          bool live; uint32_t col, it;
-          where(base_i + r * kConsumers, live, col, it);
-          raw[r] = load16<XDT>(x, (size_t)col * kdim + (size_t)(u_first + (it >> 4)) * 256 + (it & 15) * 16, live);
-      }
+        for (uint32_t r = 0; r < kFlight; r++) {
+            const uint32_t k0 = (u_first + lu) * 256 + e8 * 8;
+            const bool live = lcol < ncols && (!W::rag || k0 < kdim);
+            const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(x) +
+                                                              ((size_t)lcol * kdim + k0) * (XDT == DT_F32 ? 4 : 2));
 #pragma unroll
-      for (uint32_t r = 0; r < kFlight; r++) {
-        const uint32_t i = base_i + r * kConsumers;
-        if (i >= total) break;  // the same for the whole warp
-        bool live; uint32_t col, it;
-        where(i, live, col, it);
-        const uint32_t u = it >> 4, blk = (it >> 1) & 7, half = it & 1;  // unit, 32-wide block, 16-k half of it
-        int q[16], qsum;
-        float scale;
-        quantize16<XDT>(raw[r], q, scale, qsum);
-        if (!live) continue;
-        uint8_t *base = xs + (2 * col) * L.es + u * kXqUnit;
-        if constexpr (TY == T_Q2_0) {
-            // k = 16 * half + 4 * b + c: thread c gets four bytes (b = 0..3) from this item
+            for (int j = 0; j < (XDT == DT_F32 ? 2 : 1); j++) raw[r].v[j] = live ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
+            step(lcol, lu);
+        }
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                uint32_t t[4];
+        for (uint32_t r = 0; r < kFlight; r++, step(col, u)) {
+            if (col >= ncols) break;  // the same for the whole warp
+            float v[8];
+            x_floats<XDT>(raw[r], v);
+            uint32_t mb = 0;
 #pragma unroll
-                for (int b = 0; b < 4; b++) t[b] = (uint32_t)(q[4 * b + c] + 128);
-                const uint32_t h = __byte_perm(__byte_perm(t[0], t[1], 0x0051), __byte_perm(t[2], t[3], 0x0051), 0x5410);
-                const uint32_t l = __byte_perm(__byte_perm(t[0], t[1], 0x0040), __byte_perm(t[2], t[3], 0x0040), 0x5410) ^ 0x80808080u;
-                uint8_t *dst = base + xq_piece_offset(c, blk >> 1) + (blk & 1) * 8 + half * 4;
-                *reinterpret_cast<uint32_t *>(dst) = h;
-                *reinterpret_cast<uint32_t *>(dst + L.es) = l;
-            }
-        } else {
-            // k = 16 * half + 0..15: threads 2 * half and 2 * half + 1 get eight bytes each
+            for (int j = 0; j < 8; j++) mb = max(mb, __float_as_uint(v[j]) & 0x7FFFFFFFu);
+            mb = __reduce_max_sync(0xffffffffu, mb);
+            const float amax = __uint_as_float(mb);
+            // as in the one-column panel: below 1e-30 the unit counts as zeros, an infinite
+            // amax gives inv = 0 and an infinite scale, a NaN gives inv = 0 and a NaN scale
+            float scale;
+            uint32_t w[NB][2];  // [byte][first, second four k]
+            if constexpr (NB == 2) {
+                const float inv = amax > 1e-30f ? __fdividef(kXqMax, amax) : 0.f;
+                scale = amax * (1.f / kXqMax);
+                uint32_t t[8];
 #pragma unroll
-            for (int cc = 0; cc < 2; cc++) {
-                uint32_t h[2], l[2];
+                for (int j = 0; j < 8; j++) t[j] = __float_as_uint(fmaf(v[j], inv, __uint_as_float(kMagicBits)));
 #pragma unroll
-                for (int w = 0; w < 2; w++) {
-                    uint32_t t[4];
-#pragma unroll
-                    for (int b = 0; b < 4; b++) t[b] = (uint32_t)(q[8 * cc + 4 * w + b] + 128);
-                    h[w] = __byte_perm(__byte_perm(t[0], t[1], 0x0051), __byte_perm(t[2], t[3], 0x0051), 0x5410);
-                    l[w] = __byte_perm(__byte_perm(t[0], t[1], 0x0040), __byte_perm(t[2], t[3], 0x0040), 0x5410) ^ 0x80808080u;
+                for (int i = 0; i < 2; i++) {
+                    w[0][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0051u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0051u), 0x5410u);
+                    w[1][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0040u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0040u), 0x5410u) ^ 0x80808080u;
                 }
-                uint8_t *dst = base + xq_piece_offset(2 * half + cc, blk >> 1) + (blk & 1) * 8;
-                *reinterpret_cast<uint2 *>(dst) = make_uint2(h[0], h[1]);
-                *reinterpret_cast<uint2 *>(dst + L.es) = make_uint2(l[0], l[1]);
+            } else {
+                scale = amax * (1.f / kXq3Max);
+                const float inv = amax > 1e-30f ? __frcp_rn(scale) : 0.f;
+                uint32_t t[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) t[j] = (uint32_t)(__float2int_rn(v[j] * inv) + 0x8080);
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    w[0][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0062u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0062u), 0x5410u);
+                    w[1][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0051u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0051u), 0x5410u) ^ 0x80808080u;
+                    w[NB - 1][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0040u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0040u), 0x5410u) ^ 0x80808080u;
+                }
+            }
+            const uint32_t info = info32 + (u * ncols + col) * (IW * 4);
+            if (e8 == 0) sts32(info, __float_as_uint(scale));
+            int sums[NB];
+#pragma unroll
+            for (int b = 0; b < NB; b++) {
+                const uint32_t dst = xs32 + (col * NB + b) * es + u * kXqUnit, at = blk & 1 ? 8 : 0;
+                if constexpr (kWideOrder<TY> == O_SEQ) {
+                    sts64(dst + xq_piece_offset(e4, blk >> 1) + at, w[b][0], w[b][1]);
+                } else if constexpr (kWideOrder<TY> == O_SPLIT) {
+#pragma unroll
+                    for (int i = 0; i < 2; i++)
+                        sts32(dst + xq_piece_offset(2 * (e4 & 1) + i, blk >> 1) + at + (e4 & 2) * 2, w[b][i]);
+                } else if constexpr (kWideOrder<TY> == O_PAIRS) {
+                    // the item 16 k further on, or back, is two lanes away
+                    const uint32_t give = e4 & 2 ? w[b][0] : w[b][1], own = e4 & 2 ? w[b][1] : w[b][0];
+                    const uint32_t got = __shfl_xor_sync(0xffffffffu, give, 2);
+                    const uint32_t lo = e4 & 2 ? got : own, hi = e4 & 2 ? own : got;
+                    sts64(dst + xq_piece_offset(2 * (e4 & 1) + (e4 >> 1), blk >> 1) + at, prmt(lo, hi, 0x5140u), prmt(lo, hi, 0x7362u));
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        sts16(dst + xq_piece_offset(c, blk >> 1) + at + (e4 >> 1) * 4 + (e4 & 1) * 2, prmt(w[b][0], w[b][1], (uint32_t)(c | (4 + c) << 4)) & 0xFFFFu);
+                }
+                sums[b] = __dp4a((int)w[b][0], 0x01010101, __dp4a((int)w[b][1], 0x01010101, 0));
+            }
+            if constexpr (TY == T_Q2_0) {
+#pragma unroll
+                for (int b = 0; b < NB; b++) {
+#pragma unroll
+                    for (int o = 1; o < 16; o <<= 1) sums[b] += __shfl_xor_sync(0xffffffffu, sums[b], o);
+                    if ((e8 & 15) == 0) sts32(info + 4 + ((e8 >> 4) * NB + b) * 4, (uint32_t)-sums[b]);
+                }
+            } else if constexpr (IW > 1) {
+                constexpr uint32_t groups = TY == T_Q6_K ? 16 : 8;
+                int sum = sums[0] * 256 + sums[1];
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                if constexpr (TY != T_Q6_K) sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                if ((e8 & (32 / groups - 1)) == 0) {
+                    const uint32_t t = (uint32_t)(sum + 0x8080), g = e8 / (32 / groups);
+                    sts8(info + 4 + g, t >> 16);
+                    sts8(info + 4 + groups + g, (t >> 8 & 255u) ^ 0x80u);
+                    sts8(info + 4 + 2 * groups + g, (t & 255u) ^ 0x80u);
+                }
             }
         }
-        float *w12 = xw + ((size_t)u * 4 + col) * 12;
-        if (half == 0) {
-            reinterpret_cast<int *>(w12)[4 + blk] = qsum;
-            if (blk == 0) w12[0] = scale;
-        }
-      }
+    }
+}
+template <int TY, int MODE>
+__device__ __forceinline__ void stage_x(int xdt, uint32_t xs32, uint32_t es, uint32_t info32, const void *x, uint32_t kdim, uint32_t ncols,
+                                        uint32_t u_first, uint32_t nu, uint32_t tid) {
+    if constexpr (MODE == M_SEP) {
+        if (xdt == DT_F32) stage_x_bytes<TY, DT_F32>(xs32, es, x, u_first, nu, tid);
+        else if (xdt == DT_F16) stage_x_bytes<TY, DT_F16>(xs32, es, x, u_first, nu, tid);
+        else stage_x_bytes<TY, DT_BF16>(xs32, es, x, u_first, nu, tid);
+    } else {
+        if (xdt == DT_F32) stage_x_wide<TY, MODE, DT_F32>(xs32, es, info32, x, kdim, ncols, u_first, nu, tid);
+        else if (xdt == DT_F16) stage_x_wide<TY, MODE, DT_F16>(xs32, es, info32, x, kdim, ncols, u_first, nu, tid);
+        else stage_x_wide<TY, MODE, DT_BF16>(xs32, es, info32, x, kdim, ncols, u_first, nu, tid);
     }
 }
 
@@ -1175,23 +730,27 @@ struct RingPos {
 #ifndef OKF_GEMV_MINB
 #define OKF_GEMV_MINB 2
 #endif
-template <int TY, int XDT, bool SEP>
+template <int TY, int MODE>
 __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(GemvArgs p, GemvLayout L, GemvGather G) {
     constexpr uint32_t UB = UnitGeom<TY>::bytes;
+    constexpr bool SEP = MODE == M_SEP;
+    using W = WideMode<MODE>;
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
     uint64_t *empty = full + kMaxStages;
     volatile int *abort_flag = reinterpret_cast<volatile int *>(empty + kMaxStages);
     uint8_t *stages = smem + kBarBytes;
-    uint8_t *xs = smem + L.xs_off;
-    float4 *info = reinterpret_cast<float4 *>(smem + L.info_off);  // SEP: [unit][quarter]; WIDE: [unit][column] x 3
-    float *red = reinterpret_cast<float *>(smem + L.red_off);      // [tile in group][warp][16][nc]
+    float *part = reinterpret_cast<float *>(smem + L.part_off);  // clusters: [tile][column][16], this CTA's share of K
+    float *red = reinterpret_cast<float *>(smem + L.red_off);  // [tile in group][warp][16][nc]
     const uint32_t smem32 = smem_u32(smem);
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
-    const uint32_t t0 = (uint32_t)((uint64_t)p.tiles * blockIdx.x / gridDim.x);
-    const uint32_t t1 = (uint32_t)((uint64_t)p.tiles * (blockIdx.x + 1) / gridDim.x);
+    // the cluster's tiles and this CTA's units of them
+    const uint32_t rank = blockIdx.x & ((1u << L.clog) - 1), cid = blockIdx.x >> L.clog, ncl = gridDim.x >> L.clog;
+    const uint32_t t0 = (uint32_t)((uint64_t)p.tiles * cid / ncl);
+    const uint32_t t1 = (uint32_t)((uint64_t)p.tiles * (cid + 1) / ncl);
     const uint32_t ntl = t1 - t0;
+    const uint32_t ubeg = p.nunit * rank >> L.clog, nun = (p.nunit * (rank + 1) >> L.clog) - ubeg;
     const uint32_t spt = L.mode == 1 ? 2 : 1;  // stages per step (two half-tiles in mode 1)
 
     pdl_launch_dependents();
@@ -1205,12 +764,13 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
     }
     if (threadIdx.x < 64) reinterpret_cast<uint32_t *>(smem + kZeroOff)[threadIdx.x] = 0u;
     if constexpr (TY == T_IQ2_XXS) {
-        // The codebook, 256 entries of eight magnitude bytes, every entry `tab_copies`
-        // times side by side: a lane reads copy (lane mod copies), so with 16 copies the
-        // 16 lanes of a 64-bit access hit 16 different bank pairs whatever they look up.
-        uint64_t *tw = reinterpret_cast<uint64_t *>(smem + L.tab_off);
+        // the look-up tables, every entry `tab_copies` times side by side (see Iq2Tab)
+        uint32_t *tw = reinterpret_cast<uint32_t *>(smem + L.tab_off);
         const uint32_t sh = 31 - __clz(L.tab_copies);
-        for (uint32_t i = threadIdx.x; i < 256 * L.tab_copies; i += blockDim.x) tw[i] = g_iq2xxs_grid[i >> sh];
+        for (uint32_t i = threadIdx.x; i < 384u; i += blockDim.x) {
+            const uint32_t v = i < 256 ? iq2_code_selectors(g_iq2xxs_grid[i]) : iq2_sign_selectors(i - 256);
+            for (uint32_t k = 0; k < L.tab_copies; k++) tw[(i << sh) + ((k + threadIdx.x) & (L.tab_copies - 1))] = v;
+        }
     }
     __syncthreads();
 
@@ -1225,21 +785,24 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
         return;
     }
     if (warp == kGemvWarps) {
-        // ---- producer (one thread): weights do not depend on the previous kernel,
-        // so it does not wait for it
-        if (lane != 0) return;
+        // ---- producer: weights do not depend on the previous kernel, so it does not wait for it.
+        // One thread waits and counts; copies of whole rows are its own, those of row segments are
+        // issued by sixteen lanes, one row each (a bulk copy takes its thread some 50 ns).
         RingPos rp;
         uint32_t issued = 0;
         for (uint32_t gb = 0; gb < ntl; gb += L.group) {
             const uint32_t gn = min(L.group, ntl - gb);
             for (uint32_t j = 0; j < p.nchunk; j++) {
-                const uint32_t u0 = j * p.cb, nu = min(p.cb, p.nunit - u0);
+                const uint32_t u0 = j * p.cb, nu = nun > u0 ? min(p.cb, nun - u0) : 0u;
                 for (uint32_t tl = gb, tn; tl < gb + gn; tl += tn) {
                     const GemvSeg sg = gemv_segment(p, t0 + tl);
                     tn = min(min(L.tps, gb + gn - tl), sg.tile1 - (t0 + tl));  // a step stays inside one matrix
                     for (uint32_t half = 0; half < spt; half++, issued++) {
-                        if (rp.use > 0 &&
-                            !mbar_wait_relaxed(&empty[rp.s], (rp.use - 1) & 1, abort_flag, p.status, kStatusEmptyTimeout)) {
+                        bool ok = true;
+                        if (rp.use > 0 && lane == 0)
+                            ok = mbar_wait_relaxed(&empty[rp.s], (rp.use - 1) & 1, abort_flag, p.status, kStatusEmptyTimeout);
+                        if (!__shfl_sync(0xffffffffu, ok, 0)) {
+                            if (lane != 0) return;
                             // giving up: let the copies already issued land before the CTA goes away
                             const uint32_t first = issued > L.nstage ? issued - L.nstage : 0;
                             for (uint32_t d = first; d < issued; d++) {
@@ -1257,24 +820,21 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                             const uint32_t want = L.mode == 1 ? 8u : 16u * tn;
                             const uint32_t nrows = row0 < sg.m ? min(want, sg.m - row0) : 0u;
                             const uint32_t bytes = (nrows * p.row_bytes + 15u) & ~15u;
-                            mbar_expect_tx(&full[rp.s], bytes);
-                            if (bytes) bulk_g2s(dst, sg.w + (size_t)row0 * p.row_bytes, bytes, &full[rp.s]);
+                            if (lane == 0) {
+                                mbar_expect_tx(&full[rp.s], bytes);
+                                if (bytes) bulk_g2s(dst, sg.w + (size_t)row0 * p.row_bytes, bytes, &full[rp.s]);
+                            }
                         } else {
                             // one copy per row segment.  A segment may start anywhere (2-byte
                             // aligned layouts): the copy starts at the 16-byte boundary below it
                             // and the consumers skip the same few bytes.
                             const uint32_t seg = nu * UB;
-                            uint32_t total = 0;
-                            for (uint32_t r = 0; r < 16; r++) {
-                                const size_t src = (size_t)min(row0 + r, sg.m - 1) * p.row_bytes + (size_t)u0 * UB;
-                                total += ((uint32_t)(src & 15) + seg + 15u) & ~15u;
-                            }
-                            mbar_expect_tx(&full[rp.s], total);
-                            for (uint32_t r = 0; r < 16; r++) {
-                                const size_t src = (size_t)min(row0 + r, sg.m - 1) * p.row_bytes + (size_t)u0 * UB;
-                                const uint32_t skew = (uint32_t)(src & 15);
-                                bulk_g2s(dst + (size_t)r * L.rs, sg.w + (src - skew), (skew + seg + 15u) & ~15u, &full[rp.s]);
-                            }
+                            const size_t src = (size_t)min(row0 + (lane & 15), sg.m - 1) * p.row_bytes + (size_t)(ubeg + u0) * UB;
+                            const uint32_t skew = (uint32_t)(src & 15), bytes = seg ? (skew + seg + 15u) & ~15u : 0u;
+                            const uint32_t total = __reduce_add_sync(0xffffffffu, lane < 16 ? bytes : 0u);
+                            if (lane == 0) mbar_expect_tx(&full[rp.s], total);
+                            __syncwarp();
+                            if (lane < 16 && bytes) bulk_g2s(dst + (size_t)lane * L.rs, sg.w + (src - skew), bytes, &full[rp.s]);
                         }
                         rp.next(L.nstage);
                     }
@@ -1300,26 +860,45 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
     auto peek_full = [&](const RingPos &q) { return lane == 0 && mbar_test_wait(&full[q.s], q.use & 1); };
     auto consumer_sync = [&]() { named_bar_sync(1, kConsumers); };
 
-    // What this thread feeds into column g of the MMA's B operand.
-    //   SEP:  byte column g % 2 of x, and only in the lanes of quarter g / 2.
-    //   WIDE: byte column g of the panel (hi, lo of activation column g / 2), every lane
-    //         its own 64 bytes; lanes of columns past the last one feed zeros.
-    const bool x_active = SEP ? (g >> 1) == c : g < 2 * p.n;
-    const uint8_t *xs_mine = xs + (SEP ? (g & 1) : g) * L.es + c * 64;
-    const uint32_t xs_ustride = kXqUnit;
-    const uint32_t xq_swap = (c >> 1) * 16;
-    // The same in shared-window addresses for the one-column path.  Lanes that feed nothing
-    // read zeros (stride 0) instead of predicating every load; their zeros sit on a bank
-    // group that the two lanes carrying data in the same 8-lane phase do not touch.
-    const SepConst KC = sep_const<TY>(c, lane, smem32 + L.tab_off, L.tab_copies);
     const uint32_t stages32 = smem32 + kBarBytes;
-    const uint32_t xbase32 = SEP && x_active ? smem32 + L.xs_off + (g & 1) * L.es + c * kSepQuarter
-                                             : smem32 + kZeroOff + ((5 * (g >> 1) + 1) & 7) * 16;
-    const uint32_t xstride32 = SEP && x_active ? kSepUnit : 0u;
+    Iq2Tab tab = {0, 0, 0};
+    if constexpr (TY == T_IQ2_XXS) {
+        tab.stride = L.tab_copies * 4;
+        tab.code = smem32 + L.tab_off + (lane & (L.tab_copies - 1)) * 4;
+        tab.sign = tab.code + 256 * tab.stride;
+    }
+    // One column: what this thread feeds into column g of the MMA's B operand, byte column g % 2 of x,
+    // and only in the lanes of quarter g / 2.  Lanes that feed nothing read zeros (stride 0) instead of
+    // predicating every load; their zeros sit on a bank group that the two lanes carrying data in
+    // the same 8-lane phase do not touch.
+    const SepConst KC = sep_const<TY>(c);
+    const bool sep_active = (g >> 1) == c;
+    const uint32_t xbase32 = sep_active ? smem32 + L.xs_off + (g & 1) * L.es + c * kSepQuarter
+                                        : smem32 + kZeroOff + ((5 * (g >> 1) + 1) & 7) * 16;
+    const uint32_t xstride32 = sep_active ? kSepUnit : 0u;
     const uint32_t rec32 = smem32 + L.xs_off + c * kSepQuarter + 64;  // this quarter's record of unit 0
     const uint32_t red32 = smem32 + L.red_off + (warp * 16 + g + 8 * (c & 1)) * 4;  // this thread's slot of tile 0
-    // WIDE: this lane's copy of the IQ2_XXS codebook
-    const uint2 *tab = reinterpret_cast<const uint2 *>(smem + L.tab_off) + (lane & (L.tab_copies - 1));
+    // Several columns: the byte column of the panel this thread feeds per set (columns that stand for
+    // nothing read column 0; their sums are dropped), the records of this thread's own columns, and
+    // those behind the offsets' byte columns (Q4_K, Q5_K: eight sums, Q6_K: sixteen, per plane).
+    constexpr uint32_t kInfo = wide_info_words(TY, W::nb) * 4, kPlane = TY == T_Q6_K ? 16 : 8;
+    const uint32_t info32 = smem32 + L.info_off;
+    uint32_t wx32[W::sets], wi32[W::vals], ws32[W::vals], ws_lo = 0;
+    if constexpr (!SEP) {
+#pragma unroll
+        for (int i = 0; i < W::sets; i++) {
+            const uint32_t j = (W::rag ? 0 : 4 * i) + (g >> 1), b = W::rag && i ? 2 : g & 1;
+            wx32[i] = smem32 + L.xs_off + (j < p.n ? j * W::nb + b : 0u) * L.es + c * 64;
+        }
+#pragma unroll
+        for (int i = 0; i < W::vals; i++) {
+            const uint32_t own = 4 * i + c, fed = 4 * i + (g >> 1);
+            wi32[i] = info32 + (own < p.n ? own : 0u) * kInfo;
+            const uint32_t word = TY == T_Q6_K ? c : c & 1;
+            ws32[i] = info32 + (fed < p.n ? fed : 0u) * kInfo + 4 + (g & 1) * kPlane + 4 * word;  // s2 or s1
+            ws_lo = (2 - (g & 1)) * kPlane;                                                        // on to s0
+        }
+    }
     RingPos rp;
     uint32_t rot = 0;  // the deal of units to warps rotates from step to step
     bool seen_a = false, seen_b = false;
@@ -1340,16 +919,15 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
             for (uint32_t i = tid; i < gn * kGemvWarps * 16 * L.nc; i += kConsumers) red[i] = 0.f;
         for (uint32_t j0 = 0; j0 < p.nchunk; j0 += L.panel) {
             const uint32_t j1 = min(j0 + L.panel, p.nchunk);
-            const uint32_t pu0 = j0 * p.cb, pnu = min(j1 * p.cb, p.nunit) - pu0;
+            const uint32_t pu0 = j0 * p.cb, pnu = nun > pu0 ? min(j1 * p.cb, nun) - pu0 : 0u;
             if (gb == 0 || L.panel < p.nchunk) {
                 // the previous panel is still being read until every warp gets here
                 if (gb > 0 || j0 > 0) consumer_sync();
-                if constexpr (SEP) stage_x_bytes<TY, XDT>(smem32 + L.xs_off, L.es, p.x, pu0, pnu, tid);
-                else stage_x_wide<TY, XDT>(xs, reinterpret_cast<float *>(info), L, p.x, p.k, pu0, pnu, tid);
+                stage_x<TY, MODE>(p.xdt, smem32 + L.xs_off, L.es, smem32 + L.info_off, p.x, p.k, L.nc, ubeg + pu0, pnu, tid);
             }
             consumer_sync();
             for (uint32_t j = j0; j < j1; j++) {
-                const uint32_t u0 = j * p.cb, nu = min(p.cb, p.nunit - u0);
+                const uint32_t u0 = j * p.cb, nu = nun > u0 ? min(p.cb, nun - u0) : 0u;
                 const uint32_t pu = u0 - pu0;  // first unit of the chunk inside the panel
                 // in whole-row stages a row holds every unit; in segment stages only this chunk's
                 const uint32_t ubase = L.mode == 2 ? 0 : u0;
@@ -1370,15 +948,14 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                         q.next(L.nstage);
                         seen_b = spt == 2 && peek_full(q);
                     }
-                    // rows g and g + 8 of the step's first tile
-                    const uint8_t *ra = stages + (size_t)sA * L.stage_bytes + (size_t)g * L.rs;
-                    const uint8_t *rb = L.mode == 1 ? stages + (size_t)sB * L.stage_bytes + (size_t)g * L.rs
-                                                    : ra + (size_t)8 * L.rs;
-                    if (L.mode == 2 && L.ragged) {  // skip what the copy fetched below each segment's start
-                        const uint32_t row = (t0 + tl - sg.tile0) * 16 + g;
-                        ra += ((size_t)min(row, sg.m - 1) * p.row_bytes + (size_t)u0 * UB) & 15;
-                        rb += ((size_t)min(row + 8, sg.m - 1) * p.row_bytes + (size_t)u0 * UB) & 15;
-                    }
+                    // the step's first tile: rows 0 .. 7 and 8 .. 15; what the copies fetched below the
+                    // start of a row's segment is skipped
+                    const uint32_t top = stages32 + sA * L.stage_bytes;
+                    const uint32_t low = L.mode == 1 ? stages32 + sB * L.stage_bytes : top + 8 * L.rs;
+                    auto skew = [&](uint32_t row) {
+                        if (!(L.mode == 2 && L.ragged)) return 0u;
+                        return (uint32_t)((size_t)min((t0 + tl - sg.tile0) * 16 + row, sg.m - 1) * p.row_bytes + (size_t)(ubeg + u0) * UB) & 15u;
+                    };
                     const uint32_t tile_bytes = 16 * L.rs;
                     // Integer instructions run at half the rate of the others on this part and the
                     // unit bodies are full of them, so a warp takes a run of consecutive units of the
@@ -1394,8 +971,8 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                     uint32_t ti = 0, u = wr * share + min(wr, extra);
                     while (u >= nu && ti + 1 < tn) { u -= nu; ti++; }
                     if constexpr (SEP) {
-                        uint32_t wa = stages32 + (uint32_t)(ra - stages) + ti * tile_bytes + (ubase + u) * UB;  // row g
-                        const uint32_t wdelta = (uint32_t)(rb - ra);                                            // to row g + 8
+                        const uint32_t ra = top + g * L.rs + skew(g), wdelta = low + g * L.rs + skew(g + 8) - ra;  // row g, to row g + 8
+                        uint32_t wa = ra + ti * tile_bytes + (ubase + u) * UB;
                         uint32_t xa = xbase32 + (pu + u) * xstride32;
                         uint32_t ia = rec32 + (pu + u) * kSepUnit;
                         uint32_t da = red32 + (tl - gb + ti) * (kGemvWarps * 16 * 4);
@@ -1409,7 +986,7 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                                 const uint32_t xf[16] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w,
                                                          q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z, q3.w};
                                 const uint4 xi = lds128(ia);
-                                unit_sep<TY>(wa, wa + wdelta, KC, xf, xi, acc);
+                                unit_sep<TY>(wa, wa + wdelta, KC, tab, xf, xi, acc);
                                 wa += UB;
                                 xa += xstride32;
                                 ia += kSepUnit;
@@ -1430,37 +1007,54 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                             da += kGemvWarps * 16 * 4;
                         }
                     } else {
-                        // lanes of columns that do not exist read column 0's record; their sums are dropped
-                        const float *xw0 = reinterpret_cast<const float *>(info) + (c < L.nc ? c : 0) * 12;
+                        constexpr int NV = W::vals;
+                        uint32_t wa = top + ti * tile_bytes + (ubase + u) * UB + g * L.rs + skew(g);               // row g
+                        const uint32_t wdelta = low + g * L.rs + skew(g + 8) - (top + g * L.rs + skew(g));  // to row g + 8
                         while (left) {
                             const uint32_t run = min(left, nu - u);
                             left -= run;
-                            const uint8_t *ta = ra + (size_t)ti * tile_bytes + (size_t)(ubase + u) * UB;
-                            const uint32_t tdelta = (uint32_t)(rb - ra);
-                            const uint8_t *xp = xs_mine + (pu + u) * xs_ustride;
-                            const float *xw = xw0 + (size_t)(pu + u) * 48;
-                            float acc[2] = {0.f, 0.f};
+                            uint32_t xoff = (pu + u) * kXqUnit, ioff = (pu + u) * L.nc * kInfo;
+                            uint32_t blocks = p.k / 32 - (ubeg + u0 + u) * 8;  // left in the row
+                            float acc[NV][2];
+#pragma unroll
+                            for (int i = 0; i < NV; i++) acc[i][0] = acc[i][1] = 0.f;
 #pragma unroll 1
                             for (uint32_t i = run; i; i--) {
-                                uint32_t xf[16];
+                                WideX<TY, MODE> X;
 #pragma unroll
-                                for (int q = 0; q < 4; q++) {
-                                    uint4 w4 = make_uint4(0u, 0u, 0u, 0u);
-                                    if (x_active) w4 = lds128(xp + (q >> 1) * 32 + ((q & 1) ? 16 - xq_swap : xq_swap));
-                                    xf[4 * q] = w4.x; xf[4 * q + 1] = w4.y; xf[4 * q + 2] = w4.z; xf[4 * q + 3] = w4.w;
+                                for (int r = 0; r < W::sets; r++)
+#pragma unroll
+                                    for (int q = 0; q < 4; q++) {
+                                        const uint4 v = lds128(wx32[r] + xoff + ((q * 16) ^ ((c >> 1) * 16)));
+                                        X.f[r][4 * q] = v.x; X.f[r][4 * q + 1] = v.y; X.f[r][4 * q + 2] = v.z; X.f[r][4 * q + 3] = v.w;
+                                    }
+#pragma unroll
+                                for (int r = 0; r < NV; r++) {
+                                    X.scale[r] = __uint_as_float(lds32(wi32[r] + ioff));
+                                    if constexpr (TY == T_Q4_K || TY == T_Q5_K || TY == T_Q6_K) {
+                                        X.sum[r][0] = lds32(ws32[r] + ioff);
+                                        X.sum[r][1] = lds32(ws32[r] + ioff + ws_lo);
+                                    } else if constexpr (TY == T_Q2_0) {
+#pragma unroll
+                                        for (int e = 0; e < 2 * W::nb; e++) X.sum[r][e] = lds32(wi32[r] + ioff + 4 + 4 * e);
+                                    }
                                 }
-                                unit_wide<TY>(ta, ta + tdelta, c, xf, xw, tab, L.tab_copies, acc);
-                                ta += UB;
-                                xp += xs_ustride;
-                                xw += 48;
+                                unit_wide<TY, MODE>(wa, wa + wdelta, c, X, tab, blocks, acc);
+                                wa += UB;
+                                xoff += kXqUnit;
+                                ioff += L.nc * kInfo;
+                                if constexpr (W::rag) blocks -= 8;
                             }
-                            // thread (g, c) holds the sums of rows g, g + 8 for column c: into this
-                            // warp's own slot of the tile's partial sums
-                            if (c < L.nc) {
-                                float *dst = red + ((size_t)(tl - gb + ti) * kGemvWarps + warp) * 16 * L.nc;
-                                dst[g * L.nc + c] += acc[0];
-                                dst[(g + 8) * L.nc + c] += acc[1];
-                            }
+                            // into this warp's own slots of the tile's partial sums
+                            float *dst = red + ((size_t)(tl - gb + ti) * kGemvWarps + warp) * 16 * L.nc;
+#pragma unroll
+                            for (int i = 0; i < NV; i++)
+                                if (4 * i + c < L.nc) {
+                                    dst[g * L.nc + 4 * i + c] += acc[i][0];
+                                    dst[(g + 8) * L.nc + 4 * i + c] += acc[i][1];
+                                }
+                            // on to the first unit of the next tile
+                            wa += tile_bytes - nu * UB;
                             u = 0;
                             ti++;
                         }
@@ -1476,15 +1070,24 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
         // every warp's partials of this group are in: add them in warp order and store
         consumer_sync();
         const uint32_t per_tile = 16 * L.nc;
-        if (G.nranks == 0) {
-            for (uint32_t i = tid; i < gn * per_tile; i += kConsumers) {
-                const uint32_t tl = i / per_tile, r = (i % per_tile) / L.nc, col = i % L.nc;
-                const float *src = red + (size_t)tl * kGemvWarps * per_tile + r * L.nc + col;
-                float sum = 0.f;
+        auto total = [&](uint32_t tl, uint32_t r, uint32_t col) {
+            const float *src = red + (size_t)tl * kGemvWarps * per_tile + r * L.nc + col;
+            float sum = 0.f;
 #pragma unroll
-                for (int w = 0; w < kGemvWarps; w++) sum += src[(size_t)w * per_tile];
+            for (int w = 0; w < kGemvWarps; w++) sum += src[(size_t)w * per_tile];
+            return sum;
+        };
+        if (G.nranks == 0) {
+            // sixteen threads take the rows of one (tile, column)
+            for (uint32_t i = tid >> 4; i < gn * (SEP ? 1u : L.nc); i += kConsumers / 16) {
+                const uint32_t tl = SEP ? i : i * L.nc_inv >> 16, col = SEP ? 0u : i - tl * L.nc;
+                const float sum = total(tl, tid & 15, col);
+                if (L.clog) {
+                    part[((gb + tl) * L.nc + col) * 16 + (tid & 15)] = sum;  // this CTA's share of K
+                    continue;
+                }
                 const GemvSeg sg = gemv_segment(p, t0 + gb + tl);
-                const uint32_t row = (t0 + gb + tl - sg.tile0) * 16 + r;
+                const uint32_t row = (t0 + gb + tl - sg.tile0) * 16 + (tid & 15);
                 if (row < sg.m) sg.out[(size_t)col * sg.m + row] = sum;
             }
         } else {
@@ -1495,12 +1098,9 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
             for (uint32_t i = tid; i < runs * G.nranks; i += kConsumers) {
                 const uint32_t rk = i / runs, j = i % runs;
                 const uint32_t tl = j / (4 * L.nc), r0 = (j / L.nc) % 4 * 4, col = j % L.nc;
-                const float *src = red + (size_t)tl * kGemvWarps * per_tile + r0 * L.nc + col;
-                float sum[4] = {0.f, 0.f, 0.f, 0.f};
+                float sum[4];
 #pragma unroll
-                for (int w = 0; w < kGemvWarps; w++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) sum[e] += src[(size_t)w * per_tile + e * L.nc];
+                for (int e = 0; e < 4; e++) sum[e] = total(tl, r0 + e, col);
                 const GemvSeg sg = gemv_segment(p, t0 + gb + tl);
                 const uint32_t row = (t0 + gb + tl - sg.tile0) * 16 + r0;
                 if (row >= sg.m) continue;
@@ -1513,6 +1113,22 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
             }
         }
         if (gb + L.group < ntl) consumer_sync();  // before the buffer is zeroed again
+    }
+    if (L.clog) {
+        // The cluster's CTAs have the same tiles: each adds up every so many-th (tile, column), in rank
+        // order, reading the others' shares from their shared memory, and stores it.
+        namespace cg = cooperative_groups;
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        for (uint32_t j = ((tid >> 4) << L.clog) + rank; j < ntl * L.nc; j += kConsumers / 16 << L.clog) {
+            float sum = 0.f;
+            for (uint32_t q = 0; q < 1u << L.clog; q++) sum += cl.map_shared_rank(part, q)[j * 16 + (tid & 15)];
+            const uint32_t tl = j / L.nc, col = j - tl * L.nc;
+            const GemvSeg sg = gemv_segment(p, t0 + tl);
+            const uint32_t row = (t0 + tl - sg.tile0) * 16 + (tid & 15);
+            if (row < sg.m) sg.out[(size_t)col * sg.m + row] = sum;
+        }
+        cl.sync();  // nobody leaves while its shares may still be read
     }
     // Row shards: nobody fences or waits here.  The count the local counter has to reach for
     // the exchanges launched so far goes up by one per rank; whoever waits next reads it after
@@ -1535,64 +1151,62 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
 // any CTA of the launch gets.
 constexpr uint32_t kSharedBudget = 112 * 1024;  // two of them leave 2 KB of an SM: enough for the small kernels between matvecs
 
-static bool gemv_layout_with(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t tiles_per_cta, uint32_t tab_copies,
-                             uint32_t budget, GemvArgs &a, GemvLayout &L) {
-    const uint32_t ub = (ty == T_Q4_K || ty == T_Q4_0 || ty == T_IQ4_NL) ? 144 : ty == T_Q8_0 ? 272 : ty == T_Q2_0 ? 68 : ty == T_Q6_K ? 210 : ty == T_Q5_K ? 176 : 66;
-    L.nc = sep ? 1 : n;
-    L.ecols = sep ? 2 : 2 * n;
+static uint32_t unit_bytes(int ty) {
+    return (ty == T_Q4_K || ty == T_Q4_0 || ty == T_IQ4_NL) ? 144 : ty == T_Q8_0 ? 272 : ty == T_Q2_0 ? 68 : ty == T_Q6_K ? 210 : ty == T_Q5_K ? 176 : 66;
+}
+static bool gemv_layout_with(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t csize, uint32_t tiles_per_cta,
+                             uint32_t tab_copies, uint32_t budget, GemvArgs &a, GemvLayout &L) {
+    const uint32_t ub = unit_bytes(ty);
+    const bool sep = mode == M_SEP;
+    L.nc = n;
+    L.nc_inv = 65536 / n + 1;
+    L.clog = csize == 8 ? 3 : csize == 4 ? 2 : csize == 2 ? 1 : 0;
+    const bool rag = mode == M_R;
+    const uint32_t ecols = sep ? 2 : n * (rag ? 3 : 2);  // byte columns of the x panel
+    const uint32_t units = (nunit + csize - 1) / csize;   // the most a CTA of a cluster takes
     const uint32_t per_tile = kGemvWarps * 16 * L.nc * 4;
-    L.group = 8192 / per_tile;
+    L.group = (sep ? 8192 : 16384) / per_tile;
     if (L.group < 1) L.group = 1;
     if (L.group > tiles_per_cta) L.group = tiles_per_cta;
-    const uint32_t red_bytes = L.group * per_tile;
-    const uint32_t tab_bytes = ty == T_IQ2_XXS ? 256 * 8 * tab_copies : 0;
+    const uint32_t red_bytes = L.group * per_tile, part_bytes = csize > 1 ? tiles_per_cta * 16 * L.nc * 4 : 0;
+    const uint32_t tab_bytes = ty == T_IQ2_XXS ? 384 * 4 * tab_copies : 0;
     L.tab_copies = tab_copies;
     const uint32_t stage_cap = 46 * 1024;
-    const uint32_t row_bytes = nunit * ub;
-    // per unit: SEP 320 bytes per byte column, records included; WIDE 256 per byte column + 4 columns x 12 words
-    const uint32_t xunit = sep ? kSepUnit : kXqUnit, info_unit = sep ? 0 : 4 * 48;
-    // Candidate plans, best first: whole tiles, half tiles, then one copy per row of
-    // ever shorter segments (1, 2, ... per row).  Contiguous rows cannot be padded:
-    // when the row size is a multiple of 64 bytes the rows a warp reads together
-    // sit on the same banks, and per-row copies with a padded stride come first.
-    const bool same_banks = row_bytes % 64 == 0;
+    // per unit: SEP 320 bytes per byte column, records included; WIDE 256 per byte column and the columns' records
+    const uint32_t xunit = sep ? kSepUnit : kXqUnit, info_unit = sep ? 0 : n * wide_info_words(ty, rag ? 3 : 2) * 4;
     GemvArgs fb_a = a;
     GemvLayout fb_L = L;
     bool have_fallback = false;
-    for (uint32_t plan = 0; plan < 3 + nunit; plan++) {
-        uint32_t nchunk, cb, rs, stage;
-        L.tps = 1;
+    // One candidate; true when it is taken.
+    auto consider = [&](uint32_t kind, uint32_t tps, uint32_t nchunk) {
+        L.mode = kind;
+        L.tps = tps;
         L.ragged = 0;
-        const uint32_t kind = same_banks ? (plan == 0 ? 2 : plan <= 2 ? plan - 1 : 2) : (plan < 2 ? plan : 2);
+        uint32_t cb = units, rs = row_bytes, stage;
         if (kind == 0) {
-            L.mode = 0; nchunk = 1; cb = nunit; rs = row_bytes;
-            // several tiles per stage while they fit and the CTA still gets two steps
-            while (L.tps < 4 && (L.tps + 1) * 16 * rs <= stage_cap && (L.tps + 1) * 2 <= tiles_per_cta) L.tps++;
-            stage = (L.tps * 16 * rs + 15) & ~15u;
-        } else if (kind == 1) { L.mode = 1; nchunk = 1; cb = nunit; rs = row_bytes; stage = (8 * rs + 15) & ~15u; }
-        else {
-            L.mode = 2;
-            nchunk = same_banks ? (plan == 0 ? 1 : plan - 1) : plan - 1;  // 1, 2, 3, ...
-            if (same_banks && plan > 0 && nchunk == 1) continue;         // already tried
-            cb = (nunit + nchunk - 1) / nchunk;
-            if ((nunit + cb - 1) / cb != nchunk) continue;
+            stage = (tps * 16 * rs + 15) & ~15u;
+        } else if (kind == 1) {
+            stage = (8 * rs + 15) & ~15u;
+        } else {
+            cb = (units + nchunk - 1) / nchunk;
+            if ((units + cb - 1) / cb != nchunk) return false;
             const uint32_t seg = cb * ub;
-            L.ragged = (row_bytes % 16 || seg % 16) ? 1 : 0;
+            L.ragged = (row_bytes % 16 || ub % 16) ? 1 : 0;
             // Q4_K reads its blocks with 16-byte loads, and its rows are always aligned
-            if (L.ragged && ty != T_IQ2_XXS && ty != T_Q2_0 && ty != T_Q6_K) continue;
+            if (L.ragged && !rag && ty != T_IQ2_XXS && ty != T_Q2_0 && ty != T_Q6_K) return false;
             rs = L.ragged ? ((seg + 15 + 15) & ~15u) : seg;  // room for the skipped bytes and the round-up
             if (rs % 32 != 16) rs += 16;                      // rows g and g + 1 on different banks
             stage = 16 * rs;
         }
-        if (stage > stage_cap) continue;
+        if (stage > stage_cap) return false;
         a.nchunk = nchunk;
         a.cb = cb;
         L.rs = rs;
         L.stage_bytes = stage;
-        const uint32_t per_chunk = L.ecols * cb * xunit + cb * info_unit;  // x and what goes with it
-        const uint32_t small = kBarBytes + red_bytes + tab_bytes + 64 + 128 + L.ecols * 128;
-        const uint32_t min_stages = L.mode == 1 ? 4 : 2;
-        if (small + min_stages * stage + per_chunk > budget) continue;
+        const uint32_t per_chunk = ecols * cb * xunit + cb * info_unit;  // x and what goes with it
+        const uint32_t small = kBarBytes + red_bytes + part_bytes + tab_bytes + 64 + 128 + ecols * 128;
+        const uint32_t min_stages = kind == 1 ? 4 : 2;
+        if (small + min_stages * stage + per_chunk > budget) return false;
         uint32_t nstage, panel;
         if (small + min_stages * stage + nchunk * per_chunk <= budget) {
             panel = nchunk;  // all of x resident, the rest goes to the ring
@@ -1602,42 +1216,63 @@ static bool gemv_layout_with(int ty, uint32_t nunit, uint32_t n, bool sep, uint3
             panel = (budget - small - min_stages * stage) / per_chunk;
         }
         // no deeper than the steps a CTA takes
-        const uint32_t steps = ((tiles_per_cta + L.tps - 1) / L.tps) * nchunk * (L.mode == 1 ? 2 : 1);
+        const uint32_t steps = ((tiles_per_cta + tps - 1) / tps) * nchunk * (kind == 1 ? 2 : 1);
         if (nstage > steps) nstage = steps < min_stages ? min_stages : steps;
         if (nstage > kMaxStages) nstage = kMaxStages;
-        if (L.mode == 1) nstage &= ~1u;  // a tile takes two stages
+        if (kind == 1) nstage &= ~1u;  // a tile takes two stages
         L.nstage = nstage;
         L.panel = panel;
         L.es = sep ? sep_col_stride(panel * cb) : xq_col_stride(panel * cb);
         L.xs_off = (kBarBytes + nstage * stage + 127) & ~127u;  // the bank arithmetic of the panel counts from 128
-        L.info_off = (L.xs_off + L.ecols * L.es + 15) & ~15u;
-        L.red_off = L.info_off + panel * cb * info_unit;
+        L.info_off = (L.xs_off + ecols * L.es + 15) & ~15u;
+        L.red_off = (L.info_off + panel * cb * info_unit + 15) & ~15u;
         L.tab_off = (L.red_off + red_bytes + 15) & ~15u;
-        L.smem_bytes = L.tab_off + tab_bytes;
-        if (L.smem_bytes > budget) continue;
+        L.part_off = L.tab_off + tab_bytes;
+        L.smem_bytes = L.part_off + part_bytes;
+        if (L.smem_bytes > budget) return false;
         // A plan that keeps all of x resident stages it once per launch; one that does
-        // not stages a slice per k-chunk, every time with all warps waiting.  Prefer
-        // the first, as long as its row segments stay above 1 KB.
+        // not stages a slice per k-chunk, every time with all warps waiting.
         if (panel == nchunk) return true;
         if (!have_fallback) { fb_a = a; fb_L = L; have_fallback = true; }
-        if ((nunit / (nchunk + 1)) * ub < 1024) break;
+        return false;
+    };
+    // Candidate plans, best first: whole tiles, several per stage while they are small and the CTA
+    // still gets two steps, half tiles, then one copy per row of ever shorter segments.
+    // Contiguous rows cannot be padded: when the row size is a multiple of 64 bytes the rows a
+    // warp reads together sit on the same banks, and per-row copies with a padded stride come
+    // first.  Plans with all of x resident are preferred as long as their row segments stay
+    // above 1 KB.
+    const bool same_banks = row_bytes % 64 == 0;
+    if (csize == 1) {
+        if (same_banks && consider(2, 1, 1)) return true;
+        for (uint32_t tps = 4; tps >= 1; tps--)
+            if (tps == 1 || (tps * 16 * row_bytes <= stage_cap && tps * 2 <= tiles_per_cta))
+                if (consider(0, tps, 1)) return true;
+        if (consider(1, 1, 1)) return true;
+    }
+    for (uint32_t nchunk = 1; nchunk <= units; nchunk++) {
+        if (!(same_banks && csize == 1 && nchunk == 1) && consider(2, 1, nchunk)) return true;
+        if (have_fallback && (units / (nchunk + 1)) * ub < 1024) break;
     }
     if (have_fallback) { a = fb_a; L = fb_L; }
     return have_fallback;
 }
 
-// IQ2_XXS: as many side-by-side copies of the codebook as leave room for a plan that
-// keeps all of x resident (16 copies make every look-up free of bank conflicts).
-static bool gemv_layout_in(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t tiles_per_cta, uint32_t budget,
-                           GemvArgs &a, GemvLayout &L) {
-    if (ty != T_IQ2_XXS) return gemv_layout_with(ty, nunit, n, sep, tiles_per_cta, 1, budget, a, L);
+// IQ2_XXS: as many side-by-side copies of the look-up tables as leave room for a plan that
+// keeps all of x resident (32 copies make every look-up free of bank conflicts).
+static bool gemv_layout_search(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t csize, uint32_t tiles_per_cta, GemvArgs &a,
+                               GemvLayout &L) {
+    // (Tried for several columns of long rows, whose panel of x does not fit beside the ring in
+    // half an SM's shared memory: taking the SM alone with the whole panel resident.  Slower:
+    // the next kernel can then not prefetch under this one.)
+    if (ty != T_IQ2_XXS) return gemv_layout_with(ty, row_bytes, nunit, n, mode, csize, tiles_per_cta, 1, kSharedBudget, a, L);
     GemvArgs fa = a;
     GemvLayout fl = L;
     bool have = false;
-    for (uint32_t copies = 16; copies >= 1; copies /= 2) {
+    for (uint32_t copies = 32; copies >= 1; copies /= 2) {
         GemvArgs ta = a;
         GemvLayout tl = L;
-        if (!gemv_layout_with(ty, nunit, n, sep, tiles_per_cta, copies, budget, ta, tl)) continue;
+        if (!gemv_layout_with(ty, row_bytes, nunit, n, mode, csize, tiles_per_cta, copies, kSharedBudget, ta, tl)) continue;
         if (tl.panel == ta.nchunk) { a = ta; L = tl; return true; }
         if (!have) { fa = ta; fl = tl; have = true; }
     }
@@ -1645,34 +1280,26 @@ static bool gemv_layout_in(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_
     return have;
 }
 
-static bool gemv_layout_search(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t tiles_per_cta, GemvArgs &a,
-                               GemvLayout &L) {
-    // (Tried for several columns of long rows, whose panel of x does not fit beside the ring in
-    // half an SM's shared memory: taking the SM alone with the whole panel resident.  Slower:
-    // the next kernel can then not prefetch under this one.)
-    return gemv_layout_in(ty, nunit, n, sep, tiles_per_cta, kSharedBudget, a, L);
-}
-
 // The search costs the host about as much as a launch and an engine asks for the same few
 // shapes on every token, so each thread keeps the plans it found last.
-static bool gemv_layout(int ty, uint32_t nunit, uint32_t n, bool sep, uint32_t tiles_per_cta, GemvArgs &a,
+static bool gemv_layout(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t csize, uint32_t tiles_per_cta, GemvArgs &a,
                         GemvLayout &L) {
     struct Entry {
-        int ty;
-        uint32_t nunit, n, tiles_per_cta, cb, nchunk;
-        bool sep, used, ok;
+        int ty, mode;
+        uint32_t row_bytes, nunit, n, csize, tiles_per_cta, cb, nchunk;
+        bool used, ok;
         GemvLayout L;
     };
     constexpr uint32_t kEntries = 64;
     static thread_local Entry cache[kEntries];
-    uint32_t h = ((uint32_t)ty * 31 + nunit) * 31 + n;
-    h = (h * 31 + tiles_per_cta) * 2 + (sep ? 1 : 0);
+    uint32_t h = ((uint32_t)ty * 31 + row_bytes) * 31 + n;
+    h = ((h * 31 + tiles_per_cta) * 8 + csize) * 8 + (uint32_t)mode;
     Entry &e = cache[(h * 2654435761u) >> 26];
     static_assert(kEntries == 64, "six bits of the hash");
-    if (!(e.used && e.ty == ty && e.nunit == nunit && e.n == n && e.tiles_per_cta == tiles_per_cta && e.sep == sep)) {
+    if (!(e.used && e.ty == ty && e.mode == mode && e.row_bytes == row_bytes && e.nunit == nunit && e.n == n && e.csize == csize && e.tiles_per_cta == tiles_per_cta)) {
         GemvArgs t = {};
-        e = {ty, nunit, n, tiles_per_cta, 0, 0, sep, true, false, {}};
-        e.ok = gemv_layout_search(ty, nunit, n, sep, tiles_per_cta, t, e.L);
+        e = {ty, mode, row_bytes, nunit, n, csize, tiles_per_cta, 0, 0, true, false, {}};
+        e.ok = gemv_layout_search(ty, row_bytes, nunit, n, mode, csize, tiles_per_cta, t, e.L);
         e.cb = t.cb;
         e.nchunk = t.nchunk;
     }
@@ -1702,44 +1329,70 @@ static uint32_t gemv_ctas(uint32_t tiles, int sms, bool sep) {
     return sep && tiles <= n + n / 4 ? tiles : n;
 }
 
-template <int TY, int XDT, bool SEP>
+// Grid and shared-memory plan of a launch.  Clusters of CTAs share a tile along K where that lets every
+// CTA keep its part of x in shared memory (several columns of long rows, else staged again slice by
+// slice for every few tiles; and x is quantized once per cluster instead of once per CTA), or, for
+// IQ2_XXS, all 32 copies of its tables: the smallest cluster that does.  Q4_K 9728 -> 2560, 8 columns,
+// 34.0 -> 21.2 us, 4 columns 15.7 -> 12.9; IQ2_XXS 17408 -> 5120, one column 25.5 -> 21.7, four
+// 42.9 -> 35.0.  Where x fits anyway clusters cost time (Q4_K 9728 -> 2560, one column, 7.1 -> 7.9).
+// Row-shard launches have duties by CTA number and take no clusters.
+static bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t tiles, int sms, bool gather, GemvArgs &a,
+                      GemvLayout &L, uint32_t &ctas) {
+    const uint32_t all = gemv_ctas(tiles, sms, mode == M_SEP);
+    for (uint32_t cs = 1; cs <= 8 && !(gather && cs > 1) && cs * 4 <= nunit; cs *= 2) {
+        const uint32_t limit = (tiles >= kTwoCtasTiles * (uint32_t)sms ? 2 : 1) * (uint32_t)sms / cs;
+        const uint32_t clusters = cs == 1 ? all : tiles < limit ? tiles : limit;
+        if (!gemv_layout(ty, row_bytes, nunit, n, mode, cs, (tiles + clusters - 1) / clusters, a, L)) continue;
+        const bool last = ty == T_IQ2_XXS && cs == 2;  // shorter segments of its 66-byte units cost more than a resident x gains
+        if (!last && (L.panel < a.nchunk || (mode == M_SEP && ty == T_IQ2_XXS && nunit >= 48 && L.tab_copies < 32))) continue;
+        ctas = clusters * cs;
+        return true;
+    }
+    ctas = all;
+    return gemv_layout(ty, row_bytes, nunit, n, mode, 1, (tiles + all - 1) / all, a, L);
+}
+
+template <int TY, int MODE>
 static cudaError_t launch_t(GemvArgs a, const GemvGather &G, cudaStream_t s, int sms, int dev) {
     GemvLayout L;
-    const uint32_t ctas = gemv_ctas(a.tiles, sms, SEP);
-    if (!gemv_layout(TY, a.nunit, a.n, SEP, (a.tiles + ctas - 1) / ctas, a, L)) return cudaErrorInvalidConfiguration;
+    uint32_t ctas;
+    if (!gemv_plan(TY, a.row_bytes, a.nunit, a.n, MODE, a.tiles, sms, G.nranks != 0, a, L, ctas)) return cudaErrorInvalidConfiguration;
     static bool attr_set[64] = {};  // the opt-in is per device
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemv_kernel<TY, XDT, SEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBudget);
+        cudaError_t e = cudaFuncSetAttribute(gemv_kernel<TY, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBudget);
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    return launch_pdl(gemv_kernel<TY, XDT, SEP>, ctas, G.nranks ? kGemvThreadsMax : kGemvThreads, L.smem_bytes, s, 1, a, L, G);
+    return launch_pdl(gemv_kernel<TY, MODE>, ctas, G.nranks ? kGemvThreadsMax : kGemvThreads, L.smem_bytes, s, 1u << L.clog, a, L, G);
 }
 
 template <int TY>
-static cudaError_t launch_ty(const GemvArgs &a, const GemvGather &G, int xdt, bool sep, cudaStream_t s, int sms, int dev) {
-    if (sep) {
-        switch (xdt) {
-        case DT_F16: return launch_t<TY, DT_F16, true>(a, G, s, sms, dev);
-        case DT_BF16: return launch_t<TY, DT_BF16, true>(a, G, s, sms, dev);
-        case DT_F32: return launch_t<TY, DT_F32, true>(a, G, s, sms, dev);
-        }
-    } else {
-        switch (xdt) {
-        case DT_F16: return launch_t<TY, DT_F16, false>(a, G, s, sms, dev);
-        case DT_BF16: return launch_t<TY, DT_BF16, false>(a, G, s, sms, dev);
-        case DT_F32: return launch_t<TY, DT_F32, false>(a, G, s, sms, dev);
-        }
+static cudaError_t launch_ty(const GemvArgs &a, const GemvGather &G, int mode, cudaStream_t s, int sms, int dev) {
+    switch (mode) {
+    case M_SEP: return launch_t<TY, M_SEP>(a, G, s, sms, dev);
+    case M_W1: return launch_t<TY, M_W1>(a, G, s, sms, dev);
+    case M_W2: return launch_t<TY, M_W2>(a, G, s, sms, dev);
+    }
+    if constexpr (TY == T_Q8_0 || TY == T_Q4_0 || TY == T_IQ4_NL || TY == T_Q2_0) {
+        if (mode == M_R) return launch_t<TY, M_R>(a, G, s, sms, dev);
     }
     return cudaErrorInvalidValue;
 }
 
-bool gemv_group_supported(int ty, uint32_t k, uint32_t nseg, const uint32_t *m, const uint8_t *const *w,
-                          const void *x, int xdt, uint32_t n, int sms) {
-    if (!has_fast_kernels(ty)) return false;
+// How `n` columns are taken: the mode of the next pass and its columns.
+static int gemv_mode(uint32_t k, uint32_t n, uint32_t &take) {
+    if (k % 256) {
+        take = n < 4 ? n : 4;
+        return M_R;
+    }
+    take = n;
+    return n == 1 ? M_SEP : n <= 4 ? M_W1 : M_W2;
+}
+
+static bool group_fits(int ty, uint32_t k, uint32_t nseg, const uint32_t *m, const uint8_t *const *w,
+                       const void *x, int xdt, uint32_t n, int sms) {
     if (nseg == 0 || nseg > (uint32_t)kGemvSegs || n == 0 || n > 8) return false;
-    if (k % 256) return false;  // Q8_0 / Q2_0 rows that end inside a 256-wide unit take the simple kernel
     if ((uintptr_t)x % 16 || (k * (xdt == DT_F32 ? 4 : 2)) % 16) return false;
     uint32_t tiles = 0;
     for (uint32_t i = 0; i < nseg; i++) {
@@ -1748,10 +1401,18 @@ bool gemv_group_supported(int ty, uint32_t k, uint32_t nseg, const uint32_t *m, 
     }
     GemvArgs a = {};
     GemvLayout L;
-    const uint32_t ctas = gemv_ctas(tiles, sms, true), ctas_wide = gemv_ctas(tiles, sms, false);
-    if (!gemv_layout(ty, k / 256, 1, true, (tiles + ctas - 1) / ctas, a, L)) return false;
-    if (n > 1 && !gemv_layout(ty, k / 256, n < 4 ? n : 4, false, (tiles + ctas_wide - 1) / ctas_wide, a, L)) return false;
+    const uint32_t row_bytes = k / block_elems(ty) * block_bytes(ty);
+    for (uint32_t left = n, take; left; left -= take) {
+        const int mode = gemv_mode(k, left, take);
+        uint32_t ctas;
+        if (!gemv_plan(ty, row_bytes, (k + 255) / 256, take, mode, tiles, sms, false, a, L, ctas)) return false;
+    }
     return true;
+}
+
+bool gemv_group_supported(int ty, uint32_t k, uint32_t nseg, const uint32_t *m, const uint8_t *const *w,
+                          const void *x, int xdt, uint32_t n, int sms) {
+    return has_fast_kernels(ty) && k % 256 == 0 && group_fits(ty, k, nseg, m, w, x, xdt, n, sms);
 }
 
 bool gemv_fast_supported(int ty, uint32_t k, uint32_t m, const void *w, const void *x, int xdt, uint32_t n,
@@ -1760,17 +1421,22 @@ bool gemv_fast_supported(int ty, uint32_t k, uint32_t m, const void *w, const vo
     return gemv_group_supported(ty, k, 1, &m, &wp, x, xdt, n, sms);
 }
 
-// One launch covers one column (SEP) or up to four (WIDE); wider requests are cut
-// into passes over consecutive columns.  `nseg` matrices of the
-// same type and K share every launch.
+bool gemv_ragged_supported(int ty, uint32_t k, uint32_t m, const void *w, const void *x, int xdt, uint32_t n, int sms) {
+    if (ty != T_Q8_0 && ty != T_Q4_0 && ty != T_IQ4_NL && ty != T_Q2_0) return false;
+    const uint8_t *wp = (const uint8_t *)w;
+    return k % 256 != 0 && group_fits(ty, k, 1, &m, &wp, x, xdt, n, sms);
+}
+
+// One launch covers up to eight columns (four where rows are no multiple of 256 weights; more are
+// run as passes over consecutive columns).  `nseg` matrices of the same type and K share every launch.
 cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, const uint32_t *m, float *const *out,
                               uint32_t k, const void *x, int xdt, uint32_t n, int *status, cudaStream_t s,
                               int sms, int dev, uint64_t *launches, const GemvGatherPlan *gather) {
     if (nseg == 0 || nseg > (uint32_t)kGemvSegs) return cudaErrorInvalidValue;
     GemvArgs a = {};
-    a.status = status; a.k = k;
-    a.nunit = k / 256;
-    a.row_bytes = a.nunit * ((ty == T_Q4_K || ty == T_Q4_0 || ty == T_IQ4_NL) ? 144 : ty == T_Q8_0 ? 272 : ty == T_Q2_0 ? 68 : ty == T_Q6_K ? 210 : ty == T_Q5_K ? 176 : 66);
+    a.status = status; a.k = k; a.xdt = xdt;
+    a.nunit = (k + 255) / 256;
+    a.row_bytes = k / block_elems(ty) * block_bytes(ty);
     uint32_t tiles = 0;
     for (uint32_t i = 0; i < (uint32_t)kGemvSegs; i++) {
         const uint32_t j = i < nseg ? i : nseg - 1;  // unused slots repeat the last one
@@ -1793,9 +1459,8 @@ cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, co
     }
     const size_t xsz = xdt == DT_F32 ? 4 : 2;
     for (uint32_t c0 = 0; c0 < n;) {
-        const uint32_t left = n - c0;
-        const bool sep = left == 1;
-        const uint32_t take = sep ? 1 : (left < 4 ? left : 4);
+        uint32_t take;
+        const int mode = gemv_mode(k, n - c0, take);
         a.x = (const uint8_t *)x + (size_t)c0 * k * xsz;
         for (uint32_t i = 0; i < (uint32_t)kGemvSegs; i++) {
             const uint32_t j = i < nseg ? i : nseg - 1;
@@ -1810,14 +1475,14 @@ cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, co
         a.n = take;
         cudaError_t e;
         switch (ty) {
-        case T_Q4_K: e = launch_ty<T_Q4_K>(a, G, xdt, sep, s, sms, dev); break;
-        case T_Q8_0: e = launch_ty<T_Q8_0>(a, G, xdt, sep, s, sms, dev); break;
-        case T_Q4_0: e = launch_ty<T_Q4_0>(a, G, xdt, sep, s, sms, dev); break;
-        case T_Q6_K: e = launch_ty<T_Q6_K>(a, G, xdt, sep, s, sms, dev); break;
-        case T_Q5_K: e = launch_ty<T_Q5_K>(a, G, xdt, sep, s, sms, dev); break;
-        case T_IQ4_NL: e = launch_ty<T_IQ4_NL>(a, G, xdt, sep, s, sms, dev); break;
-        case T_Q2_0: e = launch_ty<T_Q2_0>(a, G, xdt, sep, s, sms, dev); break;
-        case T_IQ2_XXS: e = launch_ty<T_IQ2_XXS>(a, G, xdt, sep, s, sms, dev); break;
+        case T_Q4_K: e = launch_ty<T_Q4_K>(a, G, mode, s, sms, dev); break;
+        case T_Q8_0: e = launch_ty<T_Q8_0>(a, G, mode, s, sms, dev); break;
+        case T_Q4_0: e = launch_ty<T_Q4_0>(a, G, mode, s, sms, dev); break;
+        case T_Q6_K: e = launch_ty<T_Q6_K>(a, G, mode, s, sms, dev); break;
+        case T_Q5_K: e = launch_ty<T_Q5_K>(a, G, mode, s, sms, dev); break;
+        case T_IQ4_NL: e = launch_ty<T_IQ4_NL>(a, G, mode, s, sms, dev); break;
+        case T_Q2_0: e = launch_ty<T_Q2_0>(a, G, mode, s, sms, dev); break;
+        case T_IQ2_XXS: e = launch_ty<T_IQ2_XXS>(a, G, mode, s, sms, dev); break;
         default: e = cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;

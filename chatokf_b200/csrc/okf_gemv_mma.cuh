@@ -93,7 +93,8 @@ struct GemvArgs {
     const void *x;
     int *status;     // device status word: 0 = ok, else a wait gave up (see kStatus*)
     uint32_t k, n;
-    uint32_t nunit;  // 256-wide units per row
+    int xdt;
+    uint32_t nunit;  // 256-wide units per row, the last one perhaps not whole
     uint32_t tiles;  // all segments together
     uint32_t cb;     // units per chunk (one ring stage holds 16 rows x cb units)
     uint32_t nchunk; // chunks per tile
@@ -203,6 +204,57 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
 
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// Shared-memory loads by 32-bit shared-window address: all address arithmetic stays in 32 bits.
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds16(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(a));
+    return v;
+}
+// 4 * NW bytes from a 2-byte aligned shared address: aligned words and a funnel shift
+template <int NW>
+__device__ __forceinline__ void lds_a2(uint32_t a, uint32_t (&out)[NW]) {
+    const uint32_t base = a & ~3u, sh = (a & 2u) * 8u;
+    uint32_t w[NW + 1];
+#pragma unroll
+    for (int i = 0; i <= NW; i++) w[i] = lds32(base + 4 * i);
+#pragma unroll
+    for (int i = 0; i < NW; i++) out[i] = __funnelshift_r(w[i], w[i + 1], sh);
+}
+__device__ __forceinline__ int ubyte(uint32_t v, int i) { return (int)__byte_perm(v, 0, 0x4440 + i); }
+__device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t a, uint32_t x) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(x) : "memory");
+}
+__device__ __forceinline__ void sts16(uint32_t a, uint32_t x) {
+    asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "r"(x) : "memory");
+}
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t v;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(v) : "r"(a), "r"(b), "r"(sel));
+    return v;
+}
+
+__device__ __forceinline__ void sts8(uint32_t a, uint32_t x) {
+    asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(x) : "memory");
 }
 
 // byte b (0..255) of `v` as a float, without the slow int-to-float unit

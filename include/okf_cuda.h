@@ -119,7 +119,8 @@ OKF_API int okf_gemv(okf_ctx *ctx, int type, const okf_weights *w, uint64_t woff
  * in ONE scratch buffer of the context: calls of one context that may take that
  * route must be ordered on the GPU (same stream, or events between streams).
  * Numerics: for N <= 8 (fp32 out) every 256-wide run of an activation column is
- * reduced to 16-bit integers with one fp32 scale and the sums are exact integers
+ * reduced to 16-bit integers (24-bit where K is no multiple of 256) with one fp32
+ * scale and the sums are exact integers
  * (results within 1e-4 of max|y| of an fp32 evaluation on the test shapes, the
  * same for a column at every N); the tile rounds weights and activations to
  * 16-bit floats and accumulates in fp32 (within 1e-2). */
@@ -131,7 +132,7 @@ OKF_API int okf_gemm(okf_ctx *ctx, int type, const okf_weights *w, uint64_t woff
  * around gate || up and q || k || v (Qwen/QwenMetalEngine.swift:464-469, :691-696).
  * Inside a region, okf_gemv / okf_gemm calls with N <= 8 that multiply the same
  * x by matrices of one type and K (up to four) are held back and leave as ONE
- * kernel launch (one per four columns of N), at okf_parallel_end or as soon as
+ * kernel launch, at okf_parallel_end or as soon as
  * a call does not fit the set;
  * every other call runs at once, as outside a region.  A launch error of a
  * held-back call is returned by the call that sends the set off.  Regions do
@@ -358,10 +359,11 @@ OKF_API int okf_set_flags(okf_ctx *ctx, uint32_t flags);
 
 /* Number of kernels this context has launched since it was created. */
 OKF_API uint64_t okf_launch_count(const okf_ctx *ctx);
-/* Number of calls that ran on the plain warp-per-row / fp32-tile kernels because
- * the tensor-core kernels do not take the shape or alignment (K not a multiple
- * of 256 for the matvec or of 64 for the tile, x not 16-byte aligned): correct
- * but many times slower.  A caller that cares about speed checks that this
+/* Number of calls that did not run on the main kernels because of their shape or
+ * alignment: K not a multiple of 256 for the matvec (a slower form of it that
+ * keeps 24 bits of x takes Q8_0, Q4_0, IQ4_NL and Q2_0 with aligned pointers) or
+ * of 64 for the tile, x not 16-byte aligned (plain warp-per-row / fp32-tile
+ * kernels, many times slower).  A caller that cares about speed checks that this
  * stays 0.  Calls made under OKF_FLAG_SIMPLE_KERNELS are not counted.  No
  * counterpart in the reference. */
 OKF_API uint64_t okf_fallback_count(const okf_ctx *ctx);
