@@ -157,21 +157,23 @@ __global__ void __launch_bounds__(256, 6) argmax_rows_kernel(const float *__rest
 // ---- residual add + RMS norm ----------------------------------------------------------
 // x[row] += r[row] (skipped when r is null); y[row] = x[row] * scale * w with
 // scale = 1 / sqrt(mean(x^2) + eps).  One CTA per row.
+// Thread t of 256 sums elements t, t + 256, ... in this order, then come the lanes, then the warps: both
+// kernels give the same bits.
 __device__ __forceinline__ float norm_scale(float ss, uint32_t n, float eps, float *part) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
     __syncthreads();
-    float tot = (threadIdx.x & 31) < blockDim.x / 32 ? part[threadIdx.x & 31] : 0.f;
+    float tot = 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    for (int i = 0; i < 8; i++) tot += part[i];
     return 1.f / sqrtf(tot / (float)n + eps);
 }
-// any length and alignment: the row is read from HBM once, the second sweep hits L1 / L2
-__global__ void __launch_bounds__(256) add_rmsnorm_kernel(float *x, const float *__restrict__ r,
-                                                          const float *__restrict__ w, float *y, uint32_t n,
-                                                          float eps, uint32_t x_stride, uint32_t y_stride) {
-    __shared__ float part[32];
+// any length: the row is read from HBM once, the second sweep hits L1 / L2
+__global__ void __launch_bounds__(256, 6) add_rmsnorm_kernel(float *x, const float *__restrict__ r,
+                                                             const float *__restrict__ w, float *y, uint32_t n,
+                                                             float eps, uint32_t x_stride, uint32_t y_stride) {
+    __shared__ float part[8];
     pdl_launch_dependents();
     float *xr = x + (size_t)blockIdx.x * x_stride;
     const float *rr = r ? r + (size_t)blockIdx.x * x_stride : nullptr;
@@ -189,44 +191,53 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(float *x, const float 
     const float scale = norm_scale(ss, n, eps, part);
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) yr[i] = xr[i] * scale * w[i];
 }
-// Rows of up to 8192 floats, everything 16-byte aligned: a thread keeps its (at most two) groups of
-// four in registers, so there is one round trip to L2, for x, r and w together, and one sum.
-__global__ void __launch_bounds__(1024, 2) add_rmsnorm_vec_kernel(float *x, const float *__restrict__ r,
-                                                               const float *__restrict__ w, float *y, uint32_t n,
-                                                               float eps, uint32_t x_stride, uint32_t y_stride) {
-    __shared__ float part[32];
+// Rows of up to 256 V floats: a thread keeps its V elements in registers, so that there is one round
+// trip to L2, for x, r and w together (with w read after the sum four Q4_K FFN blocks took 93 us, so 80).
+template <int V>
+__global__ void __launch_bounds__(256, V <= 12 ? 4 : 2) add_rmsnorm_short_kernel(float *x, const float *__restrict__ r,
+                                                                   const float *__restrict__ w, float *y, uint32_t n,
+                                                                   float eps, uint32_t x_stride, uint32_t y_stride) {
+    __shared__ float part[8];
     pdl_launch_dependents();
-    float4 *xr = reinterpret_cast<float4 *>(x + (size_t)blockIdx.x * x_stride);
-    const float4 *rr = r ? reinterpret_cast<const float4 *>(r + (size_t)blockIdx.x * x_stride) : nullptr;
-    float4 *yr = reinterpret_cast<float4 *>(y + (size_t)blockIdx.x * y_stride);
-    const float4 *w4 = reinterpret_cast<const float4 *>(w);
-    float4 v[2], g[2];
-    float ss = 0.f;
+    float *xr = x + (size_t)blockIdx.x * x_stride;
+    const float *rr = r ? r + (size_t)blockIdx.x * x_stride : nullptr;
+    float *yr = y + (size_t)blockIdx.x * y_stride;
+    float v[V], g[V];
     pdl_wait();
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        const uint32_t i = threadIdx.x + j * blockDim.x;
-        v[j] = g[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (i < n / 4) {
-            v[j] = xr[i];
-            g[j] = w4[i];
-            if (rr) {
-                const float4 a = rr[i];
-                v[j].x += a.x; v[j].y += a.y; v[j].z += a.z; v[j].w += a.w;
-            }
-        }
+    for (int j = 0; j < V; j++) {
+        const uint32_t i = threadIdx.x + 256 * j;
+        v[j] = i < n ? xr[i] : 0.f;
     }
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        ss = fmaf(v[j].x, v[j].x, fmaf(v[j].y, v[j].y, fmaf(v[j].z, v[j].z, fmaf(v[j].w, v[j].w, ss))));
-        const uint32_t i = threadIdx.x + j * blockDim.x;
-        if (rr && i < n / 4) xr[i] = v[j];
+    for (int j = 0; j < V; j++) {
+        const uint32_t i = threadIdx.x + 256 * j;
+        g[j] = i < n ? w[i] : 0.f;
+    }
+    if (rr) {
+        float q[V];
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            const uint32_t i = threadIdx.x + 256 * j;
+            q[j] = i < n ? rr[i] : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < V; j++) v[j] += q[j];
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < V; j++) {
+        const uint32_t i = threadIdx.x + 256 * j;
+        if (i < n) {
+            if (rr) xr[i] = v[j];
+            ss = fmaf(v[j], v[j], ss);
+        }
     }
     const float s = norm_scale(ss, n, eps, part);
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        const uint32_t i = threadIdx.x + j * blockDim.x;
-        if (i < n / 4) yr[i] = make_float4(v[j].x * s * g[j].x, v[j].y * s * g[j].y, v[j].z * s * g[j].z, v[j].w * s * g[j].w);
+    for (int j = 0; j < V; j++) {
+        const uint32_t i = threadIdx.x + 256 * j;
+        if (i < n) yr[i] = v[j] * s * g[j];
     }
 }
 
@@ -318,11 +329,10 @@ int okf_add_rmsnorm(okf_ctx *ctx, float *x, const float *r, const float *weight,
     if (fault_fires(ctx)) return OKF_E_INJECTED;
     DeviceGuard g(ctx->device);
     if (!g.ok) return cuda_fail(ctx, cudaErrorInvalidDevice);
-    const bool vec = n % 4 == 0 && n <= 8192 && x_stride % 4 == 0 && y_stride % 4 == 0 &&
-                     (((uintptr_t)x | (uintptr_t)r | (uintptr_t)weight | (uintptr_t)y) & 15) == 0;
-    const unsigned threads = vec ? ((n + 7) / 8 + 31) / 32 * 32 : 256;  // two groups of four a thread
-    cudaError_t e = launch_pdl(vec ? add_rmsnorm_vec_kernel : add_rmsnorm_kernel, rows, threads, 0,
-                               (cudaStream_t)stream, 1, x, r, weight, y, n, eps, x_stride, y_stride);
+    auto *kernel = n <= 1024 ? add_rmsnorm_short_kernel<4> : n <= 2048 ? add_rmsnorm_short_kernel<8>
+                 : n <= 3072 ? add_rmsnorm_short_kernel<12> : n <= 5120 ? add_rmsnorm_short_kernel<20>
+                 : n <= 8192 ? add_rmsnorm_short_kernel<32> : add_rmsnorm_kernel;  // V covers the row
+    cudaError_t e = launch_pdl(kernel, rows, 256, 0, (cudaStream_t)stream, 1, x, r, weight, y, n, eps, x_stride, y_stride);
     if (e != cudaSuccess) return cuda_fail(ctx, e);
     ctx->launches++;
     return OKF_OK;
