@@ -30,6 +30,7 @@
 
 #include <cstring>
 #include "okf_gemv_mma.cuh"
+#include "okf_gemv_wide.cuh"
 #include "okf_internal.h"
 #include "okf_kernels.h"
 
@@ -191,39 +192,76 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
 }
 
 // ---- weights for the A tile -------------------------------------------------------
-// ARaw<TY> holds, in registers, the bytes one thread needs to unpack 32 weights
-// (half h of k-block kb of its row); load() is issued one k-block ahead of
-// decode() so the memory latency hides behind the previous block's work.
-// Q4_K and Q2_0 (the prefill shapes that are benchmarked) have register
-// forms; the other types unpack straight from memory with decode32.
-// Which 16-byte chunk of the row's 128 bytes (64 k) the thread's c4-th group of eight values is.
+// ARaw<TY> holds, in registers, the bytes one thread needs to unpack 32 weights (half h of k-block kb) of
+// its row; load() is issued a turn or two ahead of unpack() so that the latency of L2 hides behind the
+// work in between.  unpack() leaves four groups of eight 16-bit floats; chunk() says which 16-byte chunk
+// of the row's 128 bytes (64 k) each group is.
+//
+// A code byte becomes a float by one byte permute that puts it into the mantissa of a constant: 128 + b
+// for codes below 128 (mantissa bits 16 .. 22), 32768 + b for whole bytes (bits 8 .. 15).  The constant's
+// share leaves through the addend of the multiply-add that applies the scale, scale * (X + b) + add: one
+// permute, one FMA and half a conversion per weight.  The addend is exact for every type without mins
+// (a scale has 11 to 18 significant bits, the constants 3 to 9), so weights are still decoded exactly and
+// rounded once; with mins it is off by 2^-24 of 128 scales, 1 / 500 of the rounding to fp16.
+// (Before, the types other than Q4_K, Q8_0 and Q2_0 were unpacked byte by byte from memory: Q5_K 5120 ->
+// 17408 at 64 tokens took 224 us, now 53; Q6_K 197, now 78; IQ4_NL 111, now 55.)
+__device__ __forceinline__ float code_f32(uint32_t word, int byte) { return __uint_as_float(__byte_perm(word, 0x43000000u, 0x7044 | byte << 8)); }
+__device__ __forceinline__ float wide_f32(uint32_t word, int byte) { return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7404 | byte << 4)); }
+// four weights out of the bytes of a word
+template <bool F16>
+__device__ __forceinline__ uint2 unpack4(uint32_t w, float mul, float add) {
+    return make_uint2(pack16<F16>(fmaf(mul, code_f32(w, 0), add), fmaf(mul, code_f32(w, 1), add)),
+                      pack16<F16>(fmaf(mul, code_f32(w, 2), add), fmaf(mul, code_f32(w, 3), add)));
+}
+template <bool F16>
+__device__ __forceinline__ uint4 unpack8(uint32_t w0, uint32_t w1, float mul, float add) {
+    const uint2 a = unpack4<F16>(w0, mul, add), b = unpack4<F16>(w1, mul, add);
+    return make_uint4(a.x, a.y, b.x, b.y);
+}
+// 4 * NW bytes at a 2-byte aligned global address: aligned words (the last may lie past the block:
+// buffers are padded) and, in get(), a funnel shift
+template <int NW> struct Ldg2 {
+    uint32_t w[NW + 1], sh;
+    __device__ __forceinline__ void load(const uint8_t *b) {
+        const uint32_t *p = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(b) & ~(uintptr_t)3);
+        sh = ((uint32_t)reinterpret_cast<uintptr_t>(b) & 2u) * 8u;
+#pragma unroll
+        for (int i = 0; i <= NW; i++) w[i] = __ldg(p + i);
+    }
+    __device__ __forceinline__ uint32_t get(int i) const { return __funnelshift_r(w[i], w[i + 1], sh); }
+};
 __device__ __forceinline__ uint32_t chunk_in_order(uint32_t h, uint32_t c4) { return h * 4 + c4; }
 
-template <int TY> struct ARaw {
-    static constexpr int kAhead = 1;  // k-blocks of this thread in flight beside the one being unpacked
-    __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return chunk_in_order(h, c4); }
-    const uint8_t *wp; uint32_t gran;
-    __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) { wp = row; gran = kb * 2 + h; }
-    __device__ __forceinline__ void decode(float (&v)[32], const uint64_t *grid) const { decode32<TY>(wp, gran, v, grid); }
-};
-// Q4_K: a k-block is 32 bytes of a 144-byte block: low nibbles = its first 32 weights (sub-block
-// 2p), high nibbles = the other 32 (sub-block 2p + 1).  The two threads of a row take 16 bytes
-// each and unpack both nibbles, so a thread fetches 32 bytes per k-block, header included, and
-// can afford to fetch two k-blocks ahead: one turn ahead does not cover the latency of L2.
-template <> struct ARaw<T_Q4_K> {
-    static constexpr int kAhead = 2;
+template <int TY> struct ARaw;
+// Q4_K, Q5_K: a k-block is 32 bytes of qs: low nibbles = its first 32 weights (sub-block 2p), high
+// nibbles = the other 32 (sub-block 2p + 1); Q5_K's fifth bit of sub-block j is bit j of qh[l].  The two
+// threads of a row take 16 bytes each and unpack both nibbles: 32 bytes of Q4_K per k-block and thread,
+// header included, and two k-blocks in flight: one turn ahead does not cover the latency of L2.
+template <int TY> struct ARawK45 {
+    static constexpr int kAhead = 2;  // k-blocks of this thread in flight beside the one being unpacked
     // values 0..15 are k = 16h + 0..15 (chunks 2h, 2h + 1), values 16..31 the same positions 32 further on
     __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return (c4 >> 1) * 4 + 2 * h + (c4 & 1); }
-    uint4 hdr, q; uint32_t p;  // p: which 32 bytes of the block's 128
+    uint4 hdr, q, h5;
+    uint32_t p;  // which 32 bytes of the block's 128
     __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) {
-        const uint8_t *b = row + (size_t)(kb >> 2) * 144;
-        hdr = __ldg(reinterpret_cast<const uint4 *>(b));
-        q = __ldg(reinterpret_cast<const uint4 *>(b + 16 + 32 * (kb & 3) + 16 * h));
+        const uint8_t *b = row + (size_t)(kb >> 2) * (TY == T_Q4_K ? 144 : 176);
         p = kb & 3;
+        if constexpr (TY == T_Q4_K) {  // 16-byte aligned
+            hdr = __ldg(reinterpret_cast<const uint4 *>(b));
+            q = __ldg(reinterpret_cast<const uint4 *>(b + 16 + 32 * p + 16 * h));
+        } else if (((uintptr_t)b & 15) == 0) {
+            hdr = __ldg(reinterpret_cast<const uint4 *>(b));
+            h5 = __ldg(reinterpret_cast<const uint4 *>(b + 16 + 16 * h));
+            q = __ldg(reinterpret_cast<const uint4 *>(b + 48 + 32 * p + 16 * h));
+        } else {  // a tensor that does not start on a 16-byte boundary
+            auto ld = [](const uint8_t *a) { return make_uint4(ld_u32_a2(a), ld_u32_a2(a + 4), ld_u32_a2(a + 8), ld_u32_a2(a + 12)); };
+            hdr = ld(b);
+            h5 = ld(b + 16 + 16 * h);
+            q = ld(b + 48 + 32 * p + 16 * h);
+        }
     }
-    // w = (d * sc) * q - dmin * m (LLM/Quantize/KQuants.swift:104-125), here with one
-    // fused multiply-add: the result is rounded to a 16-bit float anyway
-    __device__ __forceinline__ void decode(float (&v)[32], const uint64_t *) const {
+    // w = (d * sc) * q - dmin * m (LLM/Quantize/KQuants.swift:104-158)
+    template <bool F16> __device__ __forceinline__ void unpack(uint4 (&o)[4], const uint32_t *) const {
         // 6-bit scales and mins of sub-blocks 2p and 2p + 1 (get_scale_min_k4): bytes 2p, 2p + 1 of
         // the scale field for p < 2, split fields above
         const uint32_t sh = (p & 1) * 16;
@@ -233,60 +271,167 @@ template <> struct ARaw<T_Q4_K> {
         else { sc = (e & 0x0F0Fu) | ((a >> 2) & 0x3030u); mn = ((e >> 4) & 0x0F0Fu) | ((b >> 2) & 0x3030u); }
         const float d = f16bits(hdr.x & 0xFFFF), dm = f16bits(hdr.x >> 16);
         const float d0 = d * byte_to_f32(sc, 0), d1 = d * byte_to_f32(sc, 1);
-        const float o0 = dm * byte_to_f32(mn, 0), o1 = dm * byte_to_f32(mn, 1);
-        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+        const float o0 = fmaf(d0, -128.f, -dm * byte_to_f32(mn, 0)), o1 = fmaf(d1, -128.f, -dm * byte_to_f32(mn, 1));
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w}, f[4] = {h5.x, h5.y, h5.z, h5.w};
+        uint32_t lo[4], hi[4];
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const uint32_t lo = w[i] & 0x0F0F0F0Fu, hi = (w[i] >> 4) & 0x0F0F0F0Fu;
-#pragma unroll
-            for (int e4 = 0; e4 < 4; e4++) {
-                v[4 * i + e4] = fmaf(d0, byte_to_f32(lo, e4), -o0);
-                v[16 + 4 * i + e4] = fmaf(d1, byte_to_f32(hi, e4), -o1);
+            lo[i] = w[i] & 0x0F0F0F0Fu;
+            hi[i] = (w[i] >> 4) & 0x0F0F0F0Fu;
+            if constexpr (TY == T_Q5_K) {
+                const uint32_t t = f[i] >> (2 * p);
+                lo[i] |= (t << 4) & 0x10101010u;
+                hi[i] |= (t << 3) & 0x10101010u;
             }
         }
+        o[0] = unpack8<F16>(lo[0], lo[1], d0, o0);
+        o[1] = unpack8<F16>(lo[2], lo[3], d0, o0);
+        o[2] = unpack8<F16>(hi[0], hi[1], d1, o1);
+        o[3] = unpack8<F16>(hi[2], hi[3], d1, o1);
+    }
+};
+template <> struct ARaw<T_Q4_K> : ARawK45<T_Q4_K> {};
+template <> struct ARaw<T_Q5_K> : ARawK45<T_Q5_K> {};
+// Q6_K: k-block kb is granules r = 2 (kb & 1), + 1 of half n of the block: 64 bytes of ql (low nibbles for
+// even kb, high for odd) and 32 of qh.  The two threads of a row take positions 16h .. 16h + 15 of both
+// granules, one scale each.
+template <> struct ARaw<T_Q6_K> {
+    static constexpr int kAhead = 1;
+    __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return (c4 >> 1) * 4 + 2 * h + (c4 & 1); }
+    Ldg2<4> l0, l1, hq;
+    uint32_t sc, par;
+    float d;
+    __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) {
+        const uint8_t *b = row + (size_t)(kb >> 2) * 210;
+        const uint32_t n = (kb >> 1) & 1;
+        par = kb & 1;
+        l0.load(b + 64 * n + 16 * h);
+        l1.load(b + 64 * n + 32 + 16 * h);
+        hq.load(b + 128 + 32 * n + 16 * h);
+        const uint8_t *s = b + 192 + 8 * n + 4 * par + h;
+        sc = (uint32_t)__ldg(s) | (uint32_t)__ldg(s + 2) << 8;
+        d = f16bits(__ldg(reinterpret_cast<const uint16_t *>(b + 208)));
+    }
+    // d * scale * (q - 32) (LLM/Quantize/KQuants.swift:160-177)
+    template <bool F16> __device__ __forceinline__ void unpack(uint4 (&o)[4], const uint32_t *) const {
+        const float m0 = d * (float)(int)(int8_t)(sc & 0xFF), m1 = d * (float)(int)(int8_t)(sc >> 8 & 0xFF);
+        uint32_t a[4], b[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t h = hq.get(i) >> (4 * par);
+            a[i] = ((l0.get(i) >> (4 * par)) & 0x0F0F0F0Fu) | ((h << 4) & 0x30303030u);
+            b[i] = ((l1.get(i) >> (4 * par)) & 0x0F0F0F0Fu) | ((h << 2) & 0x30303030u);
+        }
+        o[0] = unpack8<F16>(a[0], a[1], m0, -160.f * m0);
+        o[1] = unpack8<F16>(a[2], a[3], m0, -160.f * m0);
+        o[2] = unpack8<F16>(b[0], b[1], m1, -160.f * m1);
+        o[3] = unpack8<F16>(b[2], b[3], m1, -160.f * m1);
     }
 };
 template <> struct ARaw<T_Q8_0> {
     static constexpr int kAhead = 1;
     __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return chunk_in_order(h, c4); }
-    uint32_t w[10], sh;  // the 34-byte block {f16 d; i8 q[32]} and what precedes it in its first word
-    __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) {
-        const uint8_t *b = row + (size_t)(kb * 2 + h) * 34;  // 2-byte aligned
-        const uint32_t *p = reinterpret_cast<const uint32_t *>(reinterpret_cast<uintptr_t>(b) & ~(uintptr_t)3);
-        sh = ((uint32_t)reinterpret_cast<uintptr_t>(b) & 2u) * 8u;
-#pragma unroll
-        for (int i = 0; i < 10; i++) w[i] = __ldg(p + i);  // may run a few bytes past the block (buffers are padded)
-    }
-    __device__ __forceinline__ void decode(float (&v)[32], const uint64_t *) const {
+    Ldg2<9> w;  // the 34-byte block {f16 d; i8 q[32]}
+    __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) { w.load(row + (size_t)(kb * 2 + h) * 34); }
+    template <bool F16> __device__ __forceinline__ void unpack(uint4 (&o)[4], const uint32_t *) const {
         uint32_t u[9];
 #pragma unroll
-        for (int i = 0; i < 9; i++) u[i] = __funnelshift_r(w[i], w[i + 1], sh);
+        for (int i = 0; i < 9; i++) u[i] = w.get(i) ^ (i ? 0x80808080u : 0x80800000u);  // q + 128 as unsigned bytes
+        const float d = f16bits(u[0] & 0xFFFF), add = -32896.f * d;
+        auto val = [&](int j) { return fmaf(d, wide_f32(u[(j + 2) >> 2], (j + 2) & 3), add); };
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o[c] = make_uint4(pack16<F16>(val(8 * c), val(8 * c + 1)), pack16<F16>(val(8 * c + 2), val(8 * c + 3)),
+                              pack16<F16>(val(8 * c + 4), val(8 * c + 5)), pack16<F16>(val(8 * c + 6), val(8 * c + 7)));
+    }
+};
+// Q4_0, IQ4_NL: {f16 d; u8 qs[16]}, byte j = weights j (low nibble) and j + 16 (high)
+template <int TY> struct ARaw40 {
+    static constexpr int kAhead = 1;
+    __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return chunk_in_order(h, c4); }
+    Ldg2<5> w;
+    __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) { w.load(row + (size_t)(kb * 2 + h) * 18); }
+    template <bool F16> __device__ __forceinline__ void unpack(uint4 (&o)[4], const uint32_t *) const {
+        uint32_t u[5], q[4];
+#pragma unroll
+        for (int i = 0; i < 5; i++) u[i] = w.get(i);
         const float d = f16bits(u[0] & 0xFFFF);
 #pragma unroll
-        for (int j = 0; j < 32; j++) {
-            const int at = 2 + j;  // byte index in the block
-            const uint32_t word = u[at >> 2] ^ 0x80808080u;  // q + 128 as an unsigned byte
-            v[j] = d * (byte_to_f32(word, at & 3) - 128.f);
+        for (int i = 0; i < 4; i++) q[i] = __funnelshift_r(u[i], u[i + 1], 16);
+        if constexpr (TY == T_Q4_0) {
+            const float add = -136.f * d;
+            constexpr uint32_t ml = 0x0F0F0F0Fu;
+            o[0] = unpack8<F16>(q[0] & ml, q[1] & ml, d, add);
+            o[1] = unpack8<F16>(q[2] & ml, q[3] & ml, d, add);
+            o[2] = unpack8<F16>(q[0] >> 4 & ml, q[1] >> 4 & ml, d, add);
+            o[3] = unpack8<F16>(q[2] >> 4 & ml, q[3] >> 4 & ml, d, add);
+        } else {
+            // the codebook's values + 128 (LLM/Gemma/Gemma4Quant.swift:5-9), looked up eight nibbles a word in the
+            // order they follow: lo, hi of byte 0, lo, hi of byte 1, ... (see iq4nl_word)
+            constexpr uint32_t T0 = 0x3F2D1801u, T1 = 0x766A5D4Fu, T2 = 0xA6998D81u, T3 = 0xF1D9C5B5u;
+            const float add = -32896.f * d;
+            uint32_t t[8];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint32_t sel = q[i] & 0x77777777u, pick = (q[i] >> 1 & 0x44444444u) | 0x32103210u;
+                t[2 * i] = __byte_perm(__byte_perm(T0, T1, sel), __byte_perm(T2, T3, sel), pick);
+                t[2 * i + 1] = __byte_perm(__byte_perm(T0, T1, sel >> 16), __byte_perm(T2, T3, sel >> 16), pick >> 16);
+            }
+            auto val = [&](int j) { return fmaf(d, wide_f32(t[(j & 15) >> 1], (j & 1) * 2 + (j >> 4)), add); };
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                o[c] = make_uint4(pack16<F16>(val(8 * c), val(8 * c + 1)), pack16<F16>(val(8 * c + 2), val(8 * c + 3)),
+                                  pack16<F16>(val(8 * c + 4), val(8 * c + 5)), pack16<F16>(val(8 * c + 6), val(8 * c + 7)));
         }
     }
 };
+template <> struct ARaw<T_Q4_0> : ARaw40<T_Q4_0> {};
+template <> struct ARaw<T_IQ4_NL> : ARaw40<T_IQ4_NL> {};
 template <> struct ARaw<T_Q2_0> {
-    static constexpr int kAhead = 1;
+    static constexpr int kAhead = 2;
     __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return chunk_in_order(h, c4); }
-    uint32_t c0, c1, dbits;  // 32 two-bit codes and the block scale
+    Ldg2<2> w;  // 32 two-bit codes
+    uint32_t dbits;
     __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) {
-        const uint8_t *b = row + (size_t)(kb >> 1) * 34;           // block of 128 weights
-        const uint16_t *q = reinterpret_cast<const uint16_t *>(b + 2 + 16 * (kb & 1) + 8 * h);
+        const uint8_t *b = row + (size_t)(kb >> 1) * 34;  // block of 128 weights
         dbits = __ldg(reinterpret_cast<const uint16_t *>(b));
-        c0 = (uint32_t)__ldg(q) | ((uint32_t)__ldg(q + 1) << 16);
-        c1 = (uint32_t)__ldg(q + 2) | ((uint32_t)__ldg(q + 3) << 16);
+        w.load(b + 2 + 16 * (kb & 1) + 8 * h);
     }
-    __device__ __forceinline__ void decode(float (&v)[32], const uint64_t *) const {
-        const float d = f16bits(dbits);
+    template <bool F16> __device__ __forceinline__ void unpack(uint4 (&o)[4], const uint32_t *) const {
+        const float d = f16bits(dbits), add = -129.f * d;  // (code - 1) * d
+        uint32_t t[2][4];
 #pragma unroll
-        for (int e = 0; e < 16; e++) {
-            v[e] = (float)((int)((c0 >> (2 * e)) & 3u) - 1) * d;
-            v[16 + e] = (float)((int)((c1 >> (2 * e)) & 3u) - 1) * d;
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) t[i][e] = w.get(i) >> (2 * e) & 0x03030303u;  // byte b: code 4b + e
+        auto val = [&](int j) { return fmaf(d, code_f32(t[j >> 4][j & 3], (j & 15) >> 2), add); };
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            o[c] = make_uint4(pack16<F16>(val(8 * c), val(8 * c + 1)), pack16<F16>(val(8 * c + 2), val(8 * c + 3)),
+                              pack16<F16>(val(8 * c + 4), val(8 * c + 5)), pack16<F16>(val(8 * c + 6), val(8 * c + 7)));
+    }
+};
+// IQ2_XXS: sub-block = {u32: four codebook indices, u32: four 7-bit sign indices + 4-bit scale}
+// (LLM/Quantize/IQ2XXS.swift:34-53).  The tables in shared memory hold byte-permute selectors (see
+// iq2_code_selectors): over the magnitudes and their negatives, all 64 up so that they are below 128.
+template <> struct ARaw<T_IQ2_XXS> {
+    static constexpr int kAhead = 2;
+    __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return chunk_in_order(h, c4); }
+    Ldg2<2> w;
+    uint32_t dbits;
+    __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) {
+        const uint8_t *b = row + (size_t)(kb >> 2) * 66;
+        dbits = __ldg(reinterpret_cast<const uint16_t *>(b));
+        w.load(b + 2 + 8 * ((kb & 3) * 2 + h));
+    }
+    template <bool F16> __device__ __forceinline__ void unpack(uint4 (&o)[4], const uint32_t *tab) const {
+        const uint32_t a0 = w.get(0), a1 = w.get(1);
+        const float db = f16bits(dbits) * (0.5f + (float)(a1 >> 28)) * 0.25f, add = -192.f * db;
+        constexpr uint32_t P = 0x406B5948u, N = 0x40152738u;  // 64 + {8, 25, 43, 0}, 64 - {8, 25, 43, 0}
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const uint32_t s = tab[__byte_perm(a0, 0u, 0x4440 + c)] | tab[256 + (a1 >> (7 * c) & 127u)];
+            o[c] = unpack8<F16>(__byte_perm(P, N, s), __byte_perm(P, N, s >> 16), db, add);
         }
     }
 };
@@ -365,7 +510,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *a_ring = smem, *b_ring = smem + R::a_bytes;
-    uint64_t *grid = reinterpret_cast<uint64_t *>(smem + R::a_bytes + R::b_bytes);
+    uint32_t *tab = reinterpret_cast<uint32_t *>(smem + R::a_bytes + R::b_bytes);  // IQ2_XXS: 256 + 128 selector words
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + R::a_bytes + R::b_bytes + R::grid_bytes);
     uint64_t *full_a = bars, *empty_a = bars + kMaxRing;                    // A producers <-> MMA, one pair per A stage
     uint64_t *full_b = bars + 2 * kMaxRing, *empty_b = bars + 3 * kMaxRing;  // B producer(s) <-> MMA, one pair per B stage
@@ -392,7 +537,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if constexpr (TY == T_IQ2_XXS) {
-        for (uint32_t i = threadIdx.x; i < 256; i += kThreads) grid[i] = g_iq2xxs_grid[i];
+        for (uint32_t i = threadIdx.x; i < 384; i += kThreads) tab[i] = i < 256 ? iq2_code_selectors(g_iq2xxs_grid[i]) : iq2_sign_selectors(i - 256);
     }
     if (warp == kMmaWarp) {
         // the whole tensor memory of the SM: two 256-column accumulators
@@ -414,17 +559,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         const uint32_t arow = t >> 1, ahalf = t & 1;  // thread t unpacks 32 weights of row arow
         uint32_t it0 = 0;  // stage counter at the start of the work item
         Work wk;
-        // decoded values -> 16-bit floats -> this thread's four 16-byte chunks of stage s
-        auto put = [&](const float (&v)[32], bool live, uint32_t it) -> bool {
+        // this thread's four 16-byte chunks -> stage s
+        auto put = [&](const uint4 (&q)[4], uint32_t it) -> bool {
             const uint32_t s = it % kAStages, use = it / kAStages;
-            uint4 q[4];
-#pragma unroll
-            for (int c4 = 0; c4 < 4; c4++) {
-                q[c4].x = live ? pack16<F16>(v[8 * c4], v[8 * c4 + 1]) : 0u;
-                q[c4].y = live ? pack16<F16>(v[8 * c4 + 2], v[8 * c4 + 3]) : 0u;
-                q[c4].z = live ? pack16<F16>(v[8 * c4 + 4], v[8 * c4 + 5]) : 0u;
-                q[c4].w = live ? pack16<F16>(v[8 * c4 + 6], v[8 * c4 + 7]) : 0u;
-            }
             if (use > 0 && !warp_wait(&empty_a[s], (use - 1) & 1, lane, abort_flag, p.status)) return false;
             const uint32_t sa = smem_u32(a_ring) + s * kABytes;
 #pragma unroll
@@ -440,8 +577,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++) {
             const uint32_t m0 = wk.mt * kBM;
             const uint32_t kb0 = wk.kb0, kb1 = wk.kb1;
-            const bool arow_live = m0 + arow < p.m;
-            const uint32_t wrow = min(m0 + arow, p.m - 1);
+            const uint32_t wrow = min(m0 + arow, p.m - 1);  // rows past the end repeat the last one; nobody stores them
             const uint8_t *wp = p.w + (size_t)wrow * p.row_bytes;
             // this group's first k-block: the one whose stage counter has its parity
             const uint32_t first = kb0 + (kGroups == 2 ? ((grp + it0) & 1) : 0);
@@ -454,9 +590,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                 if (first + kGroups < kb1) n1.load(wp, first + kGroups, ahalf);
                 for (uint32_t kb = first; kb < kb1; kb += kGroups) {
                     if (kb + 2 * kGroups < kb1) n2.load(wp, kb + 2 * kGroups, ahalf);
-                    float v[32];
-                    cur.decode(v, grid);
-                    if (!put(v, arow_live, it0 + (kb - kb0))) goto done;
+                    uint4 v[4];
+                    cur.template unpack<F16>(v, tab);
+                    if (!put(v, it0 + (kb - kb0))) goto done;
                     cur = n1;
                     n1 = n2;
                 }
@@ -465,9 +601,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                 if (first < kb1) cur.load(wp, first, ahalf);
                 for (uint32_t kb = first; kb < kb1; kb += kGroups) {
                     if (kb + kGroups < kb1) nxt.load(wp, kb + kGroups, ahalf);  // lands while cur is unpacked
-                    float v[32];
-                    cur.decode(v, grid);
-                    if (!put(v, arow_live, it0 + (kb - kb0))) goto done;
+                    uint4 v[4];
+                    cur.template unpack<F16>(v, tab);
+                    if (!put(v, it0 + (kb - kb0))) goto done;
                     cur = nxt;
                 }
             }
@@ -510,9 +646,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                     const uint32_t s = it % kBStages, use = it / kBStages;
                     if (use > 0 && !warp_wait(&empty_b[s], (use - 1) & 1, lane, abort_flag, p.status)) goto done;
                     uint8_t *sb = b_ring + (size_t)s * kBStage;
-#pragma unroll
+                    // only as many tokens as the MMA reads, in sixteens
+                    const uint32_t rows = (min(min(wk.ntok, p.n - n0), NACC * kBN) + 15u) & ~15u;
+#pragma unroll 4
                     for (uint32_t i = 0; i < kChunks; i++) {
                         const uint32_t q = t + kBWarps * 32 * i;
+                        if ((q >> 3) >= rows) break;
                         const uint32_t row = q >> 3, c16 = q & 7;  // row over NACC x 256 tokens; blocks are 32 KB apart
                         const uint32_t tok = n0 + row;
                         uint8_t *dst = sb + (row >> 8) * kBBytes + swz(row & 255, c16);
