@@ -28,6 +28,11 @@ struct okf_ctx {
     size_t stage_x_bytes;
     void *stage_out;
     size_t stage_out_bytes;
+    // ... and its host side for callers whose buffers are pageable: page-locked, mapped, up to kPinMax
+    void *pin_x;
+    size_t pin_x_bytes;
+    void *pin_out;
+    size_t pin_out_bytes;
     // scratch for the matmul's k-range partial sums, grown on demand
     void *scratch;
     size_t scratch_bytes;

@@ -58,6 +58,25 @@ cudaError_t launch_dequant(int ty, const uint8_t *w, uint64_t count, float *out,
     }
 }
 
+// ---- x of the host-buffer operator --------------------------------------------
+// A few kilobytes over PCIe.  The copy engine would take about 5 us before the kernel behind it may
+// start; this is one PCIe round trip, and the next kernel, launched ahead of its end, has its weights on
+// their way meanwhile.
+__global__ void __launch_bounds__(128) fetch_kernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst, size_t n) {
+    pdl_launch_dependents();
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    if (i < n) {
+        uint4 v;
+        asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src + i));
+        dst[i] = v;
+    }
+}
+
+cudaError_t launch_fetch(const void *host, void *dst, size_t n16, cudaStream_t s) {
+    return launch_pdl(fetch_kernel, (unsigned)((n16 + 127) / 128), 128, 0, s, 1, (const uint4 *)host, (uint4 *)dst, n16);
+}
+
 // ---- matvec, N <= 8 columns --------------------------------------------------
 // One warp per output row; lane l takes granules l, l+32, ...; fp32 FMAs; the
 // 32 lane partials are combined with shuffles.

@@ -326,7 +326,9 @@ OKF_API int okf_linear(okf_ctx *ctx, int type, const okf_weights *w, uint64_t wo
  * GQ.matmul (Gemma/Gemma4Quant.swift:150-170), QB.dequant (Base/Quant.swift:73-76).
  * x / out are HOST pointers to fp32; each call copies x to the device, runs the
  * kernel on the context's stream, copies the result back and waits for it.
- * Pinned host memory makes the copies asynchronous; pageable memory works. */
+ * Page-locked buffers are read and written by the kernels directly; pageable ones
+ * up to 1 MiB go through page-locked memory that the context keeps (at most 2 MiB
+ * of it each way), larger ones through the copy engine. */
 OKF_API int okf_matvec_host(okf_ctx *ctx, int type, const okf_weights *w, uint64_t woff, uint32_t k,
                     uint32_t m, const float *x, float *out);
 OKF_API int okf_matmul_host(okf_ctx *ctx, int type, const okf_weights *w, uint64_t woff, uint32_t k,
@@ -357,7 +359,8 @@ OKF_API int okf_device_status(okf_ctx *ctx, int *out);
 #define OKF_FLAG_SIMPLE_KERNELS 1u
 OKF_API int okf_set_flags(okf_ctx *ctx, uint32_t flags);
 
-/* Number of kernels this context has launched since it was created. */
+/* Number of kernels this context has launched since it was created (the one that
+ * fetches x for okf_matmul_host is part of a copy and not counted). */
 OKF_API uint64_t okf_launch_count(const okf_ctx *ctx);
 /* Number of calls that did not run on the main kernels because of their shape or
  * alignment: K not a multiple of 256 for the matvec (a slower form of it that
