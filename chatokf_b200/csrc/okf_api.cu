@@ -110,6 +110,23 @@ int par_flush(okf_ctx *ctx) {
     return e == cudaSuccess ? OKF_OK : cuda_fail(ctx, e);
 }
 
+// The buffer for bf16 copies of fp32 activations on stream `s`; null: convert inside the matmul.  While a
+// stream is captured there is none: graphs captured from one stream may be replayed side by side.
+void *conv_buffer(okf_ctx *ctx, cudaStream_t s, size_t need) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    for (auto &c : ctx->conv) {
+        if (c.buf && c.stream != s) continue;
+        if (grow(ctx, &c.buf, &c.bytes, need) != OKF_OK) return nullptr;
+        c.stream = s;
+        return c.buf;
+    }
+    return nullptr;
+}
+
 int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uint32_t k, uint32_t m,
                   const void *x, int xdt, uint32_t n, void *out, int odt, okf_stream stream,
                   bool force_tile) {
@@ -152,6 +169,16 @@ int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uin
             e = launch_gemv_simple(ty, wp, k, m, x, xdt, n, (float *)out, s);
         }
     } else if (!(ctx->flags & OKF_FLAG_SIMPLE_KERNELS) && gemm_tc_supported(ty, k, m, wp, x, xdt, n)) {
+        if (xdt == DT_F32) {
+            // every slab of W would convert all of X again, and by a quarter of the warps
+            if (void *b = conv_buffer(ctx, s, (size_t)n * k * 2)) {
+                e = launch_to_bf16(x, b, (size_t)n * k, ctx->sms, s);
+                if (e != cudaSuccess) return cuda_fail(ctx, e);
+                ctx->launches++;
+                x = b;
+                xdt = DT_BF16;
+            }
+        }
         uint32_t ksplit = gemm_tc_ksplit(k, m, n, xdt, ctx->sms);
         if (ksplit > 1) {
             // Growing the scratch allocates, which is not allowed while a stream is being
@@ -234,6 +261,8 @@ void okf_destroy(okf_ctx *ctx) {
     }
     if (ctx->dev_status) cudaFree(ctx->dev_status);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    for (auto &c : ctx->conv)
+        if (c.buf) cudaFree(c.buf);
     if (ctx->stage_x) cudaFree(ctx->stage_x);
     if (ctx->stage_out) cudaFree(ctx->stage_out);
     if (ctx->pin_x) cudaFreeHost(ctx->pin_x);

@@ -54,8 +54,8 @@ constexpr uint32_t kProducerWarps = kAWarps + kBWarps;
 constexpr uint32_t kTmaWarp = kProducerWarps;          // warp 16: one thread hands B tiles to the copy engine
 constexpr uint32_t kMmaWarp = kProducerWarps + 1;      // warp 17
 constexpr uint32_t kThreads = (kProducerWarps + 2 + 4) * 32;  // + four epilogue warps
-constexpr uint32_t kMaxRing = 4;                                      // stages a ring may have
-constexpr uint32_t kBarRegion = 256;                                  // barriers, tensor-memory slot, abort flag
+constexpr uint32_t kMaxRing = 12;                                     // stages the rings may have
+constexpr uint32_t kBarRegion = 512;                                  // barriers, tensor-memory slot, abort flag
 template <int TY, int NACC> struct Rings {
     static constexpr uint32_t a_stages = NACC == 2 ? 2 : 4;
     static constexpr uint32_t b_stages = NACC == 2 ? (TY == T_IQ2_XXS ? 2 : 3) : 4;
@@ -88,6 +88,8 @@ struct Args {
 // A parameter of its own: the main loops compile to slower code (fewer registers, 12 % less
 // throughput measured) when Args grows.
 struct Outs {
+    uint32_t a_stages, b_stages, b_stage;  // stages of the rings, bytes of a B tile
+    uint32_t box;  // tokens of a B tile as the tensor map copies it: 256, or fewer when there are fewer
     uint32_t nout, out_ld, out_row0;
     void *outs[8];
     uint32_t *epoch;      // the local count the exchange is complete at goes up by epoch_inc
@@ -492,9 +494,28 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, uint32
     if (lane == 0 && !mbar_try_wait(bar, parity)) ok = mbar_wait_parked(bar, parity, abort_flag, status);
     return __shfl_sync(0xffffffffu, ok, 0);
 }
-// a single thread (the MMA issuer, the copy engine's clients)
-__device__ __forceinline__ bool thread_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status) {
-    return mbar_try_wait(bar, parity) || mbar_wait_parked(bar, parity, abort_flag, status);
+// The MMA issuer and the copy engine's client: the whole warp waits and walks the loop, converged, and one
+// elected lane issues.  Inside a branch that only one lane takes, descriptors and addresses are not uniform
+// to the compiler, and every tcgen05 instruction becomes a loop over the warp's values: 640 cycles of
+// issue per k-block, which set the pace of all k-blocks with few tokens (0.65 us each, whatever the type).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ bool warp_poll(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 64; i++)
+            if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles)) break;
+    }
+    *abort_flag = 1;
+    if (status) atomicExch(status, kStatusGemmTimeout);
+    return false;
 }
 
 // NACC: token blocks (accumulators) per work item, 1 or 2.
@@ -505,21 +526,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     constexpr bool F16 = XDT == DT_F16;
     constexpr bool ASYNC_B = XDT != DT_F32;  // 16-bit activations come by TMA, fp32 ones are converted by eight warps
     using R = Rings<TY, NACC>;
-    constexpr uint32_t kAStages = R::a_stages, kBStages = R::b_stages, kBStage = R::b_stage;
+    const uint32_t kAStages = go.a_stages, kBStages = go.b_stages, kBStage = go.b_stage;
     constexpr uint32_t kGroups = ASYNC_B ? 2 : 1;  // groups of eight unpacking warps
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t *a_ring = smem, *b_ring = smem + R::a_bytes;
+    uint8_t *a_ring = smem, *b_ring = smem + kAStages * kABytes;
     uint32_t *tab = reinterpret_cast<uint32_t *>(smem + R::a_bytes + R::b_bytes);  // IQ2_XXS: 256 + 128 selector words
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + R::a_bytes + R::b_bytes + R::grid_bytes);
     uint64_t *full_a = bars, *empty_a = bars + kMaxRing;                    // A producers <-> MMA, one pair per A stage
-    uint64_t *full_b = bars + 2 * kMaxRing, *empty_b = bars + 3 * kMaxRing;  // B producer(s) <-> MMA, one pair per B stage
-    uint64_t *acc_full = bars + 4 * kMaxRing;  // MMA -> epilogue, one per accumulator
+    uint64_t *full_b = bars + 2 * kMaxRing, *empty_b = full_b + kMaxRing;  // B producer(s) <-> MMA, one pair per B stage
+    uint64_t *acc_full = empty_b + kMaxRing;  // MMA -> epilogue, one per accumulator
     uint64_t *acc_empty = acc_full + 2;        // epilogue -> MMA
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_full + 4);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;  // (uniform, and known to be)
+    pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kAStages; s++) {
             mbar_init(&full_a[s], kAWarps);
@@ -560,8 +582,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         uint32_t it0 = 0;  // stage counter at the start of the work item
         Work wk;
         // this thread's four 16-byte chunks -> stage s
-        auto put = [&](const uint4 (&q)[4], uint32_t it) -> bool {
-            const uint32_t s = it % kAStages, use = it / kAStages;
+        // (a group's stages follow each other across work items: every kGroups-th of the ring)
+        uint32_t s = grp, use = 0;
+        auto put = [&](const uint4 (&q)[4]) -> bool {
             if (use > 0 && !warp_wait(&empty_a[s], (use - 1) & 1, lane, abort_flag, p.status)) return false;
             const uint32_t sa = smem_u32(a_ring) + s * kABytes;
 #pragma unroll
@@ -569,9 +592,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sa + swz(arow, ARaw<TY>::chunk(ahalf, c4))), "r"(q[c4].x),
                              "r"(q[c4].y), "r"(q[c4].z), "r"(q[c4].w)
                              : "memory");
-            fence_proxy_async();  // generic-proxy writes -> visible to the tensor core's async proxy
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full_a[s]);
+            if (lane == 0) mbar_arrive(&full_a[s]);  // the MMA issuer fences these stores for the tensor core
+            s += kGroups;
+            if (s >= kAStages) {
+                s -= kAStages;
+                use++;
+            }
             return true;
         };
         for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++) {
@@ -592,7 +619,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                     if (kb + 2 * kGroups < kb1) n2.load(wp, kb + 2 * kGroups, ahalf);
                     uint4 v[4];
                     cur.template unpack<F16>(v, tab);
-                    if (!put(v, it0 + (kb - kb0))) goto done;
+                    if (!put(v)) goto done;
                     cur = n1;
                     n1 = n2;
                 }
@@ -603,23 +630,22 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                     if (kb + kGroups < kb1) nxt.load(wp, kb + kGroups, ahalf);  // lands while cur is unpacked
                     uint4 v[4];
                     cur.template unpack<F16>(v, tab);
-                    if (!put(v, it0 + (kb - kb0))) goto done;
+                    if (!put(v)) goto done;
                     cur = nxt;
                 }
             }
             it0 += kb1 - kb0;
         }
     } else if (warp == kTmaWarp) {
-        // ---------------- one thread hands the B tiles to the copy engine
-        if (ASYNC_B && lane == 0) {
-            // B tiles of 16-bit activations: NACC x 256 tokens x 64 k per stage
-            uint32_t it = 0;
+        // ---------------- hands the B tiles of 16-bit activations to the copy engine: NACC x 256 tokens x 64 k a stage
+        if constexpr (ASYNC_B) {
+            pdl_wait();  // x may come from the kernel before
+            uint32_t s = 0, use = 0;
             Work wk;
             for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++) {
                 const uint32_t nblk = wk.ntok > kBN ? NACC : 1;
-                for (uint32_t kb = wk.kb0; kb < wk.kb1; kb++, it++) {
-                    const uint32_t s = it % kBStages, use = it / kBStages;
-                    if (use > 0 && !thread_wait(&empty_b[s], (use - 1) & 1, abort_flag, p.status)) {
+                for (uint32_t kb = wk.kb0; kb < wk.kb1; kb++, s = s + 1 == kBStages ? (use++, 0) : s + 1) {
+                    if (use > 0 && !warp_poll(&empty_b[s], (use - 1) & 1, abort_flag, p.status)) {
                         // giving up: the copies already handed over land within microseconds;
                         // stay for a while so that they do not write into a CTA that has gone
                         const long long t0 = clock64();
@@ -627,9 +653,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                         goto done;
                     }
                     uint8_t *sb = b_ring + (size_t)s * kBStage;
-                    mbar_expect_tx(&full_b[s], nblk * kBBytes);
-                    for (uint32_t a = 0; a < nblk; a++)
-                        tma_load_tile(sb + a * kBBytes, &xmap, kb * kBK, wk.n0 + a * kBN, &full_b[s]);
+                    if (elect_one()) {
+                        mbar_expect_tx(&full_b[s], nblk * go.box * kBK * 2);
+                        for (uint32_t a = 0; a < nblk; a++)
+                            tma_load_tile(sb + a * kBBytes, &xmap, kb * kBK, wk.n0 + a * kBN, &full_b[s]);
+                    }
+                    __syncwarp();
                 }
             }
         }
@@ -638,12 +667,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         if constexpr (!ASYNC_B) {
             const uint32_t t = threadIdx.x - kAWarps * 32;  // 0..255
             constexpr uint32_t kChunks = NACC * kBN * 8 / (kBWarps * 32);  // 16-byte chunks per thread
-            uint32_t it = 0;
+            uint32_t s = 0, use = 0;
             Work wk;
+            pdl_wait();
             for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++) {
                 const uint32_t n0 = wk.n0;
-                for (uint32_t kb = wk.kb0; kb < wk.kb1; kb++, it++) {
-                    const uint32_t s = it % kBStages, use = it / kBStages;
+                for (uint32_t kb = wk.kb0; kb < wk.kb1; kb++, s = s + 1 == kBStages ? (use++, 0) : s + 1) {
                     if (use > 0 && !warp_wait(&empty_b[s], (use - 1) & 1, lane, abort_flag, p.status)) goto done;
                     uint8_t *sb = b_ring + (size_t)s * kBStage;
                     // only as many tokens as the MMA reads, in sixteens
@@ -665,17 +694,67 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                         }
                         *reinterpret_cast<uint4 *>(dst) = v;
                     }
-                    fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&full_b[s]);
                 }
             }
         }
     } else if (warp == kMmaWarp) {
-        // ---------------- MMA issuer: one thread.  Another lane of the warp asks L2 for the CTA's
-        // whole slab of W (128 contiguous rows) ahead of the producers, which then read it
-        // k-block by k-block, 32 bytes per row at a time.
-        if (lane == 1) {
+        // ---------------- MMA issuer
+        uint32_t tile = 0, s_a = 0, use_a = 0, s_b = 0, use_b = 0;
+        Work wk;
+        for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++, tile++) {
+            // N of the instruction: the tokens each block of the item really has, in sixteens
+            const uint32_t live = min(wk.ntok, p.n - wk.n0);
+            uint32_t idesc[NACC];
+#pragma unroll
+            for (uint32_t a = 0; a < (uint32_t)NACC; a++) {
+                const uint32_t nt = live > a * kBN ? min(live - a * kBN, kBN) : 0u;
+                idesc[a] = instr_desc(F16 ? 0u : 1u, kBM, nt ? (nt + 15u) & ~15u : 16u);
+            }
+            // accumulators: both for a two-block item, alternating for one-block items
+            const uint32_t acc0 = NACC == 2 ? 0 : (tile & 1), acc_use = NACC == 2 ? tile : (tile >> 1);
+            if (acc_use > 0)
+                for (uint32_t a = 0; a < (uint32_t)NACC; a++)
+                    if (!warp_poll(&acc_empty[acc0 + a], (acc_use - 1) & 1, abort_flag, p.status)) goto done;
+            tc_fence_after();
+            const uint32_t kb0 = wk.kb0, kb1 = wk.kb1;
+            for (uint32_t kb = kb0; kb < kb1; kb++, s_a = s_a + 1 == kAStages ? (use_a++, 0) : s_a + 1,
+                          s_b = s_b + 1 == kBStages ? (use_b++, 0) : s_b + 1) {
+                if (!warp_poll(&full_a[s_a], use_a & 1, abort_flag, p.status) ||
+                    !warp_poll(&full_b[s_b], use_b & 1, abort_flag, p.status))
+                    goto done;
+                // Generic-proxy stores (unpacked weights) -> visible to the tensor core's async proxy: the
+                // fence stands on the path from the stores over the barrier to the MMAs.  Here and not in
+                // the storing threads, where it also waits for their loads in flight, a round trip to L2
+                // or HBM on every turn.
+                fence_proxy_async();
+                tc_fence_after();
+                const uint64_t da = smem_desc(smem_u32(a_ring) + s_a * kABytes);
+                const uint64_t db = smem_desc(smem_u32(b_ring) + s_b * kBStage);
+                if (elect_one()) {
+#pragma unroll
+                    for (uint32_t a = 0; a < (uint32_t)NACC; a++)
+#pragma unroll
+                        for (uint32_t k4 = 0; k4 < kBK / 16; k4++)
+                            // 16 k = 32 bytes further along the swizzled 128-byte row
+                            umma(tmem_base + (acc0 + a) * kBN, da + (uint64_t)(k4 * 2), db + (uint64_t)(a * (kBBytes >> 4) + k4 * 2), idesc[a],
+                                 (kb != kb0 || k4 != 0) ? 1u : 0u);
+                    umma_commit(&empty_a[s_a]);  // both stages are free once these MMAs have read them
+                    umma_commit(&empty_b[s_b]);
+                }
+                __syncwarp();
+            }
+            if (elect_one())
+                for (uint32_t a = 0; a < (uint32_t)NACC; a++) umma_commit(&acc_full[acc0 + a]);
+            __syncwarp();
+        }
+    } else {
+        // ---------------- epilogue: four warps, warp q reads tensor-memory lanes 32q .. 32q + 31
+        const uint32_t q = warp & 3;  // a warp may only touch the lane quarter given by warp id % 4
+        if (warp == kMmaWarp + 1 && lane == 0) {
+            // nothing to do yet: asks L2 for the CTA's whole slabs of W (128 contiguous rows) ahead of the
+            // producers, which then read them k-block by k-block, 32 bytes per row at a time
             uint32_t last_mt = 0xFFFFFFFFu;
             Work wk;
             for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++) {
@@ -693,58 +772,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                 }
             }
         }
-        if (lane == 0) {
-            uint32_t it = 0, tile = 0;
-            Work wk;
-            for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++, tile++) {
-                // N of the instruction: the tokens each block of the item really has, in sixteens
-                const uint32_t live = min(wk.ntok, p.n - wk.n0);
-                uint32_t idesc[NACC];
-#pragma unroll
-                for (uint32_t a = 0; a < (uint32_t)NACC; a++) {
-                    const uint32_t nt = live > a * kBN ? min(live - a * kBN, kBN) : 0u;
-                    idesc[a] = instr_desc(F16 ? 0u : 1u, kBM, nt ? (nt + 15u) & ~15u : 16u);
-                }
-                // accumulators: both for a two-block item, alternating for one-block items
-                const uint32_t acc0 = NACC == 2 ? 0 : (tile & 1), acc_use = NACC == 2 ? tile : (tile >> 1);
-                bool ok = true;
-                for (uint32_t a = 0; a < (uint32_t)NACC && ok; a++)
-                    if (acc_use > 0) ok = thread_wait(&acc_empty[acc0 + a], (acc_use - 1) & 1, abort_flag, p.status);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t kb0 = wk.kb0, kb1 = wk.kb1;
-                for (uint32_t kb = kb0; kb < kb1; kb++, it++) {
-                    const uint32_t s_a = it % kAStages, s_b = it % kBStages;
-                    if (!thread_wait(&full_a[s_a], (it / kAStages) & 1, abort_flag, p.status) ||
-                        !thread_wait(&full_b[s_b], (it / kBStages) & 1, abort_flag, p.status)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t sb = smem_u32(b_ring + (size_t)s_b * kBStage);
-                    const uint64_t da = smem_desc(smem_u32(a_ring + (size_t)s_a * kABytes));
-#pragma unroll
-                    for (uint32_t a = 0; a < (uint32_t)NACC; a++) {
-                        const uint64_t db = smem_desc(sb + a * kBBytes);
-                        const uint32_t d_tmem = tmem_base + (acc0 + a) * kBN;
-#pragma unroll
-                        for (uint32_t k4 = 0; k4 < kBK / 16; k4++) {
-                            // 16 k = 32 bytes further along the swizzled 128-byte row
-                            umma(d_tmem, da + (uint64_t)(k4 * 2), db + (uint64_t)(k4 * 2), idesc[a], (kb != kb0 || k4 != 0) ? 1u : 0u);
-                        }
-                    }
-                    umma_commit(&empty_a[s_a]);  // both stages are free once these MMAs have read them
-                    umma_commit(&empty_b[s_b]);
-                }
-                if (!ok) break;
-                for (uint32_t a = 0; a < (uint32_t)NACC; a++) umma_commit(&acc_full[acc0 + a]);
-            }
-        }
-    } else {
-        // ---------------- epilogue: four warps, warp q reads tensor-memory lanes 32q .. 32q + 31
-        const uint32_t q = warp & 3;  // a warp may only touch the lane quarter given by warp id % 4
+        __syncwarp();
         uint32_t tile = 0;
         Work wk;
+        pdl_wait();  // the kernel before may still read what is written here
         for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++, tile++) {
             const uint32_t mt = wk.mt, n0 = wk.n0;
             const uint32_t n_end = min(p.n, n0 + wk.ntok);
@@ -802,7 +833,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     }
 done:
     if constexpr (kIsGather<OT>)
-        if (p.ksplit == 1 && blockIdx.x == 0 && threadIdx.x == 0) go.epoch[0] += go.epoch_inc;
+        if (p.ksplit == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
+            pdl_wait();
+            go.epoch[0] += go.epoch_inc;
+        }
     tc_fence_before();
     __syncthreads();
     if (warp == kMmaWarp) {
@@ -822,6 +856,8 @@ struct ReduceOut {
 template <typename OT>
 __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ part, ReduceOut o, size_t count,
                                                             uint32_t ksplit) {
+    pdl_launch_dependents();
+    pdl_wait();
     const size_t stride = (size_t)gridDim.x * blockDim.x * 4;
     const bool vec = (o.m & 3) == 0 && (o.out_ld & 3) == 0 && (o.out_row0 & 3) == 0;
     for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < count; i += stride) {
@@ -881,9 +917,9 @@ static cudaError_t encode_map_2d(CUtensorMap *map, bool bytes, const void *base,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
-// the activations X[n][k], 16-bit elements: 64 k x 256 tokens per copy, swizzled as the MMA reads them
-static cudaError_t encode_x_map(CUtensorMap *map, const void *x, uint32_t k, uint32_t n) {
-    return encode_map_2d(map, false, x, k, n, (uint64_t)k * 2, kBK, kBN, true);
+// the activations X[n][k], 16-bit elements: 64 k x `box` tokens per copy, swizzled as the MMA reads them
+static cudaError_t encode_x_map(CUtensorMap *map, const void *x, uint32_t k, uint32_t n, uint32_t box) {
+    return encode_map_2d(map, false, x, k, n, (uint64_t)k * 2, kBK, box, true);
 }
 template <int TY, int XDT, typename OT, int NACC>
 static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int sms, int dev) {
@@ -898,19 +934,31 @@ static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int s
     const uint32_t grid = items < (uint32_t)sms ? items : (uint32_t)sms;  // a tail split always has items > sms
     alignas(64) CUtensorMap xmap;
     memset(&xmap, 0, sizeof(xmap));
+    Outs g = go;
+    // The B ring holds what is on its way from L2, so its depth sets the pace where a k-block is little work:
+    // tiles as large as the tokens present, as many as fit.  (Four stages whatever N: 0.65 us per k-block.)
+    g.box = a.n < kBN ? (a.n + 15) & ~15u : kBN;
+    g.b_stage = XDT == DT_F32 ? kBBytes : NACC * g.box * kBK * 2;
+    if (NACC == 2) {
+        g.a_stages = Rings<TY, NACC>::a_stages;
+        g.b_stages = Rings<TY, NACC>::b_stages;
+    } else {
+        const uint32_t both = (Rings<TY, NACC>::a_bytes + Rings<TY, NACC>::b_bytes) / (kABytes + g.b_stage);
+        g.a_stages = g.b_stages = both < kMaxRing ? both : kMaxRing;
+    }
     if constexpr (XDT != DT_F32) {
-        cudaError_t me = encode_x_map(&xmap, a.x, a.k, a.n);
+        cudaError_t me = encode_x_map(&xmap, a.x, a.k, a.n, g.box);
         if (me != cudaSuccess) return me;
     }
-    gemm_tc_kernel<TY, XDT, OT, NACC><<<grid, kThreads, Rings<TY, NACC>::smem, s>>>(xmap, a, go);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pdl(gemm_tc_kernel<TY, XDT, OT, NACC>, grid, kThreads, Rings<TY, NACC>::smem, s, 1, xmap, a, g);
     if (e != cudaSuccess || a.ksplit == 1) return e;
     const size_t count = (size_t)a.n * a.m;
     ReduceOut ro = {go.nout, a.m, go.out_ld, go.out_row0, {}, go.epoch, go.epoch_inc};
     for (uint32_t o = 0; o < go.nout; o++) ro.outs[o] = go.outs[o];
     using RT = std::conditional_t<kIsGather<OT>, float, OT>;
-    splitk_reduce_kernel<RT><<<sms * 4, 256, 0, s>>>(a.partial, ro, count, a.ksplit);
-    return cudaGetLastError();
+    const size_t blocks = (count + 1023) / 1024, most = (size_t)sms * 4;
+    return launch_pdl(splitk_reduce_kernel<RT>, (unsigned)(blocks < most ? blocks : most), 256, 0, s, 1, (const float *)a.partial, ro,
+                      count, a.ksplit);
 }
 
 template <int TY, int XDT, typename OT>
@@ -940,6 +988,20 @@ static cudaError_t launch_x(const Args &a, const Outs &go, uint32_t nacc, int xd
 }
 
 }  // namespace tc
+
+// fp32 activations -> bf16, once for all slabs, so that they come by TMA like the others.
+__global__ void __launch_bounds__(256) to_bf16_kernel(const float4 *__restrict__ x, uint4 *__restrict__ y, size_t n8) {
+    pdl_launch_dependents();
+    pdl_wait();
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
+        const float4 a = x[2 * i], b = x[2 * i + 1];
+        y[i] = make_uint4(tc::pack16<false>(a.x, a.y), tc::pack16<false>(a.z, a.w), tc::pack16<false>(b.x, b.y), tc::pack16<false>(b.z, b.w));
+    }
+}
+cudaError_t launch_to_bf16(const void *x, void *y, size_t count, int sms, cudaStream_t s) {
+    const size_t blocks = (count / 8 + 255) / 256, most = (size_t)sms * 8;
+    return launch_pdl(to_bf16_kernel, (unsigned)(blocks < most ? blocks : most), 256, 0, s, 1, (const float4 *)x, (uint4 *)y, count / 8);
+}
 
 // How to lay a matmul over the SMs.  A work item is a 128-row slab against one
 // or two 256-token blocks over all of K or, with a split, over one of ksplit

@@ -36,6 +36,13 @@ struct okf_ctx {
     // scratch for the matmul's k-range partial sums, grown on demand
     void *scratch;
     size_t scratch_bytes;
+    // bf16 copies of fp32 activations, one buffer per stream (calls on different streams may overlap),
+    // grown on demand; calls on further streams convert inside the matmul
+    struct {
+        cudaStream_t stream;
+        void *buf;
+        size_t bytes;
+    } conv[4];
     // staged faults (host side only)
     double fault_rate;
     uint64_t fault_state;

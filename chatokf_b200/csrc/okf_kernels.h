@@ -89,6 +89,8 @@ bool gemm_tc_supported(int ty, uint32_t k, uint32_t m, const void *w, const void
 // (ksplit * n * m floats) and are summed by a second kernel; gemm_tc_ksplit
 // proposes a split for a shape.
 uint32_t gemm_tc_ksplit(uint32_t k, uint32_t m, uint32_t n, int xdt, int sms);
+// count (a multiple of 8) floats at a 16-byte boundary to bf16.
+cudaError_t launch_to_bf16(const void *x, void *y, size_t count, int sms, cudaStream_t s);
 // `gather` (may be null): row shards, as for the matvec; results go to every rank's whole
 // output (seg[0]) instead of `out`.
 cudaError_t launch_gemm_tc(int ty, const uint8_t *w, uint32_t k, uint32_t m, const void *x, int xdt,
