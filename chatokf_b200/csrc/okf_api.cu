@@ -110,21 +110,43 @@ int par_flush(okf_ctx *ctx) {
     return e == cudaSuccess ? OKF_OK : cuda_fail(ctx, e);
 }
 
-// The buffer for bf16 copies of fp32 activations on stream `s`; null: convert inside the matmul.  While a
-// stream is captured there is none: graphs captured from one stream may be replayed side by side.
-void *conv_buffer(okf_ctx *ctx, cudaStream_t s, size_t need) {
+// Launch the tensor-core matmul with what stream `s` may use of the context's working memory.  While a
+// stream is captured nothing can be allocated: what calls outside the capture have left has to do.
+cudaError_t run_tile(okf_ctx *ctx, int ty, const uint8_t *wp, uint32_t k, uint32_t m, const void *x, int xdt, uint32_t n,
+                     void *out, int odt, cudaStream_t s, const GemvGatherPlan *gather) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-        (void)cudaGetLastError();
-        return nullptr;
+    (void)cudaStreamIsCapturing(s, &cs);
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    okf_ctx::Lane *lane = nullptr, *unused = nullptr, *largest = nullptr;
+    for (auto &l : ctx->lanes) {
+        if (l.used && l.stream == s) lane = &l;
+        if (!l.used && !unused) unused = &l;
+        if (l.used && (!largest || l.part_bytes + l.conv_bytes > largest->part_bytes + largest->conv_bytes)) largest = &l;
     }
-    for (auto &c : ctx->conv) {
-        if (c.buf && c.stream != s) continue;
-        if (grow(ctx, &c.buf, &c.bytes, need) != OKF_OK) return nullptr;
-        c.stream = s;
-        return c.buf;
+    if (!lane && capturing) lane = largest;
+    if (!lane && !capturing && unused) {
+        lane = unused;
+        lane->used = true;
+        lane->stream = s;
     }
-    return nullptr;
+    const size_t cb = (size_t)n * k * 2;
+    if (lane && xdt == DT_F32 && !gather) {
+        if (!capturing) (void)grow(ctx, &lane->conv, &lane->conv_bytes, cb);
+        if (lane->conv_bytes >= cb) {
+            // every slab of W would convert all of X again, and by a part of the warps
+            cudaError_t e = launch_to_bf16(x, lane->conv, (size_t)n * k, ctx->sms, s);
+            if (e != cudaSuccess) return e;
+            ctx->launches++;
+            x = lane->conv;
+            xdt = DT_BF16;
+        }
+    }
+    if (lane && !capturing) {
+        const size_t need = gemm_tc_scratch(ty, k, m, n, xdt, ctx->sms) * sizeof(float);
+        if (need) (void)grow(ctx, &lane->part, &lane->part_bytes, need);  // without it another plan is taken
+    }
+    return launch_gemm_tc(ty, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, lane ? (float *)lane->part : nullptr,
+                          lane ? lane->part_bytes / sizeof(float) : 0, s, ctx->sms, ctx->device, &ctx->launches, gather);
 }
 
 int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uint32_t k, uint32_t m,
@@ -169,31 +191,8 @@ int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uin
             e = launch_gemv_simple(ty, wp, k, m, x, xdt, n, (float *)out, s);
         }
     } else if (!(ctx->flags & OKF_FLAG_SIMPLE_KERNELS) && gemm_tc_supported(ty, k, m, wp, x, xdt, n)) {
-        if (xdt == DT_F32) {
-            // every slab of W would convert all of X again, and by a quarter of the warps
-            if (void *b = conv_buffer(ctx, s, (size_t)n * k * 2)) {
-                e = launch_to_bf16(x, b, (size_t)n * k, ctx->sms, s);
-                if (e != cudaSuccess) return cuda_fail(ctx, e);
-                ctx->launches++;
-                x = b;
-                xdt = DT_BF16;
-            }
-        }
-        uint32_t ksplit = gemm_tc_ksplit(k, m, n, xdt, ctx->sms);
-        if (ksplit > 1) {
-            // Growing the scratch allocates, which is not allowed while a stream is being
-            // captured into a graph: size it with one call outside the capture first.
-            const size_t need = (size_t)ksplit * n * m * sizeof(float);
-            if (ctx->scratch_bytes < need) {
-                cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-                (void)cudaStreamIsCapturing(s, &cs);
-                if (cs != cudaStreamCaptureStatusNone) ksplit = 1;
-                else if ((rc = grow(ctx, &ctx->scratch, &ctx->scratch_bytes, need))) return rc;
-            }
-        }
-        e = launch_gemm_tc(ty, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, ksplit, (float *)ctx->scratch, s,
-                           ctx->sms, ctx->device, nullptr);
-        if (e == cudaSuccess && ksplit > 1) ctx->launches++;
+        e = run_tile(ctx, ty, wp, k, m, x, xdt, n, out, odt, s, nullptr);
+        return e == cudaSuccess ? OKF_OK : cuda_fail(ctx, e);
     } else {
         if (!(ctx->flags & OKF_FLAG_SIMPLE_KERNELS)) ctx->fallbacks++;
         e = launch_gemm_simple(ty, wp, k, m, x, xdt, n, out, odt, s);
@@ -260,9 +259,10 @@ void okf_destroy(okf_ctx *ctx) {
         cudaStreamDestroy(ctx->stream);
     }
     if (ctx->dev_status) cudaFree(ctx->dev_status);
-    if (ctx->scratch) cudaFree(ctx->scratch);
-    for (auto &c : ctx->conv)
-        if (c.buf) cudaFree(c.buf);
+    for (auto &l : ctx->lanes) {
+        if (l.part) cudaFree(l.part);
+        if (l.conv) cudaFree(l.conv);
+    }
     if (ctx->stage_x) cudaFree(ctx->stage_x);
     if (ctx->stage_out) cudaFree(ctx->stage_out);
     if (ctx->pin_x) cudaFreeHost(ctx->pin_x);
@@ -466,20 +466,8 @@ int okf_gemm_gather(okf_ctx *ctx, int type, const okf_weights *w, uint64_t woff,
             if (e != cudaSuccess) return cuda_fail(ctx, e);
             ctx->launches++;
         }
-        uint32_t ksplit = gemm_tc_ksplit(k, m, n, xdt, ctx->sms);
-        if (ksplit > 1) {
-            const size_t need = (size_t)ksplit * n * m * sizeof(float);
-            if (ctx->scratch_bytes < need) {
-                cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-                (void)cudaStreamIsCapturing(s, &cs);
-                if (cs != cudaStreamCaptureStatusNone) ksplit = 1;
-                else if ((rc = grow(ctx, &ctx->scratch, &ctx->scratch_bytes, need))) return rc;
-            }
-        }
-        cudaError_t e = launch_gemm_tc(type, wp, k, m, x, xdt, n, nullptr, DT_F32, ctx->dev_status, ksplit,
-                                       (float *)ctx->scratch, s, ctx->sms, ctx->device, &plan);
+        cudaError_t e = run_tile(ctx, type, wp, k, m, x, xdt, n, nullptr, DT_F32, s, &plan);
         if (e != cudaSuccess) return cuda_fail(ctx, e);
-        ctx->launches += ksplit > 1 ? 2 : 1;
         return OKF_OK;
     }
     if (!gemv_fast_supported(type, k, m, wp, x, xdt, n, ctx->sms)) return OKF_E_ALIGN;

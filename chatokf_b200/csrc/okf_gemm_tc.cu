@@ -36,6 +36,22 @@
 
 namespace okf {
 
+// How a matmul is laid over the SMs.  A work item is a 128-row slab against one or two 256-token blocks
+// over all of K.  Full waves of items run whole, one item per CTA and wave.  What is left after them, or a
+// matmul of less than a wave, either runs whole too, on part of the SMs, or is dealt out: its k-blocks
+// laid end to end are cut into one run per CTA, pieces of items leave as fp32 partial tiles, and a
+// second kernel sums them.  The plan with the smallest estimated time wins.  The estimate, measured on
+// B200: a CTA spends 0.93 us per k-block on an item of two token blocks and 0.45 - 0.55 us on one of one
+// block (Q8_0 and Q6_K, whose rows take more loads to unpack, 1.15 and 0.8); an item of two blocks, which
+// uses all of tensor memory, exposes 3 us of epilogue; dealing costs 4 us of launch and hand-over, and
+// partial tiles move at 8 TB/s, mostly through L2.  (4096 tokens 17408 -> 5120: 320 items of two blocks
+// are 2.16 waves; three whole waves took 760 us, two and 24 dealt items 590.)
+struct GemmPlan {
+    uint32_t nacc;   // token blocks per item
+    uint32_t waves, dealt, dealers, nt;  // see tc::Args
+    size_t floats;   // of partial tiles
+};
+
 namespace tc {
 
 constexpr uint32_t kBM = 128;           // weight rows per CTA tile (UMMA M)
@@ -77,11 +93,11 @@ struct Args {
     int *status;
     uint32_t k, m, n;
     uint32_t row_bytes;
-    uint32_t ksplit;   // work items per (slab, token group): each takes a range of k-blocks
-    float *partial;    // ksplit > 1: fp32 partial results [ksplit][n][m], summed by a second kernel
-    // ksplit == 1: the last tail_items (slab, token block) items -- what is left after
-    // the full waves -- are cut into tail_parts runs of tail_tok tokens, one per CTA
-    uint32_t tail_items, tail_tok, tail_parts;
+    uint32_t waves;    // whole items every CTA takes before the dealt ones
+    uint32_t dealt;    // items whose k-blocks are dealt out evenly (0: all items are whole) ...
+    uint32_t dealers;  // ... over this many of the CTAs; every one of them gets some
+    uint32_t nt;       // tokens of a partial tile
+    float *partial;    // dealt items: fp32 partial tiles [part][dealt item][nt][128], summed by a second kernel
 };
 // Row shards: where results go instead of Args::out.  `nout` buffers (every rank's copy of
 // the whole output as mapped here), element (token, row) at [token * out_ld + out_row0 + row].
@@ -98,42 +114,42 @@ struct Outs {
 
 // One piece of work of a CTA: rows [mt * 128, +128) x tokens [n0, n0 + ntok) x k-blocks [kb0, kb1).
 struct Work {
-    uint32_t mt, n0, ntok, kb0, kb1, part;
+    uint32_t mt, n0, ntok, kb0, kb1;
+    uint32_t slot;  // which partial tile it is: part * dealt + item; kWhole: it is all of K and goes to the output
 };
+constexpr uint32_t kWhole = 0xFFFFFFFFu;
+
+// Dealing: CTA c takes k-blocks [total * c / ctas, total * (c + 1) / ctas) of the dealt items laid end to
+// end.  The CTA that takes k-block x (total * ctas stays below 2^32):
+__host__ __device__ __forceinline__ uint32_t dealt_to(uint32_t x, uint32_t total, uint32_t ctas) { return ((x + 1) * ctas - 1) / total; }
 
 // The j-th piece of work of this CTA; false when there is none.  Whole items go
-// round-robin over the CTAs; with a tail split every CTA then takes one run of
-// tokens of one of the left-over items (NACC == 1 only).
+// round-robin over the CTAs, then every CTA takes its run of the dealt k-blocks, item after item.
 template <int NACC>
 __device__ __forceinline__ bool next_work(const Args &p, uint32_t j, Work &w) {
-    const uint32_t m_tiles = (p.m + kBM - 1) / kBM;
     const uint32_t n_groups = (p.n + NACC * kBN - 1) / (NACC * kBN);
-    const uint32_t kblocks = p.k / kBK;
-    const uint32_t base = m_tiles * n_groups;
-    const uint32_t item = blockIdx.x + j * gridDim.x;
-    if (p.ksplit > 1) {  // k-range fastest, then token group, then slab
-        if (item >= base * p.ksplit) return false;
-        w.mt = item / (n_groups * p.ksplit);
-        w.n0 = ((item / p.ksplit) % n_groups) * (NACC * kBN);
-        w.ntok = NACC * kBN;
-        w.part = item % p.ksplit;
-        w.kb0 = (uint32_t)((uint64_t)kblocks * w.part / p.ksplit);
-        w.kb1 = (uint32_t)((uint64_t)kblocks * (w.part + 1) / p.ksplit);
-        return true;
+    const uint32_t base = ((p.m + kBM - 1) / kBM) * n_groups, kblocks = p.k / kBK;
+    uint32_t item;
+    w.ntok = NACC * kBN;
+    w.slot = kWhole;
+    w.kb0 = 0;
+    w.kb1 = kblocks;
+    if (!p.dealt || j < p.waves) {
+        item = blockIdx.x + j * gridDim.x;
+        if (item >= base) return false;
+    } else {
+        const uint32_t total = p.dealt * kblocks;
+        if (blockIdx.x >= p.dealers) return false;
+        const uint32_t lo = total * blockIdx.x / p.dealers, hi = total * (blockIdx.x + 1) / p.dealers;
+        const uint32_t i = lo / kblocks + (j - p.waves), start = max(lo, i * kblocks), end = min(hi, (i + 1) * kblocks);
+        if (start >= end) return false;
+        w.kb0 = start - i * kblocks;
+        w.kb1 = end - i * kblocks;
+        if (w.kb1 - w.kb0 < kblocks) w.slot = (blockIdx.x - dealt_to(i * kblocks, total, p.dealers)) * p.dealt + i;
+        item = base - p.dealt + i;
     }
-    w.part = 0; w.kb0 = 0; w.kb1 = kblocks;
-    const uint32_t whole = p.tail_tok ? base - p.tail_items : base;  // a multiple of the grid when there is a tail
-    if (item < whole) {
-        w.mt = item / n_groups;
-        w.n0 = (item % n_groups) * (NACC * kBN);
-        w.ntok = NACC * kBN;
-        return true;
-    }
-    if (!p.tail_tok || j != whole / gridDim.x || blockIdx.x >= p.tail_items * p.tail_parts) return false;
-    const uint32_t t_item = whole + blockIdx.x / p.tail_parts;
-    w.mt = t_item / n_groups;
-    w.n0 = (t_item % n_groups) * (NACC * kBN) + (blockIdx.x % p.tail_parts) * p.tail_tok;
-    w.ntok = p.tail_tok;
+    w.mt = item / n_groups;
+    w.n0 = (item % n_groups) * (NACC * kBN);
     return true;
 }
 
@@ -754,7 +770,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         const uint32_t q = warp & 3;  // a warp may only touch the lane quarter given by warp id % 4
         if (warp == kMmaWarp + 1 && lane == 0) {
             // nothing to do yet: asks L2 for the CTA's whole slabs of W (128 contiguous rows) ahead of the
-            // producers, which then read them k-block by k-block, 32 bytes per row at a time
+            // producers, which then read them k-block by k-block, 32 bytes per row at a time.  (Asking only
+            // for the k-range of dealt items, row by row, made short launches 2 us slower.)
             uint32_t last_mt = 0xFFFFFFFFu;
             Work wk;
             for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++) {
@@ -781,7 +798,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
             const uint32_t n_end = min(p.n, n0 + wk.ntok);
             const uint32_t acc0 = NACC == 2 ? 0 : (tile & 1), acc_use = NACC == 2 ? tile : (tile >> 1);
             const uint32_t row = mt * kBM + q * 32 + lane;
-            float *part = p.ksplit > 1 ? p.partial + (size_t)wk.part * p.n * p.m : nullptr;
+            // partial tiles hold all 128 rows
+            float *part = wk.slot != kWhole ? p.partial + (size_t)wk.slot * p.nt * kBM - (size_t)n0 * kBM + q * 32 + lane : nullptr;
             for (uint32_t a = 0; a < (uint32_t)NACC; a++) {
                 const uint32_t acc = acc0 + a;
                 if (!warp_wait(&acc_full[acc], acc_use & 1, lane, abort_flag, p.status)) goto done;
@@ -792,7 +810,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                     uint32_t r[32];
                     tmem_ld32(tmem_base + ((q * 32) << 16) + acc * kBN + c0, r);
                     tmem_ld_wait();
-                    if (row < p.m) {
+                    if (part) {
+#pragma unroll
+                        for (int j = 0; j < 32; j++) {
+                            const uint32_t tok = n0 + a * kBN + c0 + j;
+                            if (tok < n_end) part[(size_t)tok * kBM] = __uint_as_float(r[j]);
+                        }
+                    } else if (row < p.m) {
                         if constexpr (!kIsGather<OT>) {
                             OT *out = reinterpret_cast<OT *>(p.out);
 #pragma unroll
@@ -800,16 +824,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                                 const uint32_t tok = n0 + a * kBN + c0 + j;
                                 if (tok < n_end) {
                                     const float f = __uint_as_float(r[j]);
-                                    if (part) part[(size_t)tok * p.m + row] = f;
-                                    else if constexpr (sizeof(OT) == 4) out[(size_t)tok * p.m + row] = f;
+                                    if constexpr (sizeof(OT) == 4) out[(size_t)tok * p.m + row] = f;
                                     else out[(size_t)tok * p.m + row] = __float2bfloat16_rn(f);
                                 }
-                            }
-                        } else if (part) {
-#pragma unroll
-                            for (int j = 0; j < 32; j++) {
-                                const uint32_t tok = n0 + a * kBN + c0 + j;
-                                if (tok < n_end) part[(size_t)tok * p.m + row] = __uint_as_float(r[j]);
                             }
                         } else {
                             // row shards: a warp stores 32 consecutive rows of one token (128 bytes) into
@@ -833,7 +850,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     }
 done:
     if constexpr (kIsGather<OT>)
-        if (p.ksplit == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
+        if (!p.dealt && blockIdx.x == 0 && threadIdx.x == 0) {
             pdl_wait();
             go.epoch[0] += go.epoch_inc;
         }
@@ -845,50 +862,54 @@ done:
     }
 }
 
-// Sum the k-range partials in a fixed order: out[i] = part[0][i] + part[1][i] + ..., element
-// i = token * m + row going to [token * out_ld + out_row0 + row] of every output buffer.
+// Sum the partial tiles of the dealt items, part after part (the order of k), into every output buffer:
+// element (token, row) at [token * out_ld + out_row0 + row].  A block takes 16 tokens of an item, a thread
+// four rows of one token at a time.
 struct ReduceOut {
-    uint32_t nout, m, out_ld, out_row0;
+    uint32_t nout, m, n, out_ld, out_row0;
+    uint32_t dealt, base, kblocks, ctas, nt, groups, group_tok;  // the main kernel's dealing
     void *outs[8];
     uint32_t *epoch;
     uint32_t epoch_inc;
 };
+constexpr uint32_t kReduceTok = 16;
 template <typename OT>
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ part, ReduceOut o, size_t count,
-                                                            uint32_t ksplit) {
+__global__ void __launch_bounds__(256) reduce_kernel(const float *__restrict__ part, ReduceOut o) {
     pdl_launch_dependents();
+    const uint32_t runs = (o.nt + kReduceTok - 1) / kReduceTok;
+    const uint32_t i = blockIdx.x / runs, t0 = blockIdx.x % runs * kReduceTok, total = o.dealt * o.kblocks;
+    const uint32_t c0 = dealt_to(i * o.kblocks, total, o.ctas), c1 = dealt_to((i + 1) * o.kblocks - 1, total, o.ctas);
+    const uint32_t item = o.base - o.dealt + i, n0 = item % o.groups * o.group_tok;
+    const uint32_t r = (threadIdx.x & 31) * 4, row = item / o.groups * kBM + r;
     pdl_wait();
-    const size_t stride = (size_t)gridDim.x * blockDim.x * 4;
-    const bool vec = (o.m & 3) == 0 && (o.out_ld & 3) == 0 && (o.out_row0 & 3) == 0;
-    for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < count; i += stride) {
-        if (vec) {  // four rows of one token
-            float4 s = *reinterpret_cast<const float4 *>(part + i);
-            for (uint32_t k = 1; k < ksplit; k++) {
-                const float4 v = *reinterpret_cast<const float4 *>(part + k * count + i);
-                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-            }
-            const size_t at = o.out_ld == o.m ? i : (i / o.m) * o.out_ld + o.out_row0 + i % o.m;
-            for (uint32_t b = 0; b < o.nout; b++) {
-                if constexpr (sizeof(OT) == 4) *reinterpret_cast<float4 *>(reinterpret_cast<float *>(o.outs[b]) + at) = s;
-                else {
-                    __nv_bfloat16 *out = reinterpret_cast<__nv_bfloat16 *>(o.outs[b]) + at;
-                    out[0] = __float2bfloat16_rn(s.x); out[1] = __float2bfloat16_rn(s.y);
-                    out[2] = __float2bfloat16_rn(s.z); out[3] = __float2bfloat16_rn(s.w);
-                }
-            }
-        } else {
-            for (size_t e = i; e < count && e < i + 4; e++) {
-                float s = part[e];
-                for (uint32_t k = 1; k < ksplit; k++) s += part[k * count + e];
-                const size_t at = o.out_ld == o.m ? e : (e / o.m) * o.out_ld + o.out_row0 + e % o.m;
-                for (uint32_t b = 0; b < o.nout; b++) {
-                    if constexpr (sizeof(OT) == 4) reinterpret_cast<float *>(o.outs[b])[at] = s;
-                    else reinterpret_cast<__nv_bfloat16 *>(o.outs[b])[at] = __float2bfloat16_rn(s);
-                }
+    if (o.epoch && blockIdx.x == 0 && threadIdx.x == 0) o.epoch[0] += o.epoch_inc;
+    if (c0 == c1) return;  // one CTA took the whole item and stored it
+    const bool vec = (o.m & 3) == 0 && (o.out_ld & 3) == 0 && (o.out_row0 & 3) == 0 && sizeof(OT) == 4;
+    for (uint32_t t = t0 + (threadIdx.x >> 5); t < min(t0 + kReduceTok, o.nt); t += 8) {
+        if (n0 + t >= o.n || row >= o.m) break;
+        const float *src = part + ((size_t)i * o.nt + t) * kBM + r;
+        const size_t step = (size_t)o.dealt * o.nt * kBM;
+        float4 v = *reinterpret_cast<const float4 *>(src);
+        for (uint32_t c = c0 + 1; c <= c1; c++) {
+            const float4 a = *reinterpret_cast<const float4 *>(src + (c - c0) * step);
+            v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+        }
+        const size_t at = (size_t)(n0 + t) * o.out_ld + o.out_row0 + row;
+        const float e[4] = {v.x, v.y, v.z, v.w};
+        for (uint32_t b = 0; b < o.nout; b++) {
+            OT *out = reinterpret_cast<OT *>(o.outs[b]) + at;
+            if (vec) {
+                *reinterpret_cast<float4 *>(out) = v;
+            } else {
+#pragma unroll
+                for (uint32_t j = 0; j < 4; j++)
+                    if (row + j < o.m) {
+                        if constexpr (sizeof(OT) == 4) out[j] = e[j];
+                        else out[j] = __float2bfloat16_rn(e[j]);
+                    }
             }
         }
     }
-    if (o.epoch && blockIdx.x == 0 && threadIdx.x == 0) o.epoch[0] += o.epoch_inc;
 }
 
 // Tensor maps for tma_load_tile.  The driver's encoder is looked up once; nothing is linked
@@ -930,8 +951,8 @@ static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int s
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    const uint32_t items = ((a.m + kBM - 1) / kBM) * ((a.n + NACC * kBN - 1) / (NACC * kBN)) * a.ksplit;
-    const uint32_t grid = items < (uint32_t)sms ? items : (uint32_t)sms;  // a tail split always has items > sms
+    const uint32_t groups = (a.n + NACC * kBN - 1) / (NACC * kBN), items = ((a.m + kBM - 1) / kBM) * groups;
+    const uint32_t grid = a.waves ? (uint32_t)sms : a.dealt ? a.dealers : items < (uint32_t)sms ? items : (uint32_t)sms;
     alignas(64) CUtensorMap xmap;
     memset(&xmap, 0, sizeof(xmap));
     Outs g = go;
@@ -951,38 +972,36 @@ static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int s
         if (me != cudaSuccess) return me;
     }
     cudaError_t e = launch_pdl(gemm_tc_kernel<TY, XDT, OT, NACC>, grid, kThreads, Rings<TY, NACC>::smem, s, 1, xmap, a, g);
-    if (e != cudaSuccess || a.ksplit == 1) return e;
-    const size_t count = (size_t)a.n * a.m;
-    ReduceOut ro = {go.nout, a.m, go.out_ld, go.out_row0, {}, go.epoch, go.epoch_inc};
+    if (e != cudaSuccess || !a.dealt) return e;
+    ReduceOut ro = {go.nout, a.m, a.n, go.out_ld, go.out_row0, a.dealt, items, a.k / kBK, a.dealers, a.nt, groups, NACC * kBN, {}, go.epoch,
+                    go.epoch_inc};
     for (uint32_t o = 0; o < go.nout; o++) ro.outs[o] = go.outs[o];
     using RT = std::conditional_t<kIsGather<OT>, float, OT>;
-    const size_t blocks = (count + 1023) / 1024, most = (size_t)sms * 4;
-    return launch_pdl(splitk_reduce_kernel<RT>, (unsigned)(blocks < most ? blocks : most), 256, 0, s, 1, (const float *)a.partial, ro,
-                      count, a.ksplit);
+    return launch_pdl(reduce_kernel<RT>, a.dealt * ((a.nt + kReduceTok - 1) / kReduceTok), 256, 0, s, 1, (const float *)a.partial, ro);
 }
 
 template <int TY, int XDT, typename OT>
-static cudaError_t launch(const Args &a, const Outs &go, uint32_t nacc, cudaStream_t s, int sms, int dev) {
+static cudaError_t launch(const Args &a, const Outs &go, const GemmPlan &plan, cudaStream_t s, int sms, int dev) {
     if constexpr (XDT != DT_F32) {
-        if (nacc == 2) return launch_n<TY, XDT, OT, 2>(a, go, s, sms, dev);
+        if (plan.nacc == 2) return launch_n<TY, XDT, OT, 2>(a, go, s, sms, dev);
     }
     return launch_n<TY, XDT, OT, 1>(a, go, s, sms, dev);
 }
 
 template <int TY, int XDT>
-static cudaError_t launch_o(const Args &a, const Outs &go, uint32_t nacc, int odt, cudaStream_t s, int sms, int dev) {
-    if (odt == DT_F32 && go.epoch) return launch<TY, XDT, GatherF32>(a, go, nacc, s, sms, dev);
-    if (odt == DT_F32) return launch<TY, XDT, float>(a, go, nacc, s, sms, dev);
-    if (odt == DT_BF16) return launch<TY, XDT, __nv_bfloat16>(a, go, nacc, s, sms, dev);
+static cudaError_t launch_o(const Args &a, const Outs &go, const GemmPlan &plan, int odt, cudaStream_t s, int sms, int dev) {
+    if (odt == DT_F32 && go.epoch) return launch<TY, XDT, GatherF32>(a, go, plan, s, sms, dev);
+    if (odt == DT_F32) return launch<TY, XDT, float>(a, go, plan, s, sms, dev);
+    if (odt == DT_BF16) return launch<TY, XDT, __nv_bfloat16>(a, go, plan, s, sms, dev);
     return cudaErrorInvalidValue;
 }
 
 template <int TY>
-static cudaError_t launch_x(const Args &a, const Outs &go, uint32_t nacc, int xdt, int odt, cudaStream_t s, int sms, int dev) {
+static cudaError_t launch_x(const Args &a, const Outs &go, const GemmPlan &plan, int xdt, int odt, cudaStream_t s, int sms, int dev) {
     switch (xdt) {
-    case DT_F16: return launch_o<TY, DT_F16>(a, go, nacc, odt, s, sms, dev);
-    case DT_BF16: return launch_o<TY, DT_BF16>(a, go, nacc, odt, s, sms, dev);
-    case DT_F32: return launch_o<TY, DT_F32>(a, go, nacc, odt, s, sms, dev);
+    case DT_F16: return launch_o<TY, DT_F16>(a, go, plan, odt, s, sms, dev);
+    case DT_BF16: return launch_o<TY, DT_BF16>(a, go, plan, odt, s, sms, dev);
+    case DT_F32: return launch_o<TY, DT_F32>(a, go, plan, odt, s, sms, dev);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -1003,54 +1022,41 @@ cudaError_t launch_to_bf16(const void *x, void *y, size_t count, int sms, cudaSt
     return launch_pdl(to_bf16_kernel, (unsigned)(blocks < most ? blocks : most), 256, 0, s, 1, (const float4 *)x, (uint4 *)y, count / 8);
 }
 
-// How to lay a matmul over the SMs.  A work item is a 128-row slab against one
-// or two 256-token blocks over all of K or, with a split, over one of ksplit
-// k-ranges whose fp32 partial results a second kernel sums (ksplit * n * m floats
-// of scratch).  Without a split and with more items than SMs, the items left
-// after the full waves can be cut into short runs of tokens, one per CTA,
-// instead of costing a whole extra wave.  The plan with the smallest estimated
-// time wins.  The estimate: a CTA spends 1.04 us per k-block on an item of two
-// token blocks and 0.73 us on one of one block (the unpacking of the slab, not
-// the MMAs, sets the pace of a single block), a run of tokens costs no less than
-// 0.55 us per k-block, and the partial sums are written and read back at 5 TB/s
-// (figures measured on B200 with Q4_K weights).
-struct GemmPlan {
-    uint32_t nacc, ksplit, tail_items, tail_tok, tail_parts;
-};
-
-static GemmPlan gemm_tc_plan(uint32_t k, uint32_t m, uint32_t n, int xdt, int sms, uint32_t force_ksplit) {
-    const uint32_t slabs = (m + tc::kBM - 1) / tc::kBM, kblocks = k / tc::kBK;
-    GemmPlan best = {1, force_ksplit > 1 ? force_ksplit : 1, 0, 0, 0};
+static GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms, size_t max_floats) {
+    const uint32_t slabs = (m + tc::kBM - 1) / tc::kBM, kblocks = k / tc::kBK, all = (uint32_t)sms;
+    GemmPlan best = {};
     double best_t = 1e30;
     for (uint32_t nacc = 1; nacc <= 2; nacc++) {
         if (nacc == 2 && (xdt == DT_F32 || n <= tc::kBN)) continue;
-        const double t_kb = nacc == 2 ? 1.04e-6 : 0.73e-6;
+        const bool slow = ty == T_Q8_0 || ty == T_Q6_K;
+        const double t_kb = nacc == 2 ? (slow ? 1.15e-6 : 0.93e-6) : (slow ? 0.8e-6 : 0.45e-6 + 0.4e-9 * (n < tc::kBN ? n : tc::kBN));
         const uint32_t base = slabs * ((n + nacc * tc::kBN - 1) / (nacc * tc::kBN));
-        for (uint32_t ks = 1; ks <= 8; ks++) {
-            if (force_ksplit ? ks != force_ksplit : (ks > 1 && kblocks / ks < 8)) continue;
-            if (ks > kblocks) continue;
-            const uint32_t items = base * ks, waves = (items + sms - 1) / sms;
-            const double per_item = (double)((kblocks + ks - 1) / ks) * t_kb;
-            const double t_red = ks > 1 ? (2.0 * ks + 1) * n * (double)m * 4 / 5e12 : 0.0;
-            const double t = waves * per_item + t_red;
-            if (t < best_t) { best_t = t; best = {nacc, ks, 0, 0, 0}; }
-            if (ks == 1 && nacc == 1 && base > (uint32_t)sms && base % sms) {
-                const uint32_t full_waves = base / sms, left = base % sms;
-                uint32_t tok = 16;
-                while (left * (tc::kBN / tok) > (uint32_t)sms) tok *= 2;
-                const double run = t_kb * tok / tc::kBN;
-                const double t2 = full_waves * per_item + kblocks * (run > 0.55e-6 ? run : 0.55e-6);
-                if (t2 < best_t) { best_t = t2; best = {1, 1, left, tok, tc::kBN / tok}; }
-            }
+        const double whole = ((base + all - 1) / all) * (kblocks * t_kb + (nacc == 2 ? 3e-6 : 0));
+        if (whole < best_t) { best_t = whole; best = {nacc, 0, 0, 0, 0, 0}; }
+        // the items of the last, part-filled wave (of the only one) dealt out by k-blocks
+        const uint32_t waves = base / all, dealt = base % all, nt = n < nacc * tc::kBN ? n : nacc * tc::kBN;
+        if (dealt == 0) continue;
+        const uint64_t total = (uint64_t)dealt * kblocks;
+        if (total * (all + 1) >= 0xFFFFFFFFull) continue;
+        const uint32_t ctas = total / 4 < all ? (uint32_t)(total / 4) : all;  // four k-blocks at least
+        if (ctas <= dealt) continue;
+        uint32_t parts = 1;
+        for (uint32_t i = 0; i < dealt; i++) {
+            const uint32_t c = tc::dealt_to((i + 1) * kblocks - 1, (uint32_t)total, ctas) - tc::dealt_to(i * kblocks, (uint32_t)total, ctas) + 1;
+            if (c > parts) parts = c;
         }
+        const size_t floats = (size_t)parts * dealt * nt * tc::kBM;
+        if (floats > max_floats) continue;
+        const double moved = 2.0 * (dealt + ctas) * nt * tc::kBM * 4;
+        const double t = waves * (kblocks * t_kb + (nacc == 2 ? 3e-6 : 0)) + (double)total / ctas * t_kb + 4e-6 + moved / 8e12;
+        if (t < best_t) { best_t = t; best = {nacc, waves, dealt, ctas, nt, floats}; }
     }
     return best;
 }
 
-uint32_t gemm_tc_ksplit(uint32_t k, uint32_t m, uint32_t n, int xdt, int sms) {
-    return gemm_tc_plan(k, m, n, xdt, sms, 0).ksplit;
+size_t gemm_tc_scratch(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms) {
+    return gemm_tc_plan(ty, k, m, n, xdt, sms, kMaxScratchFloats).floats;
 }
-
 bool gemm_tc_supported(int ty, uint32_t k, uint32_t m, const void *w, const void *x, int xdt, uint32_t n) {
     if (!has_fast_kernels(ty)) return false;
     if (k % 64 || m == 0 || n == 0) return false;
@@ -1060,8 +1066,8 @@ bool gemm_tc_supported(int ty, uint32_t k, uint32_t m, const void *w, const void
 }
 
 cudaError_t launch_gemm_tc(int ty, const uint8_t *w, uint32_t k, uint32_t m, const void *x, int xdt,
-                           uint32_t n, void *out, int odt, int *status, uint32_t ksplit, float *partial,
-                           cudaStream_t s, int sms, int dev, const GemvGatherPlan *gather) {
+                           uint32_t n, void *out, int odt, int *status, float *partial, size_t partial_floats,
+                           cudaStream_t s, int sms, int dev, uint64_t *launches, const GemvGatherPlan *gather) {
     tc::Args a = {};
     a.w = w; a.x = x; a.out = out; a.status = status; a.k = k; a.m = m; a.n = n;
     tc::Outs go = {};
@@ -1076,21 +1082,20 @@ cudaError_t launch_gemm_tc(int ty, const uint8_t *w, uint32_t k, uint32_t m, con
     } else {
         go.nout = 1; go.out_ld = m; go.out_row0 = 0; go.outs[0] = out;
     }
-    // the caller decides whether there is a split (it owns the scratch); the rest is planned here
-    const GemmPlan plan = gemm_tc_plan(k, m, n, xdt, sms, ksplit > 1 && partial ? ksplit : 1);
-    a.ksplit = plan.ksplit;
+    const GemmPlan plan = gemm_tc_plan(ty, k, m, n, xdt, sms, partial ? partial_floats : 0);
+    a.waves = plan.waves; a.dealt = plan.dealt; a.dealers = plan.dealers; a.nt = plan.nt;
     a.partial = partial;
-    a.tail_items = plan.tail_items; a.tail_tok = plan.tail_tok; a.tail_parts = plan.tail_parts;
+    *launches += plan.dealt ? 2 : 1;
     a.row_bytes = (k / block_elems(ty)) * block_bytes(ty);
     switch (ty) {
-    case T_Q4_K: return tc::launch_x<T_Q4_K>(a, go, plan.nacc, xdt, odt, s, sms, dev);
-    case T_Q8_0: return tc::launch_x<T_Q8_0>(a, go, plan.nacc, xdt, odt, s, sms, dev);
-    case T_Q4_0: return tc::launch_x<T_Q4_0>(a, go, plan.nacc, xdt, odt, s, sms, dev);
-    case T_Q6_K: return tc::launch_x<T_Q6_K>(a, go, plan.nacc, xdt, odt, s, sms, dev);
-    case T_Q5_K: return tc::launch_x<T_Q5_K>(a, go, plan.nacc, xdt, odt, s, sms, dev);
-    case T_IQ4_NL: return tc::launch_x<T_IQ4_NL>(a, go, plan.nacc, xdt, odt, s, sms, dev);
-    case T_Q2_0: return tc::launch_x<T_Q2_0>(a, go, plan.nacc, xdt, odt, s, sms, dev);
-    case T_IQ2_XXS: return tc::launch_x<T_IQ2_XXS>(a, go, plan.nacc, xdt, odt, s, sms, dev);
+    case T_Q4_K: return tc::launch_x<T_Q4_K>(a, go, plan, xdt, odt, s, sms, dev);
+    case T_Q8_0: return tc::launch_x<T_Q8_0>(a, go, plan, xdt, odt, s, sms, dev);
+    case T_Q4_0: return tc::launch_x<T_Q4_0>(a, go, plan, xdt, odt, s, sms, dev);
+    case T_Q6_K: return tc::launch_x<T_Q6_K>(a, go, plan, xdt, odt, s, sms, dev);
+    case T_Q5_K: return tc::launch_x<T_Q5_K>(a, go, plan, xdt, odt, s, sms, dev);
+    case T_IQ4_NL: return tc::launch_x<T_IQ4_NL>(a, go, plan, xdt, odt, s, sms, dev);
+    case T_Q2_0: return tc::launch_x<T_Q2_0>(a, go, plan, xdt, odt, s, sms, dev);
+    case T_IQ2_XXS: return tc::launch_x<T_IQ2_XXS>(a, go, plan, xdt, odt, s, sms, dev);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -1101,7 +1106,7 @@ cudaError_t launch_gemm_tc(int ty, const uint8_t *w, uint32_t k, uint32_t m, con
 // okf_gemm_noalloc serves callers that must not allocate device memory while they
 // run: code inside a CUDA-graph capture or a real-time decode loop, a process that
 // shares the GPU under a fixed memory budget, a plugin host that forbids cudaMalloc
-// after start-up.  The split-K matmul normally takes its partial-sum buffer from
+// after start-up.  A matmul with dealt items normally takes its buffer of partial tiles from
 // the context, which grows it with cudaMalloc on demand; here the buffer is a
 // fixed array that is part of the loaded library image instead.
 namespace okf {
@@ -1121,13 +1126,8 @@ extern "C" int okf_gemm_noalloc(okf_ctx *ctx, int type, const okf_weights *w, ui
     if (rc) return rc;
     const uint8_t *wp = w->dptr + woff;
     if (!gemm_tc_supported(type, k, m, wp, x, xdt, n)) return OKF_E_ALIGN;
-    // at least two k-ranges, so the scratch really carries the partial sums
     if (k / tc::kBK < 2) return OKF_E_SHAPE;
-    uint32_t ksplit = gemm_tc_ksplit(k, m, n, xdt, ctx->sms);
-    if (ksplit < 2) ksplit = 2;
-    const size_t per_split = (size_t)n * m;
-    if (2 * per_split > kStaticScratchFloats) return OKF_E_LIMIT;  // N * M above 2 Mi outputs
-    while (ksplit * per_split > kStaticScratchFloats) ksplit--;
+    if (2 * (size_t)n * m > kStaticScratchFloats) return OKF_E_LIMIT;  // N * M above 2 Mi outputs
     if (fault_fires(ctx)) return OKF_E_INJECTED;
     DeviceGuard g(ctx->device);
     if (!g.ok) return cuda_fail(ctx, cudaErrorInvalidDevice);
@@ -1139,11 +1139,10 @@ extern "C" int okf_gemm_noalloc(okf_ctx *ctx, int type, const okf_weights *w, ui
         if (e != cudaSuccess) return cuda_fail(ctx, e);
         g_static_scratch_addr[ctx->device] = ptr;
     }
-    // every (k-range, token, row) slot the reduction reads is written by the main kernel
-    // first, so nothing in the array has to be cleared between calls
-    cudaError_t e = launch_gemm_tc(type, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, ksplit,
-                                   g_static_scratch_addr[ctx->device], (cudaStream_t)stream, ctx->sms, ctx->device, nullptr);
+    // every slot the reduction reads is written by the main kernel first, so nothing in the
+    // array has to be cleared between calls
+    cudaError_t e = launch_gemm_tc(type, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, g_static_scratch_addr[ctx->device],
+                                   kStaticScratchFloats, (cudaStream_t)stream, ctx->sms, ctx->device, &ctx->launches, nullptr);
     if (e != cudaSuccess) return cuda_fail(ctx, e);
-    ctx->launches += 2;
     return OKF_OK;
 }

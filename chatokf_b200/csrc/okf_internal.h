@@ -33,16 +33,15 @@ struct okf_ctx {
     size_t pin_x_bytes;
     void *pin_out;
     size_t pin_out_bytes;
-    // scratch for the matmul's k-range partial sums, grown on demand
-    void *scratch;
-    size_t scratch_bytes;
-    // bf16 copies of fp32 activations, one buffer per stream (calls on different streams may overlap),
-    // grown on demand; calls on further streams convert inside the matmul
-    struct {
+    // what the tensor-core matmul works in, one set per stream (calls on different streams may
+    // overlap), grown on demand: partial tiles and bf16 copies of fp32 activations.  Calls on
+    // further streams do without.
+    struct Lane {
         cudaStream_t stream;
-        void *buf;
-        size_t bytes;
-    } conv[4];
+        bool used;
+        void *part, *conv;
+        size_t part_bytes, conv_bytes;
+    } lanes[16];
     // staged faults (host side only)
     double fault_rate;
     uint64_t fault_state;

@@ -1,0 +1,66 @@
+"""The tensor-core matmul's ways of laying work over the SMs, at their edges: less than a wave dealt out by
+k-blocks (one slab, many slabs, few k-blocks, more CTAs than pieces), whole waves with a dealt rest, two
+token blocks per item with a ragged last one, heights that are no multiple of four, both output types."""
+import numpy as np
+import pytest
+import torch
+
+from chatokf_b200 import synth
+from chatokf_b200.enc import CudaEnc, GGUFTensor
+from chatokf_b200.gguf_types import GGUFType, block_elems
+from helpers import rel_err
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(256, 128, 9), (1024, 129, 33), (2560, 9728, 77), (9728, 2563, 20), (17408, 130, 300), (1536, 19001, 40),
+          (768, 19400, 513), (4096, 5120, 1300), (512, 40000, 260), (64 * 5, 7000, 100)]
+
+
+@pytest.mark.parametrize("k,m,n", SHAPES)
+@pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
+def test_dealing(ctx, k, m, n, odt):
+    """Against the fp32 tile kernel with exact decode: fp16 operands rounded once, 2^-12 each, bf16 results
+    another 2^-9.  Twice in a row, the second time with the first call's partial tiles in the buffer."""
+    ty = GGUFType.Q4_0
+    rng = np.random.default_rng(k + m + n)
+    w = ctx.upload(synth.random_blocks(ty, m * k // block_elems(ty), rng))
+    t = GGUFTensor("w", (k, m), ty)
+    enc = CudaEnc(ctx)
+    want = torch.empty(n * m, device="cuda")
+    for seed in range(2):
+        X = torch.randn(n, k, device="cuda", generator=torch.Generator("cuda").manual_seed(seed)).half()
+        got = torch.full((n * m + 8,), float("nan"), dtype=odt, device="cuda")
+        enc.gemm(t, X, got, w, n)
+        ctx.set_flags(1)
+        try:
+            enc.gemm(t, X, want, w, n)
+        finally:
+            ctx.set_flags(0)
+        torch.cuda.synchronize()
+        assert torch.isnan(got[n * m:]).all(), "wrote past the N * M outputs"
+        tol = 1e-3 + (4e-3 if odt == torch.bfloat16 else 0.0)
+        assert rel_err(got[:n * m].float().cpu().numpy(), want.cpu().numpy()) <= tol
+    assert ctx.device_status() == 0
+
+
+def test_streams_do_not_share_partial_tiles(ctx):
+    """Calls of one context on several streams at once, more streams than the context has buffers for."""
+    ty, k, m, n = GGUFType.Q4_K, 4096, 1000, 40
+    rng = np.random.default_rng(1)
+    w = ctx.upload(synth.random_blocks(ty, m * k // block_elems(ty), rng))
+    t = GGUFTensor("w", (k, m), ty)
+    X = [torch.randn(n, k, device="cuda") for _ in range(6)]
+    want = [torch.empty(n, m, device="cuda") for _ in X]
+    got = [torch.empty(n, m, device="cuda") for _ in X]
+    for x, o in zip(X, want):
+        CudaEnc(ctx).gemm(t, x, o, w, n)
+    streams = [torch.cuda.Stream() for _ in X]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for s, x, o in zip(streams, X, got):
+            CudaEnc(ctx, s).gemm(t, x, o, w, n)
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        # fp32 sums in another order at most (streams beyond the buffers take another plan)
+        assert rel_err(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5
+    assert ctx.device_status() == 0
