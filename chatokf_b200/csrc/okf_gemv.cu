@@ -703,20 +703,6 @@ __device__ __forceinline__ void stage_x_wide(uint32_t xs32, uint32_t es, uint32_
         }
     }
 }
-template <int TY, int MODE>
-__device__ __forceinline__ void stage_x(int xdt, uint32_t xs32, uint32_t es, uint32_t info32, const void *x, uint32_t kdim, uint32_t ncols,
-                                        uint32_t u_first, uint32_t nu, uint32_t tid) {
-    if constexpr (MODE == M_SEP) {
-        if (xdt == DT_F32) stage_x_bytes<TY, DT_F32>(xs32, es, x, u_first, nu, tid);
-        else if (xdt == DT_F16) stage_x_bytes<TY, DT_F16>(xs32, es, x, u_first, nu, tid);
-        else stage_x_bytes<TY, DT_BF16>(xs32, es, x, u_first, nu, tid);
-    } else {
-        if (xdt == DT_F32) stage_x_wide<TY, MODE, DT_F32>(xs32, es, info32, x, kdim, ncols, u_first, nu, tid);
-        else if (xdt == DT_F16) stage_x_wide<TY, MODE, DT_F16>(xs32, es, info32, x, kdim, ncols, u_first, nu, tid);
-        else stage_x_wide<TY, MODE, DT_BF16>(xs32, es, info32, x, kdim, ncols, u_first, nu, tid);
-    }
-}
-
 // ---- the kernel ---------------------------------------------------------------------
 // Position in the ring of stages; the producer and the consumers step through it
 // in the same order, so both keep one of these.
@@ -730,7 +716,10 @@ struct RingPos {
 #ifndef OKF_GEMV_MINB
 #define OKF_GEMV_MINB 2
 #endif
-template <int TY, int MODE>
+// XDT: element type of x.  CL: launched in clusters.  (Both were run-time once: the code a launch does not
+// need costs instruction-cache misses that every CTA's staging waits for; Q2_0 2048 -> 2048 3.12 us, so 2.8,
+// Q6_K 2560 -> 151936 90.5, so 85.8.)
+template <int TY, int MODE, int XDT, bool CL>
 __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(GemvArgs p, GemvLayout L, GemvGather G) {
     constexpr uint32_t UB = UnitGeom<TY>::bytes;
     constexpr bool SEP = MODE == M_SEP;
@@ -746,11 +735,12 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
     // the cluster's tiles and this CTA's units of them
-    const uint32_t rank = blockIdx.x & ((1u << L.clog) - 1), cid = blockIdx.x >> L.clog, ncl = gridDim.x >> L.clog;
+    const uint32_t clog = CL ? L.clog : 0;
+    const uint32_t rank = blockIdx.x & ((1u << clog) - 1), cid = blockIdx.x >> clog, ncl = gridDim.x >> clog;
     const uint32_t t0 = (uint32_t)((uint64_t)p.tiles * cid / ncl);
     const uint32_t t1 = (uint32_t)((uint64_t)p.tiles * (cid + 1) / ncl);
     const uint32_t ntl = t1 - t0;
-    const uint32_t ubeg = p.nunit * rank >> L.clog, nun = (p.nunit * (rank + 1) >> L.clog) - ubeg;
+    const uint32_t ubeg = p.nunit * rank >> clog, nun = (p.nunit * (rank + 1) >> clog) - ubeg;
     const uint32_t spt = L.mode == 1 ? 2 : 1;  // stages per step (two half-tiles in mode 1)
 
     pdl_launch_dependents();
@@ -788,6 +778,8 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
         // ---- producer: weights do not depend on the previous kernel, so it does not wait for it.
         // One thread waits and counts; copies of whole rows are its own, those of row segments are
         // issued by sixteen lanes, one row each (a bulk copy takes its thread some 50 ns).
+        if (L.mode != 2 && lane != 0) return;
+        const uint32_t all = L.mode != 2 ? 1u : 0xffffffffu;  // the lanes that are left
         RingPos rp;
         uint32_t issued = 0;
         for (uint32_t gb = 0; gb < ntl; gb += L.group) {
@@ -801,7 +793,7 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                         bool ok = true;
                         if (rp.use > 0 && lane == 0)
                             ok = mbar_wait_relaxed(&empty[rp.s], (rp.use - 1) & 1, abort_flag, p.status, kStatusEmptyTimeout);
-                        if (!__shfl_sync(0xffffffffu, ok, 0)) {
+                        if (!__shfl_sync(all, ok, 0)) {
                             if (lane != 0) return;
                             // giving up: let the copies already issued land before the CTA goes away
                             const uint32_t first = issued > L.nstage ? issued - L.nstage : 0;
@@ -923,7 +915,8 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
             if (gb == 0 || L.panel < p.nchunk) {
                 // the previous panel is still being read until every warp gets here
                 if (gb > 0 || j0 > 0) consumer_sync();
-                stage_x<TY, MODE>(p.xdt, smem32 + L.xs_off, L.es, smem32 + L.info_off, p.x, p.k, L.nc, ubeg + pu0, pnu, tid);
+                if constexpr (SEP) stage_x_bytes<TY, XDT>(smem32 + L.xs_off, L.es, p.x, ubeg + pu0, pnu, tid);
+                else stage_x_wide<TY, MODE, XDT>(smem32 + L.xs_off, L.es, smem32 + L.info_off, p.x, p.k, L.nc, ubeg + pu0, pnu, tid);
             }
             consumer_sync();
             for (uint32_t j = j0; j < j1; j++) {
@@ -952,10 +945,15 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                     // start of a row's segment is skipped
                     const uint32_t top = stages32 + sA * L.stage_bytes;
                     const uint32_t low = L.mode == 1 ? stages32 + sB * L.stage_bytes : top + 8 * L.rs;
-                    auto skew = [&](uint32_t row) {
-                        if (!(L.mode == 2 && L.ragged)) return 0u;
-                        return (uint32_t)((size_t)min((t0 + tl - sg.tile0) * 16 + row, sg.m - 1) * p.row_bytes + (size_t)(ubeg + u0) * UB) & 15u;
-                    };
+                    uint32_t ra = top + g * L.rs, wdelta = low - top;  // row g; to row g + 8
+                    if (L.mode == 2 && L.ragged) {
+                        auto skew = [&](uint32_t row) {
+                            return (uint32_t)((size_t)min((t0 + tl - sg.tile0) * 16 + row, sg.m - 1) * p.row_bytes + (size_t)(ubeg + u0) * UB) & 15u;
+                        };
+                        const uint32_t s0 = skew(g);
+                        ra += s0;
+                        wdelta += skew(g + 8) - s0;
+                    }
                     const uint32_t tile_bytes = 16 * L.rs;
                     // Integer instructions run at half the rate of the others on this part and the
                     // unit bodies are full of them, so a warp takes a run of consecutive units of the
@@ -971,7 +969,6 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                     uint32_t ti = 0, u = wr * share + min(wr, extra);
                     while (u >= nu && ti + 1 < tn) { u -= nu; ti++; }
                     if constexpr (SEP) {
-                        const uint32_t ra = top + g * L.rs + skew(g), wdelta = low + g * L.rs + skew(g + 8) - ra;  // row g, to row g + 8
                         uint32_t wa = ra + ti * tile_bytes + (ubase + u) * UB;
                         uint32_t xa = xbase32 + (pu + u) * xstride32;
                         uint32_t ia = rec32 + (pu + u) * kSepUnit;
@@ -1008,8 +1005,7 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                         }
                     } else {
                         constexpr int NV = W::vals;
-                        uint32_t wa = top + ti * tile_bytes + (ubase + u) * UB + g * L.rs + skew(g);               // row g
-                        const uint32_t wdelta = low + g * L.rs + skew(g + 8) - (top + g * L.rs + skew(g));  // to row g + 8
+                        uint32_t wa = ra + ti * tile_bytes + (ubase + u) * UB;
                         while (left) {
                             const uint32_t run = min(left, nu - u);
                             left -= run;
@@ -1082,7 +1078,7 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
             for (uint32_t i = tid >> 4; i < gn * (SEP ? 1u : L.nc); i += kConsumers / 16) {
                 const uint32_t tl = SEP ? i : i * L.nc_inv >> 16, col = SEP ? 0u : i - tl * L.nc;
                 const float sum = total(tl, tid & 15, col);
-                if (L.clog) {
+                if constexpr (CL) {
                     part[((gb + tl) * L.nc + col) * 16 + (tid & 15)] = sum;  // this CTA's share of K
                     continue;
                 }
@@ -1114,15 +1110,15 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
         }
         if (gb + L.group < ntl) consumer_sync();  // before the buffer is zeroed again
     }
-    if (L.clog) {
+    if constexpr (CL) {
         // The cluster's CTAs have the same tiles: each adds up every so many-th (tile, column), in rank
         // order, reading the others' shares from their shared memory, and stores it.
         namespace cg = cooperative_groups;
         cg::cluster_group cl = cg::this_cluster();
         cl.sync();
-        for (uint32_t j = ((tid >> 4) << L.clog) + rank; j < ntl * L.nc; j += kConsumers / 16 << L.clog) {
+        for (uint32_t j = ((tid >> 4) << clog) + rank; j < ntl * L.nc; j += kConsumers / 16 << clog) {
             float sum = 0.f;
-            for (uint32_t q = 0; q < 1u << L.clog; q++) sum += cl.map_shared_rank(part, q)[j * 16 + (tid & 15)];
+            for (uint32_t q = 0; q < 1u << clog; q++) sum += cl.map_shared_rank(part, q)[j * 16 + (tid & 15)];
             const uint32_t tl = j / L.nc, col = j - tl * L.nc;
             const GemvSeg sg = gemv_segment(p, t0 + tl);
             const uint32_t row = (t0 + tl - sg.tile0) * 16 + (tid & 15);
@@ -1165,10 +1161,7 @@ static bool gemv_layout_with(int ty, uint32_t row_bytes, uint32_t nunit, uint32_
     const uint32_t ecols = sep ? 2 : n * (rag ? 3 : 2);  // byte columns of the x panel
     const uint32_t units = (nunit + csize - 1) / csize;   // the most a CTA of a cluster takes
     const uint32_t per_tile = kGemvWarps * 16 * L.nc * 4;
-    L.group = (sep ? 8192 : 16384) / per_tile;
-    if (L.group < 1) L.group = 1;
-    if (L.group > tiles_per_cta) L.group = tiles_per_cta;
-    const uint32_t red_bytes = L.group * per_tile, part_bytes = csize > 1 ? tiles_per_cta * 16 * L.nc * 4 : 0;
+    const uint32_t part_bytes = csize > 1 ? tiles_per_cta * 16 * L.nc * 4 : 0;
     const uint32_t tab_bytes = ty == T_IQ2_XXS ? 384 * 4 * tab_copies : 0;
     L.tab_copies = tab_copies;
     const uint32_t stage_cap = 46 * 1024;
@@ -1177,8 +1170,12 @@ static bool gemv_layout_with(int ty, uint32_t row_bytes, uint32_t nunit, uint32_
     GemvArgs fb_a = a;
     GemvLayout fb_L = L;
     bool have_fallback = false;
-    // One candidate; true when it is taken.
-    auto consider = [&](uint32_t kind, uint32_t tps, uint32_t nchunk) {
+    // One candidate; true when it is taken.  `red`: bytes of partial sums, a group of tiles.
+    auto consider_with = [&](uint32_t kind, uint32_t tps, uint32_t nchunk, uint32_t red) {
+        L.group = red / per_tile;
+        if (L.group < tps) L.group = tps;
+        if (L.group > tiles_per_cta) L.group = tiles_per_cta;
+        const uint32_t red_bytes = L.group * per_tile;
         L.mode = kind;
         L.tps = tps;
         L.ragged = 0;
@@ -1234,6 +1231,12 @@ static bool gemv_layout_with(int ty, uint32_t row_bytes, uint32_t nunit, uint32_
         // not stages a slice per k-chunk, every time with all warps waiting.
         if (panel == nchunk) return true;
         if (!have_fallback) { fb_a = a; fb_L = L; have_fallback = true; }
+        return false;
+    };
+    // with fewer tiles to a group where that makes room for the plan
+    auto consider = [&](uint32_t kind, uint32_t tps, uint32_t nchunk) {
+        for (uint32_t red = sep ? 8192 : 16384; red >= (sep ? 8192u : 4096u); red /= 2)
+            if (consider_with(kind, tps, nchunk, red)) return true;
         return false;
     };
     // Candidate plans, best first: whole tiles, several per stage while they are small and the CTA
@@ -1316,16 +1319,22 @@ static bool gemv_layout(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, 
 // by side, and they do not slow each other down much (a CTA alone issues on a third of the cycles).
 // (One column only: with several columns two CTAs on an SM, each staging its slices of x at
 // barriers, were 16 % slower than two tiles in a row.)
-// From eight tiles per SM on, two CTAs share every SM: eight warps wait for one another's
-// instructions on two thirds of the cycles, sixteen fill them (Q4_K 2560 -> 65536 22.3 -> 18.5 us,
-// Q8_0 2048 -> 65536 37.2 -> 25.2, IQ2_XXS 5120 -> 34816 31.1 -> 27.7, four columns 73.7 -> 63.1).
-// Below that the second panel of x and the lost room for the next launch's first copies cost as
-// much as they gain (Q4_K 2560 -> 9728, four tiles per SM: 6.0 us both ways).
-constexpr uint32_t kTwoCtasTiles = 8;
-static uint32_t gemv_ctas(uint32_t tiles, int sms, bool sep) {
+// Where an SM has enough to do, two CTAs share it: eight warps wait for one another's instructions on two
+// thirds of the cycles, sixteen fill them; against that stand a second panel of x and the lost room for
+// the next launch's first copies.  One column: from eight tiles or 144 KB of blocks per SM on, IQ2_XXS,
+// which works longest on a byte, counted one and a half times (Q4_K 2560 -> 65536 22.3 -> 18.5 us, Q8_0
+// 4096 -> 5120, two tiles per SM, 9.4 -> 8.0; Q4_K 2560 -> 14000, 136 KB, 6.8 -> 7.2).  Several columns, with
+// more work per tile: from four tiles on (Q4_K 5120 -> 17357, 4 columns, 27.6 -> 20.0 us, 8 columns 35 -> 29;
+// down to two tiles it makes no difference).
+static bool two_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, bool sep) {
+    if (!sep) return tiles >= 4u * (uint32_t)sms;
+    const uint64_t bytes = (uint64_t)tiles * 16 * row_bytes;
+    return tiles >= 8u * (uint32_t)sms || (ty == T_IQ2_XXS ? bytes + bytes / 2 : bytes) >= 147456ull * (uint32_t)sms;
+}
+static uint32_t gemv_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, bool sep) {
     const uint32_t n = (uint32_t)sms;
     if (tiles <= n) return tiles;
-    if (tiles >= kTwoCtasTiles * n) return 2 * n;
+    if (two_ctas(ty, row_bytes, tiles, sms, sep)) return tiles < 2 * n ? tiles : 2 * n;
     return sep && tiles <= n + n / 4 ? tiles : n;
 }
 
@@ -1338,9 +1347,9 @@ static uint32_t gemv_ctas(uint32_t tiles, int sms, bool sep) {
 // Row-shard launches have duties by CTA number and take no clusters.
 static bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t tiles, int sms, bool gather, GemvArgs &a,
                       GemvLayout &L, uint32_t &ctas) {
-    const uint32_t all = gemv_ctas(tiles, sms, mode == M_SEP);
+    const uint32_t all = gemv_ctas(ty, row_bytes, tiles, sms, mode == M_SEP);
     for (uint32_t cs = 1; cs <= 8 && !(gather && cs > 1) && cs * 4 <= nunit; cs *= 2) {
-        const uint32_t limit = (tiles >= kTwoCtasTiles * (uint32_t)sms ? 2 : 1) * (uint32_t)sms / cs;
+        const uint32_t limit = (two_ctas(ty, row_bytes, tiles, sms, mode == M_SEP) ? 2 : 1) * (uint32_t)sms / cs;
         const uint32_t clusters = cs == 1 ? all : tiles < limit ? tiles : limit;
         if (!gemv_layout(ty, row_bytes, nunit, n, mode, cs, (tiles + clusters - 1) / clusters, a, L)) continue;
         const bool last = ty == T_IQ2_XXS && cs == 2;  // shorter segments of its 66-byte units cost more than a resident x gains
@@ -1352,30 +1361,42 @@ static bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, in
     return gemv_layout(ty, row_bytes, nunit, n, mode, 1, (tiles + all - 1) / all, a, L);
 }
 
-template <int TY, int MODE>
-static cudaError_t launch_t(GemvArgs a, const GemvGather &G, cudaStream_t s, int sms, int dev) {
-    GemvLayout L;
-    uint32_t ctas;
-    if (!gemv_plan(TY, a.row_bytes, a.nunit, a.n, MODE, a.tiles, sms, G.nranks != 0, a, L, ctas)) return cudaErrorInvalidConfiguration;
+template <int TY, int MODE, int XDT, bool CL>
+static cudaError_t launch_c(const GemvArgs &a, const GemvLayout &L, const GemvGather &G, uint32_t ctas, cudaStream_t s, int dev) {
     static bool attr_set[64] = {};  // the opt-in is per device
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemv_kernel<TY, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBudget);
+        cudaError_t e = cudaFuncSetAttribute(gemv_kernel<TY, MODE, XDT, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBudget);
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    return launch_pdl(gemv_kernel<TY, MODE>, ctas, G.nranks ? kGemvThreadsMax : kGemvThreads, L.smem_bytes, s, 1u << L.clog, a, L, G);
+    return launch_pdl(gemv_kernel<TY, MODE, XDT, CL>, ctas, G.nranks ? kGemvThreadsMax : kGemvThreads, L.smem_bytes, s, 1u << L.clog, a, L, G);
+}
+template <int TY, int MODE, int XDT>
+static cudaError_t launch_d(const GemvArgs &a, const GemvLayout &L, const GemvGather &G, uint32_t ctas, cudaStream_t s, int dev) {
+    return L.clog ? launch_c<TY, MODE, XDT, true>(a, L, G, ctas, s, dev) : launch_c<TY, MODE, XDT, false>(a, L, G, ctas, s, dev);
+}
+template <int TY, int MODE>
+static cudaError_t launch_t(GemvArgs a, const GemvGather &G, int xdt, cudaStream_t s, int sms, int dev) {
+    GemvLayout L;
+    uint32_t ctas;
+    if (!gemv_plan(TY, a.row_bytes, a.nunit, a.n, MODE, a.tiles, sms, G.nranks != 0, a, L, ctas)) return cudaErrorInvalidConfiguration;
+    switch (xdt) {
+    case DT_F16: return launch_d<TY, MODE, DT_F16>(a, L, G, ctas, s, dev);
+    case DT_BF16: return launch_d<TY, MODE, DT_BF16>(a, L, G, ctas, s, dev);
+    default: return launch_d<TY, MODE, DT_F32>(a, L, G, ctas, s, dev);
+    }
 }
 
 template <int TY>
-static cudaError_t launch_ty(const GemvArgs &a, const GemvGather &G, int mode, cudaStream_t s, int sms, int dev) {
+static cudaError_t launch_ty(const GemvArgs &a, const GemvGather &G, int mode, int xdt, cudaStream_t s, int sms, int dev) {
     switch (mode) {
-    case M_SEP: return launch_t<TY, M_SEP>(a, G, s, sms, dev);
-    case M_W1: return launch_t<TY, M_W1>(a, G, s, sms, dev);
-    case M_W2: return launch_t<TY, M_W2>(a, G, s, sms, dev);
+    case M_SEP: return launch_t<TY, M_SEP>(a, G, xdt, s, sms, dev);
+    case M_W1: return launch_t<TY, M_W1>(a, G, xdt, s, sms, dev);
+    case M_W2: return launch_t<TY, M_W2>(a, G, xdt, s, sms, dev);
     }
     if constexpr (TY == T_Q8_0 || TY == T_Q4_0 || TY == T_IQ4_NL || TY == T_Q2_0) {
-        if (mode == M_R) return launch_t<TY, M_R>(a, G, s, sms, dev);
+        if (mode == M_R) return launch_t<TY, M_R>(a, G, xdt, s, sms, dev);
     }
     return cudaErrorInvalidValue;
 }
@@ -1434,7 +1455,7 @@ cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, co
                               int sms, int dev, uint64_t *launches, const GemvGatherPlan *gather) {
     if (nseg == 0 || nseg > (uint32_t)kGemvSegs) return cudaErrorInvalidValue;
     GemvArgs a = {};
-    a.status = status; a.k = k; a.xdt = xdt;
+    a.status = status; a.k = k;
     a.nunit = (k + 255) / 256;
     a.row_bytes = k / block_elems(ty) * block_bytes(ty);
     uint32_t tiles = 0;
@@ -1475,14 +1496,14 @@ cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, co
         a.n = take;
         cudaError_t e;
         switch (ty) {
-        case T_Q4_K: e = launch_ty<T_Q4_K>(a, G, mode, s, sms, dev); break;
-        case T_Q8_0: e = launch_ty<T_Q8_0>(a, G, mode, s, sms, dev); break;
-        case T_Q4_0: e = launch_ty<T_Q4_0>(a, G, mode, s, sms, dev); break;
-        case T_Q6_K: e = launch_ty<T_Q6_K>(a, G, mode, s, sms, dev); break;
-        case T_Q5_K: e = launch_ty<T_Q5_K>(a, G, mode, s, sms, dev); break;
-        case T_IQ4_NL: e = launch_ty<T_IQ4_NL>(a, G, mode, s, sms, dev); break;
-        case T_Q2_0: e = launch_ty<T_Q2_0>(a, G, mode, s, sms, dev); break;
-        case T_IQ2_XXS: e = launch_ty<T_IQ2_XXS>(a, G, mode, s, sms, dev); break;
+        case T_Q4_K: e = launch_ty<T_Q4_K>(a, G, mode, xdt, s, sms, dev); break;
+        case T_Q8_0: e = launch_ty<T_Q8_0>(a, G, mode, xdt, s, sms, dev); break;
+        case T_Q4_0: e = launch_ty<T_Q4_0>(a, G, mode, xdt, s, sms, dev); break;
+        case T_Q6_K: e = launch_ty<T_Q6_K>(a, G, mode, xdt, s, sms, dev); break;
+        case T_Q5_K: e = launch_ty<T_Q5_K>(a, G, mode, xdt, s, sms, dev); break;
+        case T_IQ4_NL: e = launch_ty<T_IQ4_NL>(a, G, mode, xdt, s, sms, dev); break;
+        case T_Q2_0: e = launch_ty<T_Q2_0>(a, G, mode, xdt, s, sms, dev); break;
+        case T_IQ2_XXS: e = launch_ty<T_IQ2_XXS>(a, G, mode, xdt, s, sms, dev); break;
         default: e = cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;

@@ -93,7 +93,6 @@ struct GemvArgs {
     const void *x;
     int *status;     // device status word: 0 = ok, else a wait gave up (see kStatus*)
     uint32_t k, n;
-    int xdt;
     uint32_t nunit;  // 256-wide units per row, the last one perhaps not whole
     uint32_t tiles;  // all segments together
     uint32_t cb;     // units per chunk (one ring stage holds 16 rows x cb units)
