@@ -194,7 +194,24 @@ int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uin
         e = run_tile(ctx, ty, wp, k, m, x, xdt, n, out, odt, s, nullptr);
         return e == cudaSuccess ? OKF_OK : cuda_fail(ctx, e);
     } else {
-        if (!(ctx->flags & OKF_FLAG_SIMPLE_KERNELS)) ctx->fallbacks++;
+        const bool simple = ctx->flags & OKF_FLAG_SIMPLE_KERNELS;
+        if (!simple) ctx->fallbacks++;
+        // A few tokens of rows that the tile does not take (K not a multiple of 64): passes of the 24-bit
+        // matvec, about 3.5 us and the weights at 2 TB/s for four tokens, against the plain tile's 32-deep
+        // steps, 2.3 us each while its 64 x 64 tiles leave SMs idle, 0.74 us and as many as there are tiles
+        // per SM where they do not.  (Q4_0 4384 -> 1536, 12 tokens: 310 us on the tile.)
+        const double steps = k / 32, tiles = (double)((m + 63) / 64) * ((n + 63) / 64) / ctx->sms;
+        const double t_tile = steps * (2.3 > 0.74 * tiles ? 2.3 : 0.74 * tiles);
+        const double t_pass = 3.5 + (double)m * k / block_elems(ty) * block_bytes(ty) / 2e6;
+        if (!simple && odt == DT_F32 && !force_tile && (n + 3) / 4 * t_pass < t_tile &&
+            gemv_ragged_supported(ty, k, m, wp, x, xdt, 4, ctx->sms)) {
+            for (uint32_t c = 0; c < n; c += 4) {
+                e = launch_gemv_fast(ty, wp, k, m, (const uint8_t *)x + (size_t)c * k * dtype_size(xdt), xdt, n - c < 4 ? n - c : 4,
+                                     (float *)out + (size_t)c * m, ctx->dev_status, s, ctx->sms, ctx->device, &ctx->launches);
+                if (e != cudaSuccess) return cuda_fail(ctx, e);
+            }
+            return OKF_OK;
+        }
         e = launch_gemm_simple(ty, wp, k, m, x, xdt, n, out, odt, s);
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e);

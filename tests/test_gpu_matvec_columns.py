@@ -45,11 +45,14 @@ def test_columns(ctx, ty, n):
 
 
 @pytest.mark.parametrize("ty", [GGUFType.Q8_0, GGUFType.Q4_0, GGUFType.IQ4_NL, GGUFType.Q2_0])
-@pytest.mark.parametrize("n", [1, 3, 4, 5, 8])
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 8, 13])
 def test_rows_that_end_inside_a_unit(ctx, ty, n):
-    """From one block to several chunks, first and last block of a unit, four columns and a remainder."""
+    """From one block to several chunks, first and last block of a unit, four columns and a
+    remainder, and the passes over a few tokens more than eight that K not a multiple of 64 takes."""
     step = block_elems(ty)
     for i, (k, m) in enumerate([(step, 5), (256 + step, 16), (1024 - step, 77), (4096 + step, 1000), (16384 - step, 40)]):
+        if n > 8 and k % 64 == 0:
+            continue  # the tensor-core tile, with 16-bit operands
         assert run(ctx, ty, k, m, n, DTS[(i + n) % 3], seed=1) <= RAGGED_TOL, (k, m)
     assert ctx.device_status() == 0
 
