@@ -164,19 +164,6 @@ __device__ __forceinline__ SepConst sep_const(uint32_t c) {
     return k;
 }
 
-// IQ4_NL: the sixteen codebook values (LLM/Gemma/Gemma4Quant.swift:5-9) for four nibbles (one per
-// byte of v, 0..15) as four signed bytes.
-__device__ __forceinline__ uint32_t iq4nl_lookup(uint32_t v) {
-    // {-127, -104, -83, -65}, {-49, -35, -22, -10}, {1, 13, 25, 38}, {53, 69, 89, 113}
-    constexpr uint32_t T0 = 0xBFAD9881u, T1 = 0xF6EADDCFu, T2 = 0x26190D01u, T3 = 0x71594535u;
-    const uint32_t s = v & 0x07070707u;
-    const uint32_t t = s | (s >> 4);                       // bytes 0 and 2: two selector nibbles each
-    const uint32_t sel = (t & 0xFFu) | ((t >> 8) & 0xFF00u);
-    const uint32_t lo = prmt(T0, T1, sel), hi = prmt(T2, T3, sel);
-    const uint32_t pick = ((v >> 3) & 0x01010101u) * 0xFFu;  // bytes whose nibble is 8..15
-    return (lo & ~pick) | (hi & pick);
-}
-
 // ua / ub: shared addresses of the unit in rows g and g + 8.  xf: this thread's 64
 // bytes of x (its quarter of the unit, the byte column its MMA column stands for; zeros
 // in the lanes that feed nothing).  xi: {scale of x in this unit, scale * sum of x over
@@ -184,7 +171,7 @@ __device__ __forceinline__ uint32_t iq4nl_lookup(uint32_t v) {
 // acc: rows g and g + 8.
 template <int TY>
 __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepConst &K, const Iq2Tab &tab, const uint32_t (&xf)[16],
-                                         const uint4 &xi, float (&acc)[2]) {
+                                         const uint4 &xi, const uint4 &xj, float (&acc)[2]) {
     const float xs = __uint_as_float(xi.x);
     if constexpr (TY == T_Q4_K) {
         // {f16 d; f16 dmin; u8 scales[12]; u8 qs[128]} (LLM/Quantize/KQuants.swift:104-125).
@@ -264,9 +251,9 @@ __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepCons
         acc[0] += da0 * fmaf(xs, part[0][0], -8.f * x0) + da1 * fmaf(xs, part[1][0], -8.f * x1);
         acc[1] += db0 * fmaf(xs, part[0][1], -8.f * x0) + db1 * fmaf(xs, part[1][1], -8.f * x1);
     } else if constexpr (TY == T_IQ4_NL) {
-        // Q4_0's layout with a codebook: weight = kvalues[nibble] * d (LLM/Gemma/Gemma4Quant.swift:5-29).
-        // The sixteen signed bytes sit in four registers; a byte permute looks four nibbles up in
-        // the low or the high eight, bit 3 of each nibble picks between the two.
+        // Q4_0's layout with a codebook: weight = kvalues[nibble] * d (LLM/Gemma/Gemma4Quant.swift:5-29), looked
+        // up eight nibbles at a time (see iq4nl_word; x is staged in the order they come in).  (Four at a
+        // time, with selectors packed first: 5120 -> 65536 73 us at 2.6 TB/s.)
         uint32_t wa[9], wb[9];
 #pragma unroll
         for (int i = 0; i < 9; i++) {
@@ -285,16 +272,14 @@ __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepCons
 #pragma unroll
         for (int blk = 0; blk < 2; blk++) {
             const uint32_t *a = qa + 4 * blk, *b = qb + 4 * blk;
-            const uint32_t *xb = xf + 8 * blk;  // bytes of k 0..15 (low nibbles), then 16..31 (high)
+            const uint32_t *xb = xf + 8 * blk;
             int d[4];
-            imma0<true>(d, iq4nl_lookup(a[0] & 0x0F0F0F0Fu), iq4nl_lookup(b[0] & 0x0F0F0F0Fu), iq4nl_lookup(a[1] & 0x0F0F0F0Fu),
-                        iq4nl_lookup(b[1] & 0x0F0F0F0Fu), xb[0], xb[1]);
-            imma<true>(d, iq4nl_lookup(a[2] & 0x0F0F0F0Fu), iq4nl_lookup(b[2] & 0x0F0F0F0Fu), iq4nl_lookup(a[3] & 0x0F0F0F0Fu),
-                       iq4nl_lookup(b[3] & 0x0F0F0F0Fu), xb[2], xb[3]);
-            imma<true>(d, iq4nl_lookup((a[0] >> 4) & 0x0F0F0F0Fu), iq4nl_lookup((b[0] >> 4) & 0x0F0F0F0Fu),
-                       iq4nl_lookup((a[1] >> 4) & 0x0F0F0F0Fu), iq4nl_lookup((b[1] >> 4) & 0x0F0F0F0Fu), xb[4], xb[5]);
-            imma<true>(d, iq4nl_lookup((a[2] >> 4) & 0x0F0F0F0Fu), iq4nl_lookup((b[2] >> 4) & 0x0F0F0F0Fu),
-                       iq4nl_lookup((a[3] >> 4) & 0x0F0F0F0Fu), iq4nl_lookup((b[3] >> 4) & 0x0F0F0F0Fu), xb[6], xb[7]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const uint2 va = iq4nl_word(a[i]), vb = iq4nl_word(b[i]);
+                if (i == 0) imma0<true>(d, va.x, vb.x, va.y, vb.y, xb[0], xb[1]);
+                else imma<true>(d, va.x, vb.x, va.y, vb.y, xb[2 * i], xb[2 * i + 1]);
+            }
             part[blk][0] = join_hi_lo(d[0], d[1]);
             part[blk][1] = join_hi_lo(d[2], d[3]);
         }
@@ -352,41 +337,40 @@ __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepCons
         // d * scale[group of 16] * (q - 32), q = four bits of ql and two of qh.  Quarter c is
         // elements 64c .. 64c + 63 = the low (c even) or high (c odd) nibbles of the 64 ql bytes of
         // half c / 2, with qh bits 4(c & 1) .. +1 for its first 32 elements and the next two bits
-        // for the other 32, and scales 4c .. 4c + 3.  q - 32 is made a signed byte in place
-        // (flip bit 5, then copy it into bits 6 and 7: 0x20 * 6 = 0xC0 stays inside the byte), so
-        // the signed MMA needs no correction; one accumulator per 16-wide scale group.
-        // Units are only 2-byte aligned.
+        // for the other 32, and scales 4c .. 4c + 3.  The codes go in unsigned, one accumulator per 16-wide
+        // scale group, and 32 x the sum of x over the group leaves again.  (As signed bytes q - 32, made in
+        // place: 2560 -> 151936 86 us.)  Units are only 2-byte aligned.
         uint32_t sa[1], sb[1];
         lds_a2<1>(ua + K.m1, sa);
         lds_a2<1>(ub + K.m1, sb);
         const float da = f16bits(lds16(ua + 208)), db = f16bits(lds16(ub + 208));
-        const uint32_t sh = K.sel;
+        uint32_t ha[8], hb[8];  // 32 bytes of qh
+        lds_a2<8>(ua + K.hoff, ha);
+        lds_a2<8>(ub + K.hoff, hb);
+        const float xg[4] = {__uint_as_float(xj.x), __uint_as_float(xj.y), __uint_as_float(xj.z), __uint_as_float(xj.w)};
         float suma = 0.f, sumb = 0.f;
 #pragma unroll
         for (int grp = 0; grp < 4; grp++) {  // 16 elements: 16 bytes of ql, 16 of qh (groups 2, 3 reuse those of 0, 1)
-            uint32_t la[4], lb[4], ha[4], hb[4];
-            lds_a2<4>(ua + K.qoff + 16 * grp, la);
-            lds_a2<4>(ub + K.qoff + 16 * grp, lb);
-            lds_a2<4>(ua + K.hoff + 16 * (grp & 1), ha);
-            lds_a2<4>(ub + K.hoff + 16 * (grp & 1), hb);
-            const uint32_t hs = sh + 2 * (grp >> 1);
             uint32_t qa[4], qb[4];
+            lds_a2<4>(ua + K.qoff + 16 * grp, qa);
+            lds_a2<4>(ub + K.qoff + 16 * grp, qb);
+            // bits 4(c & 1) + 2(grp / 2) .. +1 of a byte to bits 4, 5: a rotation by 4(c & 1) + 2(grp / 2) - 4
+            const uint32_t rot = K.sel + (grp < 2 ? 28 : 30);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const uint32_t va = (((la[i] >> sh) & 0x0F0F0F0Fu) | (((ha[i] >> hs) & 0x03030303u) << 4)) ^ 0x20202020u;
-                const uint32_t vb = (((lb[i] >> sh) & 0x0F0F0F0Fu) | (((hb[i] >> hs) & 0x03030303u) << 4)) ^ 0x20202020u;
-                qa[i] = va | ((va & 0x20202020u) * 6u);
-                qb[i] = vb | ((vb & 0x20202020u) * 6u);
+                const uint32_t va = ha[4 * (grp & 1) + i], vb = hb[4 * (grp & 1) + i];
+                qa[i] = ((qa[i] >> K.sel) & 0x0F0F0F0Fu) | (__funnelshift_r(va, va, rot) & 0x30303030u);
+                qb[i] = ((qb[i] >> K.sel) & 0x0F0F0F0Fu) | (__funnelshift_r(vb, vb, rot) & 0x30303030u);
             }
             int d[4];
-            imma0<true>(d, qa[0], qb[0], qa[1], qb[1], xf[4 * grp], xf[4 * grp + 1]);
-            imma<true>(d, qa[2], qb[2], qa[3], qb[3], xf[4 * grp + 2], xf[4 * grp + 3]);
+            imma0<false>(d, qa[0], qb[0], qa[1], qb[1], xf[4 * grp], xf[4 * grp + 1]);
+            imma<false>(d, qa[2], qb[2], qa[3], qb[3], xf[4 * grp + 2], xf[4 * grp + 3]);
             const float fa = (float)((int)(sa[0] << (24 - 8 * grp)) >> 24), fb = (float)((int)(sb[0] << (24 - 8 * grp)) >> 24);
-            suma = fmaf(fa, join_hi_lo(d[0], d[1]), suma);
-            sumb = fmaf(fb, join_hi_lo(d[2], d[3]), sumb);
+            suma = fmaf(fa, fmaf(xs, join_hi_lo(d[0], d[1]), -32.f * xg[grp]), suma);
+            sumb = fmaf(fb, fmaf(xs, join_hi_lo(d[2], d[3]), -32.f * xg[grp]), sumb);
         }
-        acc[0] += (da * xs) * suma;
-        acc[1] += (db * xs) * sumb;
+        acc[0] = fmaf(da, suma, acc[0]);
+        acc[1] = fmaf(db, sumb, acc[1]);
     } else if constexpr (TY == T_Q8_0) {
         // eight blocks {f16 d; i8 q[32]} (LLM/Gemma/Gemma4Quant.swift:51-69); thread c
         // takes blocks 2c and 2c+1: {d0, q0[32], d1, q1[32]} = 17 words (units start on
@@ -557,6 +541,9 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
             }
             int qsum = (int)(tsum - 8u * kMagicBits);  // sum of the eight q
             qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
+            // Q6_K: the sums over 16-wide groups, in the second byte column
+            if constexpr (TY == T_Q6_K)
+                if ((e8 & 1) == 0) sts32(xs32 + es + (i >> 5) * kSepUnit + c * kSepQuarter + 64 + ((e8 >> 1) & 3) * 4, __float_as_uint(scale * (float)qsum));
             qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
             const uint32_t u = i >> 5;
             const uint32_t dst = xs32 + u * kSepUnit + item_off;
@@ -570,10 +557,22 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
                     sts16(at + es, (prmt(t[w], t[w + 4], 0x0040u) & 0xFFFFu) ^ 0x8080u);
                 }
             } else {
-                sts64(dst, prmt(prmt(t[0], t[1], 0x0051u), prmt(t[2], t[3], 0x0051u), 0x5410u),
-                      prmt(prmt(t[4], t[5], 0x0051u), prmt(t[6], t[7], 0x0051u), 0x5410u));
-                sts64(dst + es, prmt(prmt(t[0], t[1], 0x0040u), prmt(t[2], t[3], 0x0040u), 0x5410u) ^ 0x80808080u,
-                      prmt(prmt(t[4], t[5], 0x0040u), prmt(t[6], t[7], 0x0040u), 0x5410u) ^ 0x80808080u);
+                const uint32_t h0 = prmt(prmt(t[0], t[1], 0x0051u), prmt(t[2], t[3], 0x0051u), 0x5410u);
+                const uint32_t h1 = prmt(prmt(t[4], t[5], 0x0051u), prmt(t[6], t[7], 0x0051u), 0x5410u);
+                const uint32_t l0 = prmt(prmt(t[0], t[1], 0x0040u), prmt(t[2], t[3], 0x0040u), 0x5410u) ^ 0x80808080u;
+                const uint32_t l1 = prmt(prmt(t[4], t[5], 0x0040u), prmt(t[6], t[7], 0x0040u), 0x5410u) ^ 0x80808080u;
+                if constexpr (TY == T_IQ4_NL) {
+                    // k 4i, 16+4i, 4i+1, 17+4i, then 4i+2, ...: the item 16 k further on, or back, is two lanes away
+                    const bool high = e8 & 2;
+                    const uint32_t at = xs32 + u * kSepUnit + c * kSepQuarter + (e8 & 4) * 8 + (e8 & 1) * 16 + (e8 & 2) * 4;
+                    const uint32_t hx = __shfl_xor_sync(0xffffffffu, high ? h0 : h1, 2), lx = __shfl_xor_sync(0xffffffffu, high ? l0 : l1, 2);
+                    const uint32_t ha = high ? hx : h0, hb = high ? h1 : hx, la = high ? lx : l0, lb = high ? l1 : lx;
+                    sts64(at, prmt(ha, hb, 0x5140u), prmt(ha, hb, 0x7362u));
+                    sts64(at + es, prmt(la, lb, 0x5140u), prmt(la, lb, 0x7362u));
+                } else {
+                    sts64(dst, h0, h1);
+                    sts64(dst + es, l0, l1);
+                }
             }
             // the quarter's record, behind its 64 bytes in the first byte column
             const uint32_t rec = xs32 + u * kSepUnit + c * kSepQuarter + 64;
@@ -983,7 +982,8 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
                                 const uint32_t xf[16] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w,
                                                          q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z, q3.w};
                                 const uint4 xi = lds128(ia);
-                                unit_sep<TY>(wa, wa + wdelta, KC, tab, xf, xi, acc);
+                                const uint4 xj = TY == T_Q6_K ? lds128(ia + L.es) : make_uint4(0u, 0u, 0u, 0u);
+                                unit_sep<TY>(wa, wa + wdelta, KC, tab, xf, xi, xj, acc);
                                 wa += UB;
                                 xa += xstride32;
                                 ia += kSepUnit;
