@@ -77,8 +77,9 @@ constexpr uint32_t kXqUnit = 256;
 constexpr float kXqMax = 32512.f;  // 127 * 256: hi stays a signed byte after rounding
 constexpr float kXq3Max = 8323072.f;  // 127 * 65536, three bytes
 // SEP x panel: per byte column and unit, four quarters of 80 bytes: 64 bytes of x in k
-// order, then (first byte column only) the quarter's record {scale, scale * sum of x over
-// its first 32-wide block, over its second, -}.  One address register reaches a
+// order (two types: see stage_x_bytes), then in the first byte column the quarter's record {scale,
+// scale * sum of x over its first 32-wide block, over its second, -}, in the second one, for Q6_K,
+// the sums over its 16-wide groups.  One address register reaches a
 // quarter's x and its record with immediate offsets.  80-byte quarters put the four
 // quarters of a 16-byte access on different bank groups (0, 80, 32, 112 mod 128) and the
 // second byte column, 64 (mod 128) bytes after the first, on the other four.
@@ -141,7 +142,7 @@ __device__ __forceinline__ SepConst sep_const(uint32_t c) {
     SepConst k = {};
     if constexpr (TY == T_Q4_K || TY == T_Q5_K) {
         k.qoff = (TY == T_Q4_K ? 16 : 48) + 32 * c;
-        k.hoff = 2 * c;  // Q5_K: the bit of qh that belongs to sub-block 2c
+        k.hoff = 2 * c;  // Q5_K: the bit of qh that belongs to sub-block 2c; the next one is sub-block 2c + 1's
         k.sel = (c & 1) ? 0x7632u : 0x5410u;
         k.low = c < 2;
         k.m1 = k.low ? 0x3F3F3F3Fu : 0x0F0F0F0Fu;
@@ -151,10 +152,11 @@ __device__ __forceinline__ SepConst sep_const(uint32_t c) {
     } else if constexpr (TY == T_Q4_0 || TY == T_IQ4_NL) {
         k.qoff = 36 * c;
     } else if constexpr (TY == T_Q6_K) {
-        k.qoff = 64 * (c >> 1);         // ql of this half of the block
-        k.hoff = 128 + 32 * (c >> 1);   // qh of this half
-        k.sel = 4 * (c & 1);            // low or high nibbles of ql; bits 0-3 or 4-7 of qh
-        k.m1 = 192 + 4 * c;             // this quarter's four scales
+        k.qoff = 64 * (c >> 1) + 32 * (c & 1);      // 32 bytes of ql
+        k.hoff = 128 + 32 * (c >> 1);               // the half's 32 bytes of qh
+        k.sel = 192 + 8 * (c >> 1) + 2 * (c & 1);   // two scales, and two more 4 bytes on
+        k.m1 = 0x03030303u << (2 * (c & 1));        // this thread's two bits of qh for the low nibbles
+        k.m2 = 16u >> (2 * (c & 1));                // what puts those bits above a nibble
     } else if constexpr (TY == T_Q2_0) {
         k.hoff = 34 * (c >> 1);
         k.qoff = k.hoff + 2 + 16 * (c & 1);
@@ -289,42 +291,40 @@ __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepCons
         acc[1] += xs * (db0 * part[0][1] + db1 * part[1][1]);
     } else if constexpr (TY == T_Q5_K) {
         // {f16 d; f16 dmin; u8 scales[12]; u8 qh[32]; u8 qs[128]} (LLM/Quantize/KQuants.swift:127-158):
-        // Q4_K's header and nibbles, plus a fifth bit: bit j of qh[l] for sub-block j.  The five
-        // bits are joined into unsigned bytes (0..31) for both sub-blocks of the quarter.
+        // Q4_K's header and nibbles, plus a fifth bit: bit j of qh[l] for sub-block j.  As in Q6_K,
+        // nibbles and bits go in where they stand and their sums are put together as integers.  (Joined into
+        // bytes before the MMA: 5120 -> 65536 50 us at 4.6 TB/s.)
         const uint4 ha = lds128(ua), hb = lds128(ub);
-        int lo[4], hi[4];
+        const uint32_t bit_lo = 0x01010101u << K.hoff, bit_hi = 0x02020202u << K.hoff;
+        int lo[4], hi[4], el[4], eh[4];
 #pragma unroll
         for (int half = 0; half < 2; half++) {  // 16 bytes of qs and of qh at a time
             const uint4 a = lds128(ua + K.qoff + 16 * half), b = lds128(ub + K.qoff + 16 * half);
             const uint4 ga = lds128(ua + 16 + 16 * half), gb = lds128(ub + 16 + 16 * half);
-            const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
-            const uint32_t fa[4] = {ga.x >> K.hoff, ga.y >> K.hoff, ga.z >> K.hoff, ga.w >> K.hoff};
-            const uint32_t fb[4] = {gb.x >> K.hoff, gb.y >> K.hoff, gb.z >> K.hoff, gb.w >> K.hoff};
-            uint32_t la[4], lb[4], ua5[4], ub5[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                la[i] = (wa[i] & 0x0F0F0F0Fu) | ((fa[i] & 0x01010101u) << 4);
-                lb[i] = (wb[i] & 0x0F0F0F0Fu) | ((fb[i] & 0x01010101u) << 4);
-                ua5[i] = ((wa[i] >> 4) & 0x0F0F0F0Fu) | ((fa[i] & 0x02020202u) << 3);
-                ub5[i] = ((wb[i] >> 4) & 0x0F0F0F0Fu) | ((fb[i] & 0x02020202u) << 3);
-            }
+            const uint32_t *x0 = xf + 4 * half, *x1 = xf + 8 + 4 * half;
             if (half == 0) {
-                imma0<false>(lo, la[0], lb[0], la[1], lb[1], xf[0], xf[1]);
-                imma0<false>(hi, ua5[0], ub5[0], ua5[1], ub5[1], xf[8], xf[9]);
-                imma<false>(lo, la[2], lb[2], la[3], lb[3], xf[2], xf[3]);
-                imma<false>(hi, ua5[2], ub5[2], ua5[3], ub5[3], xf[10], xf[11]);
+                imma0<false>(lo, a.x & 0x0F0F0F0Fu, b.x & 0x0F0F0F0Fu, a.y & 0x0F0F0F0Fu, b.y & 0x0F0F0F0Fu, x0[0], x0[1]);
+                imma0<false>(el, ga.x & bit_lo, gb.x & bit_lo, ga.y & bit_lo, gb.y & bit_lo, x0[0], x0[1]);
+                imma0<false>(hi, a.x & 0xF0F0F0F0u, b.x & 0xF0F0F0F0u, a.y & 0xF0F0F0F0u, b.y & 0xF0F0F0F0u, x1[0], x1[1]);
+                imma0<false>(eh, ga.x & bit_hi, gb.x & bit_hi, ga.y & bit_hi, gb.y & bit_hi, x1[0], x1[1]);
             } else {
-                imma<false>(lo, la[0], lb[0], la[1], lb[1], xf[4], xf[5]);
-                imma<false>(hi, ua5[0], ub5[0], ua5[1], ub5[1], xf[12], xf[13]);
-                imma<false>(lo, la[2], lb[2], la[3], lb[3], xf[6], xf[7]);
-                imma<false>(hi, ua5[2], ub5[2], ua5[3], ub5[3], xf[14], xf[15]);
+                imma<false>(lo, a.x & 0x0F0F0F0Fu, b.x & 0x0F0F0F0Fu, a.y & 0x0F0F0F0Fu, b.y & 0x0F0F0F0Fu, x0[0], x0[1]);
+                imma<false>(el, ga.x & bit_lo, gb.x & bit_lo, ga.y & bit_lo, gb.y & bit_lo, x0[0], x0[1]);
+                imma<false>(hi, a.x & 0xF0F0F0F0u, b.x & 0xF0F0F0F0u, a.y & 0xF0F0F0F0u, b.y & 0xF0F0F0F0u, x1[0], x1[1]);
+                imma<false>(eh, ga.x & bit_hi, gb.x & bit_hi, ga.y & bit_hi, gb.y & bit_hi, x1[0], x1[1]);
             }
+            imma<false>(lo, a.z & 0x0F0F0F0Fu, b.z & 0x0F0F0F0Fu, a.w & 0x0F0F0F0Fu, b.w & 0x0F0F0F0Fu, x0[2], x0[3]);
+            imma<false>(el, ga.z & bit_lo, gb.z & bit_lo, ga.w & bit_lo, gb.w & bit_lo, x0[2], x0[3]);
+            imma<false>(hi, a.z & 0xF0F0F0F0u, b.z & 0xF0F0F0F0u, a.w & 0xF0F0F0F0u, b.w & 0xF0F0F0F0u, x1[2], x1[3]);
+            imma<false>(eh, ga.z & bit_hi, gb.z & bit_hi, ga.w & bit_hi, gb.w & bit_hi, x1[2], x1[3]);
         }
+        // every shift is exact: the sums are multiples of what the bits stand at (and below 32 * 240 * 32512)
+        auto put_lo = [&](int i) { return (float)((lo[i] * 256 + lo[i + 1]) + ((el[i] * 256 + el[i + 1]) >> K.hoff) * 16); };
+        auto put_hi = [&](int i) { return (float)(((hi[i] * 256 + hi[i + 1]) >> 4) + ((eh[i] * 256 + eh[i + 1]) >> (K.hoff + 1)) * 16); };
         const uint32_t pa = prmt(ha.y, hb.y, K.sel), pb = prmt(ha.z, hb.z, K.sel), pe = prmt(ha.w, hb.w, K.sel);
         const uint32_t sc = ((K.low ? pa : pe) & K.m1) | ((pa >> 2) & K.m2);
         const uint32_t mn = ((K.low ? pb : (pe >> 4)) & K.m1) | ((pb >> 2) & K.m2);
-        const float la_ = join_hi_lo(lo[0], lo[1]), ha_ = join_hi_lo(hi[0], hi[1]);
-        const float lb_ = join_hi_lo(lo[2], lo[3]), hb_ = join_hi_lo(hi[2], hi[3]);
+        const float la_ = put_lo(0), ha_ = put_hi(0), lb_ = put_lo(2), hb_ = put_hi(2);
         const float x0 = __uint_as_float(xi.y), x1 = __uint_as_float(xi.z);  // scale * sum of x per block
         const float2 fa2 = __half22float2(*reinterpret_cast<const __half2 *>(&ha.x));
         const float2 fb2 = __half22float2(*reinterpret_cast<const __half2 *>(&hb.x));
@@ -334,40 +334,46 @@ __device__ __forceinline__ void unit_sep(uint32_t ua, uint32_t ub, const SepCons
                   fb2.y * (byte_to_f32(mn, 2) * x0 + byte_to_f32(mn, 3) * x1);
     } else if constexpr (TY == T_Q6_K) {
         // {u8 ql[128]; u8 qh[64]; i8 scales[16]; f16 d} (LLM/Quantize/KQuants.swift:160-177): weight =
-        // d * scale[group of 16] * (q - 32), q = four bits of ql and two of qh.  Quarter c is
-        // elements 64c .. 64c + 63 = the low (c even) or high (c odd) nibbles of the 64 ql bytes of
-        // half c / 2, with qh bits 4(c & 1) .. +1 for its first 32 elements and the next two bits
-        // for the other 32, and scales 4c .. 4c + 3.  The codes go in unsigned, one accumulator per 16-wide
-        // scale group, and 32 x the sum of x over the group leaves again.  (As signed bytes q - 32, made in
-        // place: 2560 -> 151936 86 us.)  Units are only 2-byte aligned.
-        uint32_t sa[1], sb[1];
-        lds_a2<1>(ua + K.m1, sa);
-        lds_a2<1>(ub + K.m1, sb);
+        // d * scale[group of 16] * (q - 32), q = four bits of ql and two of qh.  Thread c takes 32 bytes
+        // of ql, both nibbles (elements 128h + 32s + l and 64 further on; h = c / 2, s = c & 1), and
+        // the two bits of the half's qh for each; x is staged to match.  Nothing is shifted or
+        // joined: nibbles and bits go in where they stand, as unsigned bytes with sums of their own
+        // per 16-wide scale group, which are put together as integers; 32 x the sum of x over the group leaves
+        // again.  (2560 -> 151936: 86 us as signed bytes made in place, 70 us unsigned but joined
+        // before the MMA and each ql byte read for one nibble.)  Units are only 2-byte aligned.
+        const uint32_t sa[2] = {lds16(ua + K.sel), lds16(ua + K.sel + 4)}, sb[2] = {lds16(ub + K.sel), lds16(ub + K.sel + 4)};
         const float da = f16bits(lds16(ua + 208)), db = f16bits(lds16(ub + 208));
-        uint32_t ha[8], hb[8];  // 32 bytes of qh
+        uint32_t qa[8], qb[8], ha[8], hb[8];
+        lds_a2<8>(ua + K.qoff, qa);
+        lds_a2<8>(ub + K.qoff, qb);
         lds_a2<8>(ua + K.hoff, ha);
         lds_a2<8>(ub + K.hoff, hb);
+        const uint32_t bits_lo = K.m1, bits_hi = K.m1 << 4;
+        const int f = (int)K.m2;
         const float xg[4] = {__uint_as_float(xj.x), __uint_as_float(xj.y), __uint_as_float(xj.z), __uint_as_float(xj.w)};
+        const float xs16 = xs * 0.0625f;
         float suma = 0.f, sumb = 0.f;
 #pragma unroll
-        for (int grp = 0; grp < 4; grp++) {  // 16 elements: 16 bytes of ql, 16 of qh (groups 2, 3 reuse those of 0, 1)
-            uint32_t qa[4], qb[4];
-            lds_a2<4>(ua + K.qoff + 16 * grp, qa);
-            lds_a2<4>(ub + K.qoff + 16 * grp, qb);
-            // bits 4(c & 1) + 2(grp / 2) .. +1 of a byte to bits 4, 5: a rotation by 4(c & 1) + 2(grp / 2) - 4
-            const uint32_t rot = K.sel + (grp < 2 ? 28 : 30);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const uint32_t va = ha[4 * (grp & 1) + i], vb = hb[4 * (grp & 1) + i];
-                qa[i] = ((qa[i] >> K.sel) & 0x0F0F0F0Fu) | (__funnelshift_r(va, va, rot) & 0x30303030u);
-                qb[i] = ((qb[i] >> K.sel) & 0x0F0F0F0Fu) | (__funnelshift_r(vb, vb, rot) & 0x30303030u);
-            }
-            int d[4];
-            imma0<false>(d, qa[0], qb[0], qa[1], qb[1], xf[4 * grp], xf[4 * grp + 1]);
-            imma<false>(d, qa[2], qb[2], qa[3], qb[3], xf[4 * grp + 2], xf[4 * grp + 3]);
-            const float fa = (float)((int)(sa[0] << (24 - 8 * grp)) >> 24), fb = (float)((int)(sb[0] << (24 - 8 * grp)) >> 24);
-            suma = fmaf(fa, fmaf(xs, join_hi_lo(d[0], d[1]), -32.f * xg[grp]), suma);
-            sumb = fmaf(fb, fmaf(xs, join_hi_lo(d[2], d[3]), -32.f * xg[grp]), sumb);
+        for (int grp = 0; grp < 2; grp++) {  // 16 bytes: the low nibbles' scale group `grp`, the high nibbles' 2 + grp
+            int dl[4], dh[4], el[4], eh[4];
+            const uint32_t *a = qa + 4 * grp, *b = qb + 4 * grp, *va = ha + 4 * grp, *vb = hb + 4 * grp;
+            const uint32_t *x0 = xf + 4 * grp, *x1 = xf + 8 + 4 * grp;
+            imma0<false>(dl, a[0] & 0x0F0F0F0Fu, b[0] & 0x0F0F0F0Fu, a[1] & 0x0F0F0F0Fu, b[1] & 0x0F0F0F0Fu, x0[0], x0[1]);
+            imma0<false>(el, va[0] & bits_lo, vb[0] & bits_lo, va[1] & bits_lo, vb[1] & bits_lo, x0[0], x0[1]);
+            imma0<false>(dh, a[0] & 0xF0F0F0F0u, b[0] & 0xF0F0F0F0u, a[1] & 0xF0F0F0F0u, b[1] & 0xF0F0F0F0u, x1[0], x1[1]);
+            imma0<false>(eh, va[0] & bits_hi, vb[0] & bits_hi, va[1] & bits_hi, vb[1] & bits_hi, x1[0], x1[1]);
+            imma<false>(dl, a[2] & 0x0F0F0F0Fu, b[2] & 0x0F0F0F0Fu, a[3] & 0x0F0F0F0Fu, b[3] & 0x0F0F0F0Fu, x0[2], x0[3]);
+            imma<false>(el, va[2] & bits_lo, vb[2] & bits_lo, va[3] & bits_lo, vb[3] & bits_lo, x0[2], x0[3]);
+            imma<false>(dh, a[2] & 0xF0F0F0F0u, b[2] & 0xF0F0F0F0u, a[3] & 0xF0F0F0F0u, b[3] & 0xF0F0F0F0u, x1[2], x1[3]);
+            imma<false>(eh, va[2] & bits_hi, vb[2] & bits_hi, va[3] & bits_hi, vb[3] & bits_hi, x1[2], x1[3]);
+            // at most 16 * 16 * 63 * 32512 in magnitude (the high ones are 16 times their value): inside 32 bits
+            auto put = [&](int i) { return (dl[i] + f * el[i]) * 256 + (dl[i + 1] + f * el[i + 1]); };
+            auto put16 = [&](int i) { return (dh[i] + f * eh[i]) * 256 + (dh[i + 1] + f * eh[i + 1]); };
+            auto scale = [&](uint32_t w) { return (float)(signed char)(grp ? w >> 8 : w & 0xFF); };
+            suma = fmaf(scale(sa[0]), fmaf(xs, (float)put(0), -32.f * xg[grp]), suma);
+            suma = fmaf(scale(sa[1]), fmaf(xs16, (float)put16(0), -32.f * xg[2 + grp]), suma);
+            sumb = fmaf(scale(sb[0]), fmaf(xs, (float)put(2), -32.f * xg[grp]), sumb);
+            sumb = fmaf(scale(sb[1]), fmaf(xs16, (float)put16(2), -32.f * xg[2 + grp]), sumb);
         }
         acc[0] = fmaf(da, suma, acc[0]);
         acc[1] = fmaf(db, sumb, acc[1]);
@@ -504,8 +510,10 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
     constexpr uint32_t kFlight = 4;  // items a thread has in flight: the loads go out first
     constexpr uint32_t kMagicBits = 0x4B400080u;  // 1.5 * 2^23 + 128 as a float
     const uint32_t e8 = tid & 31;  // this lane's item inside its unit, the same in every pass
-    const uint32_t c = e8 >> 3;
-    const uint32_t item_off = c * kSepQuarter + (e8 & 7) * 8;  // 8 bytes of the quarter's 64
+    // Its quarter, and which half of that its 32-wide block is.  Q6_K: thread 2h + s takes blocks 4h + s and 4h + s + 2.
+    const uint32_t c = TY == T_Q6_K ? (e8 >> 4) * 2 + ((e8 >> 2) & 1) : e8 >> 3;
+    const uint32_t second = TY == T_Q6_K ? (e8 >> 3) & 1 : (e8 >> 2) & 1;
+    const uint32_t item_off = c * kSepQuarter + second * 32 + (e8 & 3) * 8;  // 8 bytes of the quarter's 64
     for (uint32_t base = tid; base < items; base += kFlight * kConsumers) {
         XRaw8<XDT> raw[kFlight];
 #pragma unroll
@@ -543,7 +551,7 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
             qsum += __shfl_xor_sync(0xffffffffu, qsum, 1);
             // Q6_K: the sums over 16-wide groups, in the second byte column
             if constexpr (TY == T_Q6_K)
-                if ((e8 & 1) == 0) sts32(xs32 + es + (i >> 5) * kSepUnit + c * kSepQuarter + 64 + ((e8 >> 1) & 3) * 4, __float_as_uint(scale * (float)qsum));
+                if ((e8 & 1) == 0) sts32(xs32 + es + (i >> 5) * kSepUnit + c * kSepQuarter + 64 + second * 8 + (e8 & 2) * 2, __float_as_uint(scale * (float)qsum));
             qsum += __shfl_xor_sync(0xffffffffu, qsum, 2);
             const uint32_t u = i >> 5;
             const uint32_t dst = xs32 + u * kSepUnit + item_off;
@@ -576,8 +584,8 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
             }
             // the quarter's record, behind its 64 bytes in the first byte column
             const uint32_t rec = xs32 + u * kSepUnit + c * kSepQuarter + 64;
-            if ((e8 & 7) == 0) sts32(rec, __float_as_uint(scale));
-            if ((e8 & 3) == 0) sts32(rec + 4 + ((e8 >> 2) & 1) * 4, __float_as_uint(scale * (float)qsum));
+            if ((e8 & 3) == 0 && !second) sts32(rec, __float_as_uint(scale));
+            if ((e8 & 3) == 0) sts32(rec + 4 + second * 4, __float_as_uint(scale * (float)qsum));
         }
     }
 }
