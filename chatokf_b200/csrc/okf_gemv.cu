@@ -1331,13 +1331,18 @@ static bool gemv_layout(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, 
 // thirds of the cycles, sixteen fill them; against that stand a second panel of x and the lost room for
 // the next launch's first copies.  One column: from eight tiles or 144 KB of blocks per SM on, IQ2_XXS,
 // which works longest on a byte, counted one and a half times (Q4_K 2560 -> 65536 22.3 -> 18.5 us, Q8_0
-// 4096 -> 5120, two tiles per SM, 9.4 -> 8.0; Q4_K 2560 -> 14000, 136 KB, 6.8 -> 7.2).  Several columns, with
+// 4096 -> 5120, two tiles per SM, 9.4 -> 8.0; Q4_K 2560 -> 14000, 136 KB, 6.8 -> 7.2), and from 80 KB on
+// where that is at most three tiles, which one CTA would take one after another on some SMs (192 to
+// 320 tiles: Q8_0 4096 -> 4096 6.7 -> 5.2, Q4_K 12288 -> 3072 11.4 -> 8.7, 5120 -> 5120 6.7 -> 6.1; below, Q4_K
+// 4096 -> 4096, 64 KB, 4.15 -> 4.35; not for the two types with a look-up per weight, whose warps hardly
+// wait: IQ2_XXS 6144 -> 6144 9.6 -> 10.5, IQ4_NL 10.1 -> 11.3).  Several columns, with
 // more work per tile: from four tiles on (Q4_K 5120 -> 17357, 4 columns, 27.6 -> 20.0 us, 8 columns 35 -> 29;
 // down to two tiles it makes no difference).
 static bool two_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, bool sep) {
     if (!sep) return tiles >= 4u * (uint32_t)sms;
-    const uint64_t bytes = (uint64_t)tiles * 16 * row_bytes;
-    return tiles >= 8u * (uint32_t)sms || (ty == T_IQ2_XXS ? bytes + bytes / 2 : bytes) >= 147456ull * (uint32_t)sms;
+    const uint64_t raw = (uint64_t)tiles * 16 * row_bytes, bytes = ty == T_IQ2_XXS ? raw + raw / 2 : raw;
+    const bool few = tiles <= 3u * (uint32_t)sms && ty != T_IQ2_XXS && ty != T_IQ4_NL;
+    return tiles >= 8u * (uint32_t)sms || bytes >= (few ? 81920ull : 147456ull) * (uint32_t)sms;
 }
 static uint32_t gemv_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, bool sep) {
     const uint32_t n = (uint32_t)sms;
@@ -1351,12 +1356,17 @@ static uint32_t gemv_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, b
 // slice for every few tiles; and x is quantized once per cluster instead of once per CTA), or, for
 // IQ2_XXS, all 32 copies of its tables: the smallest cluster that does.  Q4_K 9728 -> 2560, 8 columns,
 // 34.0 -> 21.2 us, 4 columns 15.7 -> 12.9; IQ2_XXS 17408 -> 5120, one column 25.5 -> 21.7, four
-// 42.9 -> 35.0.  Where x fits anyway clusters cost time (Q4_K 9728 -> 2560, one column, 7.1 -> 7.9).
+// 42.9 -> 35.0.  Where x fits anyway clusters cost time (Q4_K 9728 -> 2560, one column, 7.1 -> 7.9), except
+// for one column of long rows with some more tiles than two to an SM: tiles halved between two CTAs spread
+// evenly over the chip, whole ones leave most CTAs one and a few of them two (Q4_K 17408 -> 5120 21.3 ->
+// 16.9 us, Q8_0 32.7 -> 24.6, Q6_K 39.6 -> 28.5, Q2_0 12288 -> 5120 10.7 -> 9.4; Q8_0 5120 -> 5120, 20 units of 272
+// bytes, 8.8 -> 9.5, Q4_K 9216 -> 5120, 36 of 144, 10.3 -> 10.8).
 // Row-shard launches have duties by CTA number and take no clusters.
 static bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t tiles, int sms, bool gather, GemvArgs &a,
                       GemvLayout &L, uint32_t &ctas) {
-    const uint32_t all = gemv_ctas(ty, row_bytes, tiles, sms, mode == M_SEP);
-    for (uint32_t cs = 1; cs <= 8 && !(gather && cs > 1) && cs * 4 <= nunit; cs *= 2) {
+    const uint32_t all = gemv_ctas(ty, row_bytes, tiles, sms, mode == M_SEP), n2 = 2u * (uint32_t)sms;
+    const bool halves = mode == M_SEP && tiles > n2 && tiles <= n2 + n2 / 2 && (row_bytes >= 6144 || nunit >= 40) && !gather;
+    for (uint32_t cs = halves ? 2 : 1; cs <= 8 && !(gather && cs > 1) && cs * 4 <= nunit; cs *= 2) {
         const uint32_t limit = (two_ctas(ty, row_bytes, tiles, sms, mode == M_SEP) ? 2 : 1) * (uint32_t)sms / cs;
         const uint32_t clusters = cs == 1 ? all : tiles < limit ? tiles : limit;
         if (!gemv_layout(ty, row_bytes, nunit, n, mode, cs, (tiles + clusters - 1) / clusters, a, L)) continue;

@@ -44,6 +44,15 @@ def test_columns(ctx, ty, n):
     assert ctx.device_status() == 0
 
 
+@pytest.mark.parametrize("ty", list(GGUFType))
+def test_one_column_of_long_rows(ctx, ty):
+    """Some more tiles than two to an SM (148 SMs), each halved between two CTAs: an odd number of units, a last
+    tile of one row; and one tile fewer, which is not halved."""
+    for k, m in [(10496, 296 * 16 + 1), (10496, 296 * 16)]:
+        assert run(ctx, ty, k, m, 1, torch.float16, seed=2) <= WIDE_TOL, (k, m)
+    assert ctx.device_status() == 0
+
+
 @pytest.mark.parametrize("ty", [GGUFType.Q8_0, GGUFType.Q4_0, GGUFType.IQ4_NL, GGUFType.Q2_0])
 @pytest.mark.parametrize("n", [1, 3, 4, 5, 8, 13])
 def test_rows_that_end_inside_a_unit(ctx, ty, n):
