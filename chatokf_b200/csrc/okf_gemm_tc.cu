@@ -248,6 +248,25 @@ template <int NW> struct Ldg2 {
     }
     __device__ __forceinline__ uint32_t get(int i) const { return __funnelshift_r(w[i], w[i + 1], sh); }
 };
+// The same from the NL aligned 8-byte words that hold it: sixteen rows a warp apart, every load costs the
+// L1 sixteen look-ups however wide it is, and the types with 2-byte aligned blocks were bound by them (5120 ->
+// 18944, 64 tokens, with 4-byte words: Q8_0 67 -> 46 us, Q6_K 64 -> 59, Q4_0 44 -> 37, IQ4_NL 47 -> 44).
+template <int NW, int NL> struct Ldg8 {
+    uint2 v[NL];
+    uint32_t off;  // the bytes' place in the first word: 0, 2, 4 or 6
+    __device__ __forceinline__ void load(const uint8_t *b) {
+        const uint2 *p = reinterpret_cast<const uint2 *>(reinterpret_cast<uintptr_t>(b) & ~(uintptr_t)7);
+        off = (uint32_t)reinterpret_cast<uintptr_t>(b) & 6u;
+#pragma unroll
+        for (int i = 0; i < NL; i++) v[i] = __ldg(p + i);
+    }
+    __device__ __forceinline__ uint32_t word(int i) const {
+        i = i < 2 * NL ? i : 2 * NL - 1;  // past the bytes that count
+        return i & 1 ? v[i >> 1].y : v[i >> 1].x;
+    }
+    __device__ __forceinline__ uint32_t half(int i) const { return off & 4u ? word(i + 1) : word(i); }
+    __device__ __forceinline__ uint32_t get(int i) const { return __funnelshift_r(half(i), half(i + 1), (off & 2u) * 8u); }
+};
 __device__ __forceinline__ uint32_t chunk_in_order(uint32_t h, uint32_t c4) { return h * 4 + c4; }
 
 template <int TY> struct ARaw;
@@ -316,7 +335,7 @@ template <> struct ARaw<T_Q5_K> : ARawK45<T_Q5_K> {};
 template <> struct ARaw<T_Q6_K> {
     static constexpr int kAhead = 1;
     __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return (c4 >> 1) * 4 + 2 * h + (c4 & 1); }
-    Ldg2<4> l0, l1, hq;
+    Ldg8<4, 3> l0, l1, hq;
     uint32_t sc, par;
     float d;
     __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) {
@@ -349,7 +368,7 @@ template <> struct ARaw<T_Q6_K> {
 template <> struct ARaw<T_Q8_0> {
     static constexpr int kAhead = 1;
     __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return chunk_in_order(h, c4); }
-    Ldg2<9> w;  // the 34-byte block {f16 d; i8 q[32]}
+    Ldg8<9, 5> w;  // the 34-byte block {f16 d; i8 q[32]}
     __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) { w.load(row + (size_t)(kb * 2 + h) * 34); }
     template <bool F16> __device__ __forceinline__ void unpack(uint4 (&o)[4], const uint32_t *) const {
         uint32_t u[9];
@@ -367,7 +386,7 @@ template <> struct ARaw<T_Q8_0> {
 template <int TY> struct ARaw40 {
     static constexpr int kAhead = 1;
     __device__ static __forceinline__ uint32_t chunk(uint32_t h, uint32_t c4) { return chunk_in_order(h, c4); }
-    Ldg2<5> w;
+    Ldg8<5, 3> w;
     __device__ __forceinline__ void load(const uint8_t *row, uint32_t kb, uint32_t h) { w.load(row + (size_t)(kb * 2 + h) * 18); }
     template <bool F16> __device__ __forceinline__ void unpack(uint4 (&o)[4], const uint32_t *) const {
         uint32_t u[5], q[4];
