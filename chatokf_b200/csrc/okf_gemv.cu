@@ -1,5 +1,4 @@
-// Decode matvec kernels (1..8 activation columns) for Q4_K, Q8_0, Q2_0 and
-// IQ2_XXS.  Replaces the reference's kq_gemv_impl / kq_gemm_nb_impl / q2_0_gemv
+// Decode matvec kernels (1..8 activation columns) for every block type.  Replaces the reference's kq_gemv_impl / kq_gemm_nb_impl / q2_0_gemv
 // families (LLM/metal/Kernels.metal:26-109, :1572-1753).  See okf_gemv_mma.cuh
 // for the data path and the MMA operand layout.
 //
@@ -21,14 +20,14 @@
 // gives the same result whatever the batch width.
 //
 // Integer tensor cores.  Weights go into the MMA as the bytes they are stored as
-// (nibbles and 2-bit codes after one AND, Q8_0 and the IQ2_XXS codebook
-// untouched), x as the hi / lo bytes, mma.sync m16n8k32 with s32 accumulators:
+// (nibbles and 2-bit codes after one AND, Q8_0 untouched, IQ2_XXS and IQ4_NL as
+// looked up), x as the hi / lo bytes, mma.sync m16n8k32 with s32 accumulators:
 // the sums are exact integers; scales, mins and biases are applied afterwards.
 //   One column ("SEP"): MMA column g stands for (quarter g / 2 of the unit, byte
 // g % 2 of x).  Thread c of a quad owns the k of quarter c and feeds x only into
 // that quarter's columns, so the accumulator a thread reads back is the sum over
 // exactly the 64 k whose block scales it decoded.
-//   Several columns ("WIDE"): x is the A operand, see okf_gemv_wide.cuh.
+//   Several columns ("WIDE"): see okf_gemv_wide.cuh.
 #include <cooperative_groups.h>
 
 #include "okf_gemv_mma.cuh"
