@@ -890,6 +890,9 @@ struct ReduceOut {
     void *outs[8];
     uint32_t *epoch;
     uint32_t epoch_inc;
+    // fp32 results leave as 16-byte words: every row of every output starts on a 16-byte boundary.  Decided
+    // from the addresses too: an fp32 output need only be 4-byte aligned (a view into a larger tensor).
+    bool vec;
 };
 constexpr uint32_t kReduceTok = 16;
 template <typename OT>
@@ -903,7 +906,6 @@ __global__ void __launch_bounds__(256) reduce_kernel(const float *__restrict__ p
     pdl_wait();
     if (o.epoch && blockIdx.x == 0 && threadIdx.x == 0) o.epoch[0] += o.epoch_inc;
     if (c0 == c1) return;  // one CTA took the whole item and stored it
-    const bool vec = (o.m & 3) == 0 && (o.out_ld & 3) == 0 && (o.out_row0 & 3) == 0 && sizeof(OT) == 4;
     for (uint32_t t = t0 + (threadIdx.x >> 5); t < min(t0 + kReduceTok, o.nt); t += 8) {
         if (n0 + t >= o.n || row >= o.m) break;
         const float *src = part + ((size_t)i * o.nt + t) * kBM + r;
@@ -917,7 +919,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const float *__restrict__ p
         const float e[4] = {v.x, v.y, v.z, v.w};
         for (uint32_t b = 0; b < o.nout; b++) {
             OT *out = reinterpret_cast<OT *>(o.outs[b]) + at;
-            if (vec) {
+            if (sizeof(OT) == 4 && o.vec) {
                 *reinterpret_cast<float4 *>(out) = v;
             } else {
 #pragma unroll
@@ -993,8 +995,11 @@ static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int s
     cudaError_t e = launch_pdl(gemm_tc_kernel<TY, XDT, OT, NACC>, grid, kThreads, Rings<TY, NACC>::smem, s, 1, xmap, a, g);
     if (e != cudaSuccess || !a.dealt) return e;
     ReduceOut ro = {go.nout, a.m, a.n, go.out_ld, go.out_row0, a.dealt, items, a.k / kBK, a.dealers, a.nt, groups, NACC * kBN, {}, go.epoch,
-                    go.epoch_inc};
-    for (uint32_t o = 0; o < go.nout; o++) ro.outs[o] = go.outs[o];
+                    go.epoch_inc, ((a.m | go.out_ld | go.out_row0) & 3) == 0};
+    for (uint32_t o = 0; o < go.nout; o++) {
+        ro.outs[o] = go.outs[o];
+        ro.vec = ro.vec && (uintptr_t)go.outs[o] % 16 == 0;
+    }
     using RT = std::conditional_t<kIsGather<OT>, float, OT>;
     return launch_pdl(reduce_kernel<RT>, a.dealt * ((a.nt + kReduceTok - 1) / kReduceTok), 256, 0, s, 1, (const float *)a.partial, ro);
 }

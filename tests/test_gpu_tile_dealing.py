@@ -64,3 +64,26 @@ def test_streams_do_not_share_partial_tiles(ctx):
         # fp32 sums in another order at most (streams beyond the buffers take another plan)
         assert rel_err(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("k,m,n", [(2560, 9728, 77), (4096, 1000, 40), (1024, 1024, 16)])
+@pytest.mark.parametrize("shift", [1, 2, 4])
+def test_outputs_that_are_only_4_byte_aligned(ctx, k, m, n, shift):
+    """Dealt matmuls (two kernels) whose fp32 output is a view at some float of a larger tensor, rows a
+    multiple of four floats: the same bits as into an aligned tensor, and nothing beside the view."""
+    ty = GGUFType.Q4_0
+    w = ctx.upload(synth.random_blocks(ty, m * k // block_elems(ty), np.random.default_rng(m)))
+    t = GGUFTensor("w", (k, m), ty)
+    enc = CudaEnc(ctx)
+    X = torch.randn(n, k, device="cuda").half()
+    for call in (enc.gemm, enc.gemm_noalloc):
+        flat = torch.full((n * m + 8,), float("nan"), device="cuda")
+        want = torch.empty(n * m, device="cuda")
+        before = ctx.launches
+        call(t, X, want, w, n)
+        assert ctx.launches - before == 2, "the shape is dealt"
+        call(t, X, flat[shift:shift + n * m], w, n)
+        torch.cuda.synchronize()
+        assert torch.equal(flat[shift:shift + n * m], want)
+        assert torch.isnan(flat[:shift]).all() and torch.isnan(flat[shift + n * m:]).all()
+    assert ctx.device_status() == 0
