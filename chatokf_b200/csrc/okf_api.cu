@@ -19,8 +19,17 @@ constexpr size_t kTailPad = 256;  // bytes readable past the last block of an up
         if (e_ != cudaSuccess) return cuda_fail((ctx), e_);   \
     } while (0)
 
+// Allocating and freeing are no part of what streams do, but by default CUDA refuses them, and gives up
+// the capture, while any stream is being captured.
+struct AllowInCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AllowInCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AllowInCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 int grow(okf_ctx *ctx, void **buf, size_t *have, size_t need) {
     if (*have >= need) return OKF_OK;
+    AllowInCapture allow;
     if (*buf) OKF_CUDA(ctx, cudaFree(*buf));
     *buf = nullptr;
     *have = 0;
@@ -110,43 +119,101 @@ int par_flush(okf_ctx *ctx) {
     return e == cudaSuccess ? OKF_OK : cuda_fail(ctx, e);
 }
 
-// Launch the tensor-core matmul with what stream `s` may use of the context's working memory.  While a
-// stream is captured nothing can be allocated: what calls outside the capture have left has to do.
+// The set of working memory of a stream outside captures, or null.
+okf_ctx::Lane *lane_of(okf_ctx *ctx, cudaStream_t s) {
+    okf_ctx::Lane *unused = nullptr;
+    for (auto &l : ctx->lanes) {
+        if (l.used && l.stream == s) return &l;
+        if (!l.used && !unused) unused = &l;
+    }
+    if (unused) {
+        unused->used = true;
+        unused->stream = s;
+    }
+    return unused;
+}
+
+void CUDART_CB graph_let_go(void *p) {
+    okf_graph_buffer *b = (okf_graph_buffer *)p;
+    if (b->holders.fetch_sub(1) == 1) delete b;
+}
+// Give back what no graph holds any more, or (`all`: the context goes) everything.
+void free_graph_buffers(okf_ctx *ctx, bool all) {
+    for (okf_graph_buffer **at = &ctx->graph_buffers; *at;) {
+        okf_graph_buffer *b = *at;
+        if (!all && b->holders.load() > 1) {
+            at = &b->next;
+            continue;
+        }
+        *at = b->next;
+        AllowInCapture allow;
+        (void)cudaFree(b->ptr);
+        (void)cudaGetLastError();
+        graph_let_go(b);
+    }
+}
+// Memory for a call that is being captured on `s`, of the capture's graph; null where there is none.
+void *graph_buffer(okf_ctx *ctx, cudaStream_t s, int kind, size_t need) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(s, &cs, &capture, &graph, nullptr, nullptr) != cudaSuccess || cs != cudaStreamCaptureStatusActive) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    for (okf_graph_buffer *b = ctx->graph_buffers; b; b = b->next)
+        if (b->capture == capture && b->stream == s && b->kind == kind && b->bytes >= need && b->holders.load() > 1) return b->ptr;
+    AllowInCapture allow;
+    okf_graph_buffer *b = new (std::nothrow) okf_graph_buffer{{1}, nullptr, need, capture, s, kind, ctx->graph_buffers};
+    if (!b) return nullptr;
+    cudaUserObject_t held;
+    if (cudaMalloc(&b->ptr, need) != cudaSuccess) {
+        (void)cudaGetLastError();
+        delete b;
+        return nullptr;
+    }
+    ctx->graph_buffers = b;
+    b->holders = 2;
+    if (cudaUserObjectCreate(&held, b, graph_let_go, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        (void)cudaGetLastError();
+        b->holders = 1;
+        return nullptr;
+    }
+    if (cudaGraphRetainUserObject(graph, held, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        (void)cudaGetLastError();
+        (void)cudaUserObjectRelease(held, 1);
+        return nullptr;
+    }
+    return b->ptr;
+}
+
+// Launch the tensor-core matmul with the working memory that stream `s`, or the graph it is captured into,
+// has for it.  Without any another plan is taken, and fp32 activations are converted by the tile itself.
 cudaError_t run_tile(okf_ctx *ctx, int ty, const uint8_t *wp, uint32_t k, uint32_t m, const void *x, int xdt, uint32_t n,
                      void *out, int odt, cudaStream_t s, const GemvGatherPlan *gather) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    (void)cudaStreamIsCapturing(s, &cs);
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) (void)cudaGetLastError();
     const bool capturing = cs != cudaStreamCaptureStatusNone;
-    okf_ctx::Lane *lane = nullptr, *unused = nullptr, *largest = nullptr;
-    for (auto &l : ctx->lanes) {
-        if (l.used && l.stream == s) lane = &l;
-        if (!l.used && !unused) unused = &l;
-        if (l.used && (!largest || l.part_bytes + l.conv_bytes > largest->part_bytes + largest->conv_bytes)) largest = &l;
-    }
-    if (!lane && capturing) lane = largest;
-    if (!lane && !capturing && unused) {
-        lane = unused;
-        lane->used = true;
-        lane->stream = s;
-    }
-    const size_t cb = (size_t)n * k * 2;
-    if (lane && xdt == DT_F32 && !gather) {
-        if (!capturing) (void)grow(ctx, &lane->conv, &lane->conv_bytes, cb);
-        if (lane->conv_bytes >= cb) {
+    if (!capturing && ctx->graph_buffers) free_graph_buffers(ctx, false);
+    okf_ctx::Lane *lane = capturing ? nullptr : lane_of(ctx, s);
+    auto memory = [&](int kind, void **buf, size_t *have, size_t need) -> void * {
+        if (capturing) return graph_buffer(ctx, s, kind, need);
+        return buf && grow(ctx, buf, have, need) == OKF_OK ? *buf : nullptr;
+    };
+    if (xdt == DT_F32 && !gather) {
+        if (void *conv = memory(1, lane ? &lane->conv : nullptr, lane ? &lane->conv_bytes : nullptr, (size_t)n * k * 2)) {
             // every slab of W would convert all of X again, and by a part of the warps
-            cudaError_t e = launch_to_bf16(x, lane->conv, (size_t)n * k, ctx->sms, s);
+            cudaError_t e = launch_to_bf16(x, conv, (size_t)n * k, ctx->sms, s);
             if (e != cudaSuccess) return e;
             ctx->launches++;
-            x = lane->conv;
+            x = conv;
             xdt = DT_BF16;
         }
     }
-    if (lane && !capturing) {
-        const size_t need = gemm_tc_scratch(ty, k, m, n, xdt, ctx->sms) * sizeof(float);
-        if (need) (void)grow(ctx, &lane->part, &lane->part_bytes, need);  // without it another plan is taken
-    }
-    return launch_gemm_tc(ty, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, lane ? (float *)lane->part : nullptr,
-                          lane ? lane->part_bytes / sizeof(float) : 0, s, ctx->sms, ctx->device, &ctx->launches, gather);
+    const size_t floats = gemm_tc_scratch(ty, k, m, n, xdt, ctx->sms);
+    void *part = floats ? memory(0, lane ? &lane->part : nullptr, lane ? &lane->part_bytes : nullptr, floats * sizeof(float)) : nullptr;
+    return launch_gemm_tc(ty, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, (float *)part, part ? floats : 0, s, ctx->sms,
+                          ctx->device, &ctx->launches, gather);
 }
 
 int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uint32_t k, uint32_t m,
@@ -280,6 +347,7 @@ void okf_destroy(okf_ctx *ctx) {
         if (l.part) cudaFree(l.part);
         if (l.conv) cudaFree(l.conv);
     }
+    free_graph_buffers(ctx, true);
     if (ctx->stage_x) cudaFree(ctx->stage_x);
     if (ctx->stage_out) cudaFree(ctx->stage_out);
     if (ctx->pin_x) cudaFreeHost(ctx->pin_x);

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/okf_cuda.h"
 #include "okf_blocks.cuh"
 
@@ -13,6 +15,19 @@ struct okf_weights {
 };
 
 #include "okf_kernels.h"
+
+// Working memory of captured matmuls.  The graph they are captured into holds it (as a user object, whose
+// references follow copies, instances and updates of the graph), so a replay never meets memory that has
+// been freed or that another call is using; the context frees it once no graph holds it.
+struct okf_graph_buffer {
+    std::atomic<int> holders;  // the context's list, the graph
+    void *ptr;
+    size_t bytes;
+    unsigned long long capture;  // calls of one stream in one capture run in order and share it
+    cudaStream_t stream;
+    int kind;                            // partial tiles, bf16 activations
+    okf_graph_buffer *next;
+};
 
 struct okf_ctx {
     int device;
@@ -42,6 +57,8 @@ struct okf_ctx {
         void *part, *conv;
         size_t part_bytes, conv_bytes;
     } lanes[16];
+    // what calls in stream captures were given: a graph's memory is its own
+    okf_graph_buffer *graph_buffers;
     // staged faults (host side only)
     double fault_rate;
     uint64_t fault_state;
