@@ -120,17 +120,37 @@ int par_flush(okf_ctx *ctx) {
 }
 
 // The set of working memory of a stream outside captures, or null.
+constexpr uint64_t kLaneIdle = 1024;
 okf_ctx::Lane *lane_of(okf_ctx *ctx, cudaStream_t s) {
-    okf_ctx::Lane *unused = nullptr;
+    unsigned long long id = 0;
+    {
+        AllowInCapture allow;
+        if (cudaStreamGetId(s, &id) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+    }
+    okf_ctx::Lane *unused = nullptr, *oldest = nullptr;
     for (auto &l : ctx->lanes) {
-        if (l.used && l.stream == s) return &l;
+        if (l.used && l.stream == id) {
+            l.last = ctx->tile_calls;
+            return &l;
+        }
         if (!l.used && !unused) unused = &l;
+        if (l.used && (!oldest || l.last < oldest->last)) oldest = &l;
     }
-    if (unused) {
-        unused->used = true;
-        unused->stream = s;
+    okf_ctx::Lane *lane = unused;
+    if (!lane) {
+        if (ctx->tile_calls - oldest->last < kLaneIdle) return nullptr;
+        lane = oldest;
+        // (cudaFree returns when the device has finished with the memory)
+        AllowInCapture allow;
+        if (lane->part) (void)cudaFree(lane->part);
+        if (lane->conv) (void)cudaFree(lane->conv);
+        (void)cudaGetLastError();
     }
-    return unused;
+    *lane = {id, true, ctx->tile_calls, nullptr, nullptr, 0, 0};
+    return lane;
 }
 
 void CUDART_CB graph_let_go(void *p) {
@@ -189,31 +209,46 @@ void *graph_buffer(okf_ctx *ctx, cudaStream_t s, int kind, size_t need) {
 
 // Launch the tensor-core matmul with the working memory that stream `s`, or the graph it is captured into,
 // has for it.  Without any another plan is taken, and fp32 activations are converted by the tile itself.
+constexpr size_t kMaxConvBytes = (size_t)256 << 20;
 cudaError_t run_tile(okf_ctx *ctx, int ty, const uint8_t *wp, uint32_t k, uint32_t m, const void *x, int xdt, uint32_t n,
                      void *out, int odt, cudaStream_t s, const GemvGatherPlan *gather) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) (void)cudaGetLastError();
     const bool capturing = cs != cudaStreamCaptureStatusNone;
     if (!capturing && ctx->graph_buffers) free_graph_buffers(ctx, false);
+    ctx->tile_calls++;
     okf_ctx::Lane *lane = capturing ? nullptr : lane_of(ctx, s);
     auto memory = [&](int kind, void **buf, size_t *have, size_t need) -> void * {
         if (capturing) return graph_buffer(ctx, s, kind, need);
         return buf && grow(ctx, buf, have, need) == OKF_OK ? *buf : nullptr;
     };
-    if (xdt == DT_F32 && !gather) {
-        if (void *conv = memory(1, lane ? &lane->conv : nullptr, lane ? &lane->conv_bytes : nullptr, (size_t)n * k * 2)) {
-            // every slab of W would convert all of X again, and by a part of the warps
-            cudaError_t e = launch_to_bf16(x, conv, (size_t)n * k, ctx->sms, s);
-            if (e != cudaSuccess) return e;
-            ctx->launches++;
-            x = conv;
-            xdt = DT_BF16;
+    // More activations than kMaxConvBytes holds are taken in runs of tokens, so that what is kept is bounded.
+    const bool convert = xdt == DT_F32 && !gather;
+    const size_t most = kMaxConvBytes / 2 / k / 512 * 512;
+    const uint32_t step = convert && most && most < n ? (uint32_t)most : n;
+    for (uint32_t n0 = 0; n0 < n; n0 += step) {
+        const uint32_t nn = n - n0 < step ? n - n0 : step;
+        const uint8_t *xp = (const uint8_t *)x + (size_t)n0 * k * dtype_size(xdt);
+        const void *xa = xp;
+        int xadt = xdt;
+        const size_t cb = (size_t)nn * k * 2;
+        if (convert && cb <= kMaxConvBytes) {
+            if (void *conv = memory(1, lane ? &lane->conv : nullptr, lane ? &lane->conv_bytes : nullptr, cb)) {
+                // every slab of W would convert all of X again, and by a part of the warps
+                cudaError_t e = launch_to_bf16(xp, conv, (size_t)nn * k, ctx->sms, s);
+                if (e != cudaSuccess) return e;
+                ctx->launches++;
+                xa = conv;
+                xadt = DT_BF16;
+            }
         }
+        const size_t floats = gemm_tc_scratch(ty, k, m, nn, xadt, ctx->sms);
+        void *part = floats ? memory(0, lane ? &lane->part : nullptr, lane ? &lane->part_bytes : nullptr, floats * sizeof(float)) : nullptr;
+        cudaError_t e = launch_gemm_tc(ty, wp, k, m, xa, xadt, nn, gather ? out : (uint8_t *)out + (size_t)n0 * m * dtype_size(odt), odt,
+                                       ctx->dev_status, (float *)part, part ? floats : 0, s, ctx->sms, ctx->device, &ctx->launches, gather);
+        if (e != cudaSuccess) return e;
     }
-    const size_t floats = gemm_tc_scratch(ty, k, m, n, xdt, ctx->sms);
-    void *part = floats ? memory(0, lane ? &lane->part : nullptr, lane ? &lane->part_bytes : nullptr, floats * sizeof(float)) : nullptr;
-    return launch_gemm_tc(ty, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, (float *)part, part ? floats : 0, s, ctx->sms,
-                          ctx->device, &ctx->launches, gather);
+    return cudaSuccess;
 }
 
 int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uint32_t k, uint32_t m,

@@ -48,15 +48,19 @@ struct okf_ctx {
     size_t pin_x_bytes;
     void *pin_out;
     size_t pin_out_bytes;
-    // what the tensor-core matmul works in, one set per stream (calls on different streams may
-    // overlap), grown on demand: partial tiles and bf16 copies of fp32 activations.  Calls on
-    // further streams do without.
+    // What the tensor-core matmul works in, one set per stream (calls on different streams may overlap),
+    // grown on demand: partial tiles and bf16 copies of fp32 activations.  Streams are told apart by their id,
+    // which unlike the handle is never given out twice and differs between threads for the per-thread
+    // default stream.  When all sets are taken, the one that has been idle for kLaneIdle matmuls
+    // is given to the stream that asks; while there is none calls on further streams do without.
     struct Lane {
-        cudaStream_t stream;
+        unsigned long long stream;
         bool used;
+        uint64_t last;  // tile_calls when it was used last
         void *part, *conv;
         size_t part_bytes, conv_bytes;
     } lanes[16];
+    uint64_t tile_calls;
     // what calls in stream captures were given: a graph's memory is its own
     okf_graph_buffer *graph_buffers;
     // staged faults (host side only)

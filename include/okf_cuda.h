@@ -116,11 +116,13 @@ OKF_API int okf_gemv(okf_ctx *ctx, int type, const okf_weights *w, uint64_t woff
  * larger N the tensor-core tile (gemmTiled, MetalEnc.swift:377-400).  X holds
  * N*K elements of xdt; out holds N*M elements of odt (OKF_F32 or OKF_BF16).
  * Where work does not fill the SMs the tile cuts K into ranges whose partial sums, and
- * bf16 copies of fp32 activations, live in buffers of the context, one set per stream:
- * calls on different streams may overlap on the GPU.  A stream capture gets memory that
- * belongs to its graph (allocated while it is captured, freed by a later call or okf_destroy
- * once the graph and its instances are gone): a graph may be replayed beside any other
- * call or graph, but not after okf_destroy.
+ * bf16 copies of fp32 activations, live in buffers of the context, one set per stream
+ * for sixteen streams: calls on different streams may overlap on the GPU.  A set keeps
+ * at most 256 MiB of each; a seventeenth stream works without one, by slower plans, until
+ * a set has been idle for 1024 matmuls and goes over to it.  A stream capture gets
+ * memory that belongs to its graph (allocated while it is captured, freed by a later call or
+ * okf_destroy once the graph and its instances are gone): a graph may be replayed beside
+ * any other call or graph, but not after okf_destroy.
  * Numerics: for N <= 8 (fp32 out) every 256-wide run of an activation column is
  * reduced to 16-bit integers (24-bit where K is no multiple of 256) with one fp32
  * scale and the sums are exact integers

@@ -44,7 +44,7 @@ def test_dealing(ctx, k, m, n, odt):
 
 
 def test_streams_do_not_share_partial_tiles(ctx):
-    """Calls of one context on several streams at once, more streams than the context has buffers for."""
+    """Calls of one context on several streams at once (streams beyond the context's sets: test_gpu_tile_memory.py)."""
     ty, k, m, n = GGUFType.Q4_K, 4096, 1000, 40
     rng = np.random.default_rng(1)
     w = ctx.upload(synth.random_blocks(ty, m * k // block_elems(ty), rng))
@@ -61,7 +61,7 @@ def test_streams_do_not_share_partial_tiles(ctx):
             CudaEnc(ctx, s).gemm(t, x, o, w, n)
     torch.cuda.synchronize()
     for a, b in zip(got, want):
-        # fp32 sums in another order at most (streams beyond the buffers take another plan)
+        # the same plan on every stream; fp32 sums in another order at most
         assert rel_err(a.cpu().numpy(), b.cpu().numpy()) <= 1e-5
     assert ctx.device_status() == 0
 

@@ -9,6 +9,7 @@ import torch
 from chatokf_b200 import synth
 from chatokf_b200.enc import Context, CudaEnc, GGUFTensor
 from chatokf_b200.gguf_types import GGUFType, block_elems
+from helpers import rel_err
 
 pytestmark = pytest.mark.gpu
 
@@ -117,3 +118,46 @@ def test_a_graphs_memory_is_given_back(own):
     torch.cuda.synchronize()
     enc.gemm(t, X, out, w, n)  # a call outside captures frees what no graph holds
     assert held - used() >= 8 * (60 << 20)
+
+
+def test_more_streams_than_sets(own):
+    """Sixteen streams have a set each; further ones convert in the tile and deal nothing out, until a set
+    has been idle for 1024 matmuls."""
+    c, w, t = own
+    n = 40
+    X, want, got = torch.randn(n, K, device="cuda"), torch.empty(n, M, device="cuda"), torch.empty(n, M, device="cuda")
+    streams = [torch.cuda.Stream() for _ in range(20)]
+    ids = {s.cuda_stream for s in streams}
+    assert len(ids) == 20
+    for i, s in enumerate(streams):
+        assert launches(c, lambda: CudaEnc(c, s).gemm(t, X, got, w, n)) == (3 if i < 16 else 1)
+        torch.cuda.synchronize()
+        if i == 0:
+            want.copy_(got)
+        # the same operands, fp32 sums in another order
+        assert rel_err(got.cpu().numpy(), want.cpu().numpy()) <= 1e-5
+    for _ in range(1024):
+        CudaEnc(c, streams[0]).gemm(t, X, got, w, n)
+    assert launches(c, lambda: CudaEnc(c, streams[19]).gemm(t, X, got, w, n)) == 3
+    assert launches(c, lambda: CudaEnc(c, streams[0]).gemm(t, X, got, w, n)) == 3
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    assert c.device_status() == 0
+
+
+def test_more_activations_than_a_set_keeps(lib_built):
+    """256 MiB of bf16 activations are kept at most: more are converted and multiplied run by run of tokens."""
+    c = Context(0)
+    k, m, n = 17408, 70, 8201
+    w = c.upload(synth.random_blocks(GGUFType.Q4_0, m * k // 32, np.random.default_rng(5)))
+    t = GGUFTensor("w", (k, m), GGUFType.Q4_0)
+    X = torch.randn(n, k, device="cuda")
+    got, want = torch.full((n * m + 8,), float("nan"), device="cuda"), torch.empty(n * m, device="cuda")
+    CudaEnc(c).gemm(t, X.bfloat16(), want, w, n)
+    CudaEnc(c).gemm(t, X, got, w, n)
+    torch.cuda.synchronize()
+    assert torch.isnan(got[n * m:]).all()
+    # the same operands, fp32 sums in another order
+    assert rel_err(got[:n * m].cpu().numpy(), want.cpu().numpy()) <= 1e-5
+    assert c.device_status() == 0
+    c.close()
