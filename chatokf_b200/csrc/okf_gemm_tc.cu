@@ -25,7 +25,6 @@
 //
 // Every mbarrier wait is bounded (about a second); a wait that gives up records
 // a code in the status word, the CTA frees its tensor memory and returns.
-#include <type_traits>
 #include <cuda.h>
 
 #include <cstring>
@@ -705,6 +704,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
             uint32_t s = 0, use = 0;
             Work wk;
             pdl_wait();
+            const float *x = dep_ptr(reinterpret_cast<const float *>(p.x));
             for (uint32_t j = 0; next_work<NACC>(p, j, wk); j++) {
                 const uint32_t n0 = wk.n0;
                 for (uint32_t kb = wk.kb0; kb < wk.kb1; kb++, s = s + 1 == kBStages ? (use++, 0) : s + 1) {
@@ -722,8 +722,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
                         const size_t e = (size_t)min(tok, p.n - 1) * p.k + (size_t)kb * kBK + c16 * 8;
                         uint4 v = make_uint4(0u, 0u, 0u, 0u);
                         if (tok < p.n && row < wk.ntok) {
-                            const float4 f0 = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.x) + e));
-                            const float4 f1 = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p.x) + e) + 1);
+                            const float4 f0 = ld_dep(reinterpret_cast<const float4 *>(x + e));
+                            const float4 f1 = ld_dep(reinterpret_cast<const float4 *>(x + e) + 1);
                             v.x = pack16<false>(f0.x, f0.y); v.y = pack16<false>(f0.z, f0.w);
                             v.z = pack16<false>(f1.x, f1.y); v.w = pack16<false>(f1.z, f1.w);
                         }
@@ -890,13 +890,14 @@ struct ReduceOut {
     void *outs[8];
     uint32_t *epoch;
     uint32_t epoch_inc;
-    // fp32 results leave as 16-byte words: every row of every output starts on a 16-byte boundary.  Decided
-    // from the addresses too: an fp32 output need only be 4-byte aligned (a view into a larger tensor).
-    bool vec;
 };
 constexpr uint32_t kReduceTok = 16;
-template <typename OT>
-__global__ void __launch_bounds__(256) reduce_kernel(const float *__restrict__ part, ReduceOut o) {
+// VEC: fp32 results leave as 16-byte words, as every row of every output starts on a 16-byte boundary.  The host
+// decides, from the addresses too: an fp32 output need only be 4-byte aligned (a view into a larger tensor).
+// (As a run-time flag the test stood between the loads of one token and the next: Q5_K 2560 -> 9728, 77 tokens,
+// 21.4 us instead of 19.1.)
+template <typename OT, bool VEC>
+__global__ void __launch_bounds__(256) reduce_kernel(const float *part, ReduceOut o) {
     pdl_launch_dependents();
     const uint32_t runs = (o.nt + kReduceTok - 1) / kReduceTok;
     const uint32_t i = blockIdx.x / runs, t0 = blockIdx.x % runs * kReduceTok, total = o.dealt * o.kblocks;
@@ -906,20 +907,21 @@ __global__ void __launch_bounds__(256) reduce_kernel(const float *__restrict__ p
     pdl_wait();
     if (o.epoch && blockIdx.x == 0 && threadIdx.x == 0) o.epoch[0] += o.epoch_inc;
     if (c0 == c1) return;  // one CTA took the whole item and stored it
+    const float *parts = dep_ptr(part);
     for (uint32_t t = t0 + (threadIdx.x >> 5); t < min(t0 + kReduceTok, o.nt); t += 8) {
         if (n0 + t >= o.n || row >= o.m) break;
-        const float *src = part + ((size_t)i * o.nt + t) * kBM + r;
+        const float *src = parts + ((size_t)i * o.nt + t) * kBM + r;
         const size_t step = (size_t)o.dealt * o.nt * kBM;
-        float4 v = *reinterpret_cast<const float4 *>(src);
+        float4 v = ld_dep(reinterpret_cast<const float4 *>(src));
         for (uint32_t c = c0 + 1; c <= c1; c++) {
-            const float4 a = *reinterpret_cast<const float4 *>(src + (c - c0) * step);
+            const float4 a = ld_dep(reinterpret_cast<const float4 *>(src + (c - c0) * step));
             v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
         }
         const size_t at = (size_t)(n0 + t) * o.out_ld + o.out_row0 + row;
         const float e[4] = {v.x, v.y, v.z, v.w};
         for (uint32_t b = 0; b < o.nout; b++) {
             OT *out = reinterpret_cast<OT *>(o.outs[b]) + at;
-            if (sizeof(OT) == 4 && o.vec) {
+            if constexpr (VEC) {
                 *reinterpret_cast<float4 *>(out) = v;
             } else {
 #pragma unroll
@@ -995,13 +997,20 @@ static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int s
     cudaError_t e = launch_pdl(gemm_tc_kernel<TY, XDT, OT, NACC>, grid, kThreads, Rings<TY, NACC>::smem, s, 1, xmap, a, g);
     if (e != cudaSuccess || !a.dealt) return e;
     ReduceOut ro = {go.nout, a.m, a.n, go.out_ld, go.out_row0, a.dealt, items, a.k / kBK, a.dealers, a.nt, groups, NACC * kBN, {}, go.epoch,
-                    go.epoch_inc, ((a.m | go.out_ld | go.out_row0) & 3) == 0};
+                    go.epoch_inc};
+    bool vec = ((a.m | go.out_ld | go.out_row0) & 3) == 0;
     for (uint32_t o = 0; o < go.nout; o++) {
         ro.outs[o] = go.outs[o];
-        ro.vec = ro.vec && (uintptr_t)go.outs[o] % 16 == 0;
+        vec = vec && (uintptr_t)go.outs[o] % 16 == 0;
     }
-    using RT = std::conditional_t<kIsGather<OT>, float, OT>;
-    return launch_pdl(reduce_kernel<RT>, a.dealt * ((a.nt + kReduceTok - 1) / kReduceTok), 256, 0, s, 1, (const float *)a.partial, ro);
+    const unsigned blocks = a.dealt * ((a.nt + kReduceTok - 1) / kReduceTok);
+    const float *part = a.partial;
+    if constexpr (sizeof(OT) == 4) {
+        if (vec) return launch_pdl(reduce_kernel<float, true>, blocks, 256, 0, s, 1, part, ro);
+        return launch_pdl(reduce_kernel<float, false>, blocks, 256, 0, s, 1, part, ro);
+    } else {
+        return launch_pdl(reduce_kernel<OT, false>, blocks, 256, 0, s, 1, part, ro);
+    }
 }
 
 template <int TY, int XDT, typename OT>
@@ -1033,11 +1042,12 @@ static cudaError_t launch_x(const Args &a, const Outs &go, const GemmPlan &plan,
 }  // namespace tc
 
 // fp32 activations -> bf16, once for all slabs, so that they come by TMA like the others.
-__global__ void __launch_bounds__(256) to_bf16_kernel(const float4 *__restrict__ x, uint4 *__restrict__ y, size_t n8) {
+__global__ void __launch_bounds__(256) to_bf16_kernel(const float4 *x, uint4 *__restrict__ y, size_t n8) {
     pdl_launch_dependents();
     pdl_wait();
+    const float4 *in = dep_ptr(x);
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
-        const float4 a = x[2 * i], b = x[2 * i + 1];
+        const float4 a = ld_dep(in + 2 * i), b = ld_dep(in + 2 * i + 1);
         y[i] = make_uint4(tc::pack16<false>(a.x, a.y), tc::pack16<false>(a.z, a.w), tc::pack16<false>(b.x, b.y), tc::pack16<false>(b.z, b.w));
     }
 }

@@ -522,7 +522,7 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
                                                               ((size_t)u_first * 256 + (size_t)i * 8) * (XDT == DT_F32 ? 4 : 2));
 #pragma unroll
             for (int j = 0; j < (XDT == DT_F32 ? 2 : 1); j++)
-                raw[r].v[j] = i < items ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
+                raw[r].v[j] = i < items ? src[j] : make_uint4(0u, 0u, 0u, 0u);
         }
 #pragma unroll
         for (uint32_t r = 0; r < kFlight; r++) {
@@ -621,7 +621,7 @@ __device__ __forceinline__ void stage_x_wide(uint32_t xs32, uint32_t es, uint32_
             const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(x) +
                                                               ((size_t)lcol * kdim + k0) * (XDT == DT_F32 ? 4 : 2));
 #pragma unroll
-            for (int j = 0; j < (XDT == DT_F32 ? 2 : 1); j++) raw[r].v[j] = live ? __ldg(src + j) : make_uint4(0u, 0u, 0u, 0u);
+            for (int j = 0; j < (XDT == DT_F32 ? 2 : 1); j++) raw[r].v[j] = live ? src[j] : make_uint4(0u, 0u, 0u, 0u);
             step(lcol, lu);
         }
 #pragma unroll

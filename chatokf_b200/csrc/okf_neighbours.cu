@@ -30,7 +30,7 @@ namespace okf {
 // and code 8 in the device status word.
 constexpr int kStatusBadId = 8;
 template <int TY>
-__global__ void __launch_bounds__(256) embed_kernel(const uint8_t *__restrict__ w, const int *__restrict__ ids,
+__global__ void __launch_bounds__(256) embed_kernel(const uint8_t *__restrict__ w, const int *ids,
                                                     uint32_t k, uint32_t n, uint32_t rows, float *__restrict__ out,
                                                     int *bad) {
     __shared__ uint64_t grid_s[256];
@@ -96,7 +96,7 @@ __device__ __forceinline__ void argmax_take(float &bv, int &bi, float ov, int oi
 // A logits row is 600 KB at a vocabulary of 151936, more than one SM can take from L2 in the time
 // of a launch; rows below kArgmaxSplit stay with one CTA.
 constexpr uint32_t kArgmaxCluster = 8, kArgmaxSplit = 16384;
-__global__ void __launch_bounds__(256, 6) argmax_rows_kernel(const float *__restrict__ x, int *__restrict__ out, uint32_t n,
+__global__ void __launch_bounds__(256, 6) argmax_rows_kernel(const float *x, int *__restrict__ out, uint32_t n,
                                                           uint32_t parts) {
     __shared__ float bestv[8 + kArgmaxCluster];  // per warp, then per CTA of the cluster
     __shared__ int besti[8 + kArgmaxCluster];
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256, 6) argmax_rows_kernel(const float *__rest
         const float4 *r4 = reinterpret_cast<const float4 *>(row);
 #pragma unroll 4
         for (uint32_t i = first; i < n / 4; i += step) {
-            const float4 v = __ldg(r4 + i);
+            const float4 v = r4[i];
             if (v.x > bv) { bv = v.x; bi = (int)(4 * i); }
             if (v.y > bv) { bv = v.y; bi = (int)(4 * i + 1); }
             if (v.z > bv) { bv = v.z; bi = (int)(4 * i + 2); }
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(256, 6) argmax_rows_kernel(const float *__rest
     } else {
 #pragma unroll 4
         for (uint32_t i = first; i < n; i += step) {
-            const float v = __ldg(row + i);
+            const float v = row[i];
             if (v > bv) { bv = v; bi = (int)i; }
         }
     }
@@ -170,8 +170,8 @@ __device__ __forceinline__ float norm_scale(float ss, uint32_t n, float eps, flo
     return 1.f / sqrtf(tot / (float)n + eps);
 }
 // any length: the row is read from HBM once, the second sweep hits L1 / L2
-__global__ void __launch_bounds__(256, 6) add_rmsnorm_kernel(float *x, const float *__restrict__ r,
-                                                             const float *__restrict__ w, float *y, uint32_t n,
+__global__ void __launch_bounds__(256, 6) add_rmsnorm_kernel(float *x, const float *r,
+                                                             const float *w, float *y, uint32_t n,
                                                              float eps, uint32_t x_stride, uint32_t y_stride) {
     __shared__ float part[8];
     pdl_launch_dependents();
@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(256, 6) add_rmsnorm_kernel(float *x, const flo
 // Rows of up to 256 V floats: a thread keeps its V elements in registers, so that there is one round
 // trip to L2, for x, r and w together (with w read after the sum four Q4_K FFN blocks took 93 us, so 80).
 template <int V>
-__global__ void __launch_bounds__(256, V <= 12 ? 4 : 2) add_rmsnorm_short_kernel(float *x, const float *__restrict__ r,
-                                                                   const float *__restrict__ w, float *y, uint32_t n,
+__global__ void __launch_bounds__(256, V <= 12 ? 4 : 2) add_rmsnorm_short_kernel(float *x, const float *r,
+                                                                   const float *w, float *y, uint32_t n,
                                                                    float eps, uint32_t x_stride, uint32_t y_stride) {
     __shared__ float part[8];
     pdl_launch_dependents();
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(256, V <= 12 ? 4 : 2) add_rmsnorm_short_kernel
 // ---- SiLU gating: a = silu(a) * b ------------------------------------------------------
 __device__ __forceinline__ float silu_times(float v, float b) { return v / (1.f + expf(-v)) * b; }
 // `vec`: both pointers 16-byte aligned; the last n % 4 elements are taken one by one
-__global__ void __launch_bounds__(256) silu_mul_kernel(float *a, const float *__restrict__ b, size_t n, bool vec) {
+__global__ void __launch_bounds__(256) silu_mul_kernel(float *a, const float *b, size_t n, bool vec) {
     pdl_launch_dependents();
     const size_t stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t n4 = vec ? n / 4 : 0;

@@ -1,0 +1,36 @@
+"""Rules of the sources that no run can show to be kept: every kernel here may be resident while the one
+before it in the stream still writes (programmatic dependent launch), so what other kernels write is
+not read through the read-only path, which is for data that nobody writes meanwhile."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "chatokf_b200" / "csrc"
+
+
+def code(name):
+    return re.sub(r"//[^\n]*", "", (CSRC / name).read_text())
+
+
+def kernels(name):
+    """(head, body) of every kernel of a source file."""
+    text = code(name)
+    for m in re.finditer(r"__global__[^{;]*\{", text):
+        depth, at = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        yield m.group(0), text[m.end():at]
+
+
+@pytest.mark.parametrize("name", ["okf_gemv.cu", "okf_gemm_tc.cu", "okf_neighbours.cu"])
+def test_results_of_other_kernels_are_not_read_through_the_read_only_path(name):
+    found = [(h, b) for h, b in kernels(name) if "pdl_wait" in b]
+    assert found
+    for head, body in found:
+        read_only = re.findall(r"const\s+(\w+)\s*\*\s*__restrict__\s*(\w+)", head)
+        assert set(read_only) <= {("uint8_t", "w")}, head  # weights
+        assert "__ldg(" not in body, head
+    if name == "okf_gemv.cu":  # x is staged by functions of their own
+        assert "__ldg(" not in code(name)
