@@ -1,5 +1,7 @@
 // C ABI of libokfcuda (include/okf_cuda.h): argument checks, dispatch by type
 // and batch width, host staging for the CPU-operator twins.
+#include <cuda.h>
+
 #include <new>
 #include <stdlib.h>
 #include <string.h>
@@ -65,15 +67,34 @@ void *pinned(void **buf, size_t *have, size_t need) {
     return *buf;
 }
 
-// The device's address of page-locked host memory on a 16-byte boundary, else null.
-void *mapped(const void *host) {
-    cudaPointerAttributes pa;
-    if (cudaPointerGetAttributes(&pa, host) == cudaSuccess) {
-        if (pa.type == cudaMemoryTypeHost && pa.devicePointer && (uintptr_t)pa.devicePointer % 16 == 0) return pa.devicePointer;
-    } else {
-        (void)cudaGetLastError();
-    }
-    return nullptr;
+// What a buffer handed to the host operator is.
+struct HostBuffer {
+    // Page-locked memory, all of it one registration and on a 16-byte boundary: its address on the device.
+    // (A buffer may begin in registered memory and run past its end.)
+    void *direct = nullptr;
+    bool cpu = false;  // the CPU may read and write it here and now; device and managed memory is the copy engine's
+};
+HostBuffer host_buffer(const void *p, size_t bytes) {
+    typedef CUresult (*GetFn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const GetFn get = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &q) != cudaSuccess) (void)cudaGetLastError();
+        return (GetFn)fn;
+    }();
+    HostBuffer h;
+    unsigned type = 0, managed = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *into[] = {&type, &managed, &dev, &start, &size};
+    if (!get || get(5, what, into, (CUdeviceptr)p) != CUDA_SUCCESS) return h;
+    h.cpu = !managed && (type == 0 || type == CU_MEMORYTYPE_HOST);
+    if (h.cpu && type == CU_MEMORYTYPE_HOST && dev && dev % 16 == 0 && (CUdeviceptr)p >= start && (CUdeviceptr)p - start <= size &&
+        bytes <= size - ((CUdeviceptr)p - start))
+        h.direct = (void *)dev;
+    return h;
 }
 
 // A gathered launch waits for the exchange launched before it and becomes the one the
@@ -692,19 +713,25 @@ int okf_matmul_host(okf_ctx *ctx, int type, const okf_weights *w, uint64_t woff,
     // a kernel from page-locked memory.  (2048 x 2048 Q8_0 between pageable buffers: 28 us with the copy
     // engine both ways, 21.5 so; page-locked buffers 22 and 20.5.)
     float *own_out = nullptr;  // set: the result still has to be copied from here
-    void *dev_out = ob <= kPinMax ? mapped(out) : nullptr;
-    if (!dev_out && ob <= kPinMax && (own_out = (float *)pinned(&ctx->pin_out, &ctx->pin_out_bytes, ob))) dev_out = mapped(own_out);
+    void *dev_out = nullptr;
+    if (ob <= kPinMax) {
+        const HostBuffer h = host_buffer(out, ob);
+        dev_out = h.direct;
+        if (!dev_out && h.cpu && (own_out = (float *)pinned(&ctx->pin_out, &ctx->pin_out_bytes, ob)))
+            dev_out = host_buffer(own_out, ob).direct;
+    }
     if (!dev_out) {
         own_out = nullptr;
         if ((rc = grow(ctx, &ctx->stage_out, &ctx->stage_out_bytes, ob))) return rc;
     }
     const void *dev_x = nullptr;
     if (xb <= kPinMax) {
-        dev_x = xb % 16 == 0 ? mapped(x) : nullptr;
-        if (!dev_x) {
+        const HostBuffer h = host_buffer(x, xb);
+        if (xb % 16 == 0) dev_x = h.direct;
+        if (!dev_x && h.cpu) {
             if (void *p = pinned(&ctx->pin_x, &ctx->pin_x_bytes, xb + 16)) {
                 memcpy(p, x, xb);
-                dev_x = mapped(p);
+                dev_x = host_buffer(p, xb + 16).direct;
             }
         }
     }
