@@ -319,8 +319,8 @@ int gemm_dispatch(okf_ctx *ctx, int ty, const okf_weights *w, uint64_t woff, uin
     } else {
         const bool simple = ctx->flags & OKF_FLAG_SIMPLE_KERNELS;
         if (!simple) ctx->fallbacks++;
-        // A few tokens of rows that the tile does not take (K not a multiple of 64): passes of the 24-bit
-        // matvec, about 3.5 us and the weights at 2 TB/s for four tokens, against the plain tile's 32-deep
+        // A few tokens of rows that the tile does not take (K not a multiple of 64): passes of the matvec
+        // for ragged rows, about 3.5 us and the weights at 2 TB/s for four tokens, against the plain tile's 32-deep
         // steps, 2.3 us each while its 64 x 64 tiles leave SMs idle, 0.74 us and as many as there are tiles
         // per SM where they do not.  (Q4_0 4384 -> 1536, 12 tokens: 310 us on the tile.)
         const double steps = k / 32, tiles = (double)((m + 63) / 64) * ((n + 63) / 64) / ctx->sms;

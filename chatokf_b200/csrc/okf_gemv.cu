@@ -74,7 +74,6 @@ constexpr uint32_t kConsumers = kGemvWarps * 32;
 // bank groups.
 constexpr uint32_t kXqUnit = 256;
 constexpr float kXqMax = 32512.f;  // 127 * 256: hi stays a signed byte after rounding
-constexpr float kXq3Max = 8323072.f;  // 127 * 65536, three bytes
 // SEP x panel: per byte column and unit, four quarters of 80 bytes: 64 bytes of x in k
 // order (two types: see stage_x_bytes), then in the first byte column the quarter's record {scale,
 // scale * sum of x over its first 32-wide block, over its second, -}, in the second one, for Q6_K,
@@ -589,9 +588,10 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
     }
 }
 
-// WIDE: every column as two or three byte columns of the panel, `es` bytes from one to the next.  An item is 8 consecutive k; the 32 items of a (column, unit)
-// pair are the lanes of one warp.  Two bytes: the integers of the one-column panel.  Three: q of 24
-// bits, |q| <= 127 * 2^16.  Inside a unit of a byte column thread c's 64 bytes start at 64c: eight bytes per
+// WIDE: every column as two to four byte columns of the panel, `es` bytes from one to the next.  An item is 8 consecutive k; the 32 items of a (column, unit)
+// pair are the lanes of one warp.  Two bytes: the integers of the one-column panel.  Three and four: v = q * 2^-s, |q| <=
+// 2^22 and 2^30, s from the largest magnitude's exponent and at most 149, so that the scale is a float however
+// small x is.  Inside a unit of a byte column thread c's 64 bytes start at 64c: eight bytes per
 // 32-wide block in the type's WideOrder, block after block, the 16-byte pieces of threads 2 and 3
 // swapped in pairs (see kXqUnit).
 template <int TY, int MODE, int XDT>
@@ -650,17 +650,26 @@ __device__ __forceinline__ void stage_x_wide(uint32_t xs32, uint32_t es, uint32_
                     w[1][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0040u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0040u), 0x5410u) ^ 0x80808080u;
                 }
             } else {
-                scale = amax * (1.f / kXq3Max);
-                const float inv = amax > 1e-30f ? __frcp_rn(scale) : 0.f;
+                // An infinity counts as its sign and everything else as zero, with an infinite scale: the sums
+                // come out as the infinity or NaN that fp32 products give.  A NaN: a NaN scale.
+                const bool finite = mb < 0x7F800000u;
+                const int sh = finite ? (NB == 4 ? 156 - (int)max(mb >> 23, 7u) : 148 - (int)max(mb >> 23, 1u)) : 0;
+                scale = !finite ? amax : __uint_as_float(sh <= 126 ? (uint32_t)(127 - sh) << 23 : 1u << (149 - sh));
+                // 2^sh in two factors: it may be beyond the largest float
+                const float f1 = __uint_as_float((uint32_t)(127 + (sh >> 1)) << 23), f2 = __uint_as_float((uint32_t)(127 + sh - (sh >> 1)) << 23);
                 uint32_t t[8];
 #pragma unroll
-                for (int j = 0; j < 8; j++) t[j] = (uint32_t)(__float2int_rn(v[j] * inv) + 0x8080);
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    w[0][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0062u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0062u), 0x5410u);
-                    w[1][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0051u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0051u), 0x5410u) ^ 0x80808080u;
-                    w[NB - 1][i] = prmt(prmt(t[4 * i], t[4 * i + 1], 0x0040u), prmt(t[4 * i + 2], t[4 * i + 3], 0x0040u), 0x5410u) ^ 0x80808080u;
+                for (int j = 0; j < 8; j++) {
+                    const float f = finite ? v[j] * f1 * f2 : isinf(v[j]) ? copysignf(1.f, v[j]) : 0.f;
+                    t[j] = (uint32_t)__float2int_rn(f) + (NB == 4 ? 0x808080u : 0x8080u);
                 }
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+#pragma unroll
+                    for (int b = 0; b < NB; b++) {
+                        const uint32_t sel = 0x0040u + 0x0011u * (NB - 1 - b);  // byte NB - 1 - b of two words
+                        w[b][i] = prmt(prmt(t[4 * i], t[4 * i + 1], sel), prmt(t[4 * i + 2], t[4 * i + 3], sel), 0x5410u) ^ (b ? 0x80808080u : 0u);
+                    }
             }
             const uint32_t info = info32 + (u * ncols + col) * (IW * 4);
             if (e8 == 0) sts32(info, __float_as_uint(scale));
@@ -885,7 +894,7 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
     if constexpr (!SEP) {
 #pragma unroll
         for (int i = 0; i < W::sets; i++) {
-            const uint32_t j = (W::rag ? 0 : 4 * i) + (g >> 1), b = W::rag && i ? 2 : g & 1;
+            const uint32_t j = (W::rag ? 0 : 4 * i) + (g >> 1), b = W::rag ? min(2u * i + (g & 1), W::nb - 1u) : g & 1;
             wx32[i] = smem32 + L.xs_off + (j < p.n ? j * W::nb + b : 0u) * L.es + c * 64;
         }
 #pragma unroll
@@ -1164,8 +1173,9 @@ static bool gemv_layout_with(int ty, uint32_t row_bytes, uint32_t nunit, uint32_
     L.nc = n;
     L.nc_inv = 65536 / n + 1;
     L.clog = csize == 8 ? 3 : csize == 4 ? 2 : csize == 2 ? 1 : 0;
-    const bool rag = mode == M_R;
-    const uint32_t ecols = sep ? 2 : n * (rag ? 3 : 2);  // byte columns of the x panel
+    const uint32_t nb = mode_bytes(mode);
+    const bool rag = nb > 2;
+    const uint32_t ecols = sep ? 2 : n * nb;  // byte columns of the x panel
     const uint32_t units = (nunit + csize - 1) / csize;   // the most a CTA of a cluster takes
     const uint32_t per_tile = kGemvWarps * 16 * L.nc * 4;
     const uint32_t part_bytes = csize > 1 ? tiles_per_cta * 16 * L.nc * 4 : 0;
@@ -1173,7 +1183,7 @@ static bool gemv_layout_with(int ty, uint32_t row_bytes, uint32_t nunit, uint32_
     L.tab_copies = tab_copies;
     const uint32_t stage_cap = 46 * 1024;
     // per unit: SEP 320 bytes per byte column, records included; WIDE 256 per byte column and the columns' records
-    const uint32_t xunit = sep ? kSepUnit : kXqUnit, info_unit = sep ? 0 : n * wide_info_words(ty, rag ? 3 : 2) * 4;
+    const uint32_t xunit = sep ? kSepUnit : kXqUnit, info_unit = sep ? 0 : n * wide_info_words(ty, nb) * 4;
     GemvArgs fb_a = a;
     GemvLayout fb_L = L;
     bool have_fallback = false;
@@ -1405,6 +1415,20 @@ static cudaError_t launch_t(GemvArgs a, const GemvGather &G, int xdt, cudaStream
     }
 }
 
+// rows that end inside a unit: never a row shard, and the element type goes with the mode
+template <int TY>
+static cudaError_t launch_r(GemvArgs a, int mode, int xdt, cudaStream_t s, int sms, int dev) {
+    GemvLayout L;
+    uint32_t ctas;
+    const GemvGather none = {};
+    if (!gemv_plan(TY, a.row_bytes, a.nunit, a.n, mode, a.tiles, sms, false, a, L, ctas)) return cudaErrorInvalidConfiguration;
+    switch (xdt) {
+    case DT_F16: return launch_d<TY, M_R3, DT_F16>(a, L, none, ctas, s, dev);
+    case DT_BF16: return launch_d<TY, M_R3, DT_BF16>(a, L, none, ctas, s, dev);
+    default: return launch_d<TY, M_R4, DT_F32>(a, L, none, ctas, s, dev);
+    }
+}
+
 template <int TY>
 static cudaError_t launch_ty(const GemvArgs &a, const GemvGather &G, int mode, int xdt, cudaStream_t s, int sms, int dev) {
     switch (mode) {
@@ -1413,16 +1437,16 @@ static cudaError_t launch_ty(const GemvArgs &a, const GemvGather &G, int mode, i
     case M_W2: return launch_t<TY, M_W2>(a, G, xdt, s, sms, dev);
     }
     if constexpr (TY == T_Q8_0 || TY == T_Q4_0 || TY == T_IQ4_NL || TY == T_Q2_0) {
-        if (mode == M_R) return launch_t<TY, M_R>(a, G, xdt, s, sms, dev);
+        if (mode == M_R4 || mode == M_R3) return launch_r<TY>(a, mode, xdt, s, sms, dev);
     }
     return cudaErrorInvalidValue;
 }
 
 // How `n` columns are taken: the mode of the next pass and its columns.
-static int gemv_mode(uint32_t k, uint32_t n, uint32_t &take) {
+static int gemv_mode(uint32_t k, int xdt, uint32_t n, uint32_t &take) {
     if (k % 256) {
         take = n < 4 ? n : 4;
-        return M_R;
+        return xdt == DT_F32 ? M_R4 : M_R3;
     }
     take = n;
     return n == 1 ? M_SEP : n <= 4 ? M_W1 : M_W2;
@@ -1441,7 +1465,7 @@ static bool group_fits(int ty, uint32_t k, uint32_t nseg, const uint32_t *m, con
     GemvLayout L;
     const uint32_t row_bytes = k / block_elems(ty) * block_bytes(ty);
     for (uint32_t left = n, take; left; left -= take) {
-        const int mode = gemv_mode(k, left, take);
+        const int mode = gemv_mode(k, xdt, left, take);
         uint32_t ctas;
         if (!gemv_plan(ty, row_bytes, (k + 255) / 256, take, mode, tiles, sms, false, a, L, ctas)) return false;
     }
@@ -1498,7 +1522,7 @@ cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, co
     const size_t xsz = xdt == DT_F32 ? 4 : 2;
     for (uint32_t c0 = 0; c0 < n;) {
         uint32_t take;
-        const int mode = gemv_mode(k, n - c0, take);
+        const int mode = gemv_mode(k, xdt, n - c0, take);
         a.x = (const uint8_t *)x + (size_t)c0 * k * xsz;
         for (uint32_t i = 0; i < (uint32_t)kGemvSegs; i++) {
             const uint32_t j = i < nseg ? i : nseg - 1;

@@ -2,12 +2,17 @@
 //
 // Weights are the A operand of the integer MMA (16 output rows), bytes of x the B operand, in one or
 // two sets of eight byte columns.  A column of x is two signed bytes per element (q = 256 * hi + lo,
-// 16 bits), or three for rows that are no multiple of 256 weights (24 bits: those shapes ran on fp32
-// arithmetic before there was a kernel for them, and keep that precision):
+// 16 bits), or three or four for rows that are no multiple of 256 weights, whose scale is a power of two.
+// (Those shapes ran on fp32 arithmetic before there was a kernel for them and keep that precision: 31 bits
+// hold an fp32 x exactly down to 2^-7 of the unit's largest, 23 bits an fp16 x down to 2^-11 and a bf16 x to 2^-14 of
+// it.  With 24 bits and a scale of any value, results of fp32 x were 1.2 to 1.6 times as far from float64 as fp32
+// sums on rows up to 2000 weights.  Four bytes for 16-bit x too: Q4_0 8224 -> 6000, 4 columns, 22.7 -> 30.3 us,
+// as less of x fits beside the ring.)
 //   W1  up to 4 columns: byte column 2j = hi, 2j + 1 = lo of column j
 //   W2  up to 8 columns: the same for columns 4 .. 7 in a second set.  Weights are unpacked and
 //       scales decoded once for both (before, eight columns were two launches over the weights)
-//   R   up to 4 columns of three bytes: hi and mid in the first set, lo in column 2j of the second
+//   R4  up to 4 columns of four bytes (fp32 x): the upper two in the first set, the lower two in the second
+//   R3  up to 4 columns of three bytes (16-bit x): hi and mid in the first set, lo in column 2j of the second
 // Thread (g = lane / 4, c = lane % 4) feeds output rows g and g + 8 at k-slots 4c .. 4c+3 and 16+4c ..
 // of a block, byte column g at the same slots, and gets back, for its own two rows, column c (and
 // 4 + c): all bytes of a column meet in one thread.  (With x as the A operand instead, 8 output rows
@@ -21,12 +26,14 @@
 
 namespace okf {
 
-enum : int { M_SEP = 0, M_W1 = 1, M_W2 = 2, M_R = 3 };
+enum : int { M_SEP = 0, M_W1 = 1, M_W2 = 2, M_R4 = 3, M_R3 = 4 };
+// bytes of an element of x
+__host__ __device__ constexpr int mode_bytes(int mode) { return mode == M_R4 ? 4 : mode == M_R3 ? 3 : 2; }
 template <int MODE> struct WideMode {
-    static constexpr int sets = MODE == M_W2 || MODE == M_R ? 2 : 1;  // sets of eight byte columns
-    static constexpr int nb = MODE == M_R ? 3 : 2;                    // bytes per element
+    static constexpr int sets = MODE == M_W2 || mode_bytes(MODE) > 2 ? 2 : 1;  // sets of eight byte columns
+    static constexpr int nb = mode_bytes(MODE);                    // bytes per element
     static constexpr int vals = MODE == M_W2 ? 2 : 1;                 // columns of a thread
-    static constexpr bool rag = nb == 3;                              // rows end inside a unit, 2-byte aligned
+    static constexpr bool rag = nb > 2;                             // rows end inside a unit, 2-byte aligned
 };
 
 // Order of a block's 32 k over the threads' slots (thread c's eight bytes, first word then second):
@@ -103,7 +110,9 @@ __device__ __forceinline__ void wide_join(const int (&d)[WideMode<MODE>::sets][4
     using W = WideMode<MODE>;
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-        if constexpr (W::nb == 3) {
+        if constexpr (W::nb == 4) {
+            v[0][r] = fmaf((float)(d[0][2 * r] * 256 + d[0][2 * r + 1]), 65536.f, (float)(d[W::sets - 1][2 * r] * 256 + d[W::sets - 1][2 * r + 1]));
+        } else if constexpr (W::nb == 3) {
             v[0][r] = fmaf((float)d[0][2 * r], 65536.f, (float)(d[0][2 * r + 1] * 256 + d[W::sets - 1][2 * r]));
         } else {
 #pragma unroll
@@ -295,8 +304,10 @@ __device__ __forceinline__ void unit_wide(uint32_t ua, uint32_t ub, uint32_t c, 
             int d[NS][4];
 #pragma unroll
             for (int s = 0; s < NS; s++) {
-                const int h = (int)(RAG ? X.sum[0][3 * blk + 2 * s] : X.sum[RAG ? 0 : s % NV][W::nb * blk]);
-                const int l = (int)(RAG ? (s ? 0u : X.sum[0][3 * blk + 1]) : X.sum[RAG ? 0 : s % NV][W::nb * blk + 1]);
+                constexpr int last = W::nb - 1;
+                const int h = (int)(RAG ? X.sum[0][W::nb * blk + 2 * s] : X.sum[RAG ? 0 : s % NV][W::nb * blk]);
+                const int l = (int)(RAG ? (2 * s < last ? X.sum[0][W::nb * blk + (2 * s < last ? 2 * s + 1 : last)] : 0u)
+                                        : X.sum[RAG ? 0 : s % NV][W::nb * blk + 1]);
                 d[s][0] = d[s][2] = h;
                 d[s][1] = d[s][3] = l;
             }

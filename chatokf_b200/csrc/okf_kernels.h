@@ -45,8 +45,8 @@ cudaError_t launch_gemm_simple(int ty, const uint8_t *w, uint32_t k, uint32_t m,
 // caller routes everything else to the simple kernel.
 bool gemv_fast_supported(int ty, uint32_t k, uint32_t m, const void *w, const void *x, int xdt, uint32_t n,
                          int sms);
-// The same kernel for rows that are no multiple of 256 weights (three bytes per activation instead of
-// two: these shapes keep the precision of the plain kernels they used to run on).
+// The same kernel for rows that are no multiple of 256 weights (more bytes per activation: these
+// shapes keep the precision of the plain kernels they used to run on).
 bool gemv_ragged_supported(int ty, uint32_t k, uint32_t m, const void *w, const void *x, int xdt, uint32_t n, int sms);
 cudaError_t launch_gemv_fast(int ty, const uint8_t *w, uint32_t k, uint32_t m, const void *x, int xdt,
                              uint32_t n, float *out, int *status, cudaStream_t s, int sms, int dev,

@@ -124,8 +124,8 @@ OKF_API int okf_gemv(okf_ctx *ctx, int type, const okf_weights *w, uint64_t woff
  * okf_destroy once the graph and its instances are gone): a graph may be replayed beside
  * any other call or graph, but not after okf_destroy.
  * Numerics: for N <= 8 (fp32 out) every 256-wide run of an activation column is
- * reduced to 16-bit integers (24-bit where K is no multiple of 256) with one fp32
- * scale and the sums are exact integers
+ * reduced to 16-bit integers (where K is no multiple of 256: 23 bits for 16-bit x,
+ * 31 for fp32 x, which hold it as it is) with one fp32 scale and the sums are exact integers
  * (results within 1e-4 of max|y| of an fp32 evaluation on the test shapes, the
  * same for a column at every N); the tile rounds weights and activations to
  * 16-bit floats and accumulates in fp32 (within 1e-2). */
@@ -369,7 +369,7 @@ OKF_API int okf_set_flags(okf_ctx *ctx, uint32_t flags);
 OKF_API uint64_t okf_launch_count(const okf_ctx *ctx);
 /* Number of calls that did not run on the main kernels because of their shape or
  * alignment: K not a multiple of 256 for the matvec (a slower form of it that
- * keeps 24 bits of x takes Q8_0, Q4_0, IQ4_NL and Q2_0 with aligned pointers) or
+ * keeps fp32 precision of x takes Q8_0, Q4_0, IQ4_NL and Q2_0 with aligned pointers) or
  * of 64 for the tile, x not 16-byte aligned (plain warp-per-row / fp32-tile
  * kernels, many times slower).  A caller that cares about speed checks that this
  * stays 0.  Calls made under OKF_FLAG_SIMPLE_KERNELS are not counted.  No

@@ -16,7 +16,7 @@ DTS = [torch.float32, torch.float16, torch.bfloat16]
 # activations carry 16 bits relative to the largest of 256: a step of 2^-15 of that, an rms error of
 # 2^-15 / sqrt(12) of it per term; 1e-4 of max|y| is the bound of every matvec test here
 WIDE_TOL = 1e-4
-# 24 bits: 2^-24 of the largest of 256 per term, below the rounding of the oracle's own sequential
+# x as it is: what is left is the rounding of the oracle's own sequential
 # fp32 sum of K terms (about sqrt(K) * 2^-24 of max|y|, 8e-6 at K = 16384)
 RAGGED_TOL = 1e-5
 
@@ -78,3 +78,56 @@ def test_the_next_rows_scales_stay_out(ctx):
     torch.cuda.synchronize()
     o, want = out.cpu().numpy(), oracle.matvec(GGUFType.Q8_0, blocks, k, m, np.ones(k, np.float32))
     assert not np.isfinite(o[1]) and rel_err(o[[0, 2]], want[[0, 2]]) <= RAGGED_TOL
+
+
+RAGGED = [GGUFType.Q8_0, GGUFType.Q4_0, GGUFType.IQ4_NL, GGUFType.Q2_0]
+
+
+@pytest.mark.parametrize("ty", RAGGED)
+@pytest.mark.parametrize("k", [128, 896, 1152, 4224])
+def test_rows_that_end_inside_a_unit_keep_fp32_precision(ctx, ty, k):
+    """No further from float64 (2-norm over M x N results) than the plain kernels' fp32 sums, from which
+    these rows were taken over; a tenth is left for the spread of the 6000 results' errors."""
+    m, n = 2000, 3
+    w = ctx.upload(synth.random_blocks(ty, m * k // block_elems(ty), np.random.default_rng(k)))
+    t = GGUFTensor("w", (k, m), ty)
+    W = torch.empty(m * k, device="cuda")
+    CudaEnc(ctx).dequantRow(w, W, m * k, ty)
+    X = torch.randn(n, k, device="cuda", generator=torch.Generator("cuda").manual_seed(k))
+    exact = X.double() @ W.view(m, k).double().T
+    err = []
+    for flag in (0, 1):
+        out = torch.empty(n, m, device="cuda")
+        ctx.set_flags(flag)
+        try:
+            CudaEnc(ctx).gemm(t, X, out, w, n)
+        finally:
+            ctx.set_flags(0)
+        err.append(float((out.double() - exact).norm() / exact.norm()))
+    assert err[0] <= 1.1 * err[1], err
+
+
+@pytest.mark.parametrize("ty", RAGGED)
+def test_rows_that_end_inside_a_unit_at_the_ends_of_the_range(ctx, ty):
+    """Activations near the smallest and the largest floats, subnormal ones, infinities and NaNs: as fp32 arithmetic
+    has them.  Results below 2^-126 are held to steps of 2^-149 in any order of sums."""
+    k, m = 1152, 64
+    w = ctx.upload(synth.random_blocks(ty, m * k // block_elems(ty), np.random.default_rng(9)))
+    t = GGUFTensor("w", (k, m), ty)
+    W = torch.empty(m * k, device="cuda")
+    CudaEnc(ctx).dequantRow(w, W, m * k, ty)
+    W = W.view(m, k).double()
+    base = torch.randn(k, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    out = torch.empty(m, device="cuda")
+    for scale in (2.0 ** 60, 1e-20, 1e-31, 1e-36, 1e-40):
+        x = base * scale
+        CudaEnc(ctx).gemm(t, x, out, w, 1)
+        exact = W @ x.double()
+        assert (out.double() - exact).abs().max() <= RAGGED_TOL * exact.abs().max() + k * 2.0 ** -149, scale
+    for value in (float("inf"), -float("inf"), float("nan")):
+        x = base.clone()
+        x[300] = value
+        CudaEnc(ctx).gemm(t, x, out, w, 1)
+        exact = (W @ x.double()).float()
+        assert torch.equal(out.isnan(), exact.isnan()) and torch.equal(out.isinf(), exact.isinf())
+        assert torch.equal(out[out.isinf()], exact[exact.isinf()])
