@@ -1063,7 +1063,9 @@ static GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt
     for (uint32_t nacc = 1; nacc <= 2; nacc++) {
         if (nacc == 2 && (xdt == DT_F32 || n <= tc::kBN)) continue;
         const bool slow = ty == T_Q8_0 || ty == T_Q6_K;
-        const double t_kb = nacc == 2 ? (slow ? 1.15e-6 : 0.93e-6) : (slow ? 0.8e-6 : 0.45e-6 + 0.4e-9 * (n < tc::kBN ? n : tc::kBN));
+        // (fp32 activations that the tile converts itself, by one group of warps while another unpacks:
+        // 0.9 us, from some 80 tokens on what the conversion takes, 2.3 us at 256)
+        const double t_kb = xdt == DT_F32 ? (n > 80 ? 0.3e-6 + 7.8e-9 * (n < tc::kBN ? n : tc::kBN) : 0.9e-6) : nacc == 2 ? (slow ? 1.15e-6 : 0.93e-6) : (slow ? 0.8e-6 : 0.45e-6 + 0.4e-9 * (n < tc::kBN ? n : tc::kBN));
         const uint32_t base = slabs * ((n + nacc * tc::kBN - 1) / (nacc * tc::kBN));
         const double whole = ((base + all - 1) / all) * (kblocks * t_kb + (nacc == 2 ? 3e-6 : 0));
         if (whole < best_t) { best_t = whole; best = {nacc, 0, 0, 0, 0, 0}; }
@@ -1072,15 +1074,24 @@ static GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt
         if (dealt == 0) continue;
         const uint64_t total = (uint64_t)dealt * kblocks;
         if (total * (all + 1) >= 0xFFFFFFFFull) continue;
-        const uint32_t ctas = total / 4 < all ? (uint32_t)(total / 4) : all;  // four k-blocks at least
+        uint32_t ctas = total / 4 < all ? (uint32_t)(total / 4) : all;  // four k-blocks at least
         if (ctas <= dealt) continue;
         uint32_t parts = 1;
         for (uint32_t i = 0; i < dealt; i++) {
             const uint32_t c = tc::dealt_to((i + 1) * kblocks - 1, (uint32_t)total, ctas) - tc::dealt_to(i * kblocks, (uint32_t)total, ctas) + 1;
             if (c > parts) parts = c;
         }
-        const size_t floats = (size_t)parts * dealt * nt * tc::kBM;
-        if (floats > max_floats) continue;
+        const size_t part = (size_t)dealt * nt * tc::kBM;  // floats
+        if (parts * part > max_floats) {
+            // as many equal parts of every item as there is room for (Q4_K 9728 -> 2560, 512 tokens, in 16 MiB: on 40
+            // of the SMs 71 us with fp16 and 358 with fp32 activations, in three parts on 120 of them 35 and 196)
+            parts = (uint32_t)(max_floats / part);
+            if (parts > kblocks / 4) parts = kblocks / 4;
+            if (parts > all / dealt) parts = all / dealt;
+            if (parts < 2) continue;
+            ctas = dealt * parts;
+        }
+        const size_t floats = parts * part;
         const double moved = 2.0 * (dealt + ctas) * nt * tc::kBM * 4;
         const double t = waves * (kblocks * t_kb + (nacc == 2 ? 3e-6 : 0)) + (double)total / ctas * t_kb + 4e-6 + moved / 8e12;
         if (t < best_t) { best_t = t; best = {nacc, waves, dealt, ctas, nt, floats}; }

@@ -87,3 +87,24 @@ def test_outputs_that_are_only_4_byte_aligned(ctx, k, m, n, shift):
         assert torch.equal(flat[shift:shift + n * m], want)
         assert torch.isnan(flat[:shift]).all() and torch.isnan(flat[shift + n * m:]).all()
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("k,m,n", [(9728, 2560, 512), (4480, 1536, 512), (2048, 2048, 512), (17408, 1000, 1500)])
+@pytest.mark.parametrize("dt", [torch.float16, torch.float32])
+def test_dealing_in_less_memory(ctx, k, m, n, dt):
+    """Partial tiles of the best plan that do not fit the fixed array: fewer parts, not the whole matmul on a few SMs."""
+    ty = GGUFType.Q4_0
+    w = ctx.upload(synth.random_blocks(ty, m * k // block_elems(ty), np.random.default_rng(m)))
+    t = GGUFTensor("w", (k, m), ty)
+    enc = CudaEnc(ctx)
+    X = torch.randn(n, k, device="cuda").to(dt)
+    got, want = torch.full((n * m + 8,), float("nan"), device="cuda"), torch.empty(n * m, device="cuda")
+    enc.gemm(t, X, want, w, n)
+    before = ctx.launches
+    enc.gemm_noalloc(t, X, got, w, n)
+    assert ctx.launches - before == 2
+    torch.cuda.synchronize()
+    assert torch.isnan(got[n * m:]).all()
+    # the same operands, fp32 sums in another order
+    assert rel_err(got[:n * m].cpu().numpy(), want.cpu().numpy()) <= 1e-5
+    assert ctx.device_status() == 0
