@@ -894,8 +894,9 @@ struct ReduceOut {
 constexpr uint32_t kReduceTok = 16;
 // VEC: fp32 results leave as 16-byte words, as every row of every output starts on a 16-byte boundary.  The host
 // decides, from the addresses too: an fp32 output need only be 4-byte aligned (a view into a larger tensor).
-// (As a run-time flag the test stood between the loads of one token and the next: Q5_K 2560 -> 9728, 77 tokens,
-// 21.4 us instead of 19.1.)
+// (As a run-time flag: Q5_K 2560 -> 9728, 77 tokens, 21.4 us instead of 19.5.  The time goes with the registers
+// per thread, which bound how many of these CTAs gather on the SMs that the matmul leaves first: forms of 32
+// to 36 registers took 19.8 to 21.7 us, of 42 to 44 19.1 to 19.5.)
 template <typename OT, bool VEC>
 __global__ void __launch_bounds__(256) reduce_kernel(const float *part, ReduceOut o) {
     pdl_launch_dependents();

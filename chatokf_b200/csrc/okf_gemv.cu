@@ -1345,10 +1345,12 @@ static bool gemv_layout(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, 
 // 320 tiles: Q8_0 4096 -> 4096 6.7 -> 5.2, Q4_K 12288 -> 3072 11.4 -> 8.7, 5120 -> 5120 6.7 -> 6.1; below, Q4_K
 // 4096 -> 4096, 64 KB, 4.15 -> 4.35; not for the two types with a look-up per weight, whose warps hardly
 // wait: IQ2_XXS 6144 -> 6144 9.6 -> 10.5, IQ4_NL 10.1 -> 11.3).  Several columns, with
-// more work per tile: from four tiles on (Q4_K 5120 -> 17357, 4 columns, 27.6 -> 20.0 us, 8 columns 35 -> 29;
-// down to two tiles it makes no difference).
+// more work per tile: from three tiles on (Q4_K 5120 -> 17357, 4 columns, 27.6 -> 20.0 us, 8 columns 35 -> 29;
+// 512 tiles, which were left to one CTA per SM: Q5_K 17408 -> 8192, 3 columns, 56.9 -> 40.6 us, Q4_K 20480 -> 8192, 4 columns, 55.6 -> 53.8 us, Q4_K 8192 -> 8192, 8
+// columns, 35.6 -> 37.6; the two-bit types, with little to wait for, from four on: IQ2_XXS 8192 -> 8192, 5 columns, 23.6 us, from three 27.5).
+static bool two_bit(int ty) { return ty == T_IQ2_XXS || ty == T_Q2_0; }
 static bool two_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, bool sep) {
-    if (!sep) return tiles >= 4u * (uint32_t)sms;
+    if (!sep) return tiles >= (two_bit(ty) ? 4u : 3u) * (uint32_t)sms;
     const uint64_t raw = (uint64_t)tiles * 16 * row_bytes, bytes = ty == T_IQ2_XXS ? raw + raw / 2 : raw;
     const bool few = tiles <= 3u * (uint32_t)sms && ty != T_IQ2_XXS && ty != T_IQ4_NL;
     return tiles >= 8u * (uint32_t)sms || bytes >= (few ? 81920ull : 147456ull) * (uint32_t)sms;
@@ -1370,7 +1372,13 @@ static uint32_t gemv_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, b
 // evenly over the chip, whole ones leave most CTAs one and a few of them two (Q4_K 17408 -> 5120 21.3 ->
 // 16.9 us, Q8_0 32.7 -> 24.6, Q6_K 39.6 -> 28.5, Q2_0 12288 -> 5120 10.7 -> 9.4; Q8_0 5120 -> 5120, 20 units of 272
 // bytes, 8.8 -> 9.5, Q4_K 9216 -> 5120, 36 of 144, 10.3 -> 10.8).
+// Several columns: x resident is not enough, copies have to be on their way as well.  A panel that leaves the ring
+// of a CTA alone less than kRingMin, in segments of about 1 KB, goes to two CTAs (Q8_0 17408 -> 8192, 2
+// columns, 88.4 -> 42.2 us, Q5_K 9728 -> 5120, 3 columns, 26.1 -> 19.2; with 36 KB the latter stays).  It is asked of a
+// CTA alone only (four CTAs instead of two for a deeper ring: Q4_0 8192 -> 14336, 8 columns, 1.9 times the time) and not of the
+// two-bit types, which get more weights out of a byte on its way (Q2_0 5120 -> 17408, 5 columns, 18.9 -> 23.0).
 // Row-shard launches have duties by CTA number and take no clusters.
+constexpr uint32_t kRingMin = 44 * 1024;
 static bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t tiles, int sms, bool gather, GemvArgs &a,
                       GemvLayout &L, uint32_t &ctas) {
     const uint32_t all = gemv_ctas(ty, row_bytes, tiles, sms, mode == M_SEP), n2 = 2u * (uint32_t)sms;
@@ -1381,6 +1389,10 @@ static bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, in
         if (!gemv_layout(ty, row_bytes, nunit, n, mode, cs, (tiles + clusters - 1) / clusters, a, L)) continue;
         const bool last = ty == T_IQ2_XXS && cs == 2;  // shorter segments of its 66-byte units cost more than a resident x gains
         if (!last && (L.panel < a.nchunk || (mode == M_SEP && ty == T_IQ2_XXS && nunit >= 48 && L.tab_copies < 32))) continue;
+        if (mode != M_SEP && cs == 1 && !gather && !two_bit(ty) && nunit >= 8) {
+            const uint32_t tpc = (tiles + clusters - 1) / clusters, steps = (tpc + L.tps - 1) / L.tps * a.nchunk * (L.mode == 1 ? 2 : 1);
+            if (L.nstage < steps && L.nstage * L.stage_bytes < kRingMin) continue;
+        }
         ctas = clusters * cs;
         return true;
     }
