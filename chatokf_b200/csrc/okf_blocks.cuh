@@ -215,6 +215,11 @@ template <typename T> __device__ __forceinline__ const T *dep_ptr(const T *p) {
     asm volatile("" : "+l"(p) : : "memory");
     return p;
 }
+__device__ __forceinline__ uint4 ld_dep(const uint4 *p) {
+    uint4 v;
+    asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ float4 ld_dep(const float4 *p) {
     float4 v;
     asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));

@@ -521,7 +521,7 @@ __device__ __forceinline__ void stage_x_bytes(uint32_t xs32, uint32_t es, const 
                                                               ((size_t)u_first * 256 + (size_t)i * 8) * (XDT == DT_F32 ? 4 : 2));
 #pragma unroll
             for (int j = 0; j < (XDT == DT_F32 ? 2 : 1); j++)
-                raw[r].v[j] = i < items ? src[j] : make_uint4(0u, 0u, 0u, 0u);
+                raw[r].v[j] = i < items ? ld_dep(src + j) : make_uint4(0u, 0u, 0u, 0u);
         }
 #pragma unroll
         for (uint32_t r = 0; r < kFlight; r++) {
@@ -621,7 +621,7 @@ __device__ __forceinline__ void stage_x_wide(uint32_t xs32, uint32_t es, uint32_
             const uint4 *src = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(x) +
                                                               ((size_t)lcol * kdim + k0) * (XDT == DT_F32 ? 4 : 2));
 #pragma unroll
-            for (int j = 0; j < (XDT == DT_F32 ? 2 : 1); j++) raw[r].v[j] = live ? src[j] : make_uint4(0u, 0u, 0u, 0u);
+            for (int j = 0; j < (XDT == DT_F32 ? 2 : 1); j++) raw[r].v[j] = live ? ld_dep(src + j) : make_uint4(0u, 0u, 0u, 0u);
             step(lcol, lu);
         }
 #pragma unroll
@@ -920,6 +920,7 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
         if (tid == 0) gather_wait(G.wait_arrivals, G.wait_epoch, p.status);
         named_bar_sync(1, kConsumers);
     }
+    const void *x = dep_ptr(reinterpret_cast<const uint8_t *>(p.x));
     for (uint32_t gb = 0; gb < ntl; gb += L.group) {
         const uint32_t gn = min(L.group, ntl - gb);
         if (gb > 0)
@@ -930,8 +931,8 @@ __global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(Ge
             if (gb == 0 || L.panel < p.nchunk) {
                 // the previous panel is still being read until every warp gets here
                 if (gb > 0 || j0 > 0) consumer_sync();
-                if constexpr (SEP) stage_x_bytes<TY, XDT>(smem32 + L.xs_off, L.es, p.x, ubeg + pu0, pnu, tid);
-                else stage_x_wide<TY, MODE, XDT>(smem32 + L.xs_off, L.es, smem32 + L.info_off, p.x, p.k, L.nc, ubeg + pu0, pnu, tid);
+                if constexpr (SEP) stage_x_bytes<TY, XDT>(smem32 + L.xs_off, L.es, x, ubeg + pu0, pnu, tid);
+                else stage_x_wide<TY, MODE, XDT>(smem32 + L.xs_off, L.es, smem32 + L.info_off, x, p.k, L.nc, ubeg + pu0, pnu, tid);
             }
             consumer_sync();
             for (uint32_t j = j0; j < j1; j++) {
