@@ -8,12 +8,13 @@
 // tile feeds two accumulators.  Per k-block of 64:
 //   - the activation tile(s), 256 tokens x 64 k each, come by TMA through a tensor
 //     map of X, already in the 128-byte-swizzled K-major layout the tensor core
-//     reads (fp32 activations are converted by eight warps instead);
+//     reads (fp32 activations are converted to bf16 once per call before; where there is no memory for
+//     that, eight warps convert them tile by tile and the other eight unpack alone);
 //   - two groups of eight warps, taking the k-blocks in turn, unpack 128 rows x 64
 //     weights to 16-bit floats into the same layout; weight bytes are fetched one
 //     or two turns ahead.  (Bringing Q4_K slabs in by TMA as stored, 128 rows x one
 //     144-byte block per copy into a ring of their own, was tried and was slower.)
-//   - one thread issues four tcgen05.mma (M = 128, N = 256, K = 16) per token block
+//   - one warp, converged, issues four tcgen05.mma (M = 128, N = 256, K = 16) per token block
 //     that accumulate in fp32 in tensor memory: lane = weight row, column = token;
 //   - tcgen05.commit hands the stage back to the producers when the MMAs that
 //     read it are done.
@@ -21,7 +22,8 @@
 // blocks of one item or alternate between items, so an epilogue (tcgen05.ld,
 // convert, coalesced stores along m) overlaps the next main loop.  Operands are
 // fp16 when the activations are fp16, bf16 otherwise (fp32 activations are
-// rounded to bf16); weights are decoded exactly to fp32 first and rounded once.
+// rounded to bf16); weights are decoded in fp32, exactly but for the mins of Q4_K and Q5_K (below), and
+// rounded once.
 //
 // Every mbarrier wait is bounded (about a second); a wait that gives up records
 // a code in the status word, the CTA frees its tensor memory and returns.
@@ -41,7 +43,8 @@ namespace okf {
 // laid end to end are cut into one run per CTA, pieces of items leave as fp32 partial tiles, and a
 // second kernel sums them.  The plan with the smallest estimated time wins.  The estimate, measured on
 // B200: a CTA spends 0.93 us per k-block on an item of two token blocks and 0.45 - 0.55 us on one of one
-// block (Q8_0 and Q6_K, whose rows take more loads to unpack, 1.15 and 0.8); an item of two blocks, which
+// block (Q8_0 and Q6_K 1.15 and 0.8: what they took when their rows were read in 4-byte words; in 8-byte words 0.5 and 0.65 at
+// up to 64 tokens, which the estimate does not know yet); an item of two blocks, which
 // uses all of tensor memory, exposes 3 us of epilogue; dealing costs 4 us of launch and hand-over, and
 // partial tiles move at 8 TB/s, mostly through L2.  (4096 tokens 17408 -> 5120: 320 items of two blocks
 // are 2.16 waves; three whole waves took 760 us, two and 24 dealt items 590.)
@@ -58,7 +61,8 @@ constexpr uint32_t kBN = 256;           // tokens per accumulator (UMMA N)
 constexpr uint32_t kBK = 64;            // k per stage: 64 x 2 bytes = one 128-byte swizzle row
 constexpr uint32_t kABytes = kBM * kBK * 2;  // 16 KB
 constexpr uint32_t kBBytes = kBN * kBK * 2;  // 32 KB per 256 tokens
-// Two rings.  With one token block per item: four stages of A (16 KB) and of B (32 KB).  With
+// Two rings.  With one token block per item: as many stages of A (16 KB) and of B (up to 32 KB, by the tokens there
+// are) as the room of four full ones holds, at most kMaxRing.  With
 // two blocks a B stage is 64 KB: three of them and two of A, so that a B tile has two MMA
 // periods to arrive while the next A tile only has to be stored (IQ2_XXS, which also keeps its
 // codebook in shared memory, stays with two B stages).
@@ -66,7 +70,7 @@ constexpr uint32_t kAWarps = 8;                        // warps 0..7 unpack weig
 constexpr uint32_t kBWarps = 8;                        // warps 8..15: fp32 activations: convert the B tile;
                                                        // 16-bit activations: a second unpacking group
 constexpr uint32_t kProducerWarps = kAWarps + kBWarps;
-constexpr uint32_t kTmaWarp = kProducerWarps;          // warp 16: one thread hands B tiles to the copy engine
+constexpr uint32_t kTmaWarp = kProducerWarps;          // warp 16: hands B tiles to the copy engine
 constexpr uint32_t kMmaWarp = kProducerWarps + 1;      // warp 17
 constexpr uint32_t kThreads = (kProducerWarps + 2 + 4) * 32;  // + four epilogue warps
 constexpr uint32_t kMaxRing = 12;                                     // stages the rings may have
@@ -221,7 +225,7 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
 // (a scale has 11 to 18 significant bits, the constants 3 to 9), so weights are still decoded exactly and
 // rounded once; with mins it is off by 2^-24 of 128 scales, 1 / 500 of the rounding to fp16.
 // (Before, the types other than Q4_K, Q8_0 and Q2_0 were unpacked byte by byte from memory: Q5_K 5120 ->
-// 17408 at 64 tokens took 224 us, now 53; Q6_K 197, now 78; IQ4_NL 111, now 55.)
+// 17408 at 64 tokens took 224 us, so 53; with the 8-byte loads below 5120 -> 18944 takes Q6_K 59, IQ4_NL 44.)
 __device__ __forceinline__ float code_f32(uint32_t word, int byte) { return __uint_as_float(__byte_perm(word, 0x43000000u, 0x7044 | byte << 8)); }
 __device__ __forceinline__ float wide_f32(uint32_t word, int byte) { return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7404 | byte << 4)); }
 // four weights out of the bytes of a word
@@ -474,11 +478,6 @@ template <> struct ARaw<T_IQ2_XXS> {
 
 // byte offset of 16-byte chunk j of row r in a 128-byte-swizzled K-major tile
 __device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t j) { return r * 128 + ((j ^ (r & 7)) << 4); }
-
-__device__ __forceinline__ void cp_async16_arrive(uint64_t *bar) {
-    // the arrival fires when this thread's earlier cp.async copies have landed
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // One 2-D tile of the activations, global -> shared, through the tensor map: box =
 // 64 k x 256 tokens, written in the 128-byte-swizzled layout the MMA reads; tokens
@@ -936,10 +935,9 @@ __global__ void __launch_bounds__(256) reduce_kernel(const float *part, ReduceOu
     }
 }
 
-// Tensor maps for tma_load_tile.  The driver's encoder is looked up once; nothing is linked
-// against libcuda.  2-D, element size 1 or 2 bytes: dims / box in elements, stride in bytes.
-static cudaError_t encode_map_2d(CUtensorMap *map, bool bytes, const void *base, uint64_t dim0, uint64_t dim1,
-                                 uint64_t stride, uint32_t box0, uint32_t box1, bool swizzle128) {
+// The tensor map for tma_load_tile: activations X[n][k], 16-bit elements, 64 k x `tokens` per copy, swizzled as the
+// MMA reads them.  The driver's encoder is looked up once; nothing is linked against libcuda.
+static cudaError_t encode_x_map(CUtensorMap *map, const void *x, uint32_t k, uint32_t n, uint32_t tokens) {
     typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -952,19 +950,14 @@ static cudaError_t encode_map_2d(CUtensorMap *map, bool bytes, const void *base,
         if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
         encode = (EncodeFn)fn;
     }
-    const cuuint64_t dims[2] = {dim0, dim1};
-    const cuuint64_t strides[1] = {stride};
-    const cuuint32_t box[2] = {box0, box1};
+    const cuuint64_t dims[2] = {k, n};
+    const cuuint64_t strides[1] = {(cuuint64_t)k * 2};  // bytes
+    const cuuint32_t box[2] = {kBK, tokens};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(map, bytes ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2,
-                              const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                              swizzle128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(x), dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-// the activations X[n][k], 16-bit elements: 64 k x `box` tokens per copy, swizzled as the MMA reads them
-static cudaError_t encode_x_map(CUtensorMap *map, const void *x, uint32_t k, uint32_t n, uint32_t box) {
-    return encode_map_2d(map, false, x, k, n, (uint64_t)k * 2, kBK, box, true);
 }
 template <int TY, int XDT, typename OT, int NACC>
 static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int sms, int dev) {

@@ -728,14 +728,11 @@ struct RingPos {
     }
 };
 
-#ifndef OKF_GEMV_MINB
-#define OKF_GEMV_MINB 2
-#endif
 // XDT: element type of x.  CL: launched in clusters.  (Both were run-time once: the code a launch does not
 // need costs instruction-cache misses that every CTA's staging waits for; Q2_0 2048 -> 2048 3.12 us, so 2.8,
 // Q6_K 2560 -> 151936 90.5, so 85.8.)
 template <int TY, int MODE, int XDT, bool CL>
-__global__ void __launch_bounds__(kGemvThreadsMax, OKF_GEMV_MINB) gemv_kernel(GemvArgs p, GemvLayout L, GemvGather G) {
+__global__ void __launch_bounds__(kGemvThreadsMax, 2) gemv_kernel(GemvArgs p, GemvLayout L, GemvGather G) {
     constexpr uint32_t UB = UnitGeom<TY>::bytes;
     constexpr bool SEP = MODE == M_SEP;
     using W = WideMode<MODE>;
@@ -1372,7 +1369,7 @@ static uint32_t gemv_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, b
 // for one column of long rows with some more tiles than two to an SM: tiles halved between two CTAs spread
 // evenly over the chip, whole ones leave most CTAs one and a few of them two (Q4_K 17408 -> 5120 21.3 ->
 // 16.9 us, Q8_0 32.7 -> 24.6, Q6_K 39.6 -> 28.5, Q2_0 12288 -> 5120 10.7 -> 9.4; Q8_0 5120 -> 5120, 20 units of 272
-// bytes, 8.8 -> 9.5, Q4_K 9216 -> 5120, 36 of 144, 10.3 -> 10.8).
+// bytes, 8.8 -> 9.5, Q4_K 9216 -> 5120, 36 of 144, 10.3 -> 10.8; the line lies somewhere between these points).
 // Several columns: x resident is not enough, copies have to be on their way as well.  A panel that leaves the ring
 // of a CTA alone less than kRingMin, in segments of about 1 KB, goes to two CTAs (Q8_0 17408 -> 8192, 2
 // columns, 88.4 -> 42.2 us, Q5_K 9728 -> 5120, 3 columns, 26.1 -> 19.2; with 36 KB the latter stays).  It is asked of a
@@ -1388,6 +1385,8 @@ static bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, in
         const uint32_t limit = (two_ctas(ty, row_bytes, tiles, sms, mode == M_SEP) ? 2 : 1) * (uint32_t)sms / cs;
         const uint32_t clusters = cs == 1 ? all : tiles < limit ? tiles : limit;
         if (!gemv_layout(ty, row_bytes, nunit, n, mode, cs, (tiles + clusters - 1) / clusters, a, L)) continue;
+        // (both rules for IQ2_XXS hold at the trunk's sizes they were set for, 5120 and 17408; where between them each starts
+        // to pay was not measured)
         const bool last = ty == T_IQ2_XXS && cs == 2;  // shorter segments of its 66-byte units cost more than a resident x gains
         if (!last && (L.panel < a.nchunk || (mode == M_SEP && ty == T_IQ2_XXS && nunit >= 48 && L.tab_copies < 32))) continue;
         if (mode != M_SEP && cs == 1 && !gather && !two_bit(ty) && nunit >= 8) {
@@ -1524,13 +1523,11 @@ cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, co
     GemvGather G = {};
     if (gather) {
         G.nranks = gather->nranks;
-        G.rank = gather->rank;
         G.epoch = gather->epoch;
         G.wait_arrivals = gather->wait_arrivals;
         G.sig_nranks = gather->sig_nranks;
         for (uint32_t r = 0; r < gather->sig_nranks; r++) G.sig_arrivals[r] = gather->sig_arrivals[r];
         G.wait_epoch = gather->wait_epoch;
-        for (uint32_t r = 0; r < gather->nranks; r++) G.arrivals[r] = gather->arrivals[r];
     }
     const size_t xsz = xdt == DT_F32 ? 4 : 2;
     for (uint32_t c0 = 0; c0 < n;) {

@@ -27,27 +27,22 @@ namespace okf {
 // one launch: their tiles are numbered through, segment after segment.
 constexpr int kGemvSegs = 4;
 constexpr int kMaxRanks = 8;
-#ifndef OKF_GEMV_WARPS
-#define OKF_GEMV_WARPS 8
-#endif
-constexpr int kGemvWarps = OKF_GEMV_WARPS;         // consumer warps
+constexpr int kGemvWarps = 8;         // consumer warps
 constexpr int kGemvThreads = (kGemvWarps + 1) * 32;  // + one producer warp
 constexpr int kGemvThreadsMax = kGemvThreads + 32;    // + one warp that announces the previous exchange (row shards only)
 constexpr long long kWaitCycles = 2000000000LL;  // about one second of SM clock
 constexpr uint32_t kSpinLimit = 1u << 16;          // polls when draining on the way out
 constexpr int kStatusFullTimeout = 1, kStatusEmptyTimeout = 2, kStatusGatherTimeout = 4;
 // Row-sharded matrices on several GPUs: every rank stores its rows straight into
-// every rank's copy of the whole output (peer-mapped pointers), counts itself in on
-// every rank, and the launch ends on a rank only when all ranks have counted in.
+// every rank's copy of the whole output (peer-mapped pointers).  The next launch counts the rank in on
+// every rank; whoever reads the output waits until all ranks have counted in.
 struct GemvGather {
     uint32_t nranks;                       // 0: single GPU, `out` below is used
     uint32_t m_total[kGemvSegs];           // rows of the whole matrix
     uint32_t row_first[kGemvSegs];         // this rank's first row in it
     float *out[kGemvSegs][kMaxRanks];      // rank r's [n][m_total] buffer as mapped here
-    uint32_t *arrivals[kMaxRanks];         // rank r's arrival counter, as mapped here: one count per rank and exchange
     uint32_t *epoch;                       // local, two words: {count the local counter reaches when the exchanges
                                            // launched so far are complete, reserved}
-    uint32_t rank;
     // The exchange launched before this one (null: none): its local counter and epoch
     // words.  The consumers wait for it to complete before they read x.
     const uint32_t *wait_arrivals;
@@ -199,10 +194,6 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
 // Shared-memory loads by 32-bit shared-window address: all address arithmetic stays in 32 bits.

@@ -29,11 +29,11 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned bloc
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Copy n16 16-byte words from mapped host memory to the device (the host twins' x).
+cudaError_t launch_fetch(const void *host, void *dst, size_t n16, cudaStream_t s);
 // Simple kernels: one warp per row (matvec), one fp32 register tile per thread
 // (matmul).  They define the numerics the fast kernels are checked against on
 // the device and serve shapes the fast kernels do not take.
-// Copy n16 16-byte words from mapped host memory to the device (the host twins' x).
-cudaError_t launch_fetch(const void *host, void *dst, size_t n16, cudaStream_t s);
 cudaError_t launch_dequant(int ty, const uint8_t *w, uint64_t count, float *out, cudaStream_t s);
 cudaError_t launch_gemv_simple(int ty, const uint8_t *w, uint32_t k, uint32_t m, const void *x,
                                int xdt, uint32_t n, float *out, cudaStream_t s);
