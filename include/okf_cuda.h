@@ -91,7 +91,9 @@ OKF_API int okf_sync(okf_ctx *ctx);
  * woff in the calls below is a byte offset into this buffer, as WeightRef.local is. */
 OKF_API int okf_weights_upload(okf_ctx *ctx, const void *host, size_t bytes, okf_weights **out);
 /* Adopt device memory the caller already owns (no copy, not freed by the
- * library).  The memory must stay valid while the handle is in use and should
+ * library).  Kernels fetch weights ahead of the kernel before them in the stream: one that
+ * writes weights has to be complete before the call (a copy, an event or a synchronisation
+ * in between).  The memory must stay valid while the handle is in use and should
  * be readable for 256 bytes past `bytes` (kernels may fetch whole 16-byte
  * words at the tail). */
 OKF_API int okf_weights_wrap(okf_ctx *ctx, const void *device, size_t bytes, okf_weights **out);
