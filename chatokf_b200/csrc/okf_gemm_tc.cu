@@ -27,10 +27,9 @@
 //
 // Every mbarrier wait is bounded (about a second); a wait that gives up records
 // a code in the status word, the CTA frees its tensor memory and returns.
-#include <cuda.h>
-
 #include <cstring>
-#include "okf_gemv_mma.cuh"
+
+#include "okf_tc.cuh"
 #include "okf_gemv_wide.cuh"
 #include "okf_internal.h"
 #include "okf_kernels.h"
@@ -56,9 +55,7 @@ struct GemmPlan {
 
 namespace tc {
 
-constexpr uint32_t kBM = 128;           // weight rows per CTA tile (UMMA M)
 constexpr uint32_t kBN = 256;           // tokens per accumulator (UMMA N)
-constexpr uint32_t kBK = 64;            // k per stage: 64 x 2 bytes = one 128-byte swizzle row
 constexpr uint32_t kABytes = kBM * kBK * 2;  // 16 KB
 constexpr uint32_t kBBytes = kBN * kBK * 2;  // 32 KB per 256 tokens
 // Two rings.  With one token block per item: as many stages of A (16 KB) and of B (up to 32 KB, by the tokens there
@@ -82,13 +79,6 @@ template <int TY, int NACC> struct Rings {
     static constexpr uint32_t grid_bytes = TY == T_IQ2_XXS ? 2048 : 0;
     static constexpr uint32_t smem = 1024 /*align*/ + a_bytes + b_bytes + grid_bytes + kBarRegion;
 };
-constexpr int kStatusGemmTimeout = 3;
-
-// Output element type that stands for "fp32, stored into every rank's whole output" (row shards).
-struct GatherF32 { float v; };
-template <typename OT> constexpr bool kIsGather = false;
-template <> constexpr bool kIsGather<GatherF32> = true;
-
 struct Args {
     const uint8_t *w;
     const void *x;
@@ -122,10 +112,6 @@ struct Work {
 };
 constexpr uint32_t kWhole = 0xFFFFFFFFu;
 
-// Dealing: CTA c takes k-blocks [total * c / ctas, total * (c + 1) / ctas) of the dealt items laid end to
-// end.  The CTA that takes k-block x (total * ctas stays below 2^32):
-__host__ __device__ __forceinline__ uint32_t dealt_to(uint32_t x, uint32_t total, uint32_t ctas) { return ((x + 1) * ctas - 1) / total; }
-
 // The j-th piece of work of this CTA; false when there is none.  Whole items go
 // round-robin over the CTAs, then every CTA takes its run of the dealt k-blocks, item after item.
 template <int NACC>
@@ -156,62 +142,6 @@ __device__ __forceinline__ bool next_work(const Args &p, uint32_t j, Work &w) {
     return true;
 }
 
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows of 128
-// bytes, groups of eight rows 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);        // start address
-    d |= (uint64_t)1 << 16;                          // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                // stride byte offset: 8 rows x 128 bytes
-    d |= (uint64_t)1 << 46;                          // descriptor version for this architecture
-    d |= (uint64_t)2 << 61;                          // layout: 128-byte swizzle
-    return d;
-}
-
-// Instruction descriptor for kind::f16: fp32 accumulate, A and B of the same
-// 16-bit float type (0 = fp16, 1 = bf16), both K-major, M x N as given.
-__host__ __device__ constexpr uint32_t instr_desc(uint32_t fmt, uint32_t mm, uint32_t nn) {
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((nn >> 3) << 17) | ((mm >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-template <bool F16>
-__device__ __forceinline__ uint32_t pack16(float a, float b) {
-    if constexpr (F16) {
-        __half2 h = __floats2half2_rn(a, b);
-        return *reinterpret_cast<uint32_t *>(&h);
-    } else {
-        __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-        return *reinterpret_cast<uint32_t *>(&h);
-    }
-}
-
 // ---- weights for the A tile -------------------------------------------------------
 // ARaw<TY> holds, in registers, the bytes one thread needs to unpack 32 weights (half h of k-block kb) of
 // its row; load() is issued a turn or two ahead of unpack() so that the latency of L2 hides behind the
@@ -226,8 +156,6 @@ __device__ __forceinline__ uint32_t pack16(float a, float b) {
 // rounded once; with mins it is off by 2^-24 of 128 scales, 1 / 500 of the rounding to fp16.
 // (Before, the types other than Q4_K, Q8_0 and Q2_0 were unpacked byte by byte from memory: Q5_K 5120 ->
 // 17408 at 64 tokens took 224 us, so 53; with the 8-byte loads below 5120 -> 18944 takes Q6_K 59, IQ4_NL 44.)
-__device__ __forceinline__ float code_f32(uint32_t word, int byte) { return __uint_as_float(__byte_perm(word, 0x43000000u, 0x7044 | byte << 8)); }
-__device__ __forceinline__ float wide_f32(uint32_t word, int byte) { return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7404 | byte << 4)); }
 // four weights out of the bytes of a word
 template <bool F16>
 __device__ __forceinline__ uint2 unpack4(uint32_t w, float mul, float add) {
@@ -475,81 +403,6 @@ template <> struct ARaw<T_IQ2_XXS> {
         }
     }
 };
-
-// byte offset of 16-byte chunk j of row r in a 128-byte-swizzled K-major tile
-__device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t j) { return r * 128 + ((j ^ (r & 7)) << 4); }
-
-// One 2-D tile of the activations, global -> shared, through the tensor map: box =
-// 64 k x 256 tokens, written in the 128-byte-swizzled layout the MMA reads; tokens
-// past the end of X come back as zeros.  x is the element index along k (a multiple
-// of 8, so the copy starts on a 16-byte boundary), y the token.
-__device__ __forceinline__ void tma_load_tile(void *dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_u32(dst)),
-        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Waiting on an mbarrier without taking issue slots from the unpacking warps: try_wait with
-// a time hint parks the thread in hardware until the phase completes or the hint runs out,
-// so a waiter costs a handful of instructions per microsecond instead of a polling loop.
-__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t *bar, uint32_t parity, uint32_t ns) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
-        : "memory");
-    return ok != 0;
-}
-// The phase was not over at the first look.  Bounded (about a second): a wait that gives
-// up sets the CTA's abort flag and the status word.
-__device__ __noinline__ bool mbar_wait_parked(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status) {
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 16; i++)
-            if (mbar_try_wait_hint(bar, parity, 2000u)) return true;
-        if (*abort_flag) return false;
-        if (clock64() - t0 > kWaitCycles) break;
-    }
-    *abort_flag = 1;
-    if (status) atomicExch(status, kStatusGemmTimeout);
-    return false;
-}
-// One lane waits, the warp follows.
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, uint32_t lane, volatile int *abort_flag,
-                                          int *status) {
-    bool ok = true;
-    if (lane == 0 && !mbar_try_wait(bar, parity)) ok = mbar_wait_parked(bar, parity, abort_flag, status);
-    return __shfl_sync(0xffffffffu, ok, 0);
-}
-// The MMA issuer and the copy engine's client: the whole warp waits and walks the loop, converged, and one
-// elected lane issues.  Inside a branch that only one lane takes, descriptors and addresses are not uniform
-// to the compiler, and every tcgen05 instruction becomes a loop over the warp's values: 640 cycles of
-// issue per k-block, which set the pace of all k-blocks with few tokens (0.65 us each, whatever the type).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-    return p != 0;
-}
-__device__ __forceinline__ bool warp_poll(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status) {
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    const long long t0 = clock64();
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 64; i++)
-            if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
-        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles)) break;
-    }
-    *abort_flag = 1;
-    if (status) atomicExch(status, kStatusGemmTimeout);
-    return false;
-}
 
 // NACC: token blocks (accumulators) per work item, 1 or 2.
 template <int TY, int XDT, typename OT, int NACC>
@@ -882,7 +735,8 @@ done:
 
 // Sum the partial tiles of the dealt items, part after part (the order of k), into every output buffer:
 // element (token, row) at [token * out_ld + out_row0 + row].  A block takes 16 tokens of an item, a thread
-// four rows of one token at a time.
+// four rows of one token at a time.  (The parameters stay where they are: indexed by a variable, a by-value copy goes to
+// local memory first, 32 stores a thread.)
 struct ReduceOut {
     uint32_t nout, m, n, out_ld, out_row0;
     uint32_t dealt, base, kblocks, ctas, nt, groups, group_tok;  // the main kernel's dealing
@@ -897,7 +751,7 @@ constexpr uint32_t kReduceTok = 16;
 // per thread, which bound how many of these CTAs gather on the SMs that the matmul leaves first: forms of 32
 // to 36 registers took 19.8 to 21.7 us, of 42 to 44 19.1 to 19.5.)
 template <typename OT, bool VEC>
-__global__ void __launch_bounds__(256) reduce_kernel(const float *part, ReduceOut o) {
+__global__ void __launch_bounds__(256) reduce_kernel(const float *part, const __grid_constant__ ReduceOut o) {
     pdl_launch_dependents();
     const uint32_t runs = (o.nt + kReduceTok - 1) / kReduceTok;
     const uint32_t i = blockIdx.x / runs, t0 = blockIdx.x % runs * kReduceTok, total = o.dealt * o.kblocks;
@@ -935,30 +789,6 @@ __global__ void __launch_bounds__(256) reduce_kernel(const float *part, ReduceOu
     }
 }
 
-// The tensor map for tma_load_tile: activations X[n][k], 16-bit elements, 64 k x `tokens` per copy, swizzled as the
-// MMA reads them.  The driver's encoder is looked up once; nothing is linked against libcuda.
-static cudaError_t encode_x_map(CUtensorMap *map, const void *x, uint32_t k, uint32_t n, uint32_t tokens) {
-    typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn encode = nullptr;
-    if (!encode) {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
-        if (e != cudaSuccess) return e;
-        if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
-        encode = (EncodeFn)fn;
-    }
-    const cuuint64_t dims[2] = {k, n};
-    const cuuint64_t strides[1] = {(cuuint64_t)k * 2};  // bytes
-    const cuuint32_t box[2] = {kBK, tokens};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void *>(x), dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
 template <int TY, int XDT, typename OT, int NACC>
 static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int sms, int dev) {
     static bool attr_set[64] = {};  // the opt-in is per device

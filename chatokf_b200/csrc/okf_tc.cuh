@@ -1,0 +1,191 @@
+// What the prefill matmul is built from: tcgen05 descriptors and instructions, waits that end, tensor maps, how
+// left-over work is dealt out.
+#pragma once
+#include <cuda.h>
+
+#include "okf_gemv_mma.cuh"
+
+namespace okf {
+namespace tc {
+
+constexpr uint32_t kBM = 128;  // weight rows per CTA tile (UMMA M)
+constexpr uint32_t kBK = 64;   // k per stage: 64 x 2 bytes = one 128-byte swizzle row
+constexpr int kStatusGemmTimeout = 3;
+
+// Output element type that stands for "fp32, stored into every rank's whole output" (row shards).
+struct GatherF32 { float v; };
+template <typename OT> constexpr bool kIsGather = false;
+template <> constexpr bool kIsGather<GatherF32> = true;
+
+// Dealing: CTA c takes k-blocks [total * c / ctas, total * (c + 1) / ctas) of the dealt items laid end to
+// end.  The CTA that takes k-block x (total * ctas stays below 2^32):
+__host__ __device__ __forceinline__ uint32_t dealt_to(uint32_t x, uint32_t total, uint32_t ctas) { return ((x + 1) * ctas - 1) / total; }
+
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows of 128
+// bytes, groups of eight rows 1024 bytes apart.
+__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);        // start address
+    d |= (uint64_t)1 << 16;                          // leading byte offset (unused for swizzled K-major)
+    d |= (uint64_t)(1024 >> 4) << 32;                // stride byte offset: 8 rows x 128 bytes
+    d |= (uint64_t)1 << 46;                          // descriptor version for this architecture
+    d |= (uint64_t)2 << 61;                          // layout: 128-byte swizzle
+    return d;
+}
+
+// Instruction descriptor for kind::f16: fp32 accumulate, A and B of the same
+// 16-bit float type (0 = fp16, 1 = bf16), both K-major, M x N as given.
+__host__ __device__ constexpr uint32_t instr_desc(uint32_t fmt, uint32_t mm, uint32_t nn) {
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((nn >> 3) << 17) | ((mm >> 4) << 24);
+}
+
+__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+template <bool F16>
+__device__ __forceinline__ uint32_t pack16(float a, float b) {
+    if constexpr (F16) {
+        __half2 h = __floats2half2_rn(a, b);
+        return *reinterpret_cast<uint32_t *>(&h);
+    } else {
+        __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+        return *reinterpret_cast<uint32_t *>(&h);
+    }
+}
+
+__device__ __forceinline__ float code_f32(uint32_t word, int byte) { return __uint_as_float(__byte_perm(word, 0x43000000u, 0x7044 | byte << 8)); }
+__device__ __forceinline__ float wide_f32(uint32_t word, int byte) { return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7404 | byte << 4)); }
+
+// byte offset of 16-byte chunk j of row r in a 128-byte-swizzled K-major tile
+__device__ __forceinline__ uint32_t swz(uint32_t r, uint32_t j) { return r * 128 + ((j ^ (r & 7)) << 4); }
+
+// One 2-D tile of the activations, global -> shared, through the tensor map: box =
+// 64 k x 256 tokens, written in the 128-byte-swizzled layout the MMA reads; tokens
+// past the end of X come back as zeros.  x is the element index along k (a multiple
+// of 8, so the copy starts on a 16-byte boundary), y the token.
+__device__ __forceinline__ void tma_load_tile(void *dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint64_t *bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
+        : "memory");
+}
+
+// Waiting on an mbarrier without taking issue slots from the unpacking warps: try_wait with
+// a time hint parks the thread in hardware until the phase completes or the hint runs out,
+// so a waiter costs a handful of instructions per microsecond instead of a polling loop.
+__device__ __forceinline__ bool mbar_try_wait_hint(uint64_t *bar, uint32_t parity, uint32_t ns) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(ns)
+        : "memory");
+    return ok != 0;
+}
+// The phase was not over at the first look.  Bounded (about a second): a wait that gives
+// up sets the CTA's abort flag and the status word.
+static __device__ __noinline__ bool mbar_wait_parked(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status) {
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 16; i++)
+            if (mbar_try_wait_hint(bar, parity, 2000u)) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > kWaitCycles) break;
+    }
+    *abort_flag = 1;
+    if (status) atomicExch(status, kStatusGemmTimeout);
+    return false;
+}
+// Over already: the usual case, and every lane sees it for itself.  Else one lane waits and the warp follows.  (One lane asking
+// and telling the others every time cost the unpacking warps some 300 cycles a turn: Q4_K 5120 -> 17408, 512 tokens, 74.3 us, so 70.8;
+// 4096 tokens 600, so 565.)
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, uint32_t lane, volatile int *abort_flag,
+                                          int *status) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    bool ok = true;
+    if (lane == 0) ok = mbar_wait_parked(bar, parity, abort_flag, status);
+    return __shfl_sync(0xffffffffu, ok, 0);
+}
+// The MMA issuer and the copy engine's client: the whole warp waits and walks the loop, converged, and one
+// elected lane issues.  Inside a branch that only one lane takes, descriptors and addresses are not uniform
+// to the compiler, and every tcgen05 instruction becomes a loop over the warp's values: 640 cycles of
+// issue per k-block, which set the pace of all k-blocks with few tokens (0.65 us each, whatever the type).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ bool warp_poll(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *status) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 64; i++)
+            if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles)) break;
+    }
+    *abort_flag = 1;
+    if (status) atomicExch(status, kStatusGemmTimeout);
+    return false;
+}
+
+// A tensor map for tma_load_tile: `rows` rows of `inner` elements, `pitch` bytes apart, copied `box_inner` x `box_rows` at a
+// time.  The driver's encoder is looked up once; nothing is linked against libcuda.
+inline cudaError_t encode_map(CUtensorMap *map, CUtensorMapDataType type, const void *base, uint64_t inner, uint64_t rows, uint64_t pitch,
+                              uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle swizzle) {
+    typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static EncodeFn encode = nullptr;
+    if (!encode) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q);
+        if (e != cudaSuccess) return e;
+        if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
+        encode = (EncodeFn)fn;
+    }
+    const cuuint64_t dims[2] = {inner, rows};
+    const cuuint64_t strides[1] = {pitch};
+    const cuuint32_t box[2] = {box_inner, box_rows};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = encode(map, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+// Activations X[n][k], 16-bit elements, 64 k x `tokens` per copy, swizzled as the MMA reads them.
+inline cudaError_t encode_x_map(CUtensorMap *map, const void *x, uint32_t k, uint32_t n, uint32_t tokens) {
+    return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, x, k, n, (uint64_t)k * 2, kBK, tokens, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+}  // namespace tc
+}  // namespace okf
