@@ -30,6 +30,7 @@
 #include <cstring>
 
 #include "okf_tc.cuh"
+#include "okf_gemm_ts.h"
 #include "okf_gemv_wide.cuh"
 #include "okf_internal.h"
 #include "okf_kernels.h"
@@ -48,6 +49,7 @@ namespace okf {
 // partial tiles move at 8 TB/s, mostly through L2.  (4096 tokens 17408 -> 5120: 320 items of two blocks
 // are 2.16 waves; three whole waves took 760 us, two and 24 dealt items 590.)
 struct GemmPlan {
+    uint32_t tok;    // tokens per item of the kernel with weights in tensor memory, 0: the other one
     uint32_t nacc;   // token blocks per item
     uint32_t waves, dealt, dealers, nt;  // see tc::Args
     size_t floats;   // of partial tiles
@@ -739,7 +741,7 @@ done:
 // local memory first, 32 stores a thread.)
 struct ReduceOut {
     uint32_t nout, m, n, out_ld, out_row0;
-    uint32_t dealt, base, kblocks, ctas, nt, groups, group_tok;  // the main kernel's dealing
+    uint32_t dealt, base, steps, ctas, nt, groups, group_tok;  // the main kernel's dealing, an item being `steps` long
     void *outs[8];
     uint32_t *epoch;
     uint32_t epoch_inc;
@@ -754,8 +756,8 @@ template <typename OT, bool VEC>
 __global__ void __launch_bounds__(256) reduce_kernel(const float *part, const __grid_constant__ ReduceOut o) {
     pdl_launch_dependents();
     const uint32_t runs = (o.nt + kReduceTok - 1) / kReduceTok;
-    const uint32_t i = blockIdx.x / runs, t0 = blockIdx.x % runs * kReduceTok, total = o.dealt * o.kblocks;
-    const uint32_t c0 = dealt_to(i * o.kblocks, total, o.ctas), c1 = dealt_to((i + 1) * o.kblocks - 1, total, o.ctas);
+    const uint32_t i = blockIdx.x / runs, t0 = blockIdx.x % runs * kReduceTok, total = o.dealt * o.steps;
+    const uint32_t c0 = dealt_to(i * o.steps, total, o.ctas), c1 = dealt_to((i + 1) * o.steps - 1, total, o.ctas);
     const uint32_t item = o.base - o.dealt + i, n0 = item % o.groups * o.group_tok;
     const uint32_t r = (threadIdx.x & 31) * 4, row = item / o.groups * kBM + r;
     pdl_wait();
@@ -818,49 +820,45 @@ static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int s
         cudaError_t me = encode_x_map(&xmap, a.x, a.k, a.n, g.box);
         if (me != cudaSuccess) return me;
     }
-    cudaError_t e = launch_pdl(gemm_tc_kernel<TY, XDT, OT, NACC>, grid, kThreads, Rings<TY, NACC>::smem, s, 1, xmap, a, g);
-    if (e != cudaSuccess || !a.dealt) return e;
-    ReduceOut ro = {go.nout, a.m, a.n, go.out_ld, go.out_row0, a.dealt, items, a.k / kBK, a.dealers, a.nt, groups, NACC * kBN, {}, go.epoch,
-                    go.epoch_inc};
+    return launch_pdl(gemm_tc_kernel<TY, XDT, OT, NACC>, grid, kThreads, Rings<TY, NACC>::smem, s, 1, xmap, a, g);
+}
+
+template <int TY, int XDT, typename OT>
+static cudaError_t launch(const Args &a, const Outs &go, cudaStream_t s, int sms, int dev) {
+    return launch_n<TY, XDT, OT, XDT == DT_F32 ? 1 : 2>(a, go, s, sms, dev);
+}
+
+template <int TY, int XDT>
+static cudaError_t launch_o(const Args &a, const Outs &go, int odt, cudaStream_t s, int sms, int dev) {
+    if (odt == DT_F32 && go.epoch) return launch<TY, XDT, GatherF32>(a, go, s, sms, dev);
+    if (odt == DT_F32) return launch<TY, XDT, float>(a, go, s, sms, dev);
+    if (odt == DT_BF16) return launch<TY, XDT, __nv_bfloat16>(a, go, s, sms, dev);
+    return cudaErrorInvalidValue;
+}
+
+template <int TY>
+static cudaError_t launch_x(const Args &a, const Outs &go, int xdt, int odt, cudaStream_t s, int sms, int dev) {
+    switch (xdt) {
+    case DT_F16: return launch_o<TY, DT_F16>(a, go, odt, s, sms, dev);
+    case DT_BF16: return launch_o<TY, DT_BF16>(a, go, odt, s, sms, dev);
+    case DT_F32: return launch_o<TY, DT_F32>(a, go, odt, s, sms, dev);
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+// `tok`, `steps`: tokens of an item and what its k is dealt by
+static cudaError_t launch_reduce(const float *part, const Args &a, const Outs &go, uint32_t tok, uint32_t steps, int odt, cudaStream_t s) {
+    const uint32_t groups = (a.n + tok - 1) / tok, items = (a.m + kBM - 1) / kBM * groups;
+    ReduceOut ro = {go.nout, a.m, a.n, go.out_ld, go.out_row0, a.dealt, items, steps, a.dealers, a.nt, groups, tok, {}, go.epoch, go.epoch_inc};
     bool vec = ((a.m | go.out_ld | go.out_row0) & 3) == 0;
     for (uint32_t o = 0; o < go.nout; o++) {
         ro.outs[o] = go.outs[o];
         vec = vec && (uintptr_t)go.outs[o] % 16 == 0;
     }
     const unsigned blocks = a.dealt * ((a.nt + kReduceTok - 1) / kReduceTok);
-    const float *part = a.partial;
-    if constexpr (sizeof(OT) == 4) {
-        if (vec) return launch_pdl(reduce_kernel<float, true>, blocks, 256, 0, s, 1, part, ro);
-        return launch_pdl(reduce_kernel<float, false>, blocks, 256, 0, s, 1, part, ro);
-    } else {
-        return launch_pdl(reduce_kernel<OT, false>, blocks, 256, 0, s, 1, part, ro);
-    }
-}
-
-template <int TY, int XDT, typename OT>
-static cudaError_t launch(const Args &a, const Outs &go, const GemmPlan &plan, cudaStream_t s, int sms, int dev) {
-    if constexpr (XDT != DT_F32) {
-        if (plan.nacc == 2) return launch_n<TY, XDT, OT, 2>(a, go, s, sms, dev);
-    }
-    return launch_n<TY, XDT, OT, 1>(a, go, s, sms, dev);
-}
-
-template <int TY, int XDT>
-static cudaError_t launch_o(const Args &a, const Outs &go, const GemmPlan &plan, int odt, cudaStream_t s, int sms, int dev) {
-    if (odt == DT_F32 && go.epoch) return launch<TY, XDT, GatherF32>(a, go, plan, s, sms, dev);
-    if (odt == DT_F32) return launch<TY, XDT, float>(a, go, plan, s, sms, dev);
-    if (odt == DT_BF16) return launch<TY, XDT, __nv_bfloat16>(a, go, plan, s, sms, dev);
-    return cudaErrorInvalidValue;
-}
-
-template <int TY>
-static cudaError_t launch_x(const Args &a, const Outs &go, const GemmPlan &plan, int xdt, int odt, cudaStream_t s, int sms, int dev) {
-    switch (xdt) {
-    case DT_F16: return launch_o<TY, DT_F16>(a, go, plan, odt, s, sms, dev);
-    case DT_BF16: return launch_o<TY, DT_BF16>(a, go, plan, odt, s, sms, dev);
-    case DT_F32: return launch_o<TY, DT_F32>(a, go, plan, odt, s, sms, dev);
-    default: return cudaErrorInvalidValue;
-    }
+    if (odt == DT_BF16) return launch_pdl(reduce_kernel<__nv_bfloat16, false>, blocks, 256, 0, s, 1, part, ro);
+    if (vec) return launch_pdl(reduce_kernel<float, true>, blocks, 256, 0, s, 1, part, ro);
+    return launch_pdl(reduce_kernel<float, false>, blocks, 256, 0, s, 1, part, ro);
 }
 
 }  // namespace tc
@@ -880,51 +878,80 @@ cudaError_t launch_to_bf16(const void *x, void *y, size_t count, int sms, cudaSt
     return launch_pdl(to_bf16_kernel, (unsigned)(blocks < most ? blocks : most), 256, 0, s, 1, (const float4 *)x, (uint4 *)y, count / 8);
 }
 
-static GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms, size_t max_floats) {
+// The better of running `slabs` x `groups` items of `tok` tokens whole and of dealing the last wave out, into `best` if it
+// beats `best_t`.  An item is `steps` of k long; t_step: seconds for one; t_item: what an item adds; `least`: steps a CTA takes at least.
+static void lay_out(GemmPlan plan, uint32_t slabs, uint32_t steps, uint32_t n, uint32_t tok, double t_step, double t_item, uint32_t least, uint32_t all,
+                    size_t max_floats, GemmPlan &best, double &best_t) {
+    const uint32_t base = slabs * ((n + tok - 1) / tok);
+    const double whole = ((base + all - 1) / all) * (steps * t_step + t_item);
+    if (whole < best_t) { best_t = whole; best = plan; }
+    // the items of the last, part-filled wave (of the only one) dealt out by steps
+    const uint32_t waves = base / all, dealt = base % all, nt = n < tok ? n : tok;
+    if (dealt == 0) return;
+    const uint64_t total = (uint64_t)dealt * steps;
+    if (total * (all + 1) >= 0xFFFFFFFFull) return;
+    uint32_t ctas = total / least < all ? (uint32_t)(total / least) : all;
+    if (ctas <= dealt) return;
+    uint32_t parts = 1;
+    for (uint32_t i = 0; i < dealt; i++) {
+        const uint32_t c = tc::dealt_to((i + 1) * steps - 1, (uint32_t)total, ctas) - tc::dealt_to(i * steps, (uint32_t)total, ctas) + 1;
+        if (c > parts) parts = c;
+    }
+    const size_t part = (size_t)dealt * nt * tc::kBM;  // floats
+    if (parts * part > max_floats) {
+        // as many equal parts of every item as there is room for (Q4_K 9728 -> 2560, 512 tokens, in 16 MiB: on 40
+        // of the SMs 71 us with fp16 and 358 with fp32 activations, in three parts on 120 of them 35 and 196)
+        parts = (uint32_t)(max_floats / part);
+        if (parts > steps / least) parts = steps / least;
+        if (parts > all / dealt) parts = all / dealt;
+        if (parts < 2) return;
+        ctas = dealt * parts;
+    }
+    const double moved = 2.0 * (dealt + ctas) * nt * tc::kBM * 4;
+    const double t = waves * (steps * t_step + t_item) + ((total + ctas - 1) / ctas) * t_step + 2.5e-6 + moved / 8e12;
+    if (t < best_t) {
+        best_t = t;
+        best = plan;
+        best.waves = waves; best.dealt = dealt; best.dealers = ctas; best.nt = nt; best.floats = parts * part;
+    }
+}
+// 16-bit activations: seconds per k-block of an item of `tok` tokens on the kernel with weights in tensor memory.  Up to
+// some 100 tokens the unpacking sets the pace, above that the activations' way through shared memory (5120 -> 17408, 80 k-blocks an SM:
+// 21.5 to 31 us at 64 tokens, Q4_K 28.9 at 128, 76 at 512 in two items).
+static double ts_kblock(int ty, uint32_t tok) {
+    const double unpack = ty == T_Q8_0 ? 0.29e-6 : ty == T_Q6_K ? 0.335e-6 : ty == T_IQ2_XXS || ty == T_IQ4_NL ? 0.3e-6 : ty == T_Q5_K ? 0.26e-6 : 0.23e-6;
+    const double stream = 0.17e-6 + 1.1e-9 * tok;
+    return unpack > stream ? unpack : stream;
+}
+// `narrow`: items may be of any number of tokens (fewer than 256 where that gives every SM one: Q2_0 2048 -> 6144, 512 tokens, in
+// 144 items of 176 tokens 16 us, in 96 of 256 17, in 48 of 512 20).  The call without allocation keeps to wide ones.
+static GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms, size_t max_floats, bool narrow) {
     const uint32_t slabs = (m + tc::kBM - 1) / tc::kBM, kblocks = k / tc::kBK, all = (uint32_t)sms;
-    GemmPlan best = {};
+    GemmPlan best = {}, plan = {};
     double best_t = 1e30;
-    for (uint32_t nacc = 1; nacc <= 2; nacc++) {
-        if (nacc == 2 && (xdt == DT_F32 || n <= tc::kBN)) continue;
-        const bool slow = ty == T_Q8_0 || ty == T_Q6_K;
-        // (fp32 activations that the tile converts itself, by one group of warps while another unpacks:
-        // 0.9 us, from some 80 tokens on what the conversion takes, 2.3 us at 256)
-        const double t_kb = xdt == DT_F32 ? (n > 80 ? 0.3e-6 + 7.8e-9 * (n < tc::kBN ? n : tc::kBN) : 0.9e-6) : nacc == 2 ? (slow ? 1.15e-6 : 0.93e-6) : (slow ? 0.8e-6 : 0.45e-6 + 0.4e-9 * (n < tc::kBN ? n : tc::kBN));
-        const uint32_t base = slabs * ((n + nacc * tc::kBN - 1) / (nacc * tc::kBN));
-        const double whole = ((base + all - 1) / all) * (kblocks * t_kb + (nacc == 2 ? 3e-6 : 0));
-        if (whole < best_t) { best_t = whole; best = {nacc, 0, 0, 0, 0, 0}; }
-        // the items of the last, part-filled wave (of the only one) dealt out by k-blocks
-        const uint32_t waves = base / all, dealt = base % all, nt = n < nacc * tc::kBN ? n : nacc * tc::kBN;
-        if (dealt == 0) continue;
-        const uint64_t total = (uint64_t)dealt * kblocks;
-        if (total * (all + 1) >= 0xFFFFFFFFull) continue;
-        uint32_t ctas = total / 4 < all ? (uint32_t)(total / 4) : all;  // four k-blocks at least
-        if (ctas <= dealt) continue;
-        uint32_t parts = 1;
-        for (uint32_t i = 0; i < dealt; i++) {
-            const uint32_t c = tc::dealt_to((i + 1) * kblocks - 1, (uint32_t)total, ctas) - tc::dealt_to(i * kblocks, (uint32_t)total, ctas) + 1;
-            if (c > parts) parts = c;
-        }
-        const size_t part = (size_t)dealt * nt * tc::kBM;  // floats
-        if (parts * part > max_floats) {
-            // as many equal parts of every item as there is room for (Q4_K 9728 -> 2560, 512 tokens, in 16 MiB: on 40
-            // of the SMs 71 us with fp16 and 358 with fp32 activations, in three parts on 120 of them 35 and 196)
-            parts = (uint32_t)(max_floats / part);
-            if (parts > kblocks / 4) parts = kblocks / 4;
-            if (parts > all / dealt) parts = all / dealt;
-            if (parts < 2) continue;
-            ctas = dealt * parts;
-        }
-        const size_t floats = parts * part;
-        const double moved = 2.0 * (dealt + ctas) * nt * tc::kBM * 4;
-        const double t = waves * (kblocks * t_kb + (nacc == 2 ? 3e-6 : 0)) + (double)total / ctas * t_kb + 4e-6 + moved / 8e12;
-        if (t < best_t) { best_t = t; best = {nacc, waves, dealt, ctas, nt, floats}; }
+    if (xdt == DT_F32) {
+        // fp32 activations that the tile converts itself, by one group of warps while another unpacks:
+        // 0.9 us, from some 80 tokens on what the conversion takes, 2.3 us at 256
+        plan.nacc = 1;
+        lay_out(plan, slabs, kblocks, n, tc::kBN, n > 80 ? 0.3e-6 + 7.8e-9 * (n < tc::kBN ? n : tc::kBN) : 0.9e-6, 0, 4, all, max_floats, best, best_t);
+        return best;
+    }
+    if (n > tc::kBN) {
+        plan.nacc = 2;
+        lay_out(plan, slabs, kblocks, n, 2 * tc::kBN, ty == T_Q8_0 || ty == T_Q6_K ? 1.1e-6 : 0.86e-6, 3e-6, 4, all, max_floats, best, best_t);
+        plan.nacc = 0;
+    }
+    const uint32_t least = (n + tc::kBN - 1) / tc::kBN;
+    for (uint32_t blocks = least; blocks <= (narrow ? least + 8 : least); blocks++) {
+        plan.tok = ((n + blocks - 1) / blocks + 15) / 16 * 16;
+        lay_out(plan, slabs, (kblocks + 3) / 4, n, plan.tok, 4 * ts_kblock(ty, plan.tok), plan.tok > 128 ? 2.5e-6 : 1e-6, 1, all, max_floats, best, best_t);
+        if (plan.tok <= 32) break;
     }
     return best;
 }
 
 size_t gemm_tc_scratch(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms) {
-    return gemm_tc_plan(ty, k, m, n, xdt, sms, kMaxScratchFloats).floats;
+    return gemm_tc_plan(ty, k, m, n, xdt, sms, kMaxScratchFloats, true).floats;
 }
 bool gemm_tc_supported(int ty, uint32_t k, uint32_t m, const void *w, const void *x, int xdt, uint32_t n) {
     if (!has_fast_kernels(ty)) return false;
@@ -936,7 +963,7 @@ bool gemm_tc_supported(int ty, uint32_t k, uint32_t m, const void *w, const void
 
 cudaError_t launch_gemm_tc(int ty, const uint8_t *w, uint32_t k, uint32_t m, const void *x, int xdt,
                            uint32_t n, void *out, int odt, int *status, float *partial, size_t partial_floats,
-                           cudaStream_t s, int sms, int dev, uint64_t *launches, const GemvGatherPlan *gather) {
+                           cudaStream_t s, int sms, int dev, uint64_t *launches, const GemvGatherPlan *gather, bool narrow) {
     tc::Args a = {};
     a.w = w; a.x = x; a.out = out; a.status = status; a.k = k; a.m = m; a.n = n;
     tc::Outs go = {};
@@ -951,22 +978,31 @@ cudaError_t launch_gemm_tc(int ty, const uint8_t *w, uint32_t k, uint32_t m, con
     } else {
         go.nout = 1; go.out_ld = m; go.out_row0 = 0; go.outs[0] = out;
     }
-    const GemmPlan plan = gemm_tc_plan(ty, k, m, n, xdt, sms, partial ? partial_floats : 0);
+    const GemmPlan plan = gemm_tc_plan(ty, k, m, n, xdt, sms, partial ? partial_floats : 0, narrow);
     a.waves = plan.waves; a.dealt = plan.dealt; a.dealers = plan.dealers; a.nt = plan.nt;
     a.partial = partial;
     *launches += plan.dealt ? 2 : 1;
     a.row_bytes = (k / block_elems(ty)) * block_bytes(ty);
-    switch (ty) {
-    case T_Q4_K: return tc::launch_x<T_Q4_K>(a, go, plan, xdt, odt, s, sms, dev);
-    case T_Q8_0: return tc::launch_x<T_Q8_0>(a, go, plan, xdt, odt, s, sms, dev);
-    case T_Q4_0: return tc::launch_x<T_Q4_0>(a, go, plan, xdt, odt, s, sms, dev);
-    case T_Q6_K: return tc::launch_x<T_Q6_K>(a, go, plan, xdt, odt, s, sms, dev);
-    case T_Q5_K: return tc::launch_x<T_Q5_K>(a, go, plan, xdt, odt, s, sms, dev);
-    case T_IQ4_NL: return tc::launch_x<T_IQ4_NL>(a, go, plan, xdt, odt, s, sms, dev);
-    case T_Q2_0: return tc::launch_x<T_Q2_0>(a, go, plan, xdt, odt, s, sms, dev);
-    case T_IQ2_XXS: return tc::launch_x<T_IQ2_XXS>(a, go, plan, xdt, odt, s, sms, dev);
-    default: return cudaErrorInvalidValue;
+    cudaError_t e = cudaErrorInvalidValue;
+    if (plan.tok) {
+        GemmTs g = {ty, xdt, odt, sms, w, x, out, status, partial, k, m, n, a.row_bytes, plan.tok, a.waves, a.dealt, a.dealers, a.nt,
+                    gather ? go.nout : 0u, go.out_ld, go.out_row0, {}, go.epoch, go.epoch_inc};
+        for (uint32_t r = 0; r < go.nout; r++) g.outs[r] = go.outs[r];
+        e = launch_gemm_ts(g, s, dev);
+    } else {
+        switch (ty) {
+        case T_Q4_K: e = tc::launch_x<T_Q4_K>(a, go, xdt, odt, s, sms, dev); break;
+        case T_Q8_0: e = tc::launch_x<T_Q8_0>(a, go, xdt, odt, s, sms, dev); break;
+        case T_Q4_0: e = tc::launch_x<T_Q4_0>(a, go, xdt, odt, s, sms, dev); break;
+        case T_Q6_K: e = tc::launch_x<T_Q6_K>(a, go, xdt, odt, s, sms, dev); break;
+        case T_Q5_K: e = tc::launch_x<T_Q5_K>(a, go, xdt, odt, s, sms, dev); break;
+        case T_IQ4_NL: e = tc::launch_x<T_IQ4_NL>(a, go, xdt, odt, s, sms, dev); break;
+        case T_Q2_0: e = tc::launch_x<T_Q2_0>(a, go, xdt, odt, s, sms, dev); break;
+        case T_IQ2_XXS: e = tc::launch_x<T_IQ2_XXS>(a, go, xdt, odt, s, sms, dev); break;
+        }
     }
+    if (e != cudaSuccess || !a.dealt) return e;
+    return tc::launch_reduce(partial, a, go, plan.tok ? plan.tok : plan.nacc * tc::kBN, plan.tok ? (k + 255) / 256 : k / tc::kBK, odt, s);
 }
 
 }  // namespace okf
@@ -1011,7 +1047,7 @@ extern "C" int okf_gemm_noalloc(okf_ctx *ctx, int type, const okf_weights *w, ui
     // every slot the reduction reads is written by the main kernel first, so nothing in the
     // array has to be cleared between calls
     cudaError_t e = launch_gemm_tc(type, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, g_static_scratch_addr[ctx->device],
-                                   kStaticScratchFloats, (cudaStream_t)stream, ctx->sms, ctx->device, &ctx->launches, nullptr);
+                                   kStaticScratchFloats, (cudaStream_t)stream, ctx->sms, ctx->device, &ctx->launches, nullptr, false);
     if (e != cudaSuccess) return cuda_fail(ctx, e);
     return OKF_OK;
 }

@@ -95,6 +95,6 @@ cudaError_t launch_to_bf16(const void *x, void *y, size_t count, int sms, cudaSt
 // output (seg[0]) instead of `out`.
 cudaError_t launch_gemm_tc(int ty, const uint8_t *w, uint32_t k, uint32_t m, const void *x, int xdt,
                            uint32_t n, void *out, int odt, int *status, float *partial, size_t partial_floats,
-                           cudaStream_t s, int sms, int dev, uint64_t *launches, const GemvGatherPlan *gather);
+                           cudaStream_t s, int sms, int dev, uint64_t *launches, const GemvGatherPlan *gather, bool narrow = true);
 
 }  // namespace okf
