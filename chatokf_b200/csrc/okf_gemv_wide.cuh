@@ -166,12 +166,25 @@ __device__ __forceinline__ uint2 iq4nl_word(uint32_t w) {
     return r;
 }
 
-// 4 bytes at a 2-byte aligned shared address
-__device__ __forceinline__ uint32_t lds_word_a2(uint32_t a) {
-    uint32_t v[1];
-    lds_a2<1>(a, v);
-    return v[0];
-}
+// Words of a row at a 2-byte aligned shared address.  Where they start inside an aligned word is worked out once
+// for all of them (anew for every few words: IQ2_XXS 5120 -> 17408 twice, 4 columns, 36.4 us, so 34.1).
+struct RowA2 {
+    uint32_t base, sh;
+    __device__ __forceinline__ explicit RowA2(uint32_t a) : base(a & ~3u), sh((a & 2u) * 8u) {}
+    // 4 * NW bytes `off` (a multiple of four) behind the start
+    template <int NW> __device__ __forceinline__ void get(uint32_t off, uint32_t (&out)[NW]) const {
+        uint32_t w[NW + 1];
+#pragma unroll
+        for (int i = 0; i <= NW; i++) w[i] = lds32(base + off + 4 * i);
+#pragma unroll
+        for (int i = 0; i < NW; i++) out[i] = __funnelshift_r(w[i], w[i + 1], sh);
+    }
+    __device__ __forceinline__ uint32_t word(uint32_t off) const {
+        uint32_t v[1];
+        get<1>(off, v);
+        return v[0];
+    }
+};
 
 // One unit of sixteen output rows.  ua, ub: shared addresses of the unit in rows g and g + 8.  left:
 // blocks of 32 weights the row still has from this unit on (R only; those past the end hold the next
@@ -248,9 +261,10 @@ __device__ __forceinline__ void unit_wide(uint32_t ua, uint32_t ub, uint32_t c, 
         // {u8 ql[128]; u8 qh[64]; i8 scales[16]; f16 d} (LLM/Quantize/KQuants.swift:160-177): granule r of half n
         // has its low four bits in ql (byte 64n + 32(r & 1) + l, low nibble for r < 2), two more in qh, and a
         // scale per 16.  The codes go in unsigned; 32 x the sum of x leaves through the offsets' MMA.
+        const RowA2 A(ua), B(ub), Ac(ua + 4 * c), Bc(ub + 4 * c);
         uint32_t sa[4], sb[4];
-        lds_a2<4>(ua + 192, sa);
-        lds_a2<4>(ub + 192, sb);
+        A.get<4>(192, sa);
+        B.get<4>(192, sb);
         auto sbyte = [](uint32_t v, int i) { return (int)prmt(v, 0u, 0x8880u + 0x1111u * i); };
         int te[NS][4];
 #pragma unroll
@@ -258,13 +272,13 @@ __device__ __forceinline__ void unit_wide(uint32_t ua, uint32_t ub, uint32_t c, 
             uint32_t qa[4], qb[4], ha[2], hb[2];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                qa[i] = lds_word_a2(ua + 64 * n + 16 * i + 4 * c);
-                qb[i] = lds_word_a2(ub + 64 * n + 16 * i + 4 * c);
+                qa[i] = Ac.word(64 * n + 16 * i);
+                qb[i] = Bc.word(64 * n + 16 * i);
             }
 #pragma unroll
             for (int i = 0; i < 2; i++) {
-                ha[i] = lds_word_a2(ua + 128 + 32 * n + 16 * i + 4 * c);
-                hb[i] = lds_word_a2(ub + 128 + 32 * n + 16 * i + 4 * c);
+                ha[i] = Ac.word(128 + 32 * n + 16 * i);
+                hb[i] = Bc.word(128 + 32 * n + 16 * i);
             }
 #pragma unroll
             for (int r = 0; r < 4; r++) {
@@ -287,7 +301,7 @@ __device__ __forceinline__ void unit_wide(uint32_t ua, uint32_t ub, uint32_t c, 
             }
         }
         int mi[NV][2];
-        X.template offsets<true>(mi, lds_word_a2(ua + 192 + 4 * c), lds_word_a2(ub + 192 + 4 * c));
+        X.template offsets<true>(mi, Ac.word(192), Bc.word(192));
         float v[NV][2];
         wide_join<MODE, false>(te, v);
         const float da = f16bits(lds16(ua + 208)), db = f16bits(lds16(ub + 208));
@@ -312,8 +326,20 @@ __device__ __forceinline__ void unit_wide(uint32_t ua, uint32_t ub, uint32_t c, 
                 d[s][1] = d[s][3] = l;
             }
             uint32_t wa[8], wb[8];
-            lds_a2<8>(ua + 34 * blk + 2, wa);
-            lds_a2<8>(ub + 34 * blk + 2, wb);
+            if constexpr (RAG) {
+                lds_a2<8>(ua + 34 * blk + 2, wa);
+                lds_a2<8>(ub + 34 * blk + 2, wb);
+            } else {  // units start on 4-byte boundaries
+                const uint32_t at = 34 * blk + 2 - (blk ? 0 : 2);
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    uint32_t w[9];
+#pragma unroll
+                    for (int i = 0; i < (blk ? 8 : 9); i++) w[i] = lds32((r ? ub : ua) + at + 4 * i);
+#pragma unroll
+                    for (int i = 0; i < 8; i++) (r ? wb : wa)[i] = blk ? w[i] : __funnelshift_r(w[i], w[i + 1], 16);
+                }
+            }
 #pragma unroll
             for (int b = 0; b < 4; b++) {  // 8 bytes = 32 codes; this thread takes code c of every byte
                 constexpr uint32_t m = 0x03030303u;
@@ -334,17 +360,22 @@ __device__ __forceinline__ void unit_wide(uint32_t ua, uint32_t ub, uint32_t c, 
         // {f16 d; 8 x (u32: four codebook indices, u32: four 7-bit sign indices + 4-bit scale)}
         // (LLM/Quantize/IQ2XXS.swift:34-53): entry c of every sub-block is this thread's eight weights.
         // Scale (0.5 + s) / 4 = (2s + 1) / 8 multiplies the integer sums.
+        const RowA2 A(ua + 2), B(ub + 2);
         int te[NS][4];
+        uint32_t na = lds32(A.base), nb = lds32(B.base);  // the word in which a sub-block starts
 #pragma unroll
         for (int b = 0; b < 8; b++) {
-            uint32_t wa[2], wb[2];
-            lds_a2<2>(ua + 2 + 8 * b, wa);
-            lds_a2<2>(ub + 2 + 8 * b, wb);
+            const uint32_t a1 = lds32(A.base + 8 * b + 4), a2 = lds32(A.base + 8 * b + 8);
+            const uint32_t b1 = lds32(B.base + 8 * b + 4), b2 = lds32(B.base + 8 * b + 8);
+            const uint32_t wa[2] = {__funnelshift_r(na, a1, A.sh), __funnelshift_r(a1, a2, A.sh)};
+            const uint32_t wb[2] = {__funnelshift_r(nb, b1, B.sh), __funnelshift_r(b1, b2, B.sh)};
+            na = a2;
+            nb = b2;
             const uint2 va = tab.bytes(prmt(wa[0], 0u, 0x4440u + c), wa[1] >> (7 * c));
             const uint2 vb = tab.bytes(prmt(wb[0], 0u, 0x4440u + c), wb[1] >> (7 * c));
             int d[NS][4];
             X.template mma<true>(d, b, va.x, vb.x, va.y, vb.y);
-            const int ea = (int)(wa[1] >> 28) * 2 + 1, eb = (int)(wb[1] >> 28) * 2 + 1;
+            const int ea = (int)(wa[1] >> 27 | 1u), eb = (int)(wb[1] >> 27 | 1u);  // 2 * (the upper four bits) + 1
 #pragma unroll
             for (int s = 0; s < NS; s++)
 #pragma unroll
@@ -370,14 +401,19 @@ __device__ __forceinline__ void unit_wide(uint32_t ua, uint32_t ub, uint32_t c, 
             for (int r = 0; r < 2; r++) {
                 const uint32_t at = (r ? ub : ua) + BB * b + 2;
                 if constexpr (TY == T_Q8_0) {
-                    if (!RAG && (b & 1)) {
+                    if constexpr (RAG) {
+                        lds_a2<2>(at + 8 * c, w[r]);
+                    } else if (b & 1) {
                         w[r][0] = lds32(at + 8 * c);
                         w[r][1] = lds32(at + 8 * c + 4);
                     } else {
-                        lds_a2<2>(at + 8 * c, w[r]);
+                        const uint32_t w0 = lds32(at + 8 * c - 2), w1 = lds32(at + 8 * c + 2), w2 = lds32(at + 8 * c + 6);
+                        w[r][0] = __funnelshift_r(w0, w1, 16);
+                        w[r][1] = __funnelshift_r(w1, w2, 16);
                     }
                 } else {
-                    const uint32_t q = !RAG && (b & 1) ? lds32(at + 4 * c) : lds_word_a2(at + 4 * c);
+                    const uint32_t q = RAG ? RowA2(at).word(4 * c) : b & 1 ? lds32(at + 4 * c)
+                                           : __funnelshift_r(lds32(at + 4 * c - 2), lds32(at + 4 * c + 2), 16);
                     if constexpr (TY == T_Q4_0) {  // q - 8 as signed bytes, without a carry between them
                         w[r][0] = (((q & ml) | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
                         w[r][1] = (((q >> 4 & ml) | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
