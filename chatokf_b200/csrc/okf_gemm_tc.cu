@@ -466,7 +466,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         // MMAs it feeds, two in flight are not.
         const uint32_t grp = warp / kAWarps;
         const uint32_t t = threadIdx.x % (kAWarps * 32);
-        const uint32_t arow = t >> 1, ahalf = t & 1;  // thread t unpacks 32 weights of row arow
+        // Thread t unpacks 32 weights of row arow.  Eight lanes in a row have eight rows and the same half, so that their 16-byte
+        // stores fall on eight bank groups (two halves of four rows: two lanes to a group for the types with super-blocks, 128
+        // cycles of a k-block's 1500 at the shared-memory port, which is what bounds items of 512 tokens).
+        const uint32_t arow = (t >> 4) * 8 + (t & 7), ahalf = t >> 3 & 1;
         uint32_t it0 = 0;  // stage counter at the start of the work item
         Work wk;
         // this thread's four 16-byte chunks -> stage s
