@@ -1,26 +1,27 @@
 // Prefill matmul on the 5th-generation tensor cores: out[n][m] = sum_k X[n][k] W[m][k]
-// for N >= 9 tokens.  Replaces the reference's gemm_mm_impl tile
+// for N >= 9 tokens; the kernel for more than 256 tokens (and for fp32 activations that nobody could convert), the
+// plans for it and for the one of okf_gemm_ts.cu, and the reduction of both.  Replaces the reference's gemm_mm_impl tile
 // (LLM/metal/Kernels.metal:226-294), which stages fp16 copies of a 64 x 32
 // weight tile and a 32 x 32 activation tile for simdgroup matrices.
 //
-// Shape of the computation.  One work item is a 128-row slab of W against one
-// block of 256 tokens or two such blocks at once, so that every unpacked weight
-// tile feeds two accumulators.  Per k-block of 64:
+// Shape of the computation.  One work item is a 128-row slab of W against two
+// blocks of 256 tokens at once, so that every unpacked weight
+// tile feeds two accumulators (fp32 activations: one block).  Per k-block of 64:
 //   - the activation tile(s), 256 tokens x 64 k each, come by TMA through a tensor
 //     map of X, already in the 128-byte-swizzled K-major layout the tensor core
 //     reads (fp32 activations are converted to bf16 once per call before; where there is no memory for
 //     that, eight warps convert them tile by tile and the other eight unpack alone);
 //   - two groups of eight warps, taking the k-blocks in turn, unpack 128 rows x 64
 //     weights to 16-bit floats into the same layout; weight bytes are fetched one
-//     or two turns ahead.  (Bringing Q4_K slabs in by TMA as stored, 128 rows x one
-//     144-byte block per copy into a ring of their own, was tried and was slower.)
+//     or two turns ahead;
 //   - one warp, converged, issues four tcgen05.mma (M = 128, N = 256, K = 16) per token block
 //     that accumulate in fp32 in tensor memory: lane = weight row, column = token;
 //   - tcgen05.commit hands the stage back to the producers when the MMAs that
 //     read it are done.
-// The two 256-column accumulators of tensor memory either serve the two token
-// blocks of one item or alternate between items, so an epilogue (tcgen05.ld,
-// convert, coalesced stores along m) overlaps the next main loop.  Operands are
+// The two 256-column accumulators of tensor memory serve the two token
+// blocks of an item (fp32 activations: alternate between items).  What bounds it: power in long runs, else the tensor core's
+// issue.  (Tried: pairs of CTAs with cta_group::2 on 256 rows x 512 tokens, half the activations' traffic: Q4_K 5120 -> 17408, 512
+// tokens, 76.7 us against 69.1, 4096 tokens 599 against 565; 71 and 551 with no unpacking at all.)  Operands are
 // fp16 when the activations are fp16, bf16 otherwise (fp32 activations are
 // rounded to bf16); weights are decoded in fp32, exactly but for the mins of Q4_K and Q5_K (below), and
 // rounded once.
@@ -37,16 +38,15 @@
 
 namespace okf {
 
-// How a matmul is laid over the SMs.  A work item is a 128-row slab against one or two 256-token blocks
-// over all of K.  Full waves of items run whole, one item per CTA and wave.  What is left after them, or a
-// matmul of less than a wave, either runs whole too, on part of the SMs, or is dealt out: its k-blocks
-// laid end to end are cut into one run per CTA, pieces of items leave as fp32 partial tiles, and a
-// second kernel sums them.  The plan with the smallest estimated time wins.  The estimate, measured on
-// B200: a CTA spends 0.93 us per k-block on an item of two token blocks and 0.45 - 0.55 us on one of one
-// block (Q8_0 and Q6_K 1.15 and 0.8: what they took when their rows were read in 4-byte words; in 8-byte words 0.5 and 0.65 at
-// up to 64 tokens, which the estimate does not know yet); an item of two blocks, which
-// uses all of tensor memory, exposes 3 us of epilogue; dealing costs 4 us of launch and hand-over, and
-// partial tiles move at 8 TB/s, mostly through L2.  (4096 tokens 17408 -> 5120: 320 items of two blocks
+// How a matmul is laid over the SMs.  A work item is a 128-row slab against some tokens over all of K.  Full waves of items
+// run whole, one item per CTA and wave.  What is left after them, or a matmul of less than a wave, either runs whole too, on
+// part of the SMs, or is dealt out: its k (k-blocks here, units of 256 in okf_gemm_ts.cu) laid end to end is cut into one run per
+// CTA, pieces of items leave as fp32 partial tiles, and a second kernel sums them.  The plan with the smallest estimated time wins.
+// The estimate, measured on B200: 0.86 us per k-block on an item of 512 tokens (Q8_0 and Q6_K 1.1), which exposes 3 us of
+// epilogue, and what ts_kblock says on one of fewer.  Dealing is counted as 2.5 us and partial tiles at 8 TB/s, mostly through L2.  (A
+// second kernel costs a chain of calls 5 us: Q5_K 9728 -> 2560, 77 tokens, 18.1 us, 12.2 of them the matmul alone.  With 5 us counted
+// some calls of half a wave would run whole, Q4_0 2560 -> 9728, 77 tokens, 13.2 us instead of 15.4; they stay
+// dealt, as callers that look at the launches of such calls know them.  4096 tokens 17408 -> 5120: 320 items of two blocks
 // are 2.16 waves; three whole waves took 760 us, two and 24 dealt items 590.)
 struct GemmPlan {
     uint32_t tok;    // tokens per item of the kernel with weights in tensor memory, 0: the other one
@@ -60,8 +60,7 @@ namespace tc {
 constexpr uint32_t kBN = 256;           // tokens per accumulator (UMMA N)
 constexpr uint32_t kABytes = kBM * kBK * 2;  // 16 KB
 constexpr uint32_t kBBytes = kBN * kBK * 2;  // 32 KB per 256 tokens
-// Two rings.  With one token block per item: as many stages of A (16 KB) and of B (up to 32 KB, by the tokens there
-// are) as the room of four full ones holds, at most kMaxRing.  With
+// Two rings.  With one token block per item (fp32 activations) four stages of A (16 KB) and of B (32 KB).  With
 // two blocks a B stage is 64 KB: three of them and two of A, so that a B tile has two MMA
 // periods to arrive while the next A tile only has to be stored (IQ2_XXS, which also keeps its
 // codebook in shared memory, stays with two B stages).
@@ -100,7 +99,7 @@ struct Args {
 // throughput measured) when Args grows.
 struct Outs {
     uint32_t a_stages, b_stages, b_stage;  // stages of the rings, bytes of a B tile
-    uint32_t box;  // tokens of a B tile as the tensor map copies it: 256, or fewer when there are fewer
+    uint32_t box;  // tokens of a B tile as the tensor map copies it
     uint32_t nout, out_ld, out_row0;
     void *outs[8];
     uint32_t *epoch;      // the local count the exchange is complete at goes up by epoch_inc
@@ -468,7 +467,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
         const uint32_t t = threadIdx.x % (kAWarps * 32);
         // Thread t unpacks 32 weights of row arow.  Eight lanes in a row have eight rows and the same half, so that their 16-byte
         // stores fall on eight bank groups (two halves of four rows: two lanes to a group for the types with super-blocks, 128
-        // cycles of a k-block's 1500 at the shared-memory port, which is what bounds items of 512 tokens).
+        // cycles of a k-block's 1500 at the shared-memory port).
         const uint32_t arow = (t >> 4) * 8 + (t & 7), ahalf = t >> 3 & 1;
         uint32_t it0 = 0;  // stage counter at the start of the work item
         Work wk;
@@ -808,17 +807,10 @@ static cudaError_t launch_n(const Args &a, const Outs &go, cudaStream_t s, int s
     alignas(64) CUtensorMap xmap;
     memset(&xmap, 0, sizeof(xmap));
     Outs g = go;
-    // The B ring holds what is on its way from L2, so its depth sets the pace where a k-block is little work:
-    // tiles as large as the tokens present, as many as fit.  (Four stages whatever N: 0.65 us per k-block.)
-    g.box = a.n < kBN ? (a.n + 15) & ~15u : kBN;
-    g.b_stage = XDT == DT_F32 ? kBBytes : NACC * g.box * kBK * 2;
-    if (NACC == 2) {
-        g.a_stages = Rings<TY, NACC>::a_stages;
-        g.b_stages = Rings<TY, NACC>::b_stages;
-    } else {
-        const uint32_t both = (Rings<TY, NACC>::a_bytes + Rings<TY, NACC>::b_bytes) / (kABytes + g.b_stage);
-        g.a_stages = g.b_stages = both < kMaxRing ? both : kMaxRing;
-    }
+    g.box = kBN;
+    g.b_stage = NACC * kBBytes;
+    g.a_stages = Rings<TY, NACC>::a_stages;
+    g.b_stages = Rings<TY, NACC>::b_stages;
     if constexpr (XDT != DT_F32) {
         cudaError_t me = encode_x_map(&xmap, a.x, a.k, a.n, g.box);
         if (me != cudaSuccess) return me;

@@ -412,7 +412,7 @@ __device__ __forceinline__ void unit_wide(uint32_t ua, uint32_t ub, uint32_t c, 
                         w[r][1] = __funnelshift_r(w1, w2, 16);
                     }
                 } else {
-                    const uint32_t q = RAG ? RowA2(at).word(4 * c) : b & 1 ? lds32(at + 4 * c)
+                    const uint32_t q = RAG ? RowA2(at + 4 * c).word(0) : b & 1 ? lds32(at + 4 * c)
                                            : __funnelshift_r(lds32(at + 4 * c - 2), lds32(at + 4 * c + 2), 16);
                     if constexpr (TY == T_Q4_0) {  // q - 8 as signed bytes, without a carry between them
                         w[r][0] = (((q & ml) | 0x80808080u) - 0x08080808u) ^ 0x80808080u;
