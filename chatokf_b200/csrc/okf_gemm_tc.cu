@@ -42,7 +42,7 @@ namespace okf {
 // run whole, one item per CTA and wave.  What is left after them, or a matmul of less than a wave, either runs whole too, on
 // part of the SMs, or is dealt out: its k (k-blocks here, units of 256 in okf_gemm_ts.cu) laid end to end is cut into one run per
 // CTA, pieces of items leave as fp32 partial tiles, and a second kernel sums them.  The plan with the smallest estimated time wins.
-// The estimate, measured on B200: 0.86 us per k-block on an item of 512 tokens (Q8_0 and Q6_K 1.1), which exposes 3 us of
+// The estimate, measured on B200: 0.86 us per k-block on an item of 512 tokens (Q8_0 0.92, Q6_K 1.1), which exposes 3 us of
 // epilogue, and what ts_kblock says on one of fewer.  Dealing is counted as 2.5 us and partial tiles at 8 TB/s, mostly through L2.  (A
 // second kernel costs a chain of calls 5 us: Q5_K 9728 -> 2560, 77 tokens, 18.1 us, 12.2 of them the matmul alone.  With 5 us counted
 // some calls of half a wave would run whole, Q4_0 2560 -> 9728, 77 tokens, 13.2 us instead of 15.4; they stay
@@ -933,7 +933,7 @@ static GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt
     }
     if (n > tc::kBN) {
         plan.nacc = 2;
-        lay_out(plan, slabs, kblocks, n, 2 * tc::kBN, ty == T_Q8_0 || ty == T_Q6_K ? 1.1e-6 : 0.86e-6, 3e-6, 4, all, max_floats, best, best_t);
+        lay_out(plan, slabs, kblocks, n, 2 * tc::kBN, ty == T_Q6_K ? 1.1e-6 : ty == T_Q8_0 ? 0.92e-6 : 0.86e-6, 3e-6, 4, all, max_floats, best, best_t);
         plan.nacc = 0;
     }
     const uint32_t least = (n + tc::kBN - 1) / tc::kBN;

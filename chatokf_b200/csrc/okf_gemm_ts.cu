@@ -13,7 +13,7 @@
 //     tensor memory holds the accumulator(s) in columns 0 .. 255 and a unit of weights per set in 256 .. 511;
 //   - activation tiles arrive by TMA, one warp issues the MMAs, a unit a turn, four run the epilogue, as in okf_gemm_tc.cu.
 // 5120 -> 17408, 64 tokens, us, there and here: Q8_0 47.6 -> 27.0, Q4_0 37.9 -> 22.5, Q6_K 59.9 -> 30.8, Q4_K 37.6 -> 23.0,
-// IQ2_XXS 38.1 -> 27.7, IQ4_NL 40.8 -> 29.0; Q5_K 2560 -> 9728, 77 tokens, 19.3 -> 15.0.  What bounds it: up to some 100 tokens instruction issue
+// IQ2_XXS 38.1 -> 25.0, IQ4_NL 40.8 -> 27.9; Q5_K 2560 -> 9728, 77 tokens, 19.3 -> 15.0.  What bounds it: up to some 100 tokens instruction issue
 // (about 260 instructions for a warp's 32 x 64 weights: widening, multiply-add, rounding), above that the shared-memory port, which
 // takes the activations in and hands them to the tensor core.
 // Tried on the way: rows copied by cp.async (two warps: 1900 cycles a unit for address arithmetic and issue, Q4_K 30.8 us against 25.9);
@@ -156,6 +156,12 @@ __device__ __forceinline__ void halves4(uint32_t even, uint32_t odd, const Affin
     const float2 e = __half22float2(*reinterpret_cast<const __half2 *>(&even)), f = __half22float2(*reinterpret_cast<const __half2 *>(&odd));
     o[0] = scale2<F16>(e.x, f.x, t);
     o[1] = scale2<F16>(e.y, f.y, t);
+}
+// two neighbours
+template <bool F16>
+__device__ __forceinline__ uint32_t pair(uint32_t w, const Affine &t) {
+    const float2 e = __half22float2(*reinterpret_cast<const __half2 *>(&w));
+    return scale2<F16>(e.x, e.y, t);
 }
 // the four bytes of a word
 template <bool F16>
@@ -302,8 +308,10 @@ template <int TY, bool SK> struct TsRaw40 {
                     const uint32_t sel = q & 0x77777777u, pick = (q >> 1 & 0x44444444u) | 0x32103210u;
                     const uint32_t t0 = prmt(prmt(T0, T1, sel), prmt(T2, T3, sel), pick);
                     const uint32_t t1 = prmt(prmt(T0, T1, sel >> 16), prmt(T2, T3, sel >> 16), pick >> 16);
-                    codes4<F16>(prmt(t0, t1, 0x6420u), t, o + 16 * b + 2 * i);
-                    codes4<F16>(prmt(t0, t1, 0x7531u), t, o + 16 * b + 8 + 2 * i);
+                    o[16 * b + 2 * i] = pair<F16>(t0 & 0x00FF00FFu, t);
+                    o[16 * b + 2 * i + 1] = pair<F16>(t1 & 0x00FF00FFu, t);
+                    o[16 * b + 8 + 2 * i] = pair<F16>(prmt(t0, 0u, 0x4341u), t);
+                    o[16 * b + 8 + 2 * i + 1] = pair<F16>(prmt(t1, 0u, 0x4341u), t);
                 }
             }
         }
@@ -398,10 +406,12 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
     }
     if constexpr (TY == T_IQ2_XXS) {
         uint32_t *tab = reinterpret_cast<uint32_t *>(smem + p.tab_off);
-        for (uint32_t i = threadIdx.x; i < 384u * kTsTabCopies; i += kTsThreads) {
-            const uint32_t e = i / kTsTabCopies;  // (the same for a warp)
-            tab[i] = e < 256 ? iq2_code_selectors(g_iq2xxs_grid[e]) : iq2_sign_selectors(e - 256);
-        }
+        // Sixteen entries a warp, worked out once and stored by all lanes side by side.  (Worked out anew for every copy, a
+        // launch started 3 us later: 6144 -> 1500, 40 tokens, 17.4 us, so 13.9.)
+        static_assert(kTsThreads / 32 * 16 == 384 && kTsTabCopies == 32, "entries to warps, copies to lanes");
+        const uint32_t e = warp * 16 + (lane & 15), v = e < 256 ? iq2_code_selectors(g_iq2xxs_grid[e]) : iq2_sign_selectors(e - 256);
+#pragma unroll
+        for (uint32_t i = 0; i < 16; i++) tab[(warp * 16 + i) * kTsTabCopies + lane] = __shfl_sync(0xffffffffu, v, i);
     }
     if (warp == kTsMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
