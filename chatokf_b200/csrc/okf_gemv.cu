@@ -1370,6 +1370,9 @@ static uint32_t gemv_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, b
 // evenly over the chip, whole ones leave most CTAs one and a few of them two (Q4_K 17408 -> 5120 21.3 ->
 // 16.9 us, Q8_0 32.7 -> 24.6, Q6_K 39.6 -> 28.5, Q2_0 12288 -> 5120 10.7 -> 9.4; Q8_0 5120 -> 5120, 20 units of 272
 // bytes, 8.8 -> 9.5, Q4_K 9216 -> 5120, 36 of 144, 10.3 -> 10.8; the line lies somewhere between these points).
+// Several columns of long rows (4 KB on) with up to half as many tiles again as SMs: the same, one CTA to an SM would take two
+// tiles on some of them (2 columns, the only ones whose x then fits a CTA alone: Q4_K 9728 -> 2560 13.0 -> 9.7 us, 12288 -> 3072 16.5 -> 11.7, Q8_0 26.1 ->
+// 18.1, Q6_K 23.7 -> 15.6, Q5_K 8192 -> 3500 13.3 -> 9.6, Q2_0 17408 -> 2560 20.8 -> 13.3; IQ2_XXS 17408 -> 2560 24.0 -> 18.2).
 // Several columns: x resident is not enough, copies have to be on their way as well.  A panel that leaves the ring
 // of a CTA alone less than kRingMin, in segments of about 1 KB, goes to two CTAs (Q8_0 17408 -> 8192, 2
 // columns, 88.4 -> 42.2 us, Q5_K 9728 -> 5120, 3 columns, 26.1 -> 19.2; with 36 KB the latter stays).  It is asked of a
@@ -1380,7 +1383,8 @@ constexpr uint32_t kRingMin = 44 * 1024;
 static bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t tiles, int sms, bool gather, GemvArgs &a,
                       GemvLayout &L, uint32_t &ctas) {
     const uint32_t all = gemv_ctas(ty, row_bytes, tiles, sms, mode == M_SEP), n2 = 2u * (uint32_t)sms;
-    const bool halves = mode == M_SEP && tiles > n2 && tiles <= n2 + n2 / 2 && (row_bytes >= 6144 || nunit >= 40) && !gather;
+    const bool few = mode != M_SEP && tiles > (uint32_t)sms && tiles <= (uint32_t)sms + (uint32_t)sms / 2 && row_bytes >= 4096;
+    const bool halves = (few || (mode == M_SEP && tiles > n2 && tiles <= n2 + n2 / 2 && (row_bytes >= 6144 || nunit >= 40))) && !gather;
     for (uint32_t cs = halves ? 2 : 1; cs <= 8 && !(gather && cs > 1) && cs * 4 <= nunit; cs *= 2) {
         const uint32_t limit = (two_ctas(ty, row_bytes, tiles, sms, mode == M_SEP) ? 2 : 1) * (uint32_t)sms / cs;
         const uint32_t clusters = cs == 1 ? all : tiles < limit ? tiles : limit;
