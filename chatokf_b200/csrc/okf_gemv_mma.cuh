@@ -103,6 +103,7 @@ struct GemvSeg {
 };
 __device__ __forceinline__ GemvSeg gemv_segment(const GemvArgs &p, uint32_t tile) {
     GemvSeg s = {p.w[0], p.out[0], p.m[0], 0u, p.tile_end[0], 0u};
+    if (tile < p.tile_end[0]) return s;
 #pragma unroll
     for (int i = 1; i < kGemvSegs; i++)
         if (tile >= p.tile_end[i - 1]) s = {p.w[i], p.out[i], p.m[i], p.tile_end[i - 1], p.tile_end[i], (uint32_t)i};

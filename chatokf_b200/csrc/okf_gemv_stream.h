@@ -1,0 +1,193 @@
+// The plan of a streaming matvec (okf_gemv_stream.cu): how its units are dealt to CTAs and warps, what lies where in shared memory,
+// and which of the possible splits a launch takes.  Host code, but for the arithmetic by which a CTA finds its share.
+#pragma once
+#include "okf_gemv_unit.cuh"
+
+namespace okf {
+
+// A warp's ring: `depth` stages of 16 row segments, `cb` units each.  Segments are copied from the 32-byte boundary below them
+// (a sector of L2 is fetched once); they lie 16 bytes into their rows of the stage, and up to 14 more where they start between 16-byte
+// boundaries.
+template <int TY, int MODE> struct StreamGeom {
+    static constexpr uint32_t ub = UnitGeom<TY>::bytes;
+    static constexpr bool rag = WideMode<MODE>::rag, aligned = ub % 16 == 0 && !rag;
+    // Units of a stage: as many as make a segment of some 100 to 300 bytes (Q2_0 2048 -> 6144 twice, one column, two and four units: 4.5
+    // and 4.2 us); in several columns' kernels, whose x takes the room, fewer.
+    static constexpr uint32_t cb = ub < 68 ? (MODE == M_SEP ? 2 : 1) : ub < 100 ? (MODE == M_SEP ? 4 : 2) : 1;
+    static constexpr uint32_t bytes = 16 + (aligned ? cb * ub : (cb * ub + 14 + 15) / 16 * 16);
+    // Rows g and g + 1 of a tile on different banks: an odd number of 16 bytes apart for 16- and 4-byte loads; where a quad's
+    // 8-byte loads lie side by side, 32 bytes modulo 64.
+    static constexpr uint32_t pitch = aligned && MODE != M_SEP ? bytes + (96 - bytes % 64) % 64 : bytes % 32 == 16 ? bytes : bytes + 16;
+    static constexpr uint32_t stage = 16 * pitch;
+};
+
+struct StreamLayout {
+    uint32_t nc, es;      // activation columns, bytes between byte columns of the x panel
+    uint32_t clog;        // log2 of the CTAs of a cluster, each with its share of K of the cluster's tiles
+    uint32_t depth;       // stages of a warp's ring: 2 to 4
+    uint32_t xs_off, info_off, slot_off, part_off, tab_off;  // byte offsets in dynamic shared memory
+    uint32_t tab_copies;  // IQ2_XXS: copies of every entry of the look-up tables, side by side
+    uint32_t tiles_each, tiles_more;     // tiles of a cluster; the first tiles_more clusters have one more
+    uint32_t unit_inv, unit_inv_more;    // v / units = v * inv >> 31, for CTAs with nunit >> clog units of a row and with one more
+    uint32_t nc_inv;                     // v / nc = v * nc_inv >> 16, v < 8192
+};
+
+// A CTA's units of its tiles laid end to end; warp w has [border(w), border(w + 1)).
+struct StreamSplit {
+    uint32_t nun, all, inv;  // units of a tile, of all tiles
+    __host__ __device__ __forceinline__ StreamSplit(uint32_t tiles, uint32_t units, uint32_t inv_) : nun(units), all(tiles * units), inv(inv_) {}
+    template <uint32_t NW> __host__ __device__ __forceinline__ uint32_t border(uint32_t w) const { return all * w / NW; }
+    __host__ __device__ __forceinline__ uint32_t tile(uint32_t v) const { return (uint32_t)((uint64_t)v * inv >> 31); }
+};
+inline uint32_t stream_inv(uint32_t units) { return (0x80000000u + units - 1) / units; }
+// Where tile(), border() and nc_inv are exact.
+inline bool stream_exact(uint32_t tiles, uint32_t units, uint32_t n) {
+    return (uint64_t)tiles * units * units < 0x80000000ull && (uint64_t)tiles * units * 16 < 0x100000000ull && (uint64_t)tiles * n < 8192;
+}
+
+// ---- which split a launch takes ----------------------------------------------------------
+// What the device has room for: clusters of 1, 2, 4 and 8 CTAs at one CTA to an SM and at two.  (GPCs do not have a multiple of eight
+// SMs, so these are fewer than SMs / size: a grid of 37 clusters of four on 148 SMs takes two waves, twice the time.)
+struct StreamRoom {
+    uint32_t one[4], two[4];
+};
+struct StreamPlan {
+    bool ok;
+    uint32_t warps, ctas, smem;
+    float us;  // estimated
+    StreamLayout L;
+};
+// (two of 112 KB leave 2 KB of an SM: enough for the small kernels between matvecs, which with 1 KB less take 0.8 us longer each)
+constexpr uint32_t stream_budget(uint32_t warps) { return warps == 8 ? 112 * 1024 : 226 * 1024; }
+
+template <int TY, int MODE>
+inline bool stream_layout(uint32_t nunit, uint32_t n, uint32_t clog, uint32_t clusters, uint32_t tiles, uint32_t warps, StreamPlan &p) {
+    using S = StreamGeom<TY, MODE>;
+    constexpr bool sep = MODE == M_SEP;
+    StreamLayout &L = p.L;
+    const uint32_t tiles_per = (tiles + clusters - 1) / clusters, units = (nunit + (1u << clog) - 1) >> clog;
+    const uint32_t nb = mode_bytes(MODE), ecols = sep ? 2 : n * nb;
+    if (!stream_exact(tiles_per, units, n)) return false;
+    L.nc = n;
+    L.clog = clog;
+    L.es = sep ? sep_col_stride(units) : xq_col_stride(units);
+    // the deepest ring that leaves room for x and, IQ2_XXS, for tables without bank conflicts; else half the tables
+    for (L.tab_copies = TY == T_IQ2_XXS ? 32 : 0;; L.tab_copies = 16) {
+        for (L.depth = 4; L.depth >= 2; L.depth--) {
+            L.xs_off = (warps * L.depth * S::stage + 127) & ~127u;
+            L.info_off = (L.xs_off + ecols * L.es + 15) & ~15u;
+            L.slot_off = (L.info_off + (sep ? 256u : units * n * wide_info_words(TY, nb) * 4) + 127) & ~127u;  // (one column: 256 bytes of zeros before it)
+            L.part_off = L.slot_off + warps * 2 * n * 64;
+            L.tab_off = L.part_off + (clog ? tiles_per * n * 64 : 0);
+            p.smem = L.tab_off + 384 * 4 * L.tab_copies;
+            if (p.smem <= stream_budget(warps)) break;
+        }
+        if (L.depth >= 2) break;
+        if (L.tab_copies != 32) return false;
+    }
+    p.warps = warps;
+    p.ctas = clusters << clog;
+    L.tiles_each = tiles / clusters;
+    L.tiles_more = tiles % clusters;
+    L.unit_inv = stream_inv(nunit >> clog);
+    L.unit_inv_more = stream_inv((nunit >> clog) + 1);
+    L.nc_inv = 65536 / n + 1;
+    return true;
+}
+
+// The time of a launch in a chain, us: what it takes whatever its size, a warp's staging of x (column, unit pairs) and a warp's units,
+// both at another rate where two CTAs share an SM, and never less than the weights take at what copies in pieces of 16 bytes reach (4.9
+// TB/s).  The constants are a fit to 21 000 timings: 1080 shapes (every type, 1 to 8 columns, rows of 512 to 18432 weights, 300 to
+// 150 000 rows), each in a chain of matvecs and in one with an elementwise kernel before every matvec, as an engine has both.  The choice made with
+// them is 0.9 % slower than the best one at one column (geometric mean over the shapes; at most 16 %), 0.7 to 1.5 % at several.  One CTA to
+// an SM where there is work for two is the faster one in the first kind of chain only (Q4_K 2560 -> 2 x 9728, one column, 8.2 and 8.4
+// us, behind an elementwise kernel 13.5 and 10.4): it leaves room for the next matvec's first copies, but the CTAs of a grid that comes while SMs
+// fall free one by one are not spread evenly, and two end up on one SM.
+inline int stream_kind(int mode) { return mode == M_SEP ? 0 : mode == M_W1 ? 1 : mode == M_W2 ? 2 : 3; }
+struct StreamUnit {
+    float stream[4];  // one column, up to four, up to eight, rows that end inside a unit
+    float ring[4];    // the same of okf_gemv.cu's kernel
+};
+inline StreamUnit stream_unit_us(int ty) {
+    switch (ty) {
+    case T_Q4_K: return {{.71f, .75f, 1.07f, 0.f}, {.44f, .58f, 0.f, 0.f}};
+    case T_Q8_0: return {{1.23f, 1.50f, 1.73f, 1.74f}, {.82f, 1.00f, 0.f, .64f}};
+    case T_Q6_K: return {{1.40f, 1.61f, 1.94f, 0.f}, {.87f, .80f, 0.f, 0.f}};
+    case T_Q5_K: return {{.90f, 1.01f, 1.30f, 0.f}, {.72f, .94f, 0.f, 0.f}};
+    case T_Q4_0: return {{.70f, 1.03f, 1.27f, 1.38f}, {.34f, .61f, 0.f, .80f}};
+    case T_IQ4_NL: return {{1.16f, 1.29f, 1.45f, 1.73f}, {.92f, .70f, 0.f, 1.22f}};
+    case T_Q2_0: return {{.51f, .71f, .94f, 1.07f}, {.28f, .33f, 0.f, .49f}};
+    default: return {{.95f, 1.20f, 1.35f, 0.f}, {.67f, .89f, 0.f, 0.f}};
+    }
+}
+inline float quad_max(float a, float b) { return sqrtf(sqrtf(a * a * a * a + b * b * b * b)); }  // the larger one, rounded off
+inline float stream_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tiles, uint32_t clog, uint32_t clusters, uint32_t warps, uint32_t sms, float floor_us) {
+    const int kind = stream_kind(mode);
+    constexpr float one[4] = {1.3f, 2.65f, 3.05f, 4.2f};   // by cluster size, one CTA to an SM
+    constexpr float two[4][4] = {{2.5f, 3.8f, 7.8f, 8.1f}, {3.2f, 4.5f, 8.5f, 8.9f}, {3.4f, 4.65f, 8.7f, 9.0f}, {1.8f, 3.05f, 7.1f, 7.45f}};
+    constexpr float wide[4] = {5.0f, 6.25f, 4.75f, 4.45f};  // sixteen warps
+    constexpr float stage[4] = {.59f, .62f, .65f, .66f}, stage_two[4] = {1.3f, .66f, .4f, 1.14f}, unit_two[4] = {.71f, .78f, 1.38f, .86f};
+    const bool shared = warps == 16 || (clusters << clog) > sms;
+    const uint32_t units = (nunit + (1u << clog) - 1) >> clog, per = (tiles + clusters - 1) / clusters * units;
+    const float busy = stream_unit_us(ty).stream[kind] * (float)((per + warps - 1) / warps) * (shared ? unit_two[kind] : 1.f) +
+                       stage[kind] * (float)((units * n + warps - 1) / warps) * (shared ? stage_two[kind] : 1.f);
+    return (warps == 16 ? wide[clog] : shared ? two[kind][clog] : one[clog]) + quad_max(busy, floor_us);
+}
+// The same of okf_gemv.cu's kernel, whose CTAs share their tiles' units between eight warps; `ctas` and `clog` as it would take them.
+// It is asked where it may be the better one: at one column, where its bulk copies of whole rows reach 6.1 TB/s (Q4_K 5120 -> 65536 33.6
+// us, 39.2 here), and at up to four where an SM gets four tiles and more, to which x is staged once.  Up to eight columns are
+// better off here (Q4_K 2560 -> 9728 twice, 17.4 -> 12.3 us, 9728 -> 2560 19.7 -> 10.8), but for the shortest rows, where there is little to share
+// (1024 -> 828, IQ4_NL 3.9 and 4.3 us; Q4_K 1024 -> 4096 4.4 and 4.1).
+inline float ring_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tiles, uint32_t ctas, uint32_t clog, uint32_t sms) {
+    const int kind = stream_kind(mode);
+    if (kind == 2) return nunit <= 6 && tiles <= 4 * sms && ty != T_Q4_K && ty != T_Q5_K ? 0.f : 1e30f;
+    if (kind != 0 && tiles < 4 * sms) return 1e30f;
+    constexpr float fixed[4] = {3.26f, 3.12f, 0.f, 5.74f};
+    const uint32_t clusters = ctas >> clog, units = (nunit + (1u << clog) - 1) >> clog;
+    const float busy = (stream_unit_us(ty).ring[kind] * (float)((tiles + clusters - 1) / clusters * units) + .9f * (float)(units * n)) / 8.f * (ctas > sms ? 1.32f : 1.f);
+    const uint32_t ub = ty == T_Q8_0 ? 272 : ty == T_Q6_K ? 210 : ty == T_Q5_K ? 176 : ty == T_Q2_0 ? 68 : ty == T_IQ2_XXS ? 66 : 144;
+    const float us = fixed[kind] + (ctas > sms ? 1.47f : 0.f) + (clog ? 3.07f : 0.f) + quad_max(busy, (float)nunit * (float)tiles * (16.f * (float)ub / 6.1e6f));
+    return tiles < 12 * sms ? us : kind == 3 && n == 1 ? .85f * us : .93f * us;  // (with so many tiles the fit favours the other kernel: ragged Q4_0 2336 -> 63677
+                                                                                 // 27.5 us here, 32.5 there)
+}
+
+template <int TY, int MODE>
+inline StreamPlan stream_search(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room) {
+    StreamPlan best = {};
+    const float floor_us = (float)nunit * (float)tiles * (16.f * UnitGeom<TY>::bytes / 4.9e6f);
+    for (uint32_t clog = 0; clog < 4 && (clog == 0 || nunit >= 2u << clog); clog++) {
+        for (uint32_t v = 0; v < (MODE == M_W2 ? 3 : 2); v++) {
+            const uint32_t warps = v == 2 ? 16 : 8, limit = v == 1 ? room.two[clog] : room.one[clog], clusters = tiles < limit ? tiles : limit;
+            if (clusters == 0 || (v == 1 && tiles <= room.one[clog])) continue;
+            StreamPlan p = {};
+            if (!stream_layout<TY, MODE>(nunit, n, clog, clusters, tiles, warps, p)) continue;
+            p.us = stream_us(TY, MODE, nunit, n, tiles, clog, clusters, warps, room.one[0], floor_us);
+            p.ok = true;
+            if (!best.ok || p.us < best.us) best = p;
+        }
+    }
+    return best;
+}
+
+// The search costs the host as much as a launch and an engine asks for the same few shapes on every token: a thread keeps
+// the plans it found last.
+template <int TY, int MODE>
+inline const StreamPlan &stream_plan(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room, int dev) {
+    struct Entry {
+        uint32_t nunit, n, tiles;
+        int dev;
+        StreamPlan p;
+    };
+    constexpr uint32_t kEntries = 16;
+    static thread_local Entry kept[kEntries];  // (tiles = 0: none yet)
+    Entry &e = kept[((nunit * 31 + n) * 31 + tiles) * 2654435761u >> 28];
+    static_assert(kEntries == 16, "four bits of the hash");
+    if (e.nunit != nunit || e.n != n || e.tiles != tiles || e.dev != dev) e = {nunit, n, tiles, dev, stream_search<TY, MODE>(nunit, n, tiles, room)};
+    return e.p;
+}
+
+// Whether a launch took this kernel; 0: it is not one for it (or does not fit), and nothing was launched.
+struct GemvArgs;
+int launch_gemv_stream(int ty, int mode, const GemvArgs &a, int xdt, cudaStream_t s, int sms, int dev, float other_us, cudaError_t &e);
+
+}  // namespace okf

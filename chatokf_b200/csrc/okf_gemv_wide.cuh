@@ -143,6 +143,24 @@ __device__ __forceinline__ uint32_t iq2_sign_selectors(uint32_t idx7) {
     for (int j = 0; j < 7; j++) s |= (idx7 >> j & 1u) << (4 * j + 2);
     return s;
 }
+// both tables, worked out by the compiler: 256 codes, then 128 signs
+struct Iq2Selectors {
+    uint32_t v[384];
+    constexpr Iq2Selectors() : v{} {
+        constexpr uint64_t grid[256] = {OKF_IQ2XXS_GRID_VALUES};
+        for (uint32_t i = 0; i < 256; i++)
+            for (int j = 0; j < 8; j++) v[i] |= (uint32_t)(grid[i] >> (8 * j + 4) & 3u) << (4 * j);  // 8, 25, 43 -> 0, 1, 2
+        for (uint32_t i = 0; i < 128; i++) {
+            uint32_t odd = 0;
+            for (int j = 0; j < 7; j++) {
+                v[256 + i] |= (i >> j & 1u) << (4 * j + 2);
+                odd ^= i >> j & 1u;
+            }
+            v[256 + i] |= odd << 30;
+        }
+    }
+};
+static __device__ constexpr Iq2Selectors g_iq2_selectors;
 struct Iq2Tab {
     uint32_t code, sign;  // shared addresses of this lane's copy of entry 0
     uint32_t stride;      // bytes between entries
