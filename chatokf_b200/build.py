@@ -6,7 +6,7 @@ The library links the CUDA runtime statically and exports only the C ABI of
 include/okf_cuda.h.  Objects go to chatokf_b200/csrc/build/ (git-ignored); the
 shared library sits beside this file so it travels with the package.  Beside it
 goes _okfcall, the C module through which Python calls the library's hot entry
-points.
+points; it is linked against torch, whose tensors it reads.
 """
 from __future__ import annotations
 
@@ -24,6 +24,7 @@ CSRC = PKG / "csrc"
 OBJ = CSRC / "build"
 LIB = PKG / "libokfcuda.so"
 PYCALL = CSRC / "okf_pycall.c"
+PYTENSOR = CSRC / "okf_pytensor.cpp"
 PYMOD = PKG / ("_okfcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -56,16 +57,30 @@ def _stale(out: Path, src_mtime: float) -> bool:
 
 def needs_build() -> bool:
     return (_stale(LIB, max(p.stat().st_mtime for p in sources()))
-            or _stale(PYMOD, PYCALL.stat().st_mtime))
+            or _stale(PYMOD, max(PYCALL.stat().st_mtime, PYTENSOR.stat().st_mtime)))
 
 
 def build_pycall() -> None:
-    cmd = [shutil.which("gcc") or "cc", "-O2", "-Wall", "-fPIC", "-shared", "-fvisibility=hidden",
-           "-I", sysconfig.get_paths()["include"], str(PYCALL), "-o", str(PYMOD) + ".tmp"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode:
-        sys.stderr.write(r.stdout + r.stderr)
-        raise RuntimeError(f"compiling {PYCALL.name} failed")
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc()).resolve().parent.parent
+    inc = ["-I", sysconfig.get_paths()["include"]]
+    obj, tobj = OBJ / "okf_pycall.o", OBJ / "okf_pytensor.o"
+    tcmd = ["-I", str(root / "include"), "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-I", str(cuda / "include"),
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    flags = ["-O2", "-Wall", "-fPIC", "-fvisibility=hidden"]
+    libs = ["-L" + str(root / "lib"), "-Wl,-rpath," + str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    cxx = shutil.which("g++") or "c++"
+    cmds = [[shutil.which("gcc") or "cc", *flags, *inc, "-c", str(PYCALL), "-o", str(obj)]]
+    if not tobj.exists() or _stale(tobj, max(PYTENSOR.stat().st_mtime, Path(torch.__file__).stat().st_mtime)):
+        cmds.append([cxx, *flags, "-std=c++17", *inc, *tcmd, "-c", str(PYTENSOR), "-o", str(tobj)])
+    cmds.append([cxx, "-shared", str(obj), str(tobj), *libs, "-o", str(PYMOD) + ".tmp"])
+    for cmd in cmds:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode:
+            sys.stderr.write(r.stdout + r.stderr)
+            raise RuntimeError(f"building {PYMOD.name} failed")
     os.replace(str(PYMOD) + ".tmp", PYMOD)
 
 

@@ -4,7 +4,7 @@
  * less time than the kernel before it runs.  Through ctypes, torch.cuda.current_stream() and the
  * properties of GGUFTensor a call cost 9 - 12 us on the host (a 16-bit two-bit trunk's layer,
  * seven calls and two regions, 69 us against 18 us on the GPU); here the arguments are read from
- * the objects in C.  The functions return the okf_status; the callers turn it into an exception.
+ * the objects in C, those of torch's from torch itself (okf_pytensor.cpp).  The functions return the okf_status; the callers turn it into an exception.
  * The library is resolved by address (bind), so this module links against nothing.
  */
 #define PY_SSIZE_T_CLEAN
@@ -34,6 +34,11 @@ static int (*matmul_host_p)(okf_ctx *, int, const okf_weights *, uint64_t, uint3
 static PyObject *dt_f32, *dt_f16, *dt_bf16;         /* torch.float32, ... */
 static PyObject *get_device_p, *raw_stream_p;       /* torch._C._cuda_getDevice, _cuda_getCurrentRawStream */
 static PyObject *s_ctx, *s_addr, *s_stream, *s_cuda_stream, *s_type, *s_dims, *s_offset, *s_dtype, *s_data_ptr;
+
+/* okf_pytensor.cpp */
+int okf_tensor_address(PyObject *o, void **out);
+int okf_tensor_dtype(PyObject *o, int *out);
+int okf_current_stream(void **out);
 
 /* ---- reading the arguments --------------------------------------------------------------- */
 
@@ -71,6 +76,7 @@ static int ctx_of(PyObject *enc, okf_ctx **out) {
     return rc;
 }
 static int data_ptr(PyObject *t, void **out) {
+    if (okf_tensor_address(t, out)) return 0;
     PyObject *v = PyObject_CallMethodNoArgs(t, s_data_ptr);
     if (!v) return -1;
     uint64_t p;
@@ -80,6 +86,7 @@ static int data_ptr(PyObject *t, void **out) {
     return rc;
 }
 static int dtype_of(PyObject *t, int *out) {
+    if (okf_tensor_dtype(t, out)) return 0;
     PyObject *d = PyObject_GetAttr(t, s_dtype);
     if (!d) return -1;
     int rc = 0;
@@ -100,6 +107,9 @@ static int stream_of(PyObject *enc, okf_stream *out) {
     uint64_t v = 0;
     int rc;
     if (s == Py_None) {
+        Py_DECREF(s);
+        if (okf_current_stream(out)) return 0;
+        s = Py_NewRef(Py_None);
         rc = -1;
         PyObject *dev = PyObject_CallNoArgs(get_device_p);
         if (dev) {
