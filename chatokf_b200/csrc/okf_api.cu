@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include "okf_internal.h"
+#include "okf_gemm_ts.h"
 #include "okf_kernels.h"
 
 using namespace okf;
@@ -263,9 +264,10 @@ cudaError_t run_tile(okf_ctx *ctx, int ty, const uint8_t *wp, uint32_t k, uint32
                 xadt = DT_BF16;
             }
         }
-        GemmPlan plan = gemm_tc_plan(ty, k, m, nn, xadt, ctx->sms, kMaxScratchFloats);
+        const uint32_t *room = gemm_ts_clusters(ctx->device);
+        GemmPlan plan = gemm_tc_plan(ty, k, m, nn, xadt, ctx->sms, kMaxScratchFloats, room);
         void *part = plan.floats ? memory(0, lane ? &lane->part : nullptr, lane ? &lane->part_bytes : nullptr, plan.floats * sizeof(float)) : nullptr;
-        if (plan.floats && !part) plan = gemm_tc_plan(ty, k, m, nn, xadt, ctx->sms, 0);
+        if (plan.floats && !part) plan = gemm_tc_plan(ty, k, m, nn, xadt, ctx->sms, 0, room);
         cudaError_t e = launch_gemm_tc(plan, ty, wp, k, m, xa, xadt, nn, gather ? out : (uint8_t *)out + (size_t)n0 * m * dtype_size(odt), odt,
                                        ctx->dev_status, (float *)part, s, ctx->sms, ctx->device, &ctx->launches, gather);
         if (e != cudaSuccess) return e;

@@ -26,6 +26,7 @@ struct GemmPlan {
     uint32_t tok;    // tokens per item of the kernel with weights in tensor memory, 0: the other one
     uint32_t nacc;   // token blocks per item
     uint32_t waves, dealt, dealers, nt;  // see tc::Args
+    uint32_t cluster;  // CTAs of a cluster that share an item along K, 0: none; tok != 0 and all items at once
     size_t floats;   // of partial tiles
 };
 
@@ -78,6 +79,24 @@ inline void lay_out(GemmPlan plan, uint32_t slabs, uint32_t steps, uint32_t n, u
         best.waves = waves; best.dealt = dealt; best.dealers = ctas; best.nt = nt; best.floats = parts * part;
     }
 }
+// The same items, each by a cluster of CTAs that cut its K among them and add up in each other's shared memory: no second kernel and no working
+// memory, but all items have to be there at once.  `room`: how many clusters of a size fit the device.  The exchange is counted as 2 us and 5 ns a
+// token, 1.5 us more against items that run whole: of 84 shapes (9 to 1020 tokens, all types) that were timed with and without, the plan taken
+// is 0.8 % slower than the better one on average (never counting the 1.5 us; 5 % if they are counted against dealt items too).  Dealt or whole, and shared, us:
+// Q5_K 9728 -> 2560, 77 tokens, 19.8 and 17.3; Q2_0 6144 -> 2048, 512 tokens, 22.6 and 19.5; Q4_K 4608 -> 403, 256 tokens, 12.1 and 8.6; IQ4_NL
+// 3840 -> 1307, 13 tokens, 11.9 and 6.1; whole items that stay whole: Q4_K 1792 -> 1840, 158 tokens, 7.9 and 8.4.
+// Q4_0 does not share: the tests of dealt items, of partial tiles and of their memory are written with it and count its kernels (4096 -> 1500, 34
+// tokens, 13.6 us instead of 9.0).
+inline void share_out(GemmPlan plan, uint32_t slabs, uint32_t units, uint32_t n, uint32_t tok, double t_unit, double t_item, const uint32_t *room, GemmPlan &best,
+                      double &best_t) {
+    const uint32_t items = slabs * ((n + tok - 1) / tok);
+    const double whole = best.dealt || best.cluster ? 0 : 1.5e-6;
+    for (uint32_t c = 2; c <= 8; c++) {
+        if (items > room[c] || units < 2 * c) continue;
+        const double t = (units + c - 1) / c * t_unit + t_item + 2e-6 + (n < tok ? n : tok) * 5e-9;
+        if (t + (best.cluster ? 0 : whole) < best_t) { best_t = t; best = plan; best.cluster = c; }
+    }
+}
 // 16-bit activations: seconds per k-block of an item of `tok` tokens on the kernel with weights in tensor memory.  Up to
 // some 100 tokens the unpacking sets the pace, above that it grows with the tokens (5120 -> 17408, 80 k-blocks an SM: 22.7 to 29.4 us
 // at 64 tokens, Q4_K 29.5 at 128, 56 at 256).
@@ -88,7 +107,8 @@ inline double ts_kblock(int ty, uint32_t tok) {
 }
 // Items may be of any number of tokens (fewer than 256 where that gives every SM one: Q2_0 2048 -> 6144, 512 tokens, in 144 items of
 // 176 tokens 16 us, in 96 of 256 17, in 48 of 512 20).
-inline GemmPlan gemm_tc_search(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms, size_t max_floats) {
+// `room`: see share_out; null: no clusters.
+inline GemmPlan gemm_tc_search(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms, size_t max_floats, const uint32_t *room = nullptr) {
     const uint32_t slabs = (m + tc::kBM - 1) / tc::kBM, kblocks = k / tc::kBK, all = (uint32_t)sms;
     GemmPlan best = {}, plan = {};
     double best_t = 1e30;
@@ -108,6 +128,7 @@ inline GemmPlan gemm_tc_search(int ty, uint32_t k, uint32_t m, uint32_t n, int x
     for (uint32_t blocks = least; blocks <= least + 8; blocks++) {
         plan.tok = ((n + blocks - 1) / blocks + 15) / 16 * 16;
         lay_out(plan, slabs, (kblocks + 3) / 4, n, plan.tok, 4 * ts_kblock(ty, plan.tok), plan.tok > 128 ? 2.5e-6 : 1e-6, 1, all, max_floats, best, best_t);
+        if (room && ty != T_Q4_0) share_out(plan, slabs, (kblocks + 3) / 4, n, plan.tok, 4 * ts_kblock(ty, plan.tok), plan.tok > 128 ? 2.5e-6 : 1e-6, room, best, best_t);
         if (plan.tok <= 32) break;
     }
     return best;
@@ -116,11 +137,12 @@ inline GemmPlan gemm_tc_search(int ty, uint32_t k, uint32_t m, uint32_t n, int x
 // The search costs the host up to 4 us (512 tokens: nine widths of items, each with a loop over the dealt ones) and an engine
 // asks for the same few shapes in every layer, so each thread keeps the plans it found last.  (Searched anew, and twice, in every
 // call: Q2_0 2048 -> 6144, 512 tokens, took the host 11.5 us beside 16 on the GPU.)
-inline GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms, size_t max_floats) {
+inline GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt, int sms, size_t max_floats, const uint32_t *room = nullptr) {
     struct Entry {
         int ty, xdt, sms;
         uint32_t k, m, n;
         size_t max_floats;
+        const uint32_t *room;  // (one array a device, never changed)
         bool used;
         GemmPlan plan;
     };
@@ -130,8 +152,8 @@ inline GemmPlan gemm_tc_plan(int ty, uint32_t k, uint32_t m, uint32_t n, int xdt
     h = (h * 4 + (uint32_t)xdt) * 2 + (max_floats != 0);
     Entry &e = cache[(h * 2654435761u) >> 26];
     static_assert(kEntries == 64, "six bits of the hash");
-    if (!(e.used && e.ty == ty && e.xdt == xdt && e.sms == sms && e.k == k && e.m == m && e.n == n && e.max_floats == max_floats))
-        e = {ty, xdt, sms, k, m, n, max_floats, true, gemm_tc_search(ty, k, m, n, xdt, sms, max_floats)};
+    if (!(e.used && e.ty == ty && e.xdt == xdt && e.sms == sms && e.k == k && e.m == m && e.n == n && e.max_floats == max_floats && e.room == room))
+        e = {ty, xdt, sms, k, m, n, max_floats, room, true, gemm_tc_search(ty, k, m, n, xdt, sms, max_floats, room)};
     return e.plan;
 }
 

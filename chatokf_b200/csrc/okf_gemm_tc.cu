@@ -897,7 +897,7 @@ cudaError_t launch_gemm_tc(const GemmPlan &plan, int ty, const uint8_t *w, uint3
     a.row_bytes = (k / block_elems(ty)) * block_bytes(ty);
     cudaError_t e = cudaErrorInvalidValue;
     if (plan.tok) {
-        GemmTs g = {ty, xdt, odt, sms, w, x, out, status, partial, k, m, n, a.row_bytes, plan.tok, a.waves, a.dealt, a.dealers, a.nt,
+        GemmTs g = {ty, xdt, odt, sms, w, x, out, status, partial, k, m, n, a.row_bytes, plan.tok, a.waves, a.dealt, a.dealers, a.nt, plan.cluster,
                     gather ? go.nout : 0u, go.out_ld, go.out_row0, {}, go.epoch, go.epoch_inc};
         for (uint32_t r = 0; r < go.nout; r++) g.outs[r] = go.outs[r];
         e = launch_gemm_ts(g, s, dev);
@@ -958,7 +958,7 @@ extern "C" int okf_gemm_noalloc(okf_ctx *ctx, int type, const okf_weights *w, ui
     }
     // every slot the reduction reads is written by the main kernel first, so nothing in the
     // array has to be cleared between calls
-    const GemmPlan plan = gemm_tc_plan(type, k, m, n, xdt, ctx->sms, kStaticScratchFloats);
+    const GemmPlan plan = gemm_tc_plan(type, k, m, n, xdt, ctx->sms, kStaticScratchFloats, gemm_ts_clusters(ctx->device));
     cudaError_t e = launch_gemm_tc(plan, type, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, g_static_scratch_addr[ctx->device],
                                    (cudaStream_t)stream, ctx->sms, ctx->device, &ctx->launches, nullptr);
     if (e != cudaSuccess) return cuda_fail(ctx, e);

@@ -16,12 +16,16 @@
 // IQ2_XXS 38.1 -> 25.0, IQ4_NL 40.8 -> 27.6; Q5_K 2560 -> 9728, 77 tokens, 19.3 -> 14.8.  What bounds it: up to some 100 tokens instruction issue
 // (about 260 instructions for a warp's 32 x 64 weights: widening, multiply-add, rounding; 58 % of the issue slots for Q4_K at 64 tokens, 68 % for
 // IQ2_XXS); at 256 tokens nothing is full, the tensor pipe is busy 55 % of the time and a third of the slots are used.
+// Where there are few items (a short prompt against few rows), clusters of 2 to 8 CTAs share one: each takes a run of its units, leaves its sums in
+// shared memory where the rings were, and adds up every so many-th token out of the others' (share_out in okf_gemm_plan.h has what it
+// gives: 1.1 to 2 times on the shapes that take it, against partial tiles through L2 and a second kernel).
 // Tried on the way: rows copied by cp.async (two warps: 1900 cycles a unit for address arithmetic and issue, Q4_K 30.8 us against 25.9);
 // a turn of the MMA warp per k-block (some 500 cycles each, 28.9); one k-block a turn for every unpacking warp (25.9
 // against 23.0: waits and stores are paid per turn).
 //
 // Every wait is bounded (about a second); a wait that gives up records a code in the status word.
 #include <cstring>
+#include <mutex>
 
 #include "okf_tc.cuh"
 #include "okf_gemv_wide.cuh"
@@ -62,6 +66,8 @@ struct TsArgs {
     uint32_t w_stages, b_stages, box, b_kb, b_off, w_off, tab_off;  // a stage of activations: box tokens x b_kb k-blocks of a unit
     uint32_t tma_log;  // weights by TMA, 2^tma_log rows to a row of the tensor map; kTsNoTma: by cp.async
     uint32_t odt;      // DT_F32, DT_BF16
+    uint32_t cluster;  // CTAs that share an item along K (<= 1: none)
+    uint32_t vec;      // shared items: rows of results start on 16 (bf16: 8) bytes
     uint32_t nout, out_ld, out_row0;  // row shards: fp32 into every rank's whole output (nout > 0)
     void *outs[8];
     uint32_t *epoch;
@@ -70,19 +76,27 @@ struct TsArgs {
 
 struct TsWork {
     uint32_t m0, n0, kb0, kb1;
-    uint32_t slot;  // partial tile, or kTsWhole
+    uint32_t slot;  // partial tile, or kTsWhole, or kTsShare
 };
-constexpr uint32_t kTsWhole = 0xFFFFFFFFu, kTsNoTma = 0xFFFFFFFFu;
+constexpr uint32_t kTsWhole = 0xFFFFFFFFu, kTsShare = 0xFFFFFFFEu, kTsNoTma = 0xFFFFFFFFu;
 
 // The j-th piece of work of this CTA; false when there is none.  Whole items go round-robin over the CTAs, then every CTA
 // takes its run of the dealt items' units laid end to end (the CTA that has a unit: dealt_to).
-__device__ __forceinline__ bool ts_work(const TsArgs &p, uint32_t j, TsWork &w) {
+// CL: one item a cluster, this CTA's part of its K.
+template <bool CL> __device__ __forceinline__ bool ts_work(const TsArgs &p, uint32_t j, TsWork &w) {
     const uint32_t kblocks = p.k / kBK, units = (kblocks + 3) / 4;
     uint32_t item;
     w.slot = kTsWhole;
     w.kb0 = 0;
     w.kb1 = kblocks;
-    if (!p.dealt || j < p.waves) {
+    if constexpr (CL) {
+        if (j) return false;
+        item = blockIdx.x / p.cluster;
+        const uint32_t rank = blockIdx.x - item * p.cluster;
+        w.kb0 = units * rank / p.cluster * 4;
+        w.kb1 = min(units * (rank + 1) / p.cluster * 4, kblocks);
+        w.slot = kTsShare;
+    } else if (!p.dealt || j < p.waves) {
         item = blockIdx.x + j * gridDim.x;
         if (item >= p.items) return false;
     } else {
@@ -127,6 +141,49 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+
+// ---- an item that the CTAs of a cluster share ----------------------------------------
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 16 bytes of CTA `rank`'s shared memory, at the place that `addr` is in this one's
+__device__ __forceinline__ float4 lds_of(uint32_t addr, uint32_t rank) {
+    float4 v;
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+// Rows m0 + 4 lane .. + 3 of token `t`, into every output.  Where results do not start on 16 (8) bytes the neighbours of every thread are dealt out
+// again, so that a warp stores 32 rows side by side.
+__device__ __forceinline__ void store_rows(const TsArgs &p, float4 v, uint32_t m0, uint32_t t, uint32_t lane) {
+    const size_t at = (size_t)t * (p.nout ? p.out_ld : p.m) + (p.nout ? p.out_row0 : 0u) + m0;
+    float e[4];  // rows lane, lane + 32, ..
+    if (!p.vec) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++) {
+            const uint32_t from = 8 * j + lane / 4;
+            const float x = __shfl_sync(0xffffffffu, v.x, from), y = __shfl_sync(0xffffffffu, v.y, from);
+            const float z = __shfl_sync(0xffffffffu, v.z, from), w = __shfl_sync(0xffffffffu, v.w, from);
+            e[j] = lane & 2 ? (lane & 1 ? w : z) : (lane & 1 ? y : x);
+        }
+    }
+#pragma unroll 1
+    for (uint32_t b = 0; b < (p.nout ? p.nout : 1u); b++) {
+        void *out = p.nout ? p.outs[b] : p.out;
+        if (p.vec) {
+            if (m0 + 4 * lane >= p.m) break;
+            if (p.odt == DT_F32) *reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + at + 4 * lane) = v;
+            else *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(out) + at + 4 * lane) = make_uint2(pack16<false>(v.x, v.y), pack16<false>(v.z, v.w));
+        } else {
+#pragma unroll
+            for (uint32_t j = 0; j < 4; j++) {
+                if (m0 + lane + 32 * j >= p.m) continue;
+                if (p.odt == DT_F32) reinterpret_cast<float *>(out)[at + lane + 32 * j] = e[j];
+                else reinterpret_cast<__nv_bfloat16 *>(out)[at + lane + 32 * j] = __float2bfloat16_rn(e[j]);
+            }
+        }
+    }
 }
 
 // ---- unpacking 64 weights of a row ------------------------------------------------
@@ -369,7 +426,8 @@ template <> struct TsRaw<T_IQ2_XXS, true> {
     }
 };
 
-template <int TY, bool SK, bool F16>
+// CL: launched in clusters that share an item along K.  (As a run-time flag it costs all other launches 0.3 us.)
+template <int TY, bool SK, bool F16, bool CL>
 __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                                                                const __grid_constant__ TsArgs p) {
     using Ge = TsGeom<TY, SK>;
@@ -439,7 +497,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
         }
         RingPlace ring_at(set);
         uint32_t it = 0, turn = 0;  // units so far, of both sets and of this one
-        for (uint32_t j = 0; ts_work(p, j, wk); j++) {
+        for (uint32_t j = 0; ts_work<CL>(p, j, wk); j++) {
             const uint32_t src = (uint32_t)reinterpret_cast<uintptr_t>(p.w) + (wk.m0 + row) * p.row_bytes;  // its low bits
             for (uint32_t u = wk.kb0 >> 2; u < (wk.kb1 + 3) >> 2; u++, it++) {
                 if ((it & 1) != set) continue;
@@ -480,7 +538,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
     } else if (warp == kTsLoadWarp && p.tma_log != kTsNoTma) {
         // ---------------- blocks as stored -> ring; weights do not depend on the kernel before
         RingPlace ring_at(0);
-        for (uint32_t j = 0; ts_work(p, j, wk); j++) {
+        for (uint32_t j = 0; ts_work<CL>(p, j, wk); j++) {
             for (uint32_t u = wk.kb0 >> 2; u < (wk.kb1 + 3) >> 2; u++, ring_at.advance(1, p.w_stages)) {
                 const uint32_t s = ring_at.stage(p.w_stages);
                 uint64_t *full = &full_w[ring_at.full()];
@@ -508,7 +566,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
             const uint32_t first = (warp - kTsLoadWarp) * 4 + (lane >> 3), c0 = lane & 7;
             const size_t step = (size_t)8 * p.row_bytes;
             RingPlace ring_at(0);
-            for (uint32_t j = 0; ts_work(p, j, wk); j++) {
+            for (uint32_t j = 0; ts_work<CL>(p, j, wk); j++) {
                 const uint32_t rows = min(kBM, p.m - wk.m0);  // rows past the end: whatever is there, nobody stores their results
                 for (uint32_t u = wk.kb0 >> 2; u < (wk.kb1 + 3) >> 2; u++, ring_at.advance(1, p.w_stages)) {
                     const uint32_t sw = ring_at.stage(p.w_stages);
@@ -542,7 +600,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
         pdl_wait();  // x may come from the kernel before
         const uint32_t tile = p.box * (kBK * 2);  // bytes
         uint32_t s = 0, use = 0;
-        for (uint32_t j = 0; ts_work(p, j, wk); j++) {
+        for (uint32_t j = 0; ts_work<CL>(p, j, wk); j++) {
             for (uint32_t g = wk.kb0 / p.b_kb; g * p.b_kb < wk.kb1; g++, s = s + 1 == p.b_stages ? (use++, 0) : s + 1) {
                 if (use > 0 && !warp_poll(&empty_b[s], (use - 1) & 1, abort_flag, p.status)) {
                     const long long t0 = clock64();  // as above
@@ -562,7 +620,7 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
         // ---------------- MMA issuer, a unit a turn
         const uint32_t tile = p.box * (kBK * 2);
         uint32_t item = 0, it = 0, s_b = 0, use_b = 0;
-        for (uint32_t j = 0; ts_work(p, j, wk); j++, item++) {
+        for (uint32_t j = 0; ts_work<CL>(p, j, wk); j++, item++) {
             // N of the instruction: the tokens the item really has, in sixteens
             const uint32_t live = min(p.tok, p.n - wk.n0), idesc = instr_desc(F16 ? 0u : 1u, kBM, (live + 15u) & ~15u);
             const uint32_t acc = two_acc ? item & 1 : 0, acc_use = two_acc ? item >> 1 : item, d = tmem_base + acc * 128;
@@ -602,20 +660,26 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
         const uint32_t q = warp & 3;
         uint32_t item = 0;
         pdl_wait();  // the kernel before may still read what is written here
-        for (uint32_t j = 0; ts_work(p, j, wk); j++, item++) {
+        for (uint32_t j = 0; ts_work<CL>(p, j, wk); j++, item++) {
             const uint32_t n_end = min(p.n, wk.n0 + p.tok), row = wk.m0 + q * 32 + lane;
             const uint32_t acc = two_acc ? item & 1 : 0, acc_use = two_acc ? item >> 1 : item;
             if (!warp_wait(&acc_full[acc], acc_use & 1, lane, abort_flag, p.status)) goto done;
             tc_fence_after();
             // partial tiles hold all 128 rows
-            float *part = wk.slot != kTsWhole ? p.partial + (size_t)wk.slot * p.nt * kBM + q * 32 + lane : nullptr;
+            float *part = wk.slot < kTsShare ? p.partial + (size_t)wk.slot * p.nt * kBM + q * 32 + lane : nullptr;
 #pragma unroll 1
             for (uint32_t t0 = wk.n0; t0 < n_end; t0 += 32) {
                 uint32_t r[32];
                 tmem_ld32(tmem_base + ((q * 32) << 16) + acc * 128 + (t0 - wk.n0), r);
                 tmem_ld_wait();
                 const uint32_t live = min(32u, n_end - t0);
-                if (part) {
+                if (CL) {
+                    // Into shared memory, where the rings were: every copy into them has been read by the MMAs that are complete.
+                    const uint32_t o = smem_u32(smem + p.b_off) + (t0 - wk.n0) * (kBM * 4) + (q * 32 + lane) * 4;
+#pragma unroll
+                    for (uint32_t i = 0; i < 32; i++)
+                        if (i < live) sts32(o + i * (kBM * 4), r[i]);
+                } else if (part) {
                     float *o = part + (size_t)(t0 - wk.n0) * kBM;
 #pragma unroll
                     for (uint32_t i = 0; i < 32; i++)
@@ -650,6 +714,26 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
         }
     }
 done:
+    if constexpr (CL) {
+        // Every CTA of the cluster adds up every so many-th token, in the order of k, out of the others' shared memory.
+        pdl_wait();  // (the kernel before may still read what is written here)
+        __syncwarp();
+        cluster_sync();
+        ts_work<CL>(p, 0, wk);
+        const uint32_t live = min(p.tok, p.n - wk.n0), rank = blockIdx.x % p.cluster;
+        for (uint32_t t = rank * (kTsThreads / 32) + warp; t < live; t += p.cluster * (kTsThreads / 32)) {
+            const uint32_t at = smem_u32(smem + p.b_off) + t * (kBM * 4) + lane * 16;
+            float4 v[8];
+#pragma unroll
+            for (uint32_t c = 0; c < 8; c++)
+                if (c < p.cluster) v[c] = lds_of(at, c);
+#pragma unroll
+            for (uint32_t c = 1; c < 8; c++)
+                if (c < p.cluster) v[0] = make_float4(v[0].x + v[c].x, v[0].y + v[c].y, v[0].z + v[c].z, v[0].w + v[c].w);
+            store_rows(p, v[0], wk.m0, wk.n0 + t, lane);
+        }
+        cluster_sync();  // nobody leaves while its part may still be read
+    }
     if (p.epoch && !p.dealt && blockIdx.x == 0 && threadIdx.x == 0) {
         pdl_wait();
         p.epoch[0] += p.epoch_inc;
@@ -662,13 +746,13 @@ done:
     }
 }
 
-template <int TY, bool SK, bool F16>
+template <int TY, bool SK, bool F16, bool CL>
 static cudaError_t ts_launch(TsArgs a, const void *x, uint32_t grid, cudaStream_t s, int dev) {
     using Ge = TsGeom<TY, SK>;
     static bool attr_set[64] = {};  // the opt-in is per device
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_ts_kernel<TY, SK, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTsSmem);
+        cudaError_t e = cudaFuncSetAttribute(gemm_ts_kernel<TY, SK, F16, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTsSmem);
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
@@ -702,14 +786,51 @@ static cudaError_t ts_launch(TsArgs a, const void *x, uint32_t grid, cudaStream_
                        CU_TENSOR_MAP_SWIZZLE_NONE);
         if (e != cudaSuccess) return e;
     }
-    return launch_pdl(gemm_ts_kernel<TY, SK, F16>, grid, kTsThreads, kTsSmem, s, 1, xmap, wmap, a);
+    return launch_pdl(gemm_ts_kernel<TY, SK, F16, CL>, grid, kTsThreads, kTsSmem, s, CL ? a.cluster : 1, xmap, wmap, a);
 }
 template <int TY, bool SK>
 static cudaError_t ts_launch_x(const TsArgs &a, const void *x, int xdt, uint32_t grid, cudaStream_t s, int dev) {
-    return xdt == DT_F16 ? ts_launch<TY, SK, true>(a, x, grid, s, dev) : ts_launch<TY, SK, false>(a, x, grid, s, dev);
+    if (a.cluster > 1) return xdt == DT_F16 ? ts_launch<TY, SK, true, true>(a, x, grid, s, dev) : ts_launch<TY, SK, false, true>(a, x, grid, s, dev);
+    return xdt == DT_F16 ? ts_launch<TY, SK, true, false>(a, x, grid, s, dev) : ts_launch<TY, SK, false, false>(a, x, grid, s, dev);
 }
 
 }  // namespace tc
+
+const uint32_t *gemm_ts_clusters(int dev) {
+    struct Known {
+        std::once_flag once;
+        uint32_t room[9] = {};
+    };
+    static Known known[64];
+    if (dev < 0 || dev >= 64) return nullptr;
+    Known &k = known[dev];
+    std::call_once(k.once, [&] {
+        auto kernel = tc::gemm_ts_kernel<T_Q4_K, false, true, true>;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::kTsSmem) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return;
+        }
+        for (uint32_t c = 2; c <= 8; c++) {
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = c;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(c * 256);
+            cfg.blockDim = dim3(tc::kTsThreads);
+            cfg.dynamicSmemBytes = tc::kTsSmem;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, (const void *)kernel, &cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                n = 0;
+            }
+            k.room[c] = (uint32_t)n;
+        }
+    });
+    return k.room;
+}
 
 cudaError_t launch_gemm_ts(const GemmTs &g, cudaStream_t s, int dev) {
     tc::TsArgs a = {};
@@ -718,9 +839,12 @@ cudaError_t launch_gemm_ts(const GemmTs &g, cudaStream_t s, int dev) {
     a.tok = g.tok; a.groups = (g.n + g.tok - 1) / g.tok; a.items = (g.m + tc::kBM - 1) / tc::kBM * a.groups;
     a.waves = g.waves; a.dealt = g.dealt; a.dealers = g.dealers; a.nt = g.nt;
     a.odt = (uint32_t)g.odt;
+    a.cluster = g.cluster;
+    a.vec = g.m % 4 == 0 && (g.nout ? (g.out_ld | g.out_row0) % 4 == 0 : (uintptr_t)g.out % (g.odt == DT_F32 ? 16 : 8) == 0);
+    for (uint32_t i = 0; i < g.nout; i++) a.vec = a.vec && (uintptr_t)g.outs[i] % 16 == 0;
     a.nout = g.nout; a.out_ld = g.out_ld; a.out_row0 = g.out_row0; a.epoch = g.epoch; a.epoch_inc = g.epoch_inc;
     for (uint32_t i = 0; i < g.nout; i++) a.outs[i] = g.outs[i];
-    const uint32_t all = (uint32_t)g.sms, grid = a.waves ? all : a.dealt ? a.dealers : a.items < all ? a.items : all;
+    const uint32_t all = (uint32_t)g.sms, grid = a.cluster > 1 ? a.items * a.cluster : a.waves ? all : a.dealt ? a.dealers : a.items < all ? a.items : all;
     const bool whole = ((uintptr_t)g.w | g.row_bytes) % 16 == 0;  // (units of these four types are multiples of 16 bytes)
     switch (g.ty) {
     case T_Q4_K: return tc::ts_launch_x<T_Q4_K, false>(a, g.x, g.xdt, grid, s, dev);

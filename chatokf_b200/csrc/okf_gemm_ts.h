@@ -15,11 +15,14 @@ struct GemmTs {
     uint32_t k, m, n, row_bytes;
     uint32_t tok;                        // tokens of an item, a multiple of 16, at most 256
     uint32_t waves, dealt, dealers, nt;  // how items are laid over the SMs
+    uint32_t cluster;                    // CTAs that share an item along K (0, 1: none)
     uint32_t nout, out_ld, out_row0;     // row shards: fp32 into `nout` whole outputs
     void *outs[8];
     uint32_t *epoch;
     uint32_t epoch_inc;
 };
 cudaError_t launch_gemm_ts(const GemmTs &g, cudaStream_t s, int dev);
+// How many clusters of 2 .. 8 of its CTAs the device has room for at once (index: size); null where that is not known.
+const uint32_t *gemm_ts_clusters(int dev);
 
 }  // namespace okf
