@@ -329,7 +329,7 @@ template <int TY, int MODE, int XDT, uint32_t NW>
 static cudaError_t stream_go(const GemvArgs &a, const StreamPlan &p, cudaStream_t s, int dev) {
     static bool attr_set[64] = {};  // the opt-in is per device
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(stream_kernel<TY, MODE, XDT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, stream_budget(NW));
+        cudaError_t e = cudaFuncSetAttribute(stream_kernel<TY, MODE, XDT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW == 8 ? kStreamAlone : stream_budget(NW));
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }

@@ -60,6 +60,13 @@ struct StreamPlan {
 // (two of 112 KB leave 2 KB of an SM: enough for the small kernels between matvecs, which with 1 KB less take 0.8 us longer each)
 constexpr uint32_t stream_budget(uint32_t warps) { return warps == 8 ? 112 * 1024 : 226 * 1024; }
 
+// What a CTA of a grid that is meant to be one to an SM asks for: two of them do not fit one SM.  Left to themselves two end up on one SM and
+// none on another where a grid comes while SMs fall free one by one: 197 such launches of all types but IQ2_XXS take 7 % longer when
+// launches follow one another, 5 % behind elementwise kernels (Q2_0 2048 -> 2048 and its like, eight layers, 131 -> 124 us; in a graph of
+// matvecs alone 1 %, 6 % the other way for grids of exactly as many CTAs as SMs).  IQ2_XXS's CTAs fill 48 KB of tables first, which they can
+// do beside their predecessors: alone 5 % slower there and 5 % faster behind elementwise kernels, so without clusters they are left.
+constexpr uint32_t kStreamAlone = 116 * 1024;
+
 template <int TY, int MODE>
 inline bool stream_layout(uint32_t nunit, uint32_t n, uint32_t clog, uint32_t clusters, uint32_t tiles, uint32_t warps, StreamPlan &p) {
     using S = StreamGeom<TY, MODE>;
@@ -97,12 +104,15 @@ inline bool stream_layout(uint32_t nunit, uint32_t n, uint32_t clog, uint32_t cl
 
 // The time of a launch in a chain, us: what it takes whatever its size, a warp's staging of x (column, unit pairs) and a warp's units,
 // both at another rate where two CTAs share an SM, and never less than the weights take at what copies in pieces of 16 bytes reach (4.9
-// TB/s).  The constants are a fit to 21 000 timings: 1080 shapes (every type, 1 to 8 columns, rows of 512 to 18432 weights, 300 to
-// 150 000 rows), each in a chain of matvecs and in one with an elementwise kernel before every matvec, as an engine has both.  The choice made with
-// them is 0.9 % slower than the best one at one column (geometric mean over the shapes; at most 16 %), 0.7 to 1.5 % at several.  One CTA to
-// an SM where there is work for two is the faster one in the first kind of chain only (Q4_K 2560 -> 2 x 9728, one column, 8.2 and 8.4
-// us, behind an elementwise kernel 13.5 and 10.4): it leaves room for the next matvec's first copies, but the CTAs of a grid that comes while SMs
-// fall free one by one are not spread evenly, and two end up on one SM.
+// TB/s).  The constants are fits, one up to four columns and one for what is left: to 21 000 and to 44 000 timings, of
+// 1080 and 1480 shapes (every type, 1 to 8 columns, rows of 384 to 18432 weights, 300 to 150 000 rows), each in a chain of matvecs, in one
+// with an elementwise kernel before every matvec and, in the second fit, in a chain of plain launches, as engines have them all.  The choice made
+// with them is 0.9 % slower than the best one at one column (geometric mean over the shapes; at most 16 %), 0.7 to 1.3 % at several.  Against
+// okf_gemv.cu's kernel alone 633 other shapes are, in the first and second kind of chain, 1.08 and 1.11 times as fast at one column, 1.18
+// and 1.20 at two to four, 1.31 and 1.34 at five to eight, 1.15 to 1.24 where rows end inside a unit; a fifth and a twentieth of
+// them at one column, a twentieth of the others, lose more than 2 %.  One CTA to an SM where there is work for two is the faster one in the
+// first kind of chain only (Q4_K 2560 -> 2 x 9728, one column, 8.2 and 8.4 us, behind an elementwise kernel 13.5 and 10.4): it leaves room
+// for the next matvec's first copies, but what comes behind a small kernel starts its copies late, and two CTAs have more of them in flight.
 inline int stream_kind(int mode) { return mode == M_SEP ? 0 : mode == M_W1 ? 1 : mode == M_W2 ? 2 : 3; }
 struct StreamUnit {
     float stream[4];  // one column, up to four, up to eight, rows that end inside a unit
@@ -110,28 +120,28 @@ struct StreamUnit {
 };
 inline StreamUnit stream_unit_us(int ty) {
     switch (ty) {
-    case T_Q4_K: return {{.71f, .75f, 1.07f, 0.f}, {.44f, .58f, 0.f, 0.f}};
-    case T_Q8_0: return {{1.23f, 1.50f, 1.73f, 1.74f}, {.82f, 1.00f, 0.f, .64f}};
-    case T_Q6_K: return {{1.40f, 1.61f, 1.94f, 0.f}, {.87f, .80f, 0.f, 0.f}};
-    case T_Q5_K: return {{.90f, 1.01f, 1.30f, 0.f}, {.72f, .94f, 0.f, 0.f}};
-    case T_Q4_0: return {{.70f, 1.03f, 1.27f, 1.38f}, {.34f, .61f, 0.f, .80f}};
-    case T_IQ4_NL: return {{1.16f, 1.29f, 1.45f, 1.73f}, {.92f, .70f, 0.f, 1.22f}};
-    case T_Q2_0: return {{.51f, .71f, .94f, 1.07f}, {.28f, .33f, 0.f, .49f}};
-    default: return {{.95f, 1.20f, 1.35f, 0.f}, {.67f, .89f, 0.f, 0.f}};
+    case T_Q4_K: return {{.71f, .75f, .83f, 0.f}, {.44f, .58f, 0.f, 0.f}};
+    case T_Q8_0: return {{1.23f, 1.50f, 1.25f, 1.18f}, {.82f, 1.00f, 0.f, .76f}};
+    case T_Q6_K: return {{1.40f, 1.61f, 1.39f, 0.f}, {.87f, .80f, 0.f, 0.f}};
+    case T_Q5_K: return {{.90f, 1.01f, 1.03f, 0.f}, {.72f, .94f, 0.f, 0.f}};
+    case T_Q4_0: return {{.70f, 1.03f, .93f, .96f}, {.34f, .61f, 0.f, .55f}};
+    case T_IQ4_NL: return {{1.16f, 1.29f, 1.04f, 1.08f}, {.92f, .70f, 0.f, .97f}};
+    case T_Q2_0: return {{.51f, .71f, .70f, .67f}, {.28f, .33f, 0.f, .44f}};
+    default: return {{.95f, 1.20f, 1.04f, 0.f}, {.67f, .89f, 0.f, 0.f}};
     }
 }
 inline float quad_max(float a, float b) { return sqrtf(sqrtf(a * a * a * a + b * b * b * b)); }  // the larger one, rounded off
 inline float stream_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tiles, uint32_t clog, uint32_t clusters, uint32_t warps, uint32_t sms, float floor_us) {
     const int kind = stream_kind(mode);
-    constexpr float one[4] = {1.3f, 2.65f, 3.05f, 4.2f};   // by cluster size, one CTA to an SM
-    constexpr float two[4][4] = {{2.5f, 3.8f, 7.8f, 8.1f}, {3.2f, 4.5f, 8.5f, 8.9f}, {3.4f, 4.65f, 8.7f, 9.0f}, {1.8f, 3.05f, 7.1f, 7.45f}};
-    constexpr float wide[4] = {5.0f, 6.25f, 4.75f, 4.45f};  // sixteen warps
-    constexpr float stage[4] = {.59f, .62f, .65f, .66f}, stage_two[4] = {1.3f, .66f, .4f, 1.14f}, unit_two[4] = {.71f, .78f, 1.38f, .86f};
+    constexpr float one[2][4] = {{1.3f, 2.65f, 3.05f, 4.2f}, {1.95f, 3.3f, 3.4f, 4.1f}};  // up to four columns, the others; by cluster size, one CTA to an SM
+    constexpr float two[4][4] = {{2.5f, 3.8f, 7.8f, 8.1f}, {3.2f, 4.5f, 8.5f, 8.9f}, {2.8f, 4.85f, 9.f, 10.f}, {1.65f, 3.7f, 7.85f, 9.f}};
+    constexpr float wide[4] = {4.35f, 6.25f, 6.5f, 8.05f};  // sixteen warps
+    constexpr float stage[4] = {.59f, .62f, .35f, .51f}, stage_two[4] = {1.3f, .66f, 1.1f, 1.75f}, unit_two[4] = {.71f, .78f, 1.42f, 1.37f};
     const bool shared = warps == 16 || (clusters << clog) > sms;
     const uint32_t units = (nunit + (1u << clog) - 1) >> clog, per = (tiles + clusters - 1) / clusters * units;
     const float busy = stream_unit_us(ty).stream[kind] * (float)((per + warps - 1) / warps) * (shared ? unit_two[kind] : 1.f) +
                        stage[kind] * (float)((units * n + warps - 1) / warps) * (shared ? stage_two[kind] : 1.f);
-    return (warps == 16 ? wide[clog] : shared ? two[kind][clog] : one[clog]) + quad_max(busy, floor_us);
+    return (warps == 16 ? wide[clog] : shared ? two[kind][clog] : one[kind / 2][clog]) + quad_max(busy, floor_us);
 }
 // The same of okf_gemv.cu's kernel, whose CTAs share their tiles' units between eight warps; `ctas` and `clog` as it would take them.
 // It is asked where it may be the better one: at one column, where its bulk copies of whole rows reach 6.1 TB/s (Q4_K 5120 -> 65536 33.6
@@ -142,11 +152,12 @@ inline float ring_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tile
     const int kind = stream_kind(mode);
     if (kind == 2) return nunit <= 6 && tiles <= 4 * sms && ty != T_Q4_K && ty != T_Q5_K ? 0.f : 1e30f;
     if (kind != 0 && tiles < 4 * sms) return 1e30f;
-    constexpr float fixed[4] = {3.26f, 3.12f, 0.f, 5.74f};
+    constexpr float fixed[4] = {3.26f, 3.12f, 0.f, 4.65f}, pair_us[2] = {.9f, .77f}, shared_x[2] = {1.32f, 1.65f}, cluster_us[2] = {3.07f, 3.5f};
+    const bool shared = ctas > (kind < 2 ? sms : sms + sms / 4);  // (up to a quarter more CTAs than SMs hardly slow each other down where rows end inside a unit)
     const uint32_t clusters = ctas >> clog, units = (nunit + (1u << clog) - 1) >> clog;
-    const float busy = (stream_unit_us(ty).ring[kind] * (float)((tiles + clusters - 1) / clusters * units) + .9f * (float)(units * n)) / 8.f * (ctas > sms ? 1.32f : 1.f);
+    const float busy = (stream_unit_us(ty).ring[kind] * (float)((tiles + clusters - 1) / clusters * units) + pair_us[kind / 2] * (float)(units * n)) / 8.f * (shared ? shared_x[kind / 2] : 1.f);
     const uint32_t ub = ty == T_Q8_0 ? 272 : ty == T_Q6_K ? 210 : ty == T_Q5_K ? 176 : ty == T_Q2_0 ? 68 : ty == T_IQ2_XXS ? 66 : 144;
-    const float us = fixed[kind] + (ctas > sms ? 1.47f : 0.f) + (clog ? 3.07f : 0.f) + quad_max(busy, (float)nunit * (float)tiles * (16.f * (float)ub / 6.1e6f));
+    const float us = fixed[kind] + (shared ? 1.45f : 0.f) + (clog ? cluster_us[kind / 2] : 0.f) + quad_max(busy, (float)nunit * (float)tiles * (16.f * (float)ub / 6.1e6f));
     return tiles < 12 * sms ? us : kind == 3 && n == 1 ? .85f * us : .93f * us;  // (with so many tiles the fit favours the other kernel: ragged Q4_0 2336 -> 63677
                                                                                  // 27.5 us here, 32.5 there)
 }
@@ -158,11 +169,15 @@ inline StreamPlan stream_search(uint32_t nunit, uint32_t n, uint32_t tiles, cons
     for (uint32_t clog = 0; clog < 4 && (clog == 0 || nunit >= 2u << clog); clog++) {
         for (uint32_t v = 0; v < (MODE == M_W2 ? 3 : 2); v++) {
             const uint32_t warps = v == 2 ? 16 : 8, limit = v == 1 ? room.two[clog] : room.one[clog], clusters = tiles < limit ? tiles : limit;
-            if (clusters == 0 || (v == 1 && tiles <= room.one[clog])) continue;
+            // Two CTAs to an SM from five columns on and at rows that end inside a unit only where they fill nine tenths of the places: fewer
+            // are spread unevenly, two on one SM and one on another (the fit without this rule chooses 1 % worse).
+            const bool fills = MODE == M_SEP || MODE == M_W1 ? tiles > room.one[clog] : (clusters << clog) * 10 >= room.two[0] * 9;
+            if (clusters == 0 || (v == 1 && !fills)) continue;
             StreamPlan p = {};
             if (!stream_layout<TY, MODE>(nunit, n, clog, clusters, tiles, warps, p)) continue;
             p.us = stream_us(TY, MODE, nunit, n, tiles, clog, clusters, warps, room.one[0], floor_us);
             p.ok = true;
+            if (warps == 8 && p.ctas <= room.one[0] && p.smem < kStreamAlone && (TY != T_IQ2_XXS || clog)) p.smem = kStreamAlone;
             if (!best.ok || p.us < best.us) best = p;
         }
     }

@@ -58,7 +58,7 @@ template <int TY, int MODE> static unsigned plans(std::mt19937 &rng, unsigned &f
         const StreamLayout &L = p.L;
         const uint32_t size = 1u << L.clog, clusters = p.ctas / size, units = (nunit + size - 1) / size, per = (tiles + clusters - 1) / clusters;
         const uint32_t panel = (MODE == M_SEP ? 2 : n * mode_bytes(MODE)) * L.es, records = MODE == M_SEP ? 256 : units * n * wide_info_words(TY, mode_bytes(MODE)) * 4;
-        bad += p.smem > stream_budget(p.warps) || p.ctas % size || nunit < size || L.depth < 2 || L.depth > 4;
+        bad += p.smem > (p.warps == 8 && p.ctas <= 148 ? kStreamAlone : stream_budget(p.warps)) || p.ctas % size || nunit < size || L.depth < 2 || L.depth > 4;
         bad += L.tiles_each * clusters + L.tiles_more != tiles || L.tiles_more >= clusters || L.tiles_each == 0;
         bad += p.warps * L.depth * StreamGeom<TY, MODE>::stage > L.xs_off || L.xs_off % 128 || L.xs_off + panel > L.info_off || L.slot_off % 128;
         bad += L.info_off + records > L.slot_off || L.slot_off + p.warps * 2 * n * 64 > L.part_off || L.part_off + (size > 1 ? per * n * 64 : 0) > L.tab_off;
