@@ -715,7 +715,7 @@ def run_ours(args):
                 "unit": "GB/s", "frac": per_launch_bytes / per_launch_us / 1e3 / pk["hbm"],
                 "traffic": traffic, "peak_source": pk["src"],
                 "bytes_per_launch": per_launch_bytes, "us_per_launch": per_launch_us,
-                "kernel": "okf gemv_kernel (decode matvec)"}
+                "kernel": "okf stream_kernel, gemv_kernel (decode matvec)"}
     result = {
         "metric": ("prefill GEMM TFLOP/s" if tensor_bound else "quant GEMV HBM GB/s at b=%d" % batch)
                   + " (%s)" % wl,
@@ -791,9 +791,9 @@ def run_ours(args):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel on ONE GPU, from the
-# ncu captures summarised under profiles/ (gemv_kernel_q4k_ffn_b1.md: gate || up 28.06 MB and down
-# 14.07 MB, the mean of the two; gemm_tc_kernel_q4k_prefill_n512.md).  Not printed for N > 1.
-TRAFFIC = {"q4k_ffn_gemv": {"value": 21.07e6, "source": "profiles/gemv_kernel_q4k_ffn_b1.md, one-GPU ncu capture"},
+# ncu captures summarised under profiles/ (stream_kernel_decode.md: gate || up 28.05 MB and down
+# 14.05 MB, the mean of the two; gemm_tc_kernel_q4k_prefill_n512.md).  Not printed for N > 1.
+TRAFFIC = {"q4k_ffn_gemv": {"value": 21.05e6, "source": "profiles/stream_kernel_decode.md, one-GPU ncu capture"},
            "q4k_prefill": {"value": 65.4e6, "source": "profiles/gemm_tc_kernel_q4k_prefill_n512.md, one-GPU ncu capture"}}
 
 
