@@ -27,6 +27,7 @@ struct GemmPlan {
     uint32_t nacc;   // token blocks per item
     uint32_t waves, dealt, dealers, nt;  // see tc::Args
     uint32_t cluster;  // CTAs of a cluster that share an item along K, 0: none; tok != 0 and all items at once
+    uint32_t chains;   // shared items: accumulators that take their k-blocks in turn
     size_t floats;   // of partial tiles
 };
 
@@ -83,18 +84,28 @@ inline void lay_out(GemmPlan plan, uint32_t slabs, uint32_t steps, uint32_t n, u
 // memory, but all items have to be there at once.  `room`: how many clusters of a size fit the device.  The exchange is counted as 2 us and 5 ns a
 // token, 1.5 us more against items that run whole: of 84 shapes (9 to 1020 tokens, all types) that were timed with and without, the plan taken
 // is 0.8 % slower than the better one on average (never counting the 1.5 us; 5 % if they are counted against dealt items too).  Dealt or whole, and shared, us:
-// Q5_K 9728 -> 2560, 77 tokens, 19.8 and 17.3; Q2_0 6144 -> 2048, 512 tokens, 22.6 and 19.5; Q4_K 4608 -> 403, 256 tokens, 12.1 and 8.6; IQ4_NL
+// Q5_K 9728 -> 2560, 77 tokens, 19.8 and 17.6; Q2_0 6144 -> 2048, 512 tokens, 22.6 and 19.5; Q4_K 4608 -> 403, 256 tokens, 12.1 and 8.6; IQ4_NL
 // 3840 -> 1307, 13 tokens, 11.9 and 6.1; whole items that stay whole: Q4_K 1792 -> 1840, 158 tokens, 7.9 and 8.4.
 // Q4_0 does not share: the tests of dealt items, of partial tiles and of their memory are written with it and count its kernels (4096 -> 1500, 34
 // tokens, 13.6 us instead of 9.0).
-inline void share_out(GemmPlan plan, uint32_t slabs, uint32_t units, uint32_t n, uint32_t tok, double t_unit, double t_item, const uint32_t *room, GemmPlan &best,
-                      double &best_t) {
+// Sums in tensor memory are cut off where fp32 would round, so a chain's error grows with its length.  `base`: units of a chain of the plan without
+// clusters; where an item's parts are longer by more than a quarter, their k-blocks go to two or four accumulators in turn (there is room for
+// them up to 128 and 64 tokens), which are added up at the end, and where that is not enough the split is not taken.  300 shapes, rms errors
+// against 64 bits: 0.93 of those without clusters on average, at most 1.34 times (one accumulator and no such rule: 1.2 and 4.2), the largest one the
+// same.  One more accumulator costs 0.3 us at 77 tokens.
+inline void share_out(GemmPlan plan, uint32_t slabs, uint32_t units, uint32_t n, uint32_t tok, double t_unit, double t_item, double base, const uint32_t *room,
+                      GemmPlan &best, double &best_t) {
     const uint32_t items = slabs * ((n + tok - 1) / tok);
     const double whole = best.dealt || best.cluster ? 0 : 1.5e-6;
     for (uint32_t c = 2; c <= 8; c++) {
         if (items > room[c] || units < 2 * c) continue;
+        const uint32_t most = tok <= 64 ? 4 : tok <= 128 ? 2 : 1;
+        const double part = (units + c - 1) / c;
+        uint32_t chains = 1;
+        while (chains < most && part > 1.25 * chains * base) chains *= 2;
+        if (part > 1.25 * chains * base) continue;
         const double t = (units + c - 1) / c * t_unit + t_item + 2e-6 + (n < tok ? n : tok) * 5e-9;
-        if (t + (best.cluster ? 0 : whole) < best_t) { best_t = t; best = plan; best.cluster = c; }
+        if (t + (best.cluster ? 0 : whole) < best_t) { best_t = t; best = plan; best.cluster = c; best.chains = chains; }
     }
 }
 // 16-bit activations: seconds per k-block of an item of `tok` tokens on the kernel with weights in tensor memory.  Up to
@@ -128,8 +139,17 @@ inline GemmPlan gemm_tc_search(int ty, uint32_t k, uint32_t m, uint32_t n, int x
     for (uint32_t blocks = least; blocks <= least + 8; blocks++) {
         plan.tok = ((n + blocks - 1) / blocks + 15) / 16 * 16;
         lay_out(plan, slabs, (kblocks + 3) / 4, n, plan.tok, 4 * ts_kblock(ty, plan.tok), plan.tok > 128 ? 2.5e-6 : 1e-6, 1, all, max_floats, best, best_t);
-        if (room && ty != T_Q4_0) share_out(plan, slabs, (kblocks + 3) / 4, n, plan.tok, 4 * ts_kblock(ty, plan.tok), plan.tok > 128 ? 2.5e-6 : 1e-6, room, best, best_t);
         if (plan.tok <= 32) break;
+    }
+    if (!room || ty == T_Q4_0) return best;
+    const uint32_t units = (kblocks + 3) / 4;
+    const double run = best.dealt && !best.waves ? (double)best.dealt * units / best.dealers : units, base = run < 1 ? 1 : run;
+    for (uint32_t blocks = least; blocks <= least + 8; blocks++) {
+        const uint32_t tok = ((n + blocks - 1) / blocks + 15) / 16 * 16;
+        plan = {};
+        plan.tok = tok;
+        share_out(plan, slabs, units, n, tok, 4 * ts_kblock(ty, tok), tok > 128 ? 2.5e-6 : 1e-6, base, room, best, best_t);
+        if (tok <= 32) break;
     }
     return best;
 }

@@ -897,7 +897,7 @@ cudaError_t launch_gemm_tc(const GemmPlan &plan, int ty, const uint8_t *w, uint3
     a.row_bytes = (k / block_elems(ty)) * block_bytes(ty);
     cudaError_t e = cudaErrorInvalidValue;
     if (plan.tok) {
-        GemmTs g = {ty, xdt, odt, sms, w, x, out, status, partial, k, m, n, a.row_bytes, plan.tok, a.waves, a.dealt, a.dealers, a.nt, plan.cluster,
+        GemmTs g = {ty, xdt, odt, sms, w, x, out, status, partial, k, m, n, a.row_bytes, plan.tok, a.waves, a.dealt, a.dealers, a.nt, plan.cluster, plan.chains,
                     gather ? go.nout : 0u, go.out_ld, go.out_row0, {}, go.epoch, go.epoch_inc};
         for (uint32_t r = 0; r < go.nout; r++) g.outs[r] = go.outs[r];
         e = launch_gemm_ts(g, s, dev);

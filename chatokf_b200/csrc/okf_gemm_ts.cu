@@ -67,6 +67,7 @@ struct TsArgs {
     uint32_t tma_log;  // weights by TMA, 2^tma_log rows to a row of the tensor map; kTsNoTma: by cp.async
     uint32_t odt;      // DT_F32, DT_BF16
     uint32_t cluster;  // CTAs that share an item along K (<= 1: none)
+    uint32_t chains;   // shared items: accumulators that take k-blocks in turn (1, 2 or 4)
     uint32_t vec;      // shared items: rows of results start on 16 (bf16: 8) bytes
     uint32_t nout, out_ld, out_row0;  // row shards: fp32 into every rank's whole output (nout > 0)
     void *outs[8];
@@ -480,6 +481,8 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t two_acc = p.tok <= 128 ? 1u : 0u;  // room for two accumulators
+    // (a CTA of a cluster has five k-blocks at least, two units but for the last one's end: every accumulator gets one)
+    const uint32_t chains = CL ? p.chains : 1, chain_cols = 256 / chains;
 
     TsWork wk;
     if (warp < kTsUnpackWarps) {
@@ -638,11 +641,13 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
 #pragma unroll 1
                     for (; kb < end; kb++, db += tile >> 4) {
                         const uint32_t a = tmem_base + kTsACol + set * kTsACols + (kb - 4 * u) * 32;
+                        const uint32_t dc = CL ? d + ((kb - wk.kb0) & (chains - 1)) * chain_cols : d;
+                        const bool begun = CL ? kb - wk.kb0 >= chains : kb != wk.kb0;
                         if (elect_one()) {
 #pragma unroll
                             for (uint32_t k4 = 0; k4 < kBK / 16; k4++)
                                 // 16 k: eight columns of A, 32 bytes further along B's swizzled 128-byte row
-                                umma_ts(d, a + k4 * 8, db + k4 * 2, idesc, (kb != wk.kb0 || k4 != 0) ? 1u : 0u);
+                                umma_ts(dc, a + k4 * 8, db + k4 * 2, idesc, (begun || k4 != 0) ? 1u : 0u);
                         }
                         __syncwarp();
                     }
@@ -679,6 +684,14 @@ __global__ void __launch_bounds__(kTsThreads, 1) gemm_ts_kernel(const __grid_con
 #pragma unroll
                     for (uint32_t i = 0; i < 32; i++)
                         if (i < live) sts32(o + i * (kBM * 4), r[i]);
+#pragma unroll 1
+                    for (uint32_t c = 1; c < chains; c++) {  // a thread's own words
+                        tmem_ld32(tmem_base + ((q * 32) << 16) + c * chain_cols + (t0 - wk.n0), r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (uint32_t i = 0; i < 32; i++)
+                            if (i < live) sts32(o + i * (kBM * 4), __float_as_uint(__uint_as_float(lds32(o + i * (kBM * 4))) + __uint_as_float(r[i])));
+                    }
                 } else if (part) {
                     float *o = part + (size_t)(t0 - wk.n0) * kBM;
 #pragma unroll
@@ -840,6 +853,7 @@ cudaError_t launch_gemm_ts(const GemmTs &g, cudaStream_t s, int dev) {
     a.waves = g.waves; a.dealt = g.dealt; a.dealers = g.dealers; a.nt = g.nt;
     a.odt = (uint32_t)g.odt;
     a.cluster = g.cluster;
+    a.chains = g.chains;
     a.vec = g.m % 4 == 0 && (g.nout ? (g.out_ld | g.out_row0) % 4 == 0 : (uintptr_t)g.out % (g.odt == DT_F32 ? 16 : 8) == 0);
     for (uint32_t i = 0; i < g.nout; i++) a.vec = a.vec && (uintptr_t)g.outs[i] % 16 == 0;
     a.nout = g.nout; a.out_ld = g.out_ld; a.out_row0 = g.out_row0; a.epoch = g.epoch; a.epoch_inc = g.epoch_inc;

@@ -15,7 +15,7 @@ struct GemmTs {
     uint32_t k, m, n, row_bytes;
     uint32_t tok;                        // tokens of an item, a multiple of 16, at most 256
     uint32_t waves, dealt, dealers, nt;  // how items are laid over the SMs
-    uint32_t cluster;                    // CTAs that share an item along K (0, 1: none)
+    uint32_t cluster, chains;            // CTAs that share an item along K (0, 1: none), accumulators each (1, 2, 4)
     uint32_t nout, out_ld, out_row0;     // row shards: fp32 into `nout` whole outputs
     void *outs[8];
     uint32_t *epoch;
