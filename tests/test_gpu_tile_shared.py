@@ -13,7 +13,8 @@ from chatokf_b200.gguf_types import GGUFType, block_elems, row_byte_count
 pytestmark = pytest.mark.gpu
 
 # k, m, n: few enough 128-row items for clusters of 2 (74 of them) to 8 (15)
-SHAPES = [(1280, 4000, 20), (1600, 5000, 33), (2112, 3001, 16), (4096, 1500, 34), (4672, 130, 97), (8192, 1023, 9), (2816, 515, 240), (6144, 2048, 500), (17408, 258, 70)]
+SHAPES = [(1280, 4000, 20), (1600, 5000, 33), (2112, 3001, 16), (4096, 1500, 34), (4672, 130, 97), (8192, 1023, 9), (2816, 515, 240), (6144, 2048, 500), (17408, 258, 70),
+          (8960, 8385, 19), (9984, 295, 1020)]
 
 
 @pytest.mark.parametrize("ty", list(GGUFType))
