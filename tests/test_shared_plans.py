@@ -1,5 +1,5 @@
-"""Plans of prefill matmuls with clusters, on the host: no partial tiles, no more clusters than there is room for, units for every CTA, k-blocks for every accumulator, and a
-search without room for any finds what it found before there were clusters."""
+"""Plans of prefill matmuls with clusters, on the host: no partial tiles, no more clusters than there is room for, units for every CTA, k-blocks for every accumulator, no longer
+chains of sums, and a search without room for any finds what it found before there were clusters."""
 import subprocess
 
 from chatokf_b200 import build
@@ -25,6 +25,9 @@ int main() {
         bad += p.tok == 0 || p.tok % 16 || p.tok > 256 || p.dealt || p.waves || p.floats || items > room[p.cluster] || units < 2 * p.cluster || xdt == DT_F32;
         const uint32_t last = units / p.cluster * 4 - 3;  // k-blocks of the shortest part at least: every accumulator gets one
         bad += (p.chains != 1 && p.chains != 2 && p.chains != 4) || p.chains * p.tok > 256 || last < p.chains;
+        // no longer chains of sums than without clusters (sums in tensor memory are cut off where fp32 would round)
+        const double chain = r.dealt && !r.waves ? (double)r.dealt * units / r.dealers : units;
+        bad += (units + p.cluster - 1) / p.cluster > p.chains * (chain < 1 ? 1 : chain);
         accs |= p.chains;
         sizes |= 1u << p.cluster;
     }
