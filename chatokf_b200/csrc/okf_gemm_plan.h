@@ -86,6 +86,13 @@ inline void lay_out(GemmPlan plan, uint32_t slabs, uint32_t steps, uint32_t n, u
 // is 0.8 % slower than the better one on average (never counting the 1.5 us; 5 % if they are counted against dealt items too).  Dealt or whole, and shared, us:
 // Q5_K 9728 -> 2560, 77 tokens, 19.8 and 17.6; Q2_0 6144 -> 2048, 512 tokens, 22.6 and 19.5; Q4_K 4608 -> 403, 256 tokens, 12.1 and 8.6; IQ4_NL
 // 3840 -> 1307, 13 tokens, 11.9 and 6.1; whole items that stay whole: Q4_K 1792 -> 1840, 158 tokens, 7.9 and 8.4.
+// Clusters of three and five, whose CTAs share a pair of SMs with another cluster's, do not take the last sixteenth of the room, and those of two that would take
+// whole items' place not all of it: while SMs fall free one by one, behind a kernel of some other grid (the one that converts x, an elementwise one),
+// the last clusters find no SMs side by side and start in a second wave (43 to 45 clusters of three, 80 shapes: 17 % slower than without behind an elementwise
+// kernel, up to 1.8 times, Q4_K 6912 -> 526, 794 tokens of fp32, 23.7 and 30.4; 39 to 42 of them 4 % faster.  Clusters of five 2 % slower and 8 % faster;
+// all the room taken by 49 grids of four, six, seven and eight CTAs 8 to 15 % faster).
+// Whole items of fewer than eight units are shared by three CTAs or more where a seventh of the room is left: 32 shapes 8 to 17 % faster; by two CTAs, or
+// with less room left, 54 shapes 1 % faster to 8 % slower (Q6_K 1536 -> 2774, 259 tokens, 10.4 and 12.5).
 // Q4_0 does not share: the tests of dealt items, of partial tiles and of their memory are written with it and count its kernels (4096 -> 1500, 34
 // tokens, 13.6 us instead of 9.0).
 // Sums in tensor memory are cut off where fp32 would round, so a chain's error grows with its length.  `base`: units of a chain of the plan without
@@ -94,18 +101,19 @@ inline void lay_out(GemmPlan plan, uint32_t slabs, uint32_t steps, uint32_t n, u
 // errors against 64 bits: the 303 that share are 0.74 of the plans without clusters on average, at most 1.04 times (chains a quarter longer
 // let through: 0.84 and 1.35).  One more accumulator costs 0.3 us at 77 tokens; 260 shapes are 0.5 % slower on average than with longer chains.
 inline void share_out(GemmPlan plan, uint32_t slabs, uint32_t units, uint32_t n, uint32_t tok, double t_unit, double t_item, double base, const uint32_t *room,
-                      GemmPlan &best, double &best_t) {
+                      bool whole, GemmPlan &best, double &best_t) {
     const uint32_t items = slabs * ((n + tok - 1) / tok);
-    const double whole = best.dealt || best.cluster ? 0 : 1.5e-6;
     for (uint32_t c = 2; c <= 8; c++) {
-        if (items > room[c] || units < 2 * c) continue;
+        const uint32_t places = c == 3 || c == 5 ? room[c] * 15 / 16 : c == 2 && whole && room[c] ? room[c] - 1 : room[c];
+        if (items > places || units < 2 * c) continue;
+        if (whole && units < 8 && (c == 2 || items > room[c] * 6 / 7)) continue;
         const uint32_t most = tok <= 64 ? 4 : tok <= 128 ? 2 : 1;
         const double part = (units + c - 1) / c;
         uint32_t chains = 1;
         while (chains < most && part > chains * base) chains *= 2;
         if (part > chains * base) continue;
         const double t = (units + c - 1) / c * t_unit + t_item + 2e-6 + (n < tok ? n : tok) * 5e-9;
-        if (t + (best.cluster ? 0 : whole) < best_t) { best_t = t; best = plan; best.cluster = c; best.chains = chains; }
+        if (t + (whole && !best.cluster ? 1.5e-6 : 0) < best_t) { best_t = t; best = plan; best.cluster = c; best.chains = chains; }
     }
 }
 // 16-bit activations: seconds per k-block of an item of `tok` tokens on the kernel with weights in tensor memory.  Up to
@@ -144,11 +152,12 @@ inline GemmPlan gemm_tc_search(int ty, uint32_t k, uint32_t m, uint32_t n, int x
     if (!room || ty == T_Q4_0) return best;
     const uint32_t units = (kblocks + 3) / 4;
     const double run = best.dealt && !best.waves ? (double)best.dealt * units / best.dealers : units, base = run < 1 ? 1 : run;
+    const bool whole = !best.dealt;
     for (uint32_t blocks = least; blocks <= least + 8; blocks++) {
         const uint32_t tok = ((n + blocks - 1) / blocks + 15) / 16 * 16;
         plan = {};
         plan.tok = tok;
-        share_out(plan, slabs, units, n, tok, 4 * ts_kblock(ty, tok), tok > 128 ? 2.5e-6 : 1e-6, base, room, best, best_t);
+        share_out(plan, slabs, units, n, tok, 4 * ts_kblock(ty, tok), tok > 128 ? 2.5e-6 : 1e-6, base, room, whole, best, best_t);
         if (tok <= 32) break;
     }
     return best;

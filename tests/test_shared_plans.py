@@ -28,6 +28,9 @@ int main() {
         // no longer chains of sums than without clusters (sums in tensor memory are cut off where fp32 would round)
         const double chain = r.dealt && !r.waves ? (double)r.dealt * units / r.dealers : units;
         bad += (units + p.cluster - 1) / p.cluster > p.chains * (chain < 1 ? 1 : chain);
+        // clusters of three and five leave room: the last ones of a full wave start late
+        bad += (p.cluster == 3 || p.cluster == 5) && items * 16 > room[p.cluster] * 15;
+        bad += !r.dealt && ((units < 8 && (p.cluster == 2 || items * 7 > room[p.cluster] * 6)) || (p.cluster == 2 && items == room[2]));
         accs |= p.chains;
         sizes |= 1u << p.cluster;
     }
