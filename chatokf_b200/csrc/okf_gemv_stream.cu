@@ -333,7 +333,7 @@ static cudaError_t stream_go(const GemvArgs &a, const StreamPlan &p, cudaStream_
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    return launch_pdl(stream_kernel<TY, MODE, XDT, NW>, p.ctas, NW * 32, p.smem, s, 1u << p.L.clog, a, p.L);
+    return launch_kernel(p.early, stream_kernel<TY, MODE, XDT, NW>, p.ctas, NW * 32, p.smem, s, 1u << p.L.clog, a, p.L);
 }
 template <int TY, int MODE, int XDT>
 static cudaError_t stream_warps(const GemvArgs &a, const StreamPlan &p, cudaStream_t s, int dev) {

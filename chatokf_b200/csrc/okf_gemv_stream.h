@@ -52,7 +52,7 @@ struct StreamRoom {
     uint32_t one[4], two[4];
 };
 struct StreamPlan {
-    bool ok;
+    bool ok, early;  // early: may start beside its predecessor
     uint32_t warps, ctas, smem;
     float us;  // estimated
     StreamLayout L;
@@ -66,6 +66,13 @@ constexpr uint32_t stream_budget(uint32_t warps) { return warps == 8 ? 112 * 102
 // matvecs alone 1 %, 6 % the other way for grids of exactly as many CTAs as SMs).  IQ2_XXS's CTAs fill 48 KB of tables first, which they can
 // do beside their predecessors: alone 5 % slower there and 5 % faster behind elementwise kernels, so without clusters they are left.
 constexpr uint32_t kStreamAlone = 116 * 1024;
+
+// Clusters of four and eight at two CTAs to an SM, all the device has room for, need every SM: beside a predecessor that still holds some (a small kernel holds
+// registers) clusters that lie across them wait, and what they leave free does not hold a cluster either, so some start when others end, half as long again
+// (IQ2_XXS 24320 -> 28385, 4 columns, behind an elementwise kernel 201.7 us, 138.5 when it starts behind it; in a chain of matvecs 131.8 and
+// 134.4).  From this estimate on they start when their predecessor is complete: 61 shapes 0.693 of the other kernel's time over three kinds of chain, 0.702
+// if all start early, 0.722 if none does; below it the 3 us that an early start hides weigh more.
+constexpr float kStreamLate = 22.f;
 
 template <int TY, int MODE>
 inline bool stream_layout(uint32_t nunit, uint32_t n, uint32_t clog, uint32_t clusters, uint32_t tiles, uint32_t warps, StreamPlan &p) {
@@ -177,6 +184,7 @@ inline StreamPlan stream_search(uint32_t nunit, uint32_t n, uint32_t tiles, cons
             if (!stream_layout<TY, MODE>(nunit, n, clog, clusters, tiles, warps, p)) continue;
             p.us = stream_us(TY, MODE, nunit, n, tiles, clog, clusters, warps, room.one[0], floor_us);
             p.ok = true;
+            p.early = clog < 2 || p.ctas <= room.one[0] || p.us < kStreamLate;
             if (warps == 8 && p.ctas <= room.one[0] && p.smem < kStreamAlone && (TY != T_IQ2_XXS || clog)) p.smem = kStreamAlone;
             if (!best.ok || p.us < best.us) best = p;
         }

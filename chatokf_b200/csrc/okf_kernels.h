@@ -11,10 +11,10 @@ namespace okf {
 // stream is finishing, and has to call pdl_wait() before it touches anything another kernel writes
 // or reads.  A chain stays in order as long as every kernel of it does: one that has passed its
 // wait knows that everything before its predecessor is complete.  `cluster` > 1 adds a cluster of
-// that many CTAs along x.
+// that many CTAs along x.  Not `early`: the kernel starts when its predecessor is complete, like any other.
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, unsigned cluster,
-                              A... args) {
+inline cudaError_t launch_kernel(bool early, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, unsigned cluster,
+                                 A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -22,13 +22,18 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned bloc
     cfg.stream = s;
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[0].val.programmaticStreamSerializationAllowed = early;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = cluster;
     at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, unsigned cluster,
+                              A... args) {
+    return launch_kernel(true, kernel, grid, block, smem, s, cluster, args...);
 }
 
 // Copy n16 16-byte words from mapped host memory to the device (the host twins' x).

@@ -46,6 +46,7 @@ template <uint32_t NW> static unsigned wrong(uint32_t tiles, uint32_t units) {
     }
     return bad;
 }
+static unsigned late = 0;
 template <int TY, int MODE> static unsigned plans(std::mt19937 &rng, unsigned &found) {
     unsigned bad = 0;
     const StreamRoom room = {{148, 74, 33, 15}, {296, 148, 71, 33}}, none = {{148, 0, 0, 0}, {296, 0, 0, 0}};
@@ -55,6 +56,9 @@ template <int TY, int MODE> static unsigned plans(std::mt19937 &rng, unsigned &f
         const StreamPlan p = stream_search<TY, MODE>(nunit, n, tiles, i & 1 ? room : none);
         if (!p.ok) continue;
         found++;
+        // grids that take every SM in clusters of four and eight, and last, wait for their predecessors; nothing else does
+        bad += p.early != !(p.ctas > 148 && p.L.clog >= 2 && p.us >= 22);
+        late += !p.early;
         const StreamLayout &L = p.L;
         const uint32_t size = 1u << L.clog, clusters = p.ctas / size, units = (nunit + size - 1) / size, per = (tiles + clusters - 1) / clusters;
         const uint32_t panel = (MODE == M_SEP ? 2 : n * mode_bytes(MODE)) * L.es, records = MODE == M_SEP ? 256 : units * n * wide_info_words(TY, mode_bytes(MODE)) * 4;
@@ -80,7 +84,7 @@ int main() {
     bad += plans<T_Q4_K, M_SEP>(rng, found) + plans<T_Q4_K, M_W1>(rng, found) + plans<T_Q4_K, M_W2>(rng, found);
     bad += plans<T_Q6_K, M_SEP>(rng, found) + plans<T_Q8_0, M_W2>(rng, found) + plans<T_Q8_0, M_R4>(rng, found) + plans<T_Q2_0, M_R3>(rng, found);
     bad += plans<T_IQ2_XXS, M_SEP>(rng, found) + plans<T_IQ2_XXS, M_W1>(rng, found) + plans<T_IQ2_XXS, M_W2>(rng, found);
-    printf("%u %u\n", bad, found);
+    printf("%u %u %u\n", bad, found, late);
 }
 """
 
@@ -95,8 +99,8 @@ def model(tmp_path_factory):
 
 
 def test_units_and_plans(model):
-    bad, found = map(int, subprocess.run([str(model)], check=True, capture_output=True, text=True).stdout.split())
-    assert bad == 0 and found > 20000
+    bad, found, late = map(int, subprocess.run([str(model)], check=True, capture_output=True, text=True).stdout.split())
+    assert bad == 0 and found > 20000 and late > 100
 
 
 def test_results_of_other_kernels_are_not_read_through_the_read_only_path():
