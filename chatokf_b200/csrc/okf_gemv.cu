@@ -609,7 +609,8 @@ cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, co
         }
         a.n = take;
         cudaError_t e;
-        if (gather || !launch_gemv_stream(ty, mode, a, xdt, s, sms, dev, ring_estimate(ty, mode, a, sms), e)) switch (ty) {
+        int count = gather ? 0 : launch_gemv_stream(ty, mode, a, xdt, s, sms, dev, ring_estimate(ty, mode, a, sms), e);
+        if (!count) switch (count = 1, ty) {
         case T_Q4_K: e = launch_ty<T_Q4_K>(a, G, mode, xdt, s, sms, dev); break;
         case T_Q8_0: e = launch_ty<T_Q8_0>(a, G, mode, xdt, s, sms, dev); break;
         case T_Q4_0: e = launch_ty<T_Q4_0>(a, G, mode, xdt, s, sms, dev); break;
@@ -621,7 +622,7 @@ cudaError_t launch_gemv_group(int ty, uint32_t nseg, const uint8_t *const *w, co
         default: e = cudaErrorInvalidValue;
         }
         if (e != cudaSuccess) return e;
-        if (launches) ++*launches;
+        if (launches) *launches += (uint64_t)count;
         if (gather) {  // a further pass over columns announces this pass's exchange and waits for it
             G.wait_arrivals = gather->arrivals[gather->rank];
             G.wait_epoch = gather->epoch;

@@ -245,7 +245,8 @@ inline uint32_t gemv_ctas(int ty, uint32_t row_bytes, uint32_t tiles, int sms, b
 // cost time (Q4_K 9728 -> 2560 7.1 -> 7.9), except for long rows with some more tiles than two to an SM: tiles halved between two CTAs
 // spread evenly over the chip, whole ones leave most CTAs one and a few of them two (Q4_K 17408 -> 5120 21.3 -> 16.9 us, Q8_0 32.7 ->
 // 24.6; Q8_0 5120 -> 5120, 20 units of 272 bytes, 8.8 -> 9.5, Q4_K 9216 -> 5120, 36 of 144, 10.3 -> 10.8; the line lies somewhere
-// between these points).  Several columns of rows that would need a cluster are okf_gemv_stream.cu's; row-shard launches have duties by CTA
+// between these points).  Several columns of rows that would need a cluster are okf_gemv_stream.cu's, in as many launches as that takes (rows of
+// Q8_0 and Q4_0 that end inside a unit come here: 7904 -> 59634, 5 columns, 258 us in clusters, 245 without); row-shard launches have duties by CTA
 // number and take none.
 inline bool gemv_plan(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, int mode, uint32_t tiles, int sms, bool gather, GemvArgs &a,
                       GemvLayout &L, uint32_t &ctas) {

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) stream_kernel(const __grid_c
     const uint32_t smem32 = smem_u32(smem);
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, g = lane >> 2, c = lane & 3;
     const uint32_t clog = L.clog, rank = blockIdx.x & ((1u << clog) - 1), cid = blockIdx.x >> clog;
-    const uint32_t t0 = cid * L.tiles_each + min(cid, L.tiles_more), ntl = L.tiles_each + (cid < L.tiles_more ? 1u : 0u);
+    const uint32_t t0 = L.tile_first + cid * L.tiles_each + min(cid, L.tiles_more), ntl = L.tiles_each + (cid < L.tiles_more ? 1u : 0u);
     const uint32_t ubeg = p.nunit * rank >> clog, nun = (p.nunit * (rank + 1) >> clog) - ubeg;
     // this warp's units of the CTA's tiles laid end to end
     const StreamSplit split(ntl, nun, nun == p.nunit >> clog ? L.unit_inv : L.unit_inv_more);
@@ -326,20 +326,29 @@ static bool stream_room(int dev, int sms, StreamRoom &room) {
 }
 
 template <int TY, int MODE, int XDT, uint32_t NW>
-static cudaError_t stream_go(const GemvArgs &a, const StreamPlan &p, cudaStream_t s, int dev) {
+static cudaError_t stream_go(const GemvArgs &a, const StreamPlan &p, const StreamLayout &L, uint32_t ctas, cudaStream_t s, int dev) {
     static bool attr_set[64] = {};  // the opt-in is per device
     if (!attr_set[dev]) {
         cudaError_t e = cudaFuncSetAttribute(stream_kernel<TY, MODE, XDT, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, NW == 8 ? kStreamAlone : stream_budget(NW));
         if (e != cudaSuccess) return e;
         attr_set[dev] = true;
     }
-    return launch_kernel(p.early, stream_kernel<TY, MODE, XDT, NW>, p.ctas, NW * 32, p.smem, s, 1u << p.L.clog, a, p.L);
+    return launch_kernel(p.early, stream_kernel<TY, MODE, XDT, NW>, ctas, NW * 32, p.smem, s, 1u << L.clog, a, L);
 }
 template <int TY, int MODE, int XDT>
 static cudaError_t stream_warps(const GemvArgs &a, const StreamPlan &p, cudaStream_t s, int dev) {
-    if constexpr (MODE == M_W2)
-        if (p.warps == 16) return stream_go<TY, MODE, XDT, 16>(a, p, s, dev);
-    return stream_go<TY, MODE, XDT, 8>(a, p, s, dev);
+    StreamLayout L = p.L;
+    for (uint32_t first = 0; first < a.tiles; first += p.tiles) {
+        const uint32_t tiles = a.tiles - first < p.tiles ? a.tiles - first : p.tiles, all = p.ctas >> L.clog, clusters = tiles < all ? tiles : all;
+        L.deal(first, tiles, clusters);
+        cudaError_t e;
+        if constexpr (MODE == M_W2)
+            e = p.warps == 16 ? stream_go<TY, MODE, XDT, 16>(a, p, L, clusters << L.clog, s, dev) : stream_go<TY, MODE, XDT, 8>(a, p, L, clusters << L.clog, s, dev);
+        else
+            e = stream_go<TY, MODE, XDT, 8>(a, p, L, clusters << L.clog, s, dev);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 template <int TY, int MODE>
 static int stream_launch(const GemvArgs &a, int xdt, const StreamRoom &room, cudaStream_t s, int dev, float other_us, cudaError_t &e) {
@@ -350,7 +359,7 @@ static int stream_launch(const GemvArgs &a, int xdt, const StreamRoom &room, cud
     else if (xdt == DT_F16) e = stream_warps<TY, MODE, DT_F16>(a, p, s, dev);
     else if (xdt == DT_BF16) e = stream_warps<TY, MODE, DT_BF16>(a, p, s, dev);
     else e = stream_warps<TY, MODE, DT_F32>(a, p, s, dev);
-    return 1;
+    return (int)((a.tiles + p.tiles - 1) / p.tiles);
 }
 template <int TY>
 static int stream_ty(int mode, const GemvArgs &a, int xdt, const StreamRoom &room, cudaStream_t s, int dev, float other_us, cudaError_t &e) {

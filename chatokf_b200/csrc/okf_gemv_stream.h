@@ -27,7 +27,13 @@ struct StreamLayout {
     uint32_t depth;       // stages of a warp's ring: 2 to 4
     uint32_t xs_off, info_off, slot_off, part_off, tab_off;  // byte offsets in dynamic shared memory
     uint32_t tab_copies;  // IQ2_XXS: copies of every entry of the look-up tables, side by side
+    uint32_t tile_first;                 // of this launch
     uint32_t tiles_each, tiles_more;     // tiles of a cluster; the first tiles_more clusters have one more
+    __host__ __device__ void deal(uint32_t first, uint32_t tiles, uint32_t clusters) {
+        tile_first = first;
+        tiles_each = tiles / clusters;
+        tiles_more = tiles % clusters;
+    }
     uint32_t unit_inv, unit_inv_more;    // v / units = v * inv >> 31, for CTAs with nunit >> clog units of a row and with one more
     uint32_t nc_inv;                     // v / nc = v * nc_inv >> 16, v < 8192
 };
@@ -54,7 +60,8 @@ struct StreamRoom {
 struct StreamPlan {
     bool ok, early;  // early: may start beside its predecessor
     uint32_t warps, ctas, smem;
-    float us;  // estimated
+    uint32_t tiles;  // of a launch: all, or (see stream_search) the launches of a matrix take that many each, the last one what is left
+    float us;  // estimated, of all launches
     StreamLayout L;
 };
 // (two of 112 KB leave 2 KB of an SM: enough for the small kernels between matvecs, which with 1 KB less take 0.8 us longer each)
@@ -101,8 +108,7 @@ inline bool stream_layout(uint32_t nunit, uint32_t n, uint32_t clog, uint32_t cl
     }
     p.warps = warps;
     p.ctas = clusters << clog;
-    L.tiles_each = tiles / clusters;
-    L.tiles_more = tiles % clusters;
+    L.deal(0, tiles, clusters);
     L.unit_inv = stream_inv(nunit >> clog);
     L.unit_inv_more = stream_inv((nunit >> clog) + 1);
     L.nc_inv = 65536 / n + 1;
@@ -170,7 +176,7 @@ inline float ring_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tile
 }
 
 template <int TY, int MODE>
-inline StreamPlan stream_search(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room) {
+inline StreamPlan stream_search_one(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room) {
     StreamPlan best = {};
     const float floor_us = (float)nunit * (float)tiles * (16.f * UnitGeom<TY>::bytes / 4.9e6f);
     for (uint32_t clog = 0; clog < 4 && (clog == 0 || nunit >= 2u << clog); clog++) {
@@ -184,10 +190,30 @@ inline StreamPlan stream_search(uint32_t nunit, uint32_t n, uint32_t tiles, cons
             if (!stream_layout<TY, MODE>(nunit, n, clog, clusters, tiles, warps, p)) continue;
             p.us = stream_us(TY, MODE, nunit, n, tiles, clog, clusters, warps, room.one[0], floor_us);
             p.ok = true;
+            p.tiles = tiles;
             p.early = clog < 2 || p.ctas <= room.one[0] || p.us < kStreamLate;
             if (warps == 8 && p.ctas <= room.one[0] && p.smem < kStreamAlone && (TY != T_IQ2_XXS || clog)) p.smem = kStreamAlone;
             if (!best.ok || p.us < best.us) best = p;
         }
+    }
+    return best;
+}
+
+// Where no split fits (tall matrices of long rows at several columns: in clusters, which x needs, a CTA keeps the sums of all its cluster's tiles) the tiles are
+// dealt to several launches, each with room for its own: as few as fit, or up to twice as many if they are estimated to be better.  Such matrices went to the other
+// kernel, which stages x anew for every few tiles: 82 shapes of all types, 2 to 8 columns, take 0.55 of its time (IQ2_XXS 23040 -> 64269, 8 columns, 802 -> 292 us, Q8_0
+// 5376 -> 80310, 8, 127 -> 110; that kernel in clusters, with all of x, 697 and 341).  Not rows of Q8_0 and Q4_0 that end inside a unit, whose x of three and four bytes
+// leaves rings of two stages (Q8_0 7904 -> 59634, 5 columns, 245 and 294).
+template <int TY, int MODE>
+inline StreamPlan stream_search(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room) {
+    StreamPlan best = stream_search_one<TY, MODE>(nunit, n, tiles, room);
+    if (best.ok || (WideMode<MODE>::rag && (TY == T_Q8_0 || TY == T_Q4_0))) return best;
+    for (uint32_t parts = 2, most = 64; parts <= most && parts <= tiles; parts++) {
+        StreamPlan p = stream_search_one<TY, MODE>(nunit, n, (tiles + parts - 1) / parts, room);
+        if (!p.ok) continue;
+        if (!best.ok) most = 2 * parts;
+        p.us *= (float)parts;
+        if (!best.ok || p.us < best.us) best = p;
     }
     return best;
 }
@@ -209,7 +235,7 @@ inline const StreamPlan &stream_plan(uint32_t nunit, uint32_t n, uint32_t tiles,
     return e.p;
 }
 
-// Whether a launch took this kernel; 0: it is not one for it (or does not fit), and nothing was launched.
+// How many launches of this kernel took the matvec; 0: it is not one for it (or does not fit), and nothing was launched.
 struct GemvArgs;
 int launch_gemv_stream(int ty, int mode, const GemvArgs &a, int xdt, cudaStream_t s, int sms, int dev, float other_us, cudaError_t &e);
 

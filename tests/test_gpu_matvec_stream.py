@@ -82,3 +82,39 @@ def test_no_bytes_behind_the_last_block_are_taken_for_weights(ctx, n):
         torch.cuda.synchronize()
         assert rel_err(out.cpu().numpy(), want.cpu().numpy()) <= 1e-4, ty
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("ty,k,rows,n", [(GGUFType.Q8_0, 105 * 256, [3000, 1483], 8), (GGUFType.Q8_0, 105 * 256, [17270], 4), (GGUFType.IQ2_XXS, 89 * 256, [40990], 8),
+                                         (GGUFType.IQ4_NL, 105 * 256 - 32, [9200], 4)])
+def test_tiles_of_several_launches(ctx, ty, k, rows, n):
+    """Matrices so tall that the sums of a cluster's tiles do not fit beside x: two launches, the border between them inside a matrix."""
+    pool = torch.from_numpy(synth.random_blocks(ty, 4096, np.random.default_rng(k)).reshape(4096, -1)).cuda()
+    gen = torch.Generator("cuda").manual_seed(n)
+    at, ts = 0, []
+    for m in rows:
+        ts.append(GGUFTensor("w", (k, m), ty, at))
+        at += (row_byte_count(ty, k) * m + 15) // 16 * 16
+    buf = torch.zeros(at + 256, dtype=torch.uint8, device="cuda")
+    for t in ts:
+        count = k // block_elems(ty) * t.M
+        buf[t.offset:t.offset + count * pool.shape[1]] = pool[torch.randint(0, 4096, (count,), device="cuda", generator=gen)].view(-1)
+    w, X, enc = ctx.wrap(buf, at), torch.randn(n, k, device="cuda", generator=gen), CudaEnc(ctx)
+    X = X.half() if k % 256 == 0 else X
+    want, got = [torch.empty(n * t.M, device="cuda") for t in ts], [torch.full((n * t.M + 4,), float("nan"), device="cuda") for t in ts]
+    ctx.set_flags(1)
+    try:
+        for t, o in zip(ts, want):
+            enc.gemm(t, X, o, w, n)
+    finally:
+        ctx.set_flags(0)
+    before = ctx.launches
+    with enc.parallel():
+        for t, o in zip(ts, got):
+            enc.gemm(t, X, o, w, n)
+    launched = ctx.launches - before
+    torch.cuda.synchronize()
+    assert launched >= 2 and ctx.device_status() == 0
+    for t, o, g in zip(ts, want, got):
+        assert torch.isnan(g[n * t.M:]).all()
+        # x carries 16 bits, as above (ragged rows: as it is)
+        assert rel_err(g[:n * t.M].cpu().numpy(), o.cpu().numpy()) <= 1e-4

@@ -51,11 +51,17 @@ template <int TY, int MODE> static unsigned plans(std::mt19937 &rng, unsigned &f
     unsigned bad = 0;
     const StreamRoom room = {{148, 74, 33, 15}, {296, 148, 71, 33}}, none = {{148, 0, 0, 0}, {296, 0, 0, 0}};
     for (int i = 0; i < 4000; i++) {
-        const uint32_t nunit = 1 + rng() % (i % 4 ? 72 : 600), tiles = 1 + rng() % (i % 3 ? 1200 : 20000);
+        const uint32_t nunit = 1 + rng() % (i % 4 ? 72 : 600), wanted = 1 + rng() % (i % 3 ? 1200 : 20000);
         const uint32_t n = MODE == M_SEP ? 1 : MODE == M_W2 ? 5 + rng() % 4 : 1 + rng() % 4;
-        const StreamPlan p = stream_search<TY, MODE>(nunit, n, tiles, i & 1 ? room : none);
+        const StreamPlan p = stream_search<TY, MODE>(nunit, n, wanted, i & 1 ? room : none);
         if (!p.ok) continue;
+        const uint32_t tiles = p.tiles;  // of a launch
+        bad += tiles == 0 || tiles > wanted;
         found++;
+        StreamLayout rest = p.L;  // the last launch takes what is left of the matrix, in as many clusters at most
+        const uint32_t left = wanted % tiles ? wanted % tiles : tiles, fit = left < p.ctas >> p.L.clog ? left : p.ctas >> p.L.clog;
+        rest.deal(wanted - left, left, fit);
+        bad += rest.tile_first + rest.tiles_each * fit + rest.tiles_more != wanted || rest.tiles_each > p.L.tiles_each || rest.tiles_each + !!rest.tiles_more > p.L.tiles_each + !!p.L.tiles_more;
         // grids that take every SM in clusters of four and eight, and last, wait for their predecessors; nothing else does
         bad += p.early != !(p.ctas > 148 && p.L.clog >= 2 && p.us >= 22);
         late += !p.early;
@@ -76,8 +82,18 @@ template <int TY, int MODE> static unsigned plans(std::mt19937 &rng, unsigned &f
     }
     return bad;
 }
+// whole rows of up to 112 units at two to eight columns: there is a plan, and it has all of x in shared memory
+template <int TY> static unsigned declined() {
+    const StreamRoom room = {{148, 74, 33, 15}, {296, 148, 71, 33}};
+    unsigned no = 0;
+    for (uint32_t nunit = 1; nunit <= 112; nunit++)
+        for (uint32_t tiles = 16; tiles <= 16384; tiles += tiles / 8)
+            for (uint32_t n = 2; n <= 8; n++) no += !(n <= 4 ? stream_search<TY, M_W1>(nunit, n, tiles, room) : stream_search<TY, M_W2>(nunit, n, tiles, room)).ok;
+    return no;
+}
 int main() {
     unsigned bad = 0, found = 0;
+    bad += declined<T_Q8_0>() + declined<T_Q4_K>() + declined<T_IQ2_XXS>() + declined<T_Q2_0>() + declined<T_Q4_0>() + declined<T_Q5_K>() + declined<T_Q6_K>() + declined<T_IQ4_NL>();
     for (uint32_t tiles = 1; tiles <= 40; tiles++)
         for (uint32_t units = 1; units <= 40; units++) bad += wrong<8>(tiles, units) + wrong<16>(tiles, units);
     std::mt19937 rng(3);
