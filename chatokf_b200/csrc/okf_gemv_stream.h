@@ -129,7 +129,7 @@ inline bool stream_layout(uint32_t nunit, uint32_t n, uint32_t clog, uint32_t cl
 inline int stream_kind(int mode) { return mode == M_SEP ? 0 : mode == M_W1 ? 1 : mode == M_W2 ? 2 : 3; }
 struct StreamUnit {
     float stream[4];  // one column, up to four, up to eight, rows that end inside a unit
-    float ring[4];    // the same of okf_gemv.cu's kernel
+    float ring[4];    // the same of okf_gemv.cu's kernel (not asked at five to eight)
 };
 inline StreamUnit stream_unit_us(int ty) {
     switch (ty) {
@@ -158,13 +158,11 @@ inline float stream_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t ti
 }
 // The same of okf_gemv.cu's kernel, whose CTAs share their tiles' units between eight warps; `ctas` and `clog` as it would take them.
 // It is asked where it may be the better one: at one column, where its bulk copies of whole rows reach 6.1 TB/s (Q4_K 5120 -> 65536 33.6
-// us, 39.2 here), and at up to four where an SM gets four tiles and more, to which x is staged once.  Up to eight columns are
-// better off here (Q4_K 2560 -> 9728 twice, 17.4 -> 12.3 us, 9728 -> 2560 19.7 -> 10.8), but for the shortest rows, where there is little to share
-// (1024 -> 828, IQ4_NL 3.9 and 4.3 us; Q4_K 1024 -> 4096 4.4 and 4.1).
+// us, 39.2 here), and at up to four where an SM gets four tiles and more, to which x is staged once.  Five to eight columns are better off here
+// (Q4_K 2560 -> 9728 twice, 17.4 -> 12.3 us, 9728 -> 2560 19.7 -> 10.8; of 240 shapes with rows of one to six units none is slower, 0.76 of the time on average).
 inline float ring_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tiles, uint32_t ctas, uint32_t clog, uint32_t sms) {
     const int kind = stream_kind(mode);
-    if (kind == 2) return nunit <= 6 && tiles <= 4 * sms && ty != T_Q4_K && ty != T_Q5_K ? 0.f : 1e30f;
-    if (kind != 0 && tiles < 4 * sms) return 1e30f;
+    if (kind == 2 || (kind != 0 && tiles < 4 * sms)) return 1e30f;
     constexpr float fixed[4] = {3.26f, 3.12f, 0.f, 4.65f}, pair_us[2] = {.9f, .77f}, shared_x[2] = {1.32f, 1.65f}, cluster_us[2] = {3.07f, 3.5f};
     const bool shared = ctas > (kind < 2 ? sms : sms + sms / 4);  // (up to a quarter more CTAs than SMs hardly slow each other down where rows end inside a unit)
     const uint32_t clusters = ctas >> clog, units = (nunit + (1u << clog) - 1) >> clog;

@@ -1,5 +1,5 @@
 """How a streaming matvec's units are dealt to warps, on the host: every unit of a CTA is in one warp's run, the parts of every tile that
-a border cuts are added up once and in order, and the divisions by multiplication are exact over what a plan may hold; every plan the search finds
+a border cuts are added up in order, every column once, and the divisions by multiplication are exact over what a plan may hold; every plan the search finds
 fits the shared memory that its kernel asks for."""
 import subprocess
 
@@ -32,13 +32,27 @@ template <uint32_t NW> static unsigned wrong(uint32_t tiles, uint32_t units) {
         }
     }
     bad += split.border<NW>(0) != 0 || split.border<NW>(NW) != tiles * units;
-    for (uint32_t w = 0; w + 1 < NW; w++) {
-        const uint32_t first = split.border<NW>(w), at = split.border<NW>(w + 1), tile = split.tile(at), lo = tile * units, hi = lo + units;
-        if (!(at < split.all && at > lo && first <= lo)) continue;
-        bad += !got[tile].empty();
-        got[tile] = slot[2 * w + (first < lo)];
-        for (uint32_t v = w + 1; v < NW && split.border<NW>(v) < hi; v++)
-            if (split.border<NW>(v + 1) > split.border<NW>(v)) got[tile].insert(got[tile].end(), slot[2 * v].begin(), slot[2 * v].end());
+    for (uint32_t nc : {1u, 3u, 8u}) {
+        std::vector<unsigned> taken(tiles * nc);  // how many warps add a column of a tile up
+        for (uint32_t w = 0; w + 1 < NW; w++) {
+            const uint32_t last = split.border<NW>(w + 1), tile = split.tile(last), lo = tile * units, hi = lo + units;
+            if (!(last < split.all && last > lo)) continue;
+            uint32_t w0 = w, w1 = w + 1;
+            while (split.border<NW>(w0) > lo) w0--;
+            while (w1 + 1 < NW && split.border<NW>(w1 + 1) < hi) w1++;
+            std::vector<uint32_t> sum = slot[2 * w0 + (split.border<NW>(w0) < lo)];
+            for (uint32_t v = w0 + 1; v <= w1; v++)
+                if (split.border<NW>(v + 1) > split.border<NW>(v)) sum.insert(sum.end(), slot[2 * v].begin(), slot[2 * v].end());
+            for (uint32_t half = 0; half < 2; half++)
+                for (uint32_t col = half + 2 * (w - w0); col < nc; col += 2 * (w1 - w0)) taken[tile * nc + col]++;
+            bad += !got[tile].empty() && got[tile] != sum;
+            got[tile] = sum;
+        }
+        for (uint32_t t = 0; t < tiles; t++) {
+            bool cut = false;
+            for (uint32_t w = 1; w < NW; w++) cut |= split.border<NW>(w) > t * units && split.border<NW>(w) < (t + 1) * units;
+            for (uint32_t c = 0; c < nc; c++) bad += taken[t * nc + c] != cut;
+        }
     }
     for (uint32_t t = 0; t < tiles; t++) {
         bad += got[t].size() != units;
