@@ -285,7 +285,8 @@ inline float ring_estimate(int ty, int mode, const GemvArgs &a, int sms) {
     uint32_t ctas;
     if (!gemv_plan(ty, a.row_bytes, a.nunit, a.n, mode, a.tiles, sms, false, t, L, ctas)) return 1e30f;
     // Several columns: x resident is not enough, copies have to be on their way as well (Q8_0 17408 -> 8192, 2 columns, with less than 44 KB
-    // of ring 88.4 us, shared by two CTAs 42.2).
+    // of ring 88.4 us, shared by two CTAs 42.2).  Asked of every plan: 27 shapes of two to four columns whose ring holds a CTA's whole share, or of two-bit
+    // types, that the estimates alone would leave here take 0.62 to 0.98 of this kernel's time on the other one.
     if (mode != M_SEP && (L.panel < t.nchunk || L.nstage * L.stage_bytes < 44 * 1024)) return 1e30f;
     return ring_us(ty, mode, a.nunit, a.n, a.tiles, ctas, L.clog, (uint32_t)sms);
 }
