@@ -14,6 +14,17 @@ from pathlib import Path
 LIB_PATH = Path(__file__).resolve().parent / "libokfcuda.so"
 CALL_PATH = LIB_PATH.with_name("_okfcall" + sysconfig.get_config_var("EXT_SUFFIX"))
 
+
+
+def tensor_path(torch) -> Path | None:
+    """The library that reads this torch's tensors without Python calls (csrc/okf_pytensor.cpp).  It has torch's object layouts compiled in, so
+    there is one a torch; None for a torch without CUDA."""
+    if torch is None or torch.version.cuda is None:
+        return None
+    commit = (torch.version.git_version or "")[:8]
+    return LIB_PATH.with_name(f"_okftensor-torch{torch.__version__}-{commit}" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
 OKF_OK = 0
 STATUS = {
     0: "OKF_OK", -1: "OKF_E_ARG", -2: "OKF_E_TYPE", -3: "OKF_E_SHAPE", -4: "OKF_E_RANGE",
@@ -169,8 +180,14 @@ class _Call:
         spec.loader.exec_module(mod)
         # a torch without CUDA lacks these two; nothing that needs a stream runs there
         dev, raw = (getattr(torch._C, n, None) for n in ("_cuda_getDevice", "_cuda_getCurrentRawStream"))
+        # nothing built for this torch: tensors are read by look-ups, 0.25 us a call slower
+        direct, path = None, tensor_path(torch)
+        if path is not None and path.exists():
+            T = ctypes.CDLL(str(path))
+            direct = tuple(ctypes.cast(getattr(T, n), ctypes.c_void_p).value
+                           for n in ("okf_tensor_address", "okf_tensor_dtype", "okf_current_stream"))
         mod.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in SIGNATURES},
-                 (torch.float32, torch.float16, torch.bfloat16), dev, raw)
+                 (torch.float32, torch.float16, torch.bfloat16), dev, raw, direct)
         for name in ("gemm", "gemv", "parallel_begin", "parallel_end", "dequant", "embed", "argmax", "norm", "silu",
                      "matmul_at", "matmul_host"):
             setattr(self, name, getattr(mod, name))

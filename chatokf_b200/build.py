@@ -6,7 +6,7 @@ The library links the CUDA runtime statically and exports only the C ABI of
 include/okf_cuda.h.  Objects go to chatokf_b200/csrc/build/ (git-ignored); the
 shared library sits beside this file so it travels with the package.  Beside it
 goes _okfcall, the C module through which Python calls the library's hot entry
-points; it is linked against torch, whose tensors it reads.
+points, and for a torch with CUDA a library that reads this very torch's tensors.
 """
 from __future__ import annotations
 
@@ -18,6 +18,8 @@ import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
+
+from ._lib import tensor_path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
@@ -55,33 +57,42 @@ def _stale(out: Path, src_mtime: float) -> bool:
     return not out.exists() or out.stat().st_mtime < max(src_mtime, _headers_mtime())
 
 
+def _torch():
+    try:
+        import torch
+    except ImportError:
+        return None
+    return torch
+
+
 def needs_build() -> bool:
-    return (_stale(LIB, max(p.stat().st_mtime for p in sources()))
-            or _stale(PYMOD, max(PYCALL.stat().st_mtime, PYTENSOR.stat().st_mtime)))
+    tensor = tensor_path(_torch())
+    return (_stale(LIB, max(p.stat().st_mtime for p in sources())) or _stale(PYMOD, PYCALL.stat().st_mtime)
+            or (tensor is not None and _stale(tensor, PYTENSOR.stat().st_mtime)))
 
 
-def build_pycall() -> None:
-    import torch
+def _run(cmd: list[str], what: str) -> None:
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError(f"building {what} failed")
 
+
+def build_pycall(force: bool = False) -> None:
+    flags = ["-O2", "-Wall", "-fPIC", "-shared", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"]]
+    _run([shutil.which("gcc") or "cc", *flags, str(PYCALL), "-o", str(PYMOD) + ".tmp"], PYMOD.name)
+    os.replace(str(PYMOD) + ".tmp", PYMOD)
+    torch = _torch()
+    out = tensor_path(torch)
+    if out is None or not (force or _stale(out, PYTENSOR.stat().st_mtime)):
+        return
     root = Path(torch.__file__).resolve().parent
     cuda = Path(nvcc()).resolve().parent.parent
-    inc = ["-I", sysconfig.get_paths()["include"]]
-    obj, tobj = OBJ / "okf_pycall.o", OBJ / "okf_pytensor.o"
-    tcmd = ["-I", str(root / "include"), "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-I", str(cuda / "include"),
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
-    flags = ["-O2", "-Wall", "-fPIC", "-fvisibility=hidden"]
+    inc = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include"]
     libs = ["-L" + str(root / "lib"), "-Wl,-rpath," + str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
-    cxx = shutil.which("g++") or "c++"
-    cmds = [[shutil.which("gcc") or "cc", *flags, *inc, "-c", str(PYCALL), "-o", str(obj)]]
-    if not tobj.exists() or _stale(tobj, max(PYTENSOR.stat().st_mtime, Path(torch.__file__).stat().st_mtime)):
-        cmds.append([cxx, *flags, "-std=c++17", *inc, *tcmd, "-c", str(PYTENSOR), "-o", str(tobj)])
-    cmds.append([cxx, "-shared", str(obj), str(tobj), *libs, "-o", str(PYMOD) + ".tmp"])
-    for cmd in cmds:
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode:
-            sys.stderr.write(r.stdout + r.stderr)
-            raise RuntimeError(f"building {PYMOD.name} failed")
-    os.replace(str(PYMOD) + ".tmp", PYMOD)
+    _run([shutil.which("g++") or "c++", *flags, "-std=c++17", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          *(a for i in inc for a in ("-I", str(i))), str(PYTENSOR), *libs, "-o", str(out) + ".tmp"], out.name)
+    os.replace(str(out) + ".tmp", out)
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -114,7 +125,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         sys.stderr.write(r.stdout + r.stderr)
         raise RuntimeError("link of libokfcuda.so failed")
     os.replace(tmp, LIB)
-    build_pycall()
+    build_pycall(force)
     return LIB
 
 

@@ -4,8 +4,9 @@
  * less time than the kernel before it runs.  Through ctypes, torch.cuda.current_stream() and the
  * properties of GGUFTensor a call cost 9 - 12 us on the host (a 16-bit two-bit trunk's layer,
  * seven calls and two regions, 69 us against 18 us on the GPU); here the arguments are read from
- * the objects in C, those of torch's from torch itself (okf_pytensor.cpp).  The functions return the okf_status; the callers turn it into an exception.
- * The library is resolved by address (bind), so this module links against nothing.
+ * the objects in C, those of torch's from torch itself where there is a module for it (okf_pytensor.cpp), else by method and
+ * attribute look-ups.  The functions return the okf_status; the callers turn it into an exception.
+ * The library and that module are resolved by address (bind), so this one links against nothing.
  */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -35,10 +36,10 @@ static PyObject *dt_f32, *dt_f16, *dt_bf16;         /* torch.float32, ... */
 static PyObject *get_device_p, *raw_stream_p;       /* torch._C._cuda_getDevice, _cuda_getCurrentRawStream */
 static PyObject *s_ctx, *s_addr, *s_stream, *s_cuda_stream, *s_type, *s_dims, *s_offset, *s_dtype, *s_data_ptr;
 
-/* okf_pytensor.cpp */
-int okf_tensor_address(PyObject *o, void **out);
-int okf_tensor_dtype(PyObject *o, int *out);
-int okf_current_stream(void **out);
+/* okf_pytensor.cpp's functions for the torch that is loaded, NULL: there are none */
+static int (*tensor_address_p)(PyObject *o, void **out);
+static int (*tensor_dtype_p)(PyObject *o, int *out);
+static int (*current_stream_p)(void **out);
 
 /* ---- reading the arguments --------------------------------------------------------------- */
 
@@ -76,7 +77,7 @@ static int ctx_of(PyObject *enc, okf_ctx **out) {
     return rc;
 }
 static int data_ptr(PyObject *t, void **out) {
-    if (okf_tensor_address(t, out)) return 0;
+    if (tensor_address_p && tensor_address_p(t, out)) return 0;
     PyObject *v = PyObject_CallMethodNoArgs(t, s_data_ptr);
     if (!v) return -1;
     uint64_t p;
@@ -86,7 +87,7 @@ static int data_ptr(PyObject *t, void **out) {
     return rc;
 }
 static int dtype_of(PyObject *t, int *out) {
-    if (okf_tensor_dtype(t, out)) return 0;
+    if (tensor_dtype_p && tensor_dtype_p(t, out)) return 0;
     PyObject *d = PyObject_GetAttr(t, s_dtype);
     if (!d) return -1;
     int rc = 0;
@@ -107,9 +108,10 @@ static int stream_of(PyObject *enc, okf_stream *out) {
     uint64_t v = 0;
     int rc;
     if (s == Py_None) {
-        Py_DECREF(s);
-        if (okf_current_stream(out)) return 0;
-        s = Py_NewRef(Py_None);
+        if (current_stream_p && current_stream_p(out)) {
+            Py_DECREF(s);
+            return 0;
+        }
         rc = -1;
         PyObject *dev = PyObject_CallNoArgs(get_device_p);
         if (dev) {
@@ -290,7 +292,7 @@ static PyObject *py_matmul_host(PyObject *self, PyObject *const *a, Py_ssize_t n
     return got;
 }
 
-/* bind(addresses: dict of name -> int, (float32, float16, bfloat16), get_device, raw_stream) */
+/* bind(addresses: dict of name -> int, (float32, float16, bfloat16), get_device, raw_stream, (okf_pytensor.cpp's three addresses) or None) */
 static int resolve(PyObject *d, const char *name, void *slot) {
     PyObject *v = PyDict_GetItemString(d, name);
     uint64_t p;
@@ -303,8 +305,10 @@ static int resolve(PyObject *d, const char *name, void *slot) {
     return 0;
 }
 static PyObject *py_bind(PyObject *self, PyObject *args) {
-    PyObject *d, *f32, *f16, *bf16, *dev, *raw;
-    if (!PyArg_ParseTuple(args, "O!(OOO)OO", &PyDict_Type, &d, &f32, &f16, &bf16, &dev, &raw)) return NULL;
+    PyObject *d, *f32, *f16, *bf16, *dev, *raw, *direct;
+    unsigned long long at[3] = {0, 0, 0};
+    if (!PyArg_ParseTuple(args, "O!(OOO)OOO", &PyDict_Type, &d, &f32, &f16, &bf16, &dev, &raw, &direct)) return NULL;
+    if (direct != Py_None && !PyArg_ParseTuple(direct, "KKK", &at[0], &at[1], &at[2])) return NULL;
     if (resolve(d, "okf_gemm", &gemm_fns[FN_GEMM]) || resolve(d, "okf_gemm_tile", &gemm_fns[FN_GEMM_TILE]) ||
         resolve(d, "okf_gemm_noalloc", &gemm_fns[FN_GEMM_NOALLOC]) || resolve(d, "okf_gemv", &gemv_p) ||
         resolve(d, "okf_parallel_begin", &parallel_begin_p) || resolve(d, "okf_parallel_end", &parallel_end_p) ||
@@ -317,6 +321,9 @@ static PyObject *py_bind(PyObject *self, PyObject *args) {
     dt_bf16 = Py_NewRef(bf16);
     get_device_p = Py_NewRef(dev);
     raw_stream_p = Py_NewRef(raw);
+    tensor_address_p = (int (*)(PyObject *, void **))(uintptr_t)at[0];
+    tensor_dtype_p = (int (*)(PyObject *, int *))(uintptr_t)at[1];
+    current_stream_p = (int (*)(void **))(uintptr_t)at[2];
     Py_RETURN_NONE;
 }
 
