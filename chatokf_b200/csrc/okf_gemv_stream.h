@@ -78,8 +78,8 @@ constexpr uint32_t kStreamAlone = 116 * 1024;
 // registers) clusters that lie across them wait, and what they leave free does not hold a cluster either, so some start when others end, half as long again
 // (IQ2_XXS 24320 -> 28385, 4 columns, behind an elementwise kernel 201.7 us, 138.5 when it starts behind it; in a chain of matvecs 131.8 and
 // 134.4).  From this estimate on they start when their predecessor is complete: 61 shapes 0.693 of the other kernel's time over three kinds of chain, 0.702
-// if all start early, 0.722 if none does; below it the 3 us that an early start hides weigh more.
-constexpr float kStreamLate = 22.f;
+// if all start early, 0.722 if none does; below it the 3 us that an early start hides weigh more (IQ2_XXS 17408 -> 5120, 4 columns, 19.8 and 22.4 in a chain of matvecs).
+constexpr float kStreamLate = 27.f;
 
 template <int TY, int MODE>
 inline bool stream_layout(uint32_t nunit, uint32_t n, uint32_t clog, uint32_t clusters, uint32_t tiles, uint32_t warps, StreamPlan &p) {

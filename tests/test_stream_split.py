@@ -77,7 +77,7 @@ template <int TY, int MODE> static unsigned plans(std::mt19937 &rng, unsigned &f
         rest.deal(wanted - left, left, fit);
         bad += rest.tile_first + rest.tiles_each * fit + rest.tiles_more != wanted || rest.tiles_each > p.L.tiles_each || rest.tiles_each + !!rest.tiles_more > p.L.tiles_each + !!p.L.tiles_more;
         // grids that take every SM in clusters of four and eight, and last, wait for their predecessors; nothing else does
-        bad += p.early != !(p.ctas > 148 && p.L.clog >= 2 && p.us >= 22);
+        bad += p.early != !(p.ctas > 148 && p.L.clog >= 2 && p.us >= kStreamLate);
         late += !p.early;
         const StreamLayout &L = p.L;
         const uint32_t size = 1u << L.clog, clusters = p.ctas / size, units = (nunit + size - 1) / size, per = (tiles + clusters - 1) / clusters;
