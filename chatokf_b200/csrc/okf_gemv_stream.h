@@ -144,13 +144,12 @@ inline StreamUnit stream_unit_us(int ty) {
     }
 }
 inline float quad_max(float a, float b) { return sqrtf(sqrtf(a * a * a * a + b * b * b * b)); }  // the larger one, rounded off
-inline float stream_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tiles, uint32_t clog, uint32_t clusters, uint32_t warps, uint32_t sms, float floor_us) {
+inline float stream_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tiles, uint32_t clog, uint32_t clusters, uint32_t warps, bool shared, float floor_us) {
     const int kind = stream_kind(mode);
     constexpr float one[2][4] = {{1.3f, 2.65f, 3.05f, 4.2f}, {1.95f, 3.3f, 3.4f, 4.1f}};  // up to four columns, the others; by cluster size, one CTA to an SM
     constexpr float two[4][4] = {{2.5f, 3.8f, 7.8f, 8.1f}, {3.2f, 4.5f, 8.5f, 8.9f}, {2.8f, 4.85f, 9.f, 10.f}, {1.65f, 3.7f, 7.85f, 9.f}};
     constexpr float wide[4] = {4.35f, 6.25f, 6.5f, 8.05f};  // sixteen warps
     constexpr float stage[4] = {.59f, .62f, .35f, .51f}, stage_two[4] = {1.3f, .66f, 1.1f, 1.75f}, unit_two[4] = {.71f, .78f, 1.42f, 1.37f};
-    const bool shared = warps == 16 || (clusters << clog) > sms;
     const uint32_t units = (nunit + (1u << clog) - 1) >> clog, per = (tiles + clusters - 1) / clusters * units;
     const float busy = stream_unit_us(ty).stream[kind] * (float)((per + warps - 1) / warps) * (shared ? unit_two[kind] : 1.f) +
                        stage[kind] * (float)((units * n + warps - 1) / warps) * (shared ? stage_two[kind] : 1.f);
@@ -186,11 +185,14 @@ inline StreamPlan stream_search_one(uint32_t nunit, uint32_t n, uint32_t tiles, 
             if (clusters == 0 || (v == 1 && !fills)) continue;
             StreamPlan p = {};
             if (!stream_layout<TY, MODE>(nunit, n, clog, clusters, tiles, warps, p)) continue;
-            p.us = stream_us(TY, MODE, nunit, n, tiles, clog, clusters, warps, room.one[0], floor_us);
+            // There is an SM for every CTA.  (Asked of the number of CTAs, 34 to 37 clusters of four and 16 to 18 of eight went out as grids with an SM a CTA, of which 33 and 15
+            // fit at once: 25 shapes took 1.8 times as long.)
+            const bool alone = clusters <= room.one[clog];
+            p.us = stream_us(TY, MODE, nunit, n, tiles, clog, clusters, warps, warps == 16 || !alone, floor_us);
             p.ok = true;
             p.tiles = tiles;
-            p.early = clog < 2 || p.ctas <= room.one[0] || p.us < kStreamLate;
-            if (warps == 8 && p.ctas <= room.one[0] && p.smem < kStreamAlone && (TY != T_IQ2_XXS || clog)) p.smem = kStreamAlone;
+            p.early = clog < 2 || alone || p.us < kStreamLate;
+            if (warps == 8 && alone && p.smem < kStreamAlone && (TY != T_IQ2_XXS || clog)) p.smem = kStreamAlone;
             if (!best.ok || p.us < best.us) best = p;
         }
     }

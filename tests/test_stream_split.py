@@ -67,7 +67,8 @@ template <int TY, int MODE> static unsigned plans(std::mt19937 &rng, unsigned &f
     for (int i = 0; i < 4000; i++) {
         const uint32_t nunit = 1 + rng() % (i % 4 ? 72 : 600), wanted = 1 + rng() % (i % 3 ? 1200 : 20000);
         const uint32_t n = MODE == M_SEP ? 1 : MODE == M_W2 ? 5 + rng() % 4 : 1 + rng() % 4;
-        const StreamPlan p = stream_search<TY, MODE>(nunit, n, wanted, i & 1 ? room : none);
+        const StreamRoom &fits = i & 1 ? room : none;
+        const StreamPlan p = stream_search<TY, MODE>(nunit, n, wanted, fits);
         if (!p.ok) continue;
         const uint32_t tiles = p.tiles;  // of a launch
         bad += tiles == 0 || tiles > wanted;
@@ -77,12 +78,13 @@ template <int TY, int MODE> static unsigned plans(std::mt19937 &rng, unsigned &f
         rest.deal(wanted - left, left, fit);
         bad += rest.tile_first + rest.tiles_each * fit + rest.tiles_more != wanted || rest.tiles_each > p.L.tiles_each || rest.tiles_each + !!rest.tiles_more > p.L.tiles_each + !!p.L.tiles_more;
         // grids that take every SM in clusters of four and eight, and last, wait for their predecessors; nothing else does
-        bad += p.early != !(p.ctas > 148 && p.L.clog >= 2 && p.us >= kStreamLate);
+        bad += p.early != !(p.ctas >> p.L.clog > fits.one[p.L.clog] && p.L.clog >= 2 && p.us >= kStreamLate);
         late += !p.early;
         const StreamLayout &L = p.L;
         const uint32_t size = 1u << L.clog, clusters = p.ctas / size, units = (nunit + size - 1) / size, per = (tiles + clusters - 1) / clusters;
         const uint32_t panel = (MODE == M_SEP ? 2 : n * mode_bytes(MODE)) * L.es, records = MODE == M_SEP ? 256 : units * n * wide_info_words(TY, mode_bytes(MODE)) * 4;
-        bad += p.smem > (p.warps == 8 && p.ctas <= 148 ? kStreamAlone : stream_budget(p.warps)) || p.ctas % size || nunit < size || L.depth < 2 || L.depth > 4;
+        // only where there is an SM for every CTA of a cluster does a grid ask for SMs of its own: the last clusters would wait for the first else
+        bad += p.smem > (p.warps == 8 && clusters <= fits.one[L.clog] ? kStreamAlone : stream_budget(p.warps)) || p.ctas % size || nunit < size || L.depth < 2 || L.depth > 4;
         bad += L.tiles_each * clusters + L.tiles_more != tiles || L.tiles_more >= clusters || L.tiles_each == 0;
         bad += p.warps * L.depth * StreamGeom<TY, MODE>::stage > L.xs_off || L.xs_off % 128 || L.xs_off + panel > L.info_off || L.slot_off % 128;
         bad += L.info_off + records > L.slot_off || L.slot_off + p.warps * 2 * n * 64 > L.part_off || L.part_off + (size > 1 ? per * n * 64 : 0) > L.tab_off;
