@@ -167,7 +167,11 @@ inline float ring_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tile
     const uint32_t clusters = ctas >> clog, units = (nunit + (1u << clog) - 1) >> clog;
     const float busy = (stream_unit_us(ty).ring[kind] * (float)((tiles + clusters - 1) / clusters * units) + pair_us[kind / 2] * (float)(units * n)) / 8.f * (shared ? shared_x[kind / 2] : 1.f);
     const uint32_t ub = ty == T_Q8_0 ? 272 : ty == T_Q6_K ? 210 : ty == T_Q5_K ? 176 : ty == T_Q2_0 ? 68 : ty == T_IQ2_XXS ? 66 : 144;
-    const float us = fixed[kind] + (shared ? 1.45f : 0.f) + (clog ? cluster_us[kind / 2] : 0.f) + quad_max(busy, (float)nunit * (float)tiles * (16.f * (float)ub / 6.1e6f));
+    float us = fixed[kind] + (shared ? 1.45f : 0.f) + (clog ? cluster_us[kind / 2] : 0.f) + quad_max(busy, (float)nunit * (float)tiles * (16.f * (float)ub / 6.1e6f));
+    // One column: where this is too high by 1300 shapes in three kinds of chain.  A tile to a CTA and two CTAs on some SMs only (73 shapes that would all be on the
+    // other kernel: 0.960 of this one's time on average and 22 slower by more than 3 % in plain chains, 25 in graphs; with the factor 0.953, 5 and 6; Q8_0 2304 -> 2729 3.7 us,
+    // 4.7 there); clusters (31: 0.918 -> 0.915); two CTAs on every SM, three types (101: 0.944 -> 0.947, slower by more than 3 % 18 -> 8; Q6_K 3072 -> 27634 17.7, 21.9 there).
+    if (kind == 0 && ctas > sms) us *= ctas < 2 * sms ? .7f : clog || ty == T_Q8_0 ? .85f : ty == T_Q6_K || ty == T_IQ4_NL ? .9f : 1.f;
     return tiles < 12 * sms ? us : kind == 3 && n == 1 ? .85f * us : .93f * us;  // (with so many tiles the fit favours the other kernel: ragged Q4_0 2336 -> 63677
                                                                                  // 27.5 us here, 32.5 there)
 }
