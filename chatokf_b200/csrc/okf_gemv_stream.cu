@@ -321,8 +321,11 @@ static bool stream_room(int dev, int sms, StreamRoom &room) {
     std::call_once(k.once, [&] {
         auto one = stream_kernel<T_Q4_K, M_W2, DT_F32, 16>;
         auto two = stream_kernel<T_Q4_K, M_W2, DT_F32, 8>;
-        if (cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, stream_budget(16)) != cudaSuccess) return;
-        if (cudaFuncSetAttribute(two, cudaFuncAttributeMaxDynamicSharedMemorySize, stream_budget(8)) != cudaSuccess) return;
+        if (cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, stream_budget(16)) != cudaSuccess ||
+            cudaFuncSetAttribute(two, cudaFuncAttributeMaxDynamicSharedMemorySize, stream_budget(8)) != cudaSuccess) {
+            (void)cudaGetLastError();  // not for whoever asks next
+            return;
+        }
         k.room.one[0] = (uint32_t)sms;
         k.room.two[0] = 2 * (uint32_t)sms;
         for (uint32_t clog = 1; clog < 4; clog++) {
@@ -338,7 +341,10 @@ static bool stream_room(int dev, int sms, StreamRoom &room) {
                 cfg.attrs = &at;
                 cfg.numAttrs = 1;
                 int n = 0;
-                if (cudaOccupancyMaxActiveClusters(&n, w ? (const void *)two : (const void *)one, &cfg) != cudaSuccess) n = 0;  // none of that size
+                if (cudaOccupancyMaxActiveClusters(&n, w ? (const void *)two : (const void *)one, &cfg) != cudaSuccess) {
+                    (void)cudaGetLastError();
+                    n = 0;  // none of that size
+                }
                 (w ? k.room.two : k.room.one)[clog] = (uint32_t)n;
             }
         }
