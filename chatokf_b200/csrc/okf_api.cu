@@ -264,7 +264,7 @@ cudaError_t run_tile(okf_ctx *ctx, int ty, const uint8_t *wp, uint32_t k, uint32
                 xadt = DT_BF16;
             }
         }
-        const uint32_t *room = gemm_ts_clusters(ctx->device);
+        const uint32_t *room = ctx->flags & OKF_FLAG_DEAL_ITEMS ? nullptr : gemm_ts_clusters(ctx->device);
         GemmPlan plan = gemm_tc_plan(ty, k, m, nn, xadt, ctx->sms, kMaxScratchFloats, room);
         void *part = plan.floats ? memory(0, lane ? &lane->part : nullptr, lane ? &lane->part_bytes : nullptr, plan.floats * sizeof(float)) : nullptr;
         if (plan.floats && !part) plan = gemm_tc_plan(ty, k, m, nn, xadt, ctx->sms, 0, room);

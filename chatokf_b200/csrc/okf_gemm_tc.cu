@@ -958,7 +958,8 @@ extern "C" int okf_gemm_noalloc(okf_ctx *ctx, int type, const okf_weights *w, ui
     }
     // every slot the reduction reads is written by the main kernel first, so nothing in the
     // array has to be cleared between calls
-    const GemmPlan plan = gemm_tc_plan(type, k, m, n, xdt, ctx->sms, kStaticScratchFloats, gemm_ts_clusters(ctx->device));
+    const GemmPlan plan = gemm_tc_plan(type, k, m, n, xdt, ctx->sms, kStaticScratchFloats,
+                                       ctx->flags & OKF_FLAG_DEAL_ITEMS ? nullptr : gemm_ts_clusters(ctx->device));
     cudaError_t e = launch_gemm_tc(plan, type, wp, k, m, x, xdt, n, out, odt, ctx->dev_status, g_static_scratch_addr[ctx->device],
                                    (cudaStream_t)stream, ctx->sms, ctx->device, &ctx->launches, nullptr);
     if (e != cudaSuccess) return cuda_fail(ctx, e);

@@ -94,7 +94,7 @@ class Context:
         return v.value
 
     def set_flags(self, flags: int):
-        """okf_set_flags: 1 = simple kernels only (device-side yardstick)."""
+        """okf_set_flags: 1 = simple kernels only (device-side yardstick), 2 = no items shared by clusters."""
         self._check(self.lib.okf_set_flags(self.h, int(flags)), "okf_set_flags")
 
     def fault_inject(self, rate: float, seed: int = 0):

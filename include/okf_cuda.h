@@ -364,6 +364,10 @@ OKF_API int okf_device_status(okf_ctx *ctx, int *out);
  * the plain warp-per-row / fp32-tile kernels, which the fast kernels are
  * checked against on the device.  No counterpart in the reference. */
 #define OKF_FLAG_SIMPLE_KERNELS 1u
+/* ... OKF_FLAG_DEAL_ITEMS keeps the tensor-core matmul from letting clusters of CTAs
+ * share an item: what does not fill the device is dealt out along K, with partial tiles
+ * in working memory and a second kernel, as where items do not fit at once. */
+#define OKF_FLAG_DEAL_ITEMS 2u
 OKF_API int okf_set_flags(okf_ctx *ctx, uint32_t flags);
 
 /* Number of kernels this context has launched since it was created (the one that
