@@ -131,33 +131,27 @@ __device__ __forceinline__ void wide_join(const int (&d)[WideMode<MODE>::sets][4
 // `copies` times side by side, lane l reads copy l mod copies: 32 copies make every access free of
 // bank conflicts.
 constexpr uint32_t kIq2Pos = 0x002B1908u, kIq2Neg = 0x00D5E7F8u;
-__device__ __forceinline__ uint32_t iq2_code_selectors(uint64_t entry) {
+__host__ __device__ constexpr uint32_t iq2_code_selectors(uint64_t entry) {
     uint32_t s = 0;
 #pragma unroll
     for (int j = 0; j < 8; j++) s |= (uint32_t)(entry >> (8 * j + 4) & 3u) << (4 * j);  // 8, 25, 43 -> 0, 1, 2
     return s;
 }
-__device__ __forceinline__ uint32_t iq2_sign_selectors(uint32_t idx7) {
-    uint32_t s = (__popc(idx7) & 1u) << 30;
+__host__ __device__ constexpr uint32_t iq2_sign_selectors(uint32_t idx7) {
+    const uint32_t a = idx7 ^ idx7 >> 4, b = a ^ a >> 2;
+    uint32_t s = ((b ^ b >> 1) & 1u) << 30;
 #pragma unroll
     for (int j = 0; j < 7; j++) s |= (idx7 >> j & 1u) << (4 * j + 2);
     return s;
 }
-// both tables, worked out by the compiler: 256 codes, then 128 signs
+// both tables, worked out by the compiler: 256 codes, then 128 signs (for okf_gemv_stream.cu; in the other kernels, whose threads have an entry or two
+// each to work out, loads of these made launches 0.1 to 0.3 % longer)
 struct Iq2Selectors {
     uint32_t v[384];
     constexpr Iq2Selectors() : v{} {
         constexpr uint64_t grid[256] = {OKF_IQ2XXS_GRID_VALUES};
-        for (uint32_t i = 0; i < 256; i++)
-            for (int j = 0; j < 8; j++) v[i] |= (uint32_t)(grid[i] >> (8 * j + 4) & 3u) << (4 * j);  // 8, 25, 43 -> 0, 1, 2
-        for (uint32_t i = 0; i < 128; i++) {
-            uint32_t odd = 0;
-            for (int j = 0; j < 7; j++) {
-                v[256 + i] |= (i >> j & 1u) << (4 * j + 2);
-                odd ^= i >> j & 1u;
-            }
-            v[256 + i] |= odd << 30;
-        }
+        for (uint32_t i = 0; i < 256; i++) v[i] = iq2_code_selectors(grid[i]);
+        for (uint32_t i = 0; i < 128; i++) v[256 + i] = iq2_sign_selectors(i);
     }
 };
 static __device__ constexpr Iq2Selectors g_iq2_selectors;
