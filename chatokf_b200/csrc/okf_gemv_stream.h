@@ -60,7 +60,7 @@ struct StreamRoom {
 struct StreamPlan {
     bool ok, early;  // early: may start beside its predecessor
     uint32_t warps, ctas, smem;
-    uint32_t tiles;  // of a launch: all, or (see stream_search) the launches of a matrix take that many each, the last one what is left
+    uint32_t tiles;  // of a launch: all, or (see stream_launches) the launches of a matrix take that many each, the last one what is left
     float us;  // estimated, of all launches
     StreamLayout L;
 };
@@ -177,7 +177,7 @@ inline float ring_us(int ty, int mode, uint32_t nunit, uint32_t n, uint32_t tile
 }
 
 template <int TY, int MODE>
-inline StreamPlan stream_search_one(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room) {
+inline StreamPlan stream_search(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room) {
     StreamPlan best = {};
     const float floor_us = (float)nunit * (float)tiles * (16.f * UnitGeom<TY>::bytes / 4.9e6f);
     for (uint32_t clog = 0; clog < 4 && (clog == 0 || nunit >= 2u << clog); clog++) {
@@ -209,11 +209,11 @@ inline StreamPlan stream_search_one(uint32_t nunit, uint32_t n, uint32_t tiles, 
 // 5376 -> 80310, 8, 127 -> 110; that kernel in clusters, with all of x, 697 and 341).  Not rows of Q8_0 and Q4_0 that end inside a unit, whose x of three and four bytes
 // leaves rings of two stages (Q8_0 7904 -> 59634, 5 columns, 245 and 294).
 template <int TY, int MODE>
-inline StreamPlan stream_search(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room) {
-    StreamPlan best = stream_search_one<TY, MODE>(nunit, n, tiles, room);
+inline StreamPlan stream_launches(uint32_t nunit, uint32_t n, uint32_t tiles, const StreamRoom &room) {
+    StreamPlan best = stream_search<TY, MODE>(nunit, n, tiles, room);
     if (best.ok || (WideMode<MODE>::rag && (TY == T_Q8_0 || TY == T_Q4_0))) return best;
     for (uint32_t parts = 2, most = 64; parts <= most && parts <= tiles; parts++) {
-        StreamPlan p = stream_search_one<TY, MODE>(nunit, n, (tiles + parts - 1) / parts, room);
+        StreamPlan p = stream_search<TY, MODE>(nunit, n, (tiles + parts - 1) / parts, room);
         if (!p.ok) continue;
         if (!best.ok) most = 2 * parts;
         p.us *= (float)parts;
@@ -235,7 +235,7 @@ inline const StreamPlan &stream_plan(uint32_t nunit, uint32_t n, uint32_t tiles,
     static thread_local Entry kept[kEntries];  // (tiles = 0: none yet)
     Entry &e = kept[((nunit * 31 + n) * 31 + tiles) * 2654435761u >> 28];
     static_assert(kEntries == 16, "four bits of the hash");
-    if (e.nunit != nunit || e.n != n || e.tiles != tiles || e.dev != dev) e = {nunit, n, tiles, dev, stream_search<TY, MODE>(nunit, n, tiles, room)};
+    if (e.nunit != nunit || e.n != n || e.tiles != tiles || e.dev != dev) e = {nunit, n, tiles, dev, stream_launches<TY, MODE>(nunit, n, tiles, room)};
     return e.p;
 }
 

@@ -10,11 +10,11 @@ MODEL = r"""
 using namespace okf;
 static const StreamRoom room = {{148, 74, 33, 15}, {296, 148, 71, 33}};
 template <int TY> static StreamPlan plan(int mode, uint32_t nunit, uint32_t n, uint32_t tiles) {
-    if (mode == M_SEP) return stream_search<TY, M_SEP>(nunit, n, tiles, room);
-    if (mode == M_W1) return stream_search<TY, M_W1>(nunit, n, tiles, room);
-    if (mode == M_W2) return stream_search<TY, M_W2>(nunit, n, tiles, room);
+    if (mode == M_SEP) return stream_launches<TY, M_SEP>(nunit, n, tiles, room);
+    if (mode == M_W1) return stream_launches<TY, M_W1>(nunit, n, tiles, room);
+    if (mode == M_W2) return stream_launches<TY, M_W2>(nunit, n, tiles, room);
     if constexpr (TY == T_Q8_0 || TY == T_Q4_0 || TY == T_IQ4_NL || TY == T_Q2_0)
-        return mode == M_R3 ? stream_search<TY, M_R3>(nunit, n, tiles, room) : stream_search<TY, M_R4>(nunit, n, tiles, room);
+        return mode == M_R3 ? stream_launches<TY, M_R3>(nunit, n, tiles, room) : stream_launches<TY, M_R4>(nunit, n, tiles, room);
     return {};
 }
 int main() {
