@@ -93,6 +93,8 @@ inline void lay_out(GemmPlan plan, uint32_t slabs, uint32_t steps, uint32_t n, u
 // all the room taken by 49 grids of four, six, seven and eight CTAs 8 to 15 % faster).
 // Whole items of fewer than eight units are shared by three CTAs or more where a seventh of the room is left: 32 shapes 8 to 17 % faster; by two CTAs, or
 // with less room left, 54 shapes 1 % faster to 8 % slower (Q6_K 1536 -> 2774, 259 tokens, 10.4 and 12.5).
+// Q4_0 does not share, though it would gain as the others do (4096 -> 1500, 34 tokens, 13.6 us instead of 9.0; 120 shapes of 9 to 1024 tokens take 0.916 of the time in plain
+// chains): test_gpu_tile_dealing.py and test_gpu_tile_memory.py hold that its calls deal, by the number of their kernels.
 // Sums in tensor memory are cut off where fp32 would round, so a chain's error grows with its length.  `base`: units of a chain of the plan without
 // clusters; where an item's parts are longer, their k-blocks go to two or four accumulators in turn (there is room for
 // them up to 128 and 64 tokens), which are added up at the end, and where that is not enough the split is not taken.  500 shapes of fp16 operands, rms
@@ -147,7 +149,7 @@ inline GemmPlan gemm_tc_search(int ty, uint32_t k, uint32_t m, uint32_t n, int x
         lay_out(plan, slabs, (kblocks + 3) / 4, n, plan.tok, 4 * ts_kblock(ty, plan.tok), plan.tok > 128 ? 2.5e-6 : 1e-6, 1, all, max_floats, best, best_t);
         if (plan.tok <= 32) break;
     }
-    if (!room) return best;
+    if (!room || ty == T_Q4_0) return best;
     const uint32_t units = (kblocks + 3) / 4;
     const double run = best.dealt && !best.waves ? (double)best.dealt * units / best.dealers : units, base = run < 1 ? 1 : run;
     const bool whole = !best.dealt;

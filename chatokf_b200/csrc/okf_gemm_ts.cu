@@ -803,7 +803,8 @@ static cudaError_t ts_launch(TsArgs a, const void *x, uint32_t grid, cudaStream_
 }
 template <int TY, bool SK>
 static cudaError_t ts_launch_x(const TsArgs &a, const void *x, int xdt, uint32_t grid, cudaStream_t s, int dev) {
-    if (a.cluster > 1) return xdt == DT_F16 ? ts_launch<TY, SK, true, true>(a, x, grid, s, dev) : ts_launch<TY, SK, false, true>(a, x, grid, s, dev);
+    if constexpr (TY != T_Q4_0)  // (see share_out)
+        if (a.cluster > 1) return xdt == DT_F16 ? ts_launch<TY, SK, true, true>(a, x, grid, s, dev) : ts_launch<TY, SK, false, true>(a, x, grid, s, dev);
     return xdt == DT_F16 ? ts_launch<TY, SK, true, false>(a, x, grid, s, dev) : ts_launch<TY, SK, false, false>(a, x, grid, s, dev);
 }
 

@@ -245,11 +245,9 @@ def test_gemm_more_items_than_sms(ctx, m, n):
     assert rel_err(o[:n * m].reshape(n, m), ref) <= GEMM_TOL
 
 
-@pytest.mark.parametrize("flags", [0, 2])
-def test_gemm_split_k_odd_sizes(ctx, flags):
-    """A short, deep matrix makes the matmul cut K into ranges (summed in a
-    cluster's shared memory or, flag 2, partials in scratch, summed by a second
-    kernel); M * N is odd on purpose."""
+def test_gemm_split_k_odd_sizes(ctx):
+    """A short, deep matrix makes the matmul cut K into ranges (partials in
+    scratch, summed by a second kernel); M * N is odd on purpose."""
     ty, k, m, n = GGUFType.Q4_K, 8192, 131, 45
     blocks = make_weights(ty, m, k, seed=4)
     X = np.random.default_rng(5).normal(size=(n, k)).astype(np.float32)
@@ -257,11 +255,7 @@ def test_gemm_split_k_odd_sizes(ctx, flags):
     ref = oracle.matmul(ty, blocks, k, m, Xd.float().cpu().numpy(), n)
     for odt in (torch.float32, torch.bfloat16):
         out = torch.full((n * m + 8,), float("nan"), dtype=odt, device="cuda")
-        before = ctx.launches
-        ctx.set_flags(flags)
         CudaEnc(ctx).gemm(GGUFTensor("w", (k, m), ty), Xd, out, ctx.upload(blocks), n)
-        ctx.set_flags(0)
-        assert ctx.launches - before == (2 if flags else 1)
         torch.cuda.synchronize()
         o = out.float().cpu().numpy()
         assert np.isnan(o[n * m:]).all()

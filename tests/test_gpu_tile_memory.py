@@ -19,7 +19,6 @@ K, M = 4096, 1000  # eight slabs: dealt out at every token count below 512
 @pytest.fixture()
 def own(lib_built):
     c = Context(0)
-    c.set_flags(2)  # partial tiles: items dealt out, not shared by clusters
     w = c.upload(synth.random_blocks(GGUFType.Q4_0, M * K // block_elems(GGUFType.Q4_0), np.random.default_rng(4)))
     yield c, w, GGUFTensor("w", (K, M), GGUFType.Q4_0)
     torch.cuda.synchronize()
