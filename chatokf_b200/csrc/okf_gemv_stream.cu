@@ -276,9 +276,10 @@ __global__ void __launch_bounds__(NW * 32, 16 / NW) stream_kernel(const __grid_c
     // the first of them, up to seven parts of eight columns one after the other: rows of two to six units, 5 to 8 columns, 160 shapes, took 1.22 times as long;
     // IQ4_NL 1024 -> 209, 8 columns, 4.8 and 3.6 us.)
     const uint32_t tile = split.tile(last), lo = tile * nun;
-    if (warp + 1 < NW && last < split.all && last > lo) {
+    if (warp + 1 < NW && last < split.all && last > lo && (!SEP || first <= lo)) {  // (a single column is the first one's)
         uint32_t w0 = warp, w1 = warp + 1;  // the first and the last warp with a part
-        while (split.border<NW>(w0) > lo) w0--;
+        if constexpr (!SEP)
+            while (split.border<NW>(w0) > lo) w0--;
         while (w1 + 1 < NW && split.border<NW>(w1 + 1) < lo + nun) w1++;
         const float *slots = reinterpret_cast<const float *>(smem + L.slot_off) + (lane & 15);
         const GemvSeg sg = gemv_segment(p, t0 + tile);
@@ -365,16 +366,19 @@ static cudaError_t stream_go(const GemvArgs &a, const StreamPlan &p, const Strea
     return launch_kernel(p.early, stream_kernel<TY, MODE, XDT, NW>, ctas, NW * 32, p.smem, s, 1u << L.clog, a, L);
 }
 template <int TY, int MODE, int XDT>
-static cudaError_t stream_warps(const GemvArgs &a, const StreamPlan &p, cudaStream_t s, int dev) {
+static cudaError_t stream_warps(const GemvArgs &a, const StreamPlan &p, const StreamLayout &L, uint32_t ctas, cudaStream_t s, int dev) {
+    if constexpr (MODE == M_W2)
+        if (p.warps == 16) return stream_go<TY, MODE, XDT, 16>(a, p, L, ctas, s, dev);
+    return stream_go<TY, MODE, XDT, 8>(a, p, L, ctas, s, dev);
+}
+template <int TY, int MODE, int XDT>
+static cudaError_t stream_all(const GemvArgs &a, const StreamPlan &p, cudaStream_t s, int dev) {
+    if (p.tiles == a.tiles) return stream_warps<TY, MODE, XDT>(a, p, p.L, p.ctas, s, dev);
     StreamLayout L = p.L;
     for (uint32_t first = 0; first < a.tiles; first += p.tiles) {
         const uint32_t tiles = a.tiles - first < p.tiles ? a.tiles - first : p.tiles, all = p.ctas >> L.clog, clusters = tiles < all ? tiles : all;
         L.deal(first, tiles, clusters);
-        cudaError_t e;
-        if constexpr (MODE == M_W2)
-            e = p.warps == 16 ? stream_go<TY, MODE, XDT, 16>(a, p, L, clusters << L.clog, s, dev) : stream_go<TY, MODE, XDT, 8>(a, p, L, clusters << L.clog, s, dev);
-        else
-            e = stream_go<TY, MODE, XDT, 8>(a, p, L, clusters << L.clog, s, dev);
+        const cudaError_t e = stream_warps<TY, MODE, XDT>(a, p, L, clusters << L.clog, s, dev);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -383,12 +387,12 @@ template <int TY, int MODE>
 static int stream_launch(const GemvArgs &a, int xdt, const StreamRoom &room, cudaStream_t s, int dev, float other_us, cudaError_t &e) {
     const StreamPlan &p = stream_plan<TY, MODE>(a.nunit, a.n, a.tiles, room, dev);
     if (!p.ok || p.us >= other_us) return 0;
-    if constexpr (MODE == M_R4) e = stream_warps<TY, MODE, DT_F32>(a, p, s, dev);
-    else if constexpr (MODE == M_R3) e = xdt == DT_F16 ? stream_warps<TY, MODE, DT_F16>(a, p, s, dev) : stream_warps<TY, MODE, DT_BF16>(a, p, s, dev);
-    else if (xdt == DT_F16) e = stream_warps<TY, MODE, DT_F16>(a, p, s, dev);
-    else if (xdt == DT_BF16) e = stream_warps<TY, MODE, DT_BF16>(a, p, s, dev);
-    else e = stream_warps<TY, MODE, DT_F32>(a, p, s, dev);
-    return (int)((a.tiles + p.tiles - 1) / p.tiles);
+    if constexpr (MODE == M_R4) e = stream_all<TY, MODE, DT_F32>(a, p, s, dev);
+    else if constexpr (MODE == M_R3) e = xdt == DT_F16 ? stream_all<TY, MODE, DT_F16>(a, p, s, dev) : stream_all<TY, MODE, DT_BF16>(a, p, s, dev);
+    else if (xdt == DT_F16) e = stream_all<TY, MODE, DT_F16>(a, p, s, dev);
+    else if (xdt == DT_BF16) e = stream_all<TY, MODE, DT_BF16>(a, p, s, dev);
+    else e = stream_all<TY, MODE, DT_F32>(a, p, s, dev);
+    return p.tiles == a.tiles ? 1 : (int)((a.tiles + p.tiles - 1) / p.tiles);
 }
 template <int TY>
 static int stream_ty(int mode, const GemvArgs &a, int xdt, const StreamRoom &room, cudaStream_t s, int dev, float other_us, cudaError_t &e) {
