@@ -222,8 +222,8 @@ inline bool gemv_layout(int ty, uint32_t row_bytes, uint32_t nunit, uint32_t n, 
 // where that is at most three tiles, which one CTA would take one after another on some SMs (192 to
 // 320 tiles: Q8_0 4096 -> 4096 6.7 -> 5.2, Q4_K 12288 -> 3072 11.4 -> 8.7, 5120 -> 5120 6.7 -> 6.1; below, Q4_K
 // 4096 -> 4096, 64 KB, 4.15 -> 4.35; not for the two types with a look-up per weight, whose warps hardly
-// wait: IQ2_XXS 6144 -> 6144 9.6 -> 10.5, IQ4_NL 10.1 -> 11.3).  Several columns, with
-// more work per tile: from three tiles on (Q4_K 5120 -> 17357, 4 columns, 27.6 -> 20.0 us, 8 columns 35 -> 29;
+// wait: IQ2_XXS 6144 -> 6144 9.6 -> 10.5, IQ4_NL 10.1 -> 11.3).  Several columns (up to four, and row shards; five to eight are okf_gemv_stream.cu's else, and
+// the figures of eight are this kernel's, before there was that one), with more work per tile: from three tiles on (Q4_K 5120 -> 17357, 4 columns, 27.6 -> 20.0 us, 8 columns 35 -> 29;
 // 512 tiles, which were left to one CTA per SM: Q5_K 17408 -> 8192, 3 columns, 56.9 -> 40.6 us, Q4_K 20480 -> 8192, 4 columns, 55.6 -> 53.8 us, Q4_K 8192 -> 8192, 8
 // columns, 35.6 -> 37.6; the two-bit types, with little to wait for, from four on: IQ2_XXS 8192 -> 8192, 5 columns, 23.6 us, from three 27.5).
 inline bool two_bit(int ty) { return ty == T_IQ2_XXS || ty == T_Q2_0; }
